@@ -27,6 +27,7 @@ SOURCES = [
     "gemv.cu",
     "gemv_mma.cu",
     "gemm_tcgen05.cu",
+    "gemm_rows.cu",
     "elementwise.cu",
     "sample.cu",
     "ragged_rows.cu",

@@ -1,0 +1,423 @@
+// bf16 projections of a few to some thousand rows on the 5th-generation tensor cores: the K range of an output tile is
+// split over the CTAs of a thread-block cluster and the partial tiles meet in distributed shared memory.
+//
+//   y[M,N] = epi( x[M,K] . w[N,K]^T )
+//
+// The operands are swapped: 128 weight rows of a tile sit on the tensor core's M side, BN activation rows on its N side,
+// so a batch is padded to a multiple of 16 rows and not of 128.  Warp 0 = TMA producer, warp 1 = TMEM owner and MMA
+// issuer, warps 2-5 drain TMEM; all six warps add the partial tiles and run the epilogue with 16-byte accesses.
+//
+// What bounds it: up to ~64 rows the weight stream (2 N K bytes), above it the operand feed of the 128 x BN tiles; at
+// either end a matrix of 768 ... 4096 outputs has 6 ... 32 weight tiles for 148 SMs, so K must be split, and then the
+// chain at the end of a tile counts.  Through global memory (partials, fence, counter, the last CTA reads all of them
+// back) that chain was ~10 of the 14 us of a 4096 x 4096 projection of 16 rows; through distributed shared memory it is
+// two cluster barriers, and every CTA finishes its own share of the columns.  Two CTAs fit an SM (at most 108 KB of ring,
+// at most 256 TMEM columns each), and the dependents are released as soon as all CTAs run, so their weight loads
+// start beside this kernel's tail.  Measured on B200 in a chain of launches over rotating weights, us, before -> now:
+//   rows           16            128            301            1024
+//   4096 x 4096    11.6 ->  8.6   19.8 -> 12.5   35.0 -> 17.7   36.0 -> 36.0 (persistent kernel)
+//   4096 x 14336   24.6 -> 21.7   35.2 -> 27.4   94.5 -> 40.1   97.4 -> 97.4 (persistent kernel)
+//   28672 gated    42.4 -> 39.8   62.8 -> 48.9   87.2 -> 79.2  181   -> 181  (persistent kernel)
+//   768 x 3072      9.7 ->  4.6   30.6 ->  6.0   29.2 ->  7.6   28.8 -> 11.8
+// (before: split-K through global memory up to 128 rows, the persistent kernel of 128-row tiles above.)
+#include "gemm_rows.cuh"
+
+namespace dli {
+
+constexpr int kRowsThreads = 192;
+constexpr int kRowsMaxCluster = 8;
+
+__device__ __forceinline__ void tmem_ld_32x8(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr)
+               : "memory");
+}
+__device__ __forceinline__ uint32_t cluster_map(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void cluster_store(uint32_t addr, uint32_t v) {
+  asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// One tile per cluster: gridDim.x = cluster size c (the K splits), y = activation-row tiles, z = weight-row tiles (so the
+// clusters that share a weight tile run side by side and HBM reads it once).
+//   kRowsGated: w is the [gate128 | up128]-interleaved matrix; the tile's 128 weight rows are 64 gate rows and the 64 up
+//   rows that belong to them (two TMA boxes), so gate and up of an output meet in the same tile's sums.
+//   kRowsRope: the qkv projection of a prompt pass; the epilogue rotates q and k as rope_kv_append_kernel does on the
+//   stored bf16 values (a tile holds one 128-wide or two 64-wide heads, so a rotation pair meets in the tile's sums) and
+//   writes k and v to the cache pages too.
+template <int kMode>
+__global__ void __launch_bounds__(kRowsThreads, 2)
+gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX,
+                 const bf16* __restrict__ bias, const bf16* residual, bf16* y, int M, int N, int K, int epilogue, int BN,
+                 int stages, int tmem_cols, const __grid_constant__ RopeArgs rope, int hd) {
+  constexpr bool kGated = kMode == kRowsGated;
+  extern __shared__ uint8_t smem_raw[];
+  // SWIZZLE_128B operands need 1024-byte alignment (the same offset in every CTA of the cluster)
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  const int stage_bytes = (128 + BN) * (kBlockK * 2);
+  uint8_t* bar_mem = smem + stages * stage_bytes;
+  const uint32_t full_bar = smem_addr(bar_mem);
+  const uint32_t empty_bar = full_bar + 8 * stages;
+  const uint32_t done_bar = empty_bar + 8 * stages;
+  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(bar_mem + 8 * (2 * stages + 1));
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int splits = gridDim.x, rank = blockIdx.x;
+  const int total_kb = K / kBlockK;
+  const int kb0 = (int)((long long)total_kb * rank / splits);  // splits <= total_kb: no empty range
+  const int num_kb = (int)((long long)total_kb * (rank + 1) / splits) - kb0;
+  const int m0 = blockIdx.y * BN;
+  const int n_tile = blockIdx.z;
+  const int rows = min(BN, M - m0);  // activation rows of this tile
+
+  if (warp == 0 && lane == 0) {
+    tma_prefetch_desc(&tmW);
+    tma_prefetch_desc(&tmX);
+    for (int s = 0; s < stages; ++s) {
+      mbar_init(full_bar + 8 * s, 1);
+      mbar_init(empty_bar + 8 * s, 1);
+    }
+    mbar_init(done_bar, 1);
+    fence_barrier_init();
+  }
+  if (warp == 1) tmem_alloc(smem_addr(tmem_ptr_smem), tmem_cols);
+  tcgen05_fence_before();
+  __syncthreads();
+  tcgen05_fence_after();
+  const uint32_t tmem_base = *tmem_ptr_smem;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      auto load_w = [&](int kb, int s) {
+        const uint32_t dst = smem_addr(smem) + s * stage_bytes;
+        if (kGated) {
+          const int row = (n_tile >> 1) * 256 + (n_tile & 1) * 64;  // 64 gate rows; their up rows are 128 further
+          tma_load_2d(dst, &tmW, full_bar + 8 * s, (kb0 + kb) * kBlockK, row);
+          tma_load_2d(dst + 64 * kBlockK * 2, &tmW, full_bar + 8 * s, (kb0 + kb) * kBlockK, row + 128);
+        } else {
+          tma_load_2d(dst, &tmW, full_bar + 8 * s, (kb0 + kb) * kBlockK, n_tile * 128);
+        }
+      };
+      auto load_x = [&](int kb, int s) {
+        tma_load_2d(smem_addr(smem) + s * stage_bytes + 128 * kBlockK * 2, &tmX, full_bar + 8 * s, (kb0 + kb) * kBlockK, m0);
+      };
+      // weights do not depend on the previous kernel: the first ring of them goes out before the dependency wait
+      const int pre = min(stages, num_kb);
+      for (int kb = 0; kb < pre; ++kb) {
+        mbar_expect_tx(full_bar + 8 * kb, stage_bytes);
+        load_w(kb, kb);
+      }
+      pdl_wait();
+      // every predecessor is complete here, and this CTA is resident: the next kernel's CTAs may come in beside the
+      // running ones (their weights before their own wait)
+      pdl_trigger();
+      for (int kb = 0; kb < pre; ++kb) load_x(kb, kb);
+      int s = 0;
+      uint32_t ph = 0;  // parity of the empty barrier's phase this lap waits for
+      for (int kb = pre; kb < num_kb; ++kb) {  // runs only when the ring was filled: pre == stages
+        mbar_wait(empty_bar + 8 * s, ph);
+        mbar_expect_tx(full_bar + 8 * s, stage_bytes);
+        load_w(kb, s);
+        load_x(kb, s);
+        if (++s == stages) s = 0, ph ^= 1;
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    const uint32_t idesc = make_idesc(BN);
+    const uint64_t adesc0 = make_smem_desc(smem_addr(smem));
+    const uint64_t bdesc0 = make_smem_desc(smem_addr(smem) + 128 * kBlockK * 2);
+    int s = 0;
+    uint32_t ph = 0;
+    for (int kb = 0; kb < num_kb; ++kb) {
+      mbar_wait(full_bar + 8 * s, ph);
+      tcgen05_fence_after();
+      const uint64_t off = (uint64_t)(s * (stage_bytes >> 4));  // start-address field: bytes >> 4
+      if (elect_one()) {
+#pragma unroll
+        for (int k = 0; k < kBlockK / kUmmaK; ++k)
+          umma_bf16(tmem_base, adesc0 + off + 2 * k, bdesc0 + off + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+        umma_commit(empty_bar + 8 * s);
+        if (kb == num_kb - 1) umma_commit(done_bar);
+      }
+      __syncwarp();
+      if (++s == stages) s = 0, ph ^= 1;
+    }
+  } else {
+    pdl_wait();  // residual and bias may come from the previous kernel
+    mbar_wait(done_bar, 0);
+    tcgen05_fence_after();
+  }
+  // Every MMA of every CTA of the cluster is done: the operand rings are free and take the partial sums.
+  if (splits > 1) cluster_barrier();
+  else __syncthreads();
+
+  // The tile's columns (activation rows) are dealt to the CTAs in groups of `per`; each CTA sends every owner its fp32
+  // partial of the owner's columns: [source rank][column][128 weight rows], lanes on consecutive weight rows.
+  const int per = (((rows + splits - 1) / splits) + 7) & ~7;
+  const uint32_t red = smem_addr(smem);
+  if (warp >= 2) {
+    const int quad = warp & 3;
+    const uint32_t lane_base = tmem_base + ((uint32_t)(quad * 32) << 16);
+    for (int o = 0; o < splits; ++o) {
+      const int c_end = min((o + 1) * per, rows);
+      const uint32_t base = (splits > 1 ? cluster_map(red, o) : red) + (rank * per * 128 + quad * 32 + lane) * 4;
+      for (int c0 = o * per; c0 < c_end; c0 += 16) {
+        uint32_t r1[8], r2[8];
+        tmem_ld_32x8(lane_base + c0, r1);
+        const bool two = c0 + 8 < c_end;
+        if (two) tmem_ld_32x8(lane_base + c0 + 8, r2);
+        tmem_ld_wait();
+        const uint32_t dst = base + (c0 - o * per) * 512;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) cluster_store(dst + j * 512, r1[j]);
+        if (two) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) cluster_store(dst + (8 + j) * 512, r2[j]);
+        }
+      }
+    }
+    tcgen05_fence_before();
+  } else {
+    pdl_wait();  // these warps take part in the epilogue, which reads the residual
+  }
+  if (splits > 1) cluster_barrier();
+  else __syncthreads();
+
+  // ---- epilogue over this CTA's columns: an item is 8 consecutive outputs of one activation row (two groups of 8 where
+  // two belong together: gate and up, or the halves of a rotation pair) ----
+  constexpr int kGroups = kMode == kRowsPlain ? 16 : 8;
+  const int n_out = kGated ? N / 2 : N;
+  const int col0 = rank * per;
+  const int items = max(0, min(per, rows - col0)) * kGroups;
+  const float* sums = reinterpret_cast<const float*>(smem);
+  for (int id = threadIdx.x; id < items; id += kRowsThreads) {
+    const int c = id / kGroups, g = id - c * kGroups;
+    const int m = m0 + col0 + c;
+    // first weight row of the item inside the tile, and how much further its second group starts
+    const int half = hd >> 1;
+    const int r0 = kMode == kRowsRope && hd == 64 ? (g >> 2) * 64 + (g & 3) * 8 : g * 8;
+    const int r1 = kMode == kRowsRope ? half : 64;
+    const int n = kGated ? n_tile * 64 + r0 : n_tile * 128 + r0;
+    if (n >= n_out) continue;  // n_out is a multiple of 16 (of hd with heads): a group is whole or absent
+    const size_t at = (size_t)m * n_out + n;
+    uint4 res = make_uint4(0u, 0u, 0u, 0u), bv = res, bv2 = res;
+    if (kMode == kRowsPlain && (epilogue & DLI_EPI_RESIDUAL)) res = ld_16B(residual + at);
+    if (!kGated && (epilogue & DLI_EPI_BIAS)) {
+      bv = ld_16B(bias + n);
+      if (kMode == kRowsRope) bv2 = ld_16B(bias + n + half);
+    }
+    float a[8], b[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) a[e] = 0.f, b[e] = 0.f;
+    for (int sp = 0; sp < splits; ++sp) {  // in split order: deterministic
+      const float4* p = reinterpret_cast<const float4*>(sums + (size_t)(sp * per + c) * 128 + r0);
+      const float4 u = p[0], v = p[1];
+      a[0] += u.x; a[1] += u.y; a[2] += u.z; a[3] += u.w;
+      a[4] += v.x; a[5] += v.y; a[6] += v.z; a[7] += v.w;
+      if (kMode != kRowsPlain) {
+        const float4 u2 = p[r1 / 4], v2 = p[r1 / 4 + 1];
+        b[0] += u2.x; b[1] += u2.y; b[2] += u2.z; b[3] += u2.w;
+        b[4] += v2.x; b[5] += v2.y; b[6] += v2.z; b[7] += v2.w;
+      }
+    }
+    if (kGated) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) a[e] = round_bf16(a[e]), b[e] = round_bf16(b[e]);
+      gated_combine_n(a, b, reinterpret_cast<const float*>(bias));
+      st_16B(y + at, pack8(a));
+      continue;
+    }
+    float bb[8];
+    unpack8(bv, bb);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) a[e] = round_bf16(a[e] + bb[e]);
+    if (kMode == kRowsPlain) {
+      float rr[8];
+      unpack8(res, rr);
+      if (epilogue & DLI_EPI_GELU_NEW) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) a[e] = round_bf16(gelu_new_f(a[e]));
+      }
+#pragma unroll
+      for (int e = 0; e < 8; ++e) a[e] += rr[e];
+      st_16B(y + at, pack8(a));
+    } else {
+      unpack8(bv2, bb);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) b[e] = round_bf16(b[e] + bb[e]);
+      const int head = hd == 64 ? n_tile * 2 + (g >> 2) : n_tile;  // q heads, then k heads, then v heads
+      const int i = hd == 64 ? (g & 3) * 8 : g * 8;                // element of the head's first half
+      const int pos = rope.positions[m];
+      if (rope.cos_t && head < rope.H + rope.KV) {
+        float cs[8], sn[8];
+        unpack8(ld_16B(rope.cos_t + (size_t)pos * half + i), cs);
+        unpack8(ld_16B(rope.sin_t + (size_t)pos * half + i), sn);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          const float x1 = a[e], x2 = b[e];
+          a[e] = round_bf16(x1 * cs[e]) + round_bf16(-x2 * sn[e]);
+          b[e] = round_bf16(x2 * cs[e]) + round_bf16(x1 * sn[e]);
+        }
+      }
+      const uint4 u1 = pack8(a), u2 = pack8(b);
+      st_16B(y + at, u1);
+      st_16B(y + at + half, u2);
+      if (head >= rope.H) {
+        const bool is_k = head < rope.H + rope.KV;
+        const int kvh = head - rope.H - (is_k ? 0 : rope.KV);
+        const int page = rope.page_table[(size_t)rope.seq_ids[m] * rope.max_pages + (pos >> rope.page_shift)];
+        const size_t row = (((size_t)page * rope.KV + kvh) << rope.page_shift) + (pos & ((1 << rope.page_shift) - 1));
+        bf16* dst = (is_k ? rope.k_cache : rope.v_cache) + row * hd + i;
+        st_16B(dst, u1);
+        st_16B(dst + half, u2);
+      }
+    }
+  }
+  __syncthreads();
+  if (warp == 1) {
+    tcgen05_fence_after();
+    tmem_dealloc(tmem_base, tmem_cols);
+  }
+}
+
+// ---- host side -------------------------------------------------------------------------------------------------------
+constexpr int kRowsMaxSmem = 227 * 1024;
+constexpr size_t kSmemPerSm = 228 * 1024;  // of which each resident CTA also takes 1 KB for the system
+
+static size_t rows_smem(int bn, int stages) { return (size_t)stages * (128 + bn) * kBlockK * 2 + 1024 + 256; }
+static int rows_per_owner(int bn, int splits) { return (((bn + splits - 1) / splits) + 7) & ~7; }
+static bool rows_fits(int bn, int splits, int stages) {
+  // the ring also takes the partial sums: `splits` times the columns a CTA owns
+  return rows_smem(bn, stages) <= (size_t)kRowsMaxSmem &&
+         (size_t)splits * rows_per_owner(bn, splits) * 512 <= (size_t)stages * (128 + bn) * kBlockK * 2;
+}
+
+static int rows_setup(int* capacity /*[kRowsMaxCluster + 1]: CTAs that run at once with one CTA per SM*/) {
+  static PerDeviceOnce once;
+  static int cap[kMaxDevices][kRowsMaxCluster + 1];
+  DLI_ONCE_PER_DEVICE(once, dev, {
+    DLI_CUDA_CALL(cudaFuncSetAttribute(gemm_rows_kernel<kRowsPlain>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowsMaxSmem));
+    DLI_CUDA_CALL(cudaFuncSetAttribute(gemm_rows_kernel<kRowsGated>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowsMaxSmem));
+    DLI_CUDA_CALL(cudaFuncSetAttribute(gemm_rows_kernel<kRowsRope>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowsMaxSmem));
+    for (int c = 1; c <= kRowsMaxCluster; ++c) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(c, 64, 64);
+      cfg.blockDim = dim3(kRowsThreads);
+      cfg.dynamicSmemBytes = 200 * 1024;  // one CTA per SM
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = c;
+      attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      int n = 0;
+      DLI_CUDA_CALL(cudaOccupancyMaxActiveClusters(&n, gemm_rows_kernel<kRowsPlain>, &cfg));
+      cap[dev][c] = n * c;
+    }
+  });
+  for (int c = 1; c <= kRowsMaxCluster; ++c) capacity[c] = cap[dev][c];
+  return DLI_OK;
+}
+
+// The cut is the cheapest by a model of the kernel's time, fitted to 12 matrices (768 x 768 ... 28672 x 4096) x 18 row
+// counts (3 ... 2048) x all cuts, B200: what it picks is 3.4 % slower than the best cut on average.
+//   time = max(weight bytes / 5.5 TB/s,
+//              CTAs an SM works through x k-blocks each x (0.104 + 0.00127 bn) us,     operand feed and MMAs
+//              waves x k-blocks x 0.234 us)                                            one CTA's own chain
+//          + 2.55 + 0.0323 bn us (set-up; partial sums and epilogue) + 5 us per further wave
+// Clusters do not fill the chip: with one CTA per SM 148 / 148 / 135 / 132 / 130 / 132 / 120 CTAs of clusters of 1, 2, 3, 4,
+// 5, 6, 8 run at once (asked of the driver; 7 only 105, not used), and a few CTAs beyond that cost a whole wave.
+// Rings of at most 108 KB let two CTAs share an SM, so that one's epilogue hides behind the other's loads and MMAs.
+static double rows_cost(int M, int N, int K, const RowsShape& sh, const int* cap) {
+  const int kb = K / kBlockK, kbp = (kb + sh.splits - 1) / sh.splits;
+  const long long ctas = (long long)((M + sh.bn - 1) / sh.bn) * ((N + 127) / 128) * sh.splits;
+  const int r = 2 * (rows_smem(sh.bn, sh.stages) + 1024) <= kSmemPerSm ? 2 : 1;
+  const long long at_once = (long long)cap[sh.splits] * r;
+  const long long waves = (ctas + at_once - 1) / at_once, rest = ctas - (waves - 1) * at_once;
+  const long long last = (rest + cap[sh.splits] - 1) / cap[sh.splits];
+  const double rounds = (double)(waves - 1) * r + (double)(last < r ? last : r);
+  const double mma = rounds * kbp * (0.104 + 0.00127 * sh.bn), chain = (double)waves * kbp * 0.234;
+  const double mem = (double)N * K * 2 / 5.54e6;
+  double t = mma > chain ? mma : chain;
+  if (mem > t) t = mem;
+  return t + 2.55 + 0.0323 * sh.bn + 5.0 * (double)(waves - 1);
+}
+
+int plan_gemm_rows(int M, int N, int K, RowsShape* shape, double* us) {
+  // a plan is a pure function of the sizes (and the device): the last few are kept per thread
+  struct Slot { int dev, M, N, K; RowsShape sh; double us; };
+  constexpr int kSlots = 64;
+  static thread_local Slot cache[kSlots] = {};
+  const int dev = current_device_slot();
+  if (dev < 0) return DLI_ERR_CUDA;
+  Slot& slot = cache[((unsigned)M * 31u + (unsigned)N * 7u + (unsigned)K) % kSlots];
+  if (!(slot.M == M && slot.N == N && slot.K == K && slot.dev == dev)) {
+    int cap[kRowsMaxCluster + 1];
+    const int rc = rows_setup(cap);
+    if (rc != DLI_OK) return rc;
+    static const int kWidths[] = {32, 48, 64, 96, 128, 160, 192, 224, 256};
+    static const int kSplits[] = {1, 2, 3, 4, 5, 6, 8};
+    double best = 1e30;
+    RowsShape pick = {};
+    for (int width : kWidths) {
+      const int tiles = (M + width - 1) / width;
+      const int bn = ((M + tiles - 1) / tiles + 15) / 16 * 16;  // rows spread evenly over the tiles
+      for (int splits : kSplits) {
+        // at least 512 elements of K per split: shorter ranges end before the ring has filled
+        if ((splits > 1 && splits > K / (8 * kBlockK)) || cap[splits] <= 0) continue;
+        for (int budget : {108, 216}) {
+          int stages = budget * 1024 / ((128 + bn) * kBlockK * 2);
+          if (stages > 8) stages = 8;
+          if (!rows_fits(bn, splits, stages)) continue;
+          const RowsShape sh{bn, splits, stages};
+          const double t = rows_cost(M, N, K, sh, cap);
+          if (t < best) best = t, pick = sh;
+        }
+      }
+    }
+    slot = Slot{dev, M, N, K, pick, best};
+  }
+  *shape = slot.sh;
+  *us = slot.us;
+  return DLI_OK;
+}
+
+template <int kMode>
+static int launch_rows(const CUtensorMap& tmW, const CUtensorMap& tmX, const void* bias, const void* residual, void* y, int M,
+                       int N, int K, int epilogue, const RowsShape& sh, cudaStream_t s, const RopeArgs& rope, int hd) {
+  const int cols = sh.bn <= 32 ? 32 : sh.bn <= 64 ? 64 : sh.bn <= 128 ? 128 : 256;
+  const dim3 grid(sh.splits, (M + sh.bn - 1) / sh.bn, (N + 127) / 128);
+  const cudaError_t e = launch_kernel_cluster(gemm_rows_kernel<kMode>, grid, dim3(kRowsThreads), rows_smem(sh.bn, sh.stages), s,
+                                              (unsigned)sh.splits, tmW, tmX, (const bf16*)bias, (const bf16*)residual,
+                                              (bf16*)y, M, N, K, epilogue, sh.bn, sh.stages, cols, rope, hd);
+  if (e != cudaSuccess) return fail(DLI_ERR_CUDA, "gemm_rows_kernel: %s", cudaGetErrorString(e));
+  return DLI_OK;
+}
+
+int launch_gemm_rows(RowsMode mode, const void* x, const void* w, const void* bias, const void* residual, void* y, int M,
+                     int N, int K, int epilogue, const RowsShape& sh, cudaStream_t s, const RopeArgs& rope, int hd) {
+  int cap[kRowsMaxCluster + 1];
+  int rc = rows_setup(cap);
+  if (rc != DLI_OK) return rc;
+  if (sh.bn < 16 || sh.bn > 256 || sh.bn % 16 || sh.splits < 1 || sh.splits > kRowsMaxCluster || sh.splits > K / kBlockK ||
+      !rows_fits(sh.bn, sh.splits, sh.stages) || (N + 127) / 128 > 65535 || (M + sh.bn - 1) / sh.bn > 65535)
+    return fail(DLI_ERR_INVALID, "gemm_rows: M=%d N=%d K=%d in tiles of %d rows, %d splits, %d stages does not fit", M, N, K,
+                sh.bn, sh.splits, sh.stages);
+  CUtensorMap tmW, tmX;
+  if ((rc = make_tmap(&tmW, w, N, K, mode == kRowsGated ? 64 : 128)) != DLI_OK) return rc;
+  if ((rc = make_tmap(&tmX, x, M, K, sh.bn)) != DLI_OK) return rc;
+  if (mode == kRowsGated) return launch_rows<kRowsGated>(tmW, tmX, bias, residual, y, M, N, K, epilogue, sh, s, rope, hd);
+  if (mode == kRowsRope) return launch_rows<kRowsRope>(tmW, tmX, bias, residual, y, M, N, K, epilogue, sh, s, rope, hd);
+  return launch_rows<kRowsPlain>(tmW, tmX, bias, residual, y, M, N, K, epilogue, sh, s, rope, hd);
+}
+
+}  // namespace dli

@@ -340,8 +340,8 @@ def gemm_splitk_scratch_bytes(M, N) -> int:
 
 
 def linear_splitk(x, w, scratch, bias=None, residual=None, out=None, epilogue=EPI_NONE):
-    """Batched-decode projection (4 < M <= 128): split-K tcgen05 weight stream.  `scratch` is a
-    zero-initialised uint8/float tensor of gemm_splitk_scratch_bytes(M, N) bytes."""
+    """Batched-decode projection: the split-K tcgen05 weight stream gemm() takes for few rows.  `scratch` (a tensor of
+    gemm_splitk_scratch_bytes(M, N) bytes) is accepted and not used: partial sums meet in shared memory."""
     global launch_count
     _req(x), _req(w), _req(bias), _req(residual), _req(out)
     M, K = x.shape

@@ -291,15 +291,13 @@ int dli_gemm_qkv_rope_append_bf16(const void* x, const void* w_qkv, void* qkv, i
                                   int max_pages, void* k_cache, void* v_cache, int H, int KV,
                                   int hd, int page_size, dli_stream_t stream);
 
-/* Split-K variants of the tensor-core GEMM for batched decode (4 < M <= 128),
- * where the kernel is a weight stream and a matrix with few 128-row tiles would
- * leave most SMs (and most of HBM's bandwidth) idle: K is split over about
- * SMs/tiles CTAs per tile, each parks its fp32 partial in `scratch`, and the CTA
- * that finishes a tile last adds the partials in split order (deterministic) and
- * runs the epilogue.  scratch: dli_gemm_splitk_scratch_bytes(M, N) bytes (N = rows
- * of w; 2F for the gated form), ZERO-FILLED before its first use; every call
- * leaves its counters zero again.  Calls sharing a scratch buffer must be ordered
- * on one stream.  M > 128 or scratch == NULL falls through to dli_gemm_bf16. */
+/* The tensor-core GEMM as batched decode calls it (2 < M <= 128), where the kernel is
+ * a weight stream and a matrix with few 128-row tiles would leave most SMs (and most
+ * of HBM's bandwidth) idle.  K is split over the CTAs of a thread-block cluster, the
+ * fp32 partials meet in distributed shared memory and are added in split order
+ * (deterministic), so `scratch` is no longer read or written: it may be any 16-byte
+ * aligned buffer or NULL, and dli_gemm_bf16 / dli_gemm_gated_silu_bf16 run the same
+ * kernel.  dli_gemm_splitk_scratch_bytes keeps the size it has always returned. */
 size_t dli_gemm_splitk_scratch_bytes(int M, int N);
 int dli_gemm_splitk_bf16(const void* x, const void* w, const void* bias,
                          const void* residual, void* y, int M, int N, int K,
