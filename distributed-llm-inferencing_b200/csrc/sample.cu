@@ -1,4 +1,4 @@
-// Sampling epilogue: temperature -> top-k -> top-p -> multinomial, one CTA per row.
+// Sampling epilogue: temperature -> top-k -> top-p -> multinomial, one cluster of CTAs per row.
 //
 // This is what the reference worker asks of generate() by default
 // (worker/app.py:297-305: do_sample=True, top_k=50, top_p=0.95, temperature=0.8), i.e.
@@ -15,8 +15,13 @@
 //         draws agree in distribution, not bit for bit; the kept set and its probabilities
 //         are what the parity test compares.
 //
-// HBM-bound: the row (V * 2 bytes) is read three times (two radix-select passes over the
-// 16-bit keys + the gather); 0.77 MB per row at V = 128 256, negligible next to lm_head.
+// What bounds it: latency.  A row is 64 ... 256 KB, a few us of one SM's load bandwidth, so it is cut over a cluster of up
+// to 8 CTAs (16 384 logits each) and read ONCE, with 16-byte loads, into registers.  The k-th largest logit is found
+// without a histogram of the row: the k-th largest of a CTA's 512 per-thread maxima is a lower bound of it (k threads hold
+// an element at least that large), the largest such bound of the cluster leaves a few hundred candidates, and these meet
+// in the first CTA's shared memory, where the exact threshold is a binary search over keys.  (The two 256-bin
+// histograms with shared-memory atomics and their serial scans, three passes of 2-byte loads by one CTA per row, took
+// 62 us for one row as for 48, V = 128 256.)
 #include "common.cuh"
 
 namespace dli {
@@ -58,7 +63,37 @@ __device__ __forceinline__ float philox_uniform(uint64_t seed, uint32_t step, ui
   return (float)(p.c[0] >> 8) * (1.0f / 16777216.0f);
 }
 
-// Largest key t such that at least `k` elements have key >= t (two 8-bit radix passes).
+// ---- clusters -----------------------------------------------------------------------------------------------------
+constexpr int kSliceVecs = 4;                                  // 16-byte vectors a thread keeps in registers
+constexpr int kSliceElems = kSampleThreads * kSliceVecs * 8;   // logits of a CTA that are read once
+constexpr int kMaxRowCtas = 8;
+
+__device__ __forceinline__ uint32_t cluster_addr(const void* p, uint32_t rank) {
+  uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(p)), r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void cluster_st(uint32_t addr, uint32_t v) {
+  asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
+__device__ __forceinline__ uint32_t cluster_add(uint32_t addr, uint32_t v) {
+  uint32_t old;
+  asm volatile("atom.shared::cluster.add.u32 %0, [%1], %2;" : "=r"(old) : "r"(addr), "r"(v) : "memory");
+  return old;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// Larger of the two 16-bit halves' keys, and the keys of a vector's elements.
+__device__ __forceinline__ uint32_t vec_elem(const uint4& u, int e) {
+  const uint32_t w = e < 2 ? u.x : e < 4 ? u.y : e < 6 ? u.z : u.w;
+  return (e & 1) ? w >> 16 : w & 0xffffu;
+}
+
+// Largest key t such that at least `k` elements of the row have key >= t (two 8-bit radix passes over global memory): the
+// general form, for k above the number of threads and rows with more candidates than fit.
 __device__ uint32_t kth_largest_key(const uint16_t* __restrict__ row, int V, int k, uint32_t* hist /*256*/,
                                     uint32_t* sh /*2*/) {
   const int tid = threadIdx.x;
@@ -90,57 +125,189 @@ __device__ uint32_t kth_largest_key(const uint16_t* __restrict__ row, int V, int
   return prefix;
 }
 
+// grid: rows x CTAs of a row (a cluster)
 __global__ void __launch_bounds__(kSampleThreads)
 sample_kernel(const bf16* __restrict__ logits, int ld, int32_t* __restrict__ out, int V, float inv_temperature,
               int top_k, float top_p, const uint64_t* __restrict__ seed, const int32_t* __restrict__ step,
               float* __restrict__ dbg_probs, int32_t* __restrict__ dbg_ids, int dbg_cap, int per_row,
-              const int32_t* __restrict__ row_mask) {
+              const int32_t* __restrict__ row_mask, int ctas) {
   __shared__ uint32_t hist[256];
   __shared__ uint32_t sh[2];
   __shared__ float cval[kMaxCand];
   __shared__ int cidx[kMaxCand];
+  __shared__ uint32_t gkey[kMaxCand];  // first CTA: the row's candidates
+  __shared__ int gidx[kMaxCand];
+  __shared__ uint32_t bounds[kMaxRowCtas];
+  __shared__ uint32_t gcount;
+  __shared__ uint32_t gbase;
   __shared__ int ncand;
   __shared__ float red[kSampleThreads / 32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int b = blockIdx.x / ctas, rank = blockIdx.x - b * ctas;
+  if (tid == 0) gcount = 0, ncand = 0;
   pdl_wait();
   pdl_trigger();
-  if (row_mask != nullptr && row_mask[blockIdx.x] == 0) return;  // this row keeps the token already in out[]
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const uint16_t* row = reinterpret_cast<const uint16_t*>(logits + (size_t)blockIdx.x * ld);
+  if (row_mask != nullptr && row_mask[b] == 0) return;  // this row keeps the token already in out[]
+  const uint16_t* row = reinterpret_cast<const uint16_t*>(logits + (size_t)b * ld);
   const int k = top_k > 0 ? min(top_k, V) : V;
 
-  // ---- top-k threshold and candidate gather ------------------------------------------------
-  const uint32_t thr = kth_largest_key(row, V, min(k, kMaxCand), hist, sh);
+  // ---- this CTA's share of the row: whole 16-byte vectors; what lies before and after them goes to the first CTA --------
+  const int head = min(V, (int)(((16u - (uint32_t)(reinterpret_cast<uintptr_t>(row) & 15u)) & 15u) >> 1));
+  const int n_vec = (V - head) >> 3, tail0 = head + n_vec * 8;
+  const int v0 = (int)((long long)n_vec * rank / ctas), v1 = (int)((long long)n_vec * (rank + 1) / ctas);
+  const uint4* vecs = reinterpret_cast<const uint4*>(row + head);
+  uint4 held[kSliceVecs];
+#pragma unroll
+  for (int i = 0; i < kSliceVecs; ++i) {
+    const int v = v0 + i * kSampleThreads + tid;
+    // beyond the slice: the lowest key (a negative NaN), never at or above a bound
+    held[i] = v < v1 ? vecs[v] : make_uint4(0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu);
+  }
+  int edge = -1;  // an element of the unaligned ends
+  if (rank == 0) {
+    if (tid < head) edge = tid;
+    else if (tail0 + tid - head < V) edge = tail0 + tid - head;
+  }
+  uint32_t top = 0;
+#pragma unroll
+  for (int i = 0; i < kSliceVecs; ++i)
+#pragma unroll
+    for (int e = 0; e < 8; ++e) top = max(top, bf16_key((uint16_t)vec_elem(held[i], e)));
+  for (int v = v0 + kSliceVecs * kSampleThreads + tid; v < v1; v += kSampleThreads) {
+    const uint4 u = vecs[v];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) top = max(top, bf16_key((uint16_t)vec_elem(u, e)));
+  }
+  if (edge >= 0) top = max(top, bf16_key(row[edge]));
+
+  // ---- lower bound of the k-th largest key: the k-th largest of the per-thread maxima, bit by bit ---------------------
+  uint32_t bound = 0;
+  const bool narrow = k <= kSampleThreads;
+  if (narrow) {
+#pragma unroll 1
+    for (uint32_t bit = 0x8000u; bit; bit >>= 1)
+      if (__syncthreads_count(top >= (bound | bit)) >= k) bound |= bit;
+    if (tid < ctas) cluster_st(cluster_addr(&bounds[rank], tid), bound);
+    cluster_sync_all();
+    for (int c = 0; c < ctas; ++c) bound = max(bound, bounds[c]);
+    // ---- candidates: this CTA's elements at or above the bound, then all of the row's in the first CTA ----------------
+    auto take = [&](uint32_t raw, int i) {
+      const uint32_t key = bf16_key((uint16_t)raw);
+      if (key >= bound) {
+        const int slot = atomicAdd(&ncand, 1);
+        if (slot < kMaxCand) { cval[slot] = __uint_as_float(key); cidx[slot] = i; }
+      }
+    };
+#pragma unroll
+    for (int i = 0; i < kSliceVecs; ++i) {
+      const int v = v0 + i * kSampleThreads + tid;
+      if (v < v1) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) take(vec_elem(held[i], e), head + v * 8 + e);
+      }
+    }
+    for (int v = v0 + kSliceVecs * kSampleThreads + tid; v < v1; v += kSampleThreads) {
+      const uint4 u = vecs[v];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) take(vec_elem(u, e), head + v * 8 + e);
+    }
+    if (edge >= 0) take(row[edge], edge);
+    __syncthreads();
+    const uint32_t mine = (uint32_t)ncand;
+    if (tid == 0) gbase = cluster_add(cluster_addr(&gcount, 0), min(mine, (uint32_t)kMaxCand + 1));  // too many: too many there too
+    __syncthreads();
+    const uint32_t base = gbase, kb = cluster_addr(gkey, 0), ib = cluster_addr(gidx, 0);
+    if (mine <= (uint32_t)kMaxCand && base + mine <= (uint32_t)kMaxCand) {
+      for (uint32_t i = tid; i < mine; i += kSampleThreads) {
+        cluster_st(kb + (base + i) * 4, __float_as_uint(cval[i]));
+        cluster_st(ib + (base + i) * 4, (uint32_t)cidx[i]);
+      }
+    }
+    cluster_sync_all();
+  }
+  if (rank != 0) return;
+
+  // ---- first CTA: the exact threshold, and everything at or above it (ties are kept) ----------------------------------
   if (tid == 0) ncand = 0;
-  __syncthreads();
-  for (int i = tid; i < V; i += kSampleThreads) {
-    const uint32_t key = bf16_key(row[i]);
-    if (key >= thr) {
-      const int slot = atomicAdd(&ncand, 1);
-      if (slot < kMaxCand) { cval[slot] = key_value(key) * inv_temperature; cidx[slot] = i; }
+  if (narrow && gcount <= (uint32_t)kMaxCand) {
+    const int n_c = (int)gcount;
+    uint32_t keys[kMaxCand / kSampleThreads];
+#pragma unroll
+    for (int q = 0; q < kMaxCand / kSampleThreads; ++q)
+      keys[q] = q * kSampleThreads + tid < n_c ? gkey[q * kSampleThreads + tid] : 0u;
+    uint32_t thr = 0;
+#pragma unroll 1
+    for (uint32_t bit = 0x8000u; bit; bit >>= 1) {
+      int count = 0;
+#pragma unroll
+      for (int q = 0; q < kMaxCand / kSampleThreads; ++q)
+        if (q * kSampleThreads < n_c) count += __syncthreads_count(keys[q] >= (thr | bit));
+      if (count >= k) thr |= bit;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < kMaxCand / kSampleThreads; ++q) {
+      const int i = q * kSampleThreads + tid;
+      if (i < n_c && keys[q] >= thr) {
+        const int slot = atomicAdd(&ncand, 1);
+        cval[slot] = key_value(keys[q]) * inv_temperature;
+        cidx[slot] = gidx[i];
+      }
+    }
+  } else {
+    const uint32_t thr = kth_largest_key(row, V, min(k, kMaxCand), hist, sh);
+    // what lies above the threshold first (fewer than k elements): ties beyond the capacity are dropped, never those
+    for (int ties = 0; ties < 2; ++ties) {
+      for (int i = tid; i < V; i += kSampleThreads) {
+        const uint32_t key = bf16_key(row[i]);
+        if (ties ? key == thr : key > thr) {
+          const int slot = atomicAdd(&ncand, 1);
+          if (slot < kMaxCand) { cval[slot] = key_value(key) * inv_temperature; cidx[slot] = i; }
+        }
+      }
+      __syncthreads();
     }
   }
   __syncthreads();
   const int n = min(ncand, kMaxCand);
-  int npow = 1;
-  while (npow < n) npow <<= 1;
-  for (int i = n + tid; i < npow; i += kSampleThreads) { cval[i] = -INFINITY; cidx[i] = -1; }
-  __syncthreads();
-  // bitonic sort, descending by value, equal values by ascending token id.  Which of several
-  // EQUAL-probability tokens survive at the nucleus boundary depends on torch.sort's tie order
-  // in the reference (not specified); here the lower token ids stay.
-  for (int size = 2; size <= npow; size <<= 1) {
-    for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      for (int i = tid; i < npow; i += kSampleThreads) {
-        const int j = i ^ stride;
-        if (j > i) {
-          const bool desc = (i & size) == 0;
-          const float a = cval[i], b = cval[j];
-          const int ia = cidx[i], ib = cidx[j];
-          const bool a_first = (a > b) || (a == b && (unsigned)ia < (unsigned)ib);
-          if (a_first != desc) { cval[i] = b; cval[j] = a; cidx[i] = ib; cidx[j] = ia; }
-        }
+  // Descending by value, equal values by ascending token id.  Which of several EQUAL-probability tokens survive at the
+  // nucleus boundary depends on torch.sort's tie order in the reference (not specified); here the lower token ids stay.
+  if (n <= kSampleThreads) {
+    // every candidate counts those before it (a NaN goes before every number)
+    float a = 0.f;
+    int ia = 0, place = 0;
+    if (tid < n) {
+      a = cval[tid];
+      ia = cidx[tid];
+      for (int j = 0; j < n; ++j) {
+        const float c = cval[j];
+        const bool tie = c == a || (c != c && a != a);
+        place += (c > a || (c != c && a == a) || (tie && cidx[j] < ia)) ? 1 : 0;
       }
-      __syncthreads();
+    }
+    __syncthreads();
+    if (tid < n) { cval[place] = a; cidx[place] = ia; }
+    __syncthreads();
+  } else {
+    int npow = 1;
+    while (npow < n) npow <<= 1;
+    for (int i = n + tid; i < npow; i += kSampleThreads) { cval[i] = -INFINITY; cidx[i] = -1; }
+    __syncthreads();
+    // bitonic sort
+    for (int size = 2; size <= npow; size <<= 1) {
+      for (int stride = size >> 1; stride > 0; stride >>= 1) {
+        for (int i = tid; i < npow; i += kSampleThreads) {
+          const int j = i ^ stride;
+          if (j > i) {
+            const bool desc = (i & size) == 0;
+            const float a = cval[i], b = cval[j];
+            const int ia = cidx[i], ib = cidx[j];
+            const bool a_first = (a > b) || (a == b && (unsigned)ia < (unsigned)ib);
+            if (a_first != desc) { cval[i] = b; cval[j] = a; cidx[i] = ib; cidx[j] = ia; }
+          }
+        }
+        __syncthreads();
+      }
     }
   }
   // ---- softmax over the top-k set, nucleus cut, renormalise, draw (n <= 2048: one warp scans) ----
@@ -181,25 +348,47 @@ sample_kernel(const bf16* __restrict__ logits, int ld, int32_t* __restrict__ out
     mass = warp_sum(mass);
     if (dbg_probs) {
       for (int i = lane; i < dbg_cap; i += 32) {
-        dbg_probs[(size_t)blockIdx.x * dbg_cap + i] = i < kept ? cval[i] / mass : 0.f;
-        dbg_ids[(size_t)blockIdx.x * dbg_cap + i] = i < kept ? cidx[i] : -1;
+        dbg_probs[(size_t)b * dbg_cap + i] = i < kept ? cval[i] / mass : 0.f;
+        dbg_ids[(size_t)b * dbg_cap + i] = i < kept ? cidx[i] : -1;
       }
     }
     if (lane == 0) {
       // per_row: every row has its own (seed, step) and the row index stays out of the key, so a sequence's
       // draws do not depend on the batch row it happens to occupy
-      const int r = per_row ? blockIdx.x : 0;
-      const float u = philox_uniform(seed ? seed[r] : 0ull, step ? (uint32_t)step[r] : 0u,
-                                     per_row ? 0u : blockIdx.x) * mass;
+      const int r = per_row ? b : 0;
+      const float u = philox_uniform(seed ? seed[r] : 0ull, step ? (uint32_t)step[r] : 0u, per_row ? 0u : b) * mass;
       float acc = 0.f;
       int pick = kept - 1;
-      for (int i = 0; i < kept; ++i) {
-        acc += cval[i];
-        if (u < acc) { pick = i; break; }
+      for (int i0 = 0; i0 < kept; i0 += 8) {  // eight loads in flight, the sums in order
+        float p[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) p[e] = cval[min(i0 + e, kept - 1)];
+        int first = kept;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          acc += p[e];
+          if (first == kept && i0 + e < kept && u < acc) first = i0 + e;
+        }
+        if (first < kept) { pick = first; break; }
       }
-      out[blockIdx.x] = cidx[pick];
+      out[b] = cidx[pick];
     }
   }
+}
+
+// A cluster of as many CTAs as the row has slices of 16 384 logits, at most the portable 8 (beyond 131 072 logits a
+// thread reads the rest of its slice twice).
+static int launch_sample(const char* what, const void* logits, int ld, int32_t* out, int B, int V, float temperature,
+                         int top_k, float top_p, const uint64_t* seed, const int32_t* step, float* dbg_probs,
+                         int32_t* dbg_ids, int dbg_cap, int per_row, const int32_t* row_mask, cudaStream_t s) {
+  int ctas = (V - 1) / kSliceElems + 1;
+  if (ctas > kMaxRowCtas) ctas = kMaxRowCtas;
+  if ((long long)B * ctas > 0x7fffffffLL) ctas = 1;
+  const cudaError_t e = launch_kernel_cluster(sample_kernel, dim3((unsigned)B * ctas), dim3(kSampleThreads), (size_t)0, s,
+                                              (unsigned)ctas, (const bf16*)logits, ld, out, V, 1.0f / temperature, top_k,
+                                              top_p, seed, step, dbg_probs, dbg_ids, dbg_cap, per_row, row_mask, ctas);
+  if (e != cudaSuccess) return fail(DLI_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
+  return DLI_OK;
 }
 
 }  // namespace dli
@@ -216,10 +405,8 @@ extern "C" int dli_sample_bf16(const void* logits, int ld, int32_t* out, int B, 
                 "dli_sample_bf16: top_k must be 1..%d when the vocabulary is larger than that", kMaxCand);
   DLI_CHECK_ARG((dbg_probs == nullptr) == (dbg_ids == nullptr) && dbg_cap >= 0, "dli_sample_bf16: bad debug buffers");
   if (B == 0) return DLI_OK;
-  DLI_LAUNCH("dli_sample_bf16", sample_kernel, dim3(B), dim3(kSampleThreads), (size_t)0, static_cast<cudaStream_t>(stream),
-             (const bf16*)logits, ld, out, V, 1.0f / temperature, top_k, top_p, seed, step, dbg_probs, dbg_ids, dbg_cap,
-             0, (const int32_t*)nullptr);
-  return DLI_OK;
+  return launch_sample("dli_sample_bf16", logits, ld, out, B, V, temperature, top_k, top_p, seed, step, dbg_probs, dbg_ids,
+                       dbg_cap, 0, nullptr, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int dli_sample_rows_bf16(const void* logits, int ld, int32_t* out, int B, int V, float temperature,
@@ -233,8 +420,6 @@ extern "C" int dli_sample_rows_bf16(const void* logits, int ld, int32_t* out, in
   DLI_CHECK_ARG((top_k > 0 && top_k <= kMaxCand) || V <= kMaxCand,
                 "dli_sample_rows_bf16: top_k must be 1..%d when the vocabulary is larger than that", kMaxCand);
   if (B == 0) return DLI_OK;
-  DLI_LAUNCH("dli_sample_rows_bf16", sample_kernel, dim3(B), dim3(kSampleThreads), (size_t)0,
-             static_cast<cudaStream_t>(stream), (const bf16*)logits, ld, out, V, 1.0f / temperature, top_k, top_p, seeds,
-             steps, (float*)nullptr, (int32_t*)nullptr, 0, 1, row_mask);
-  return DLI_OK;
+  return launch_sample("dli_sample_rows_bf16", logits, ld, out, B, V, temperature, top_k, top_p, seeds, steps, nullptr,
+                       nullptr, 0, 1, row_mask, static_cast<cudaStream_t>(stream));
 }
