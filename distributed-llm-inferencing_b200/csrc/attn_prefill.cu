@@ -215,6 +215,24 @@ static int launch_prefill(const void* qkv, void* out, int B, int T, int H, int K
   return DLI_OK;
 }
 
+// attn_prefill_tc.cu: both attention GEMMs on tcgen05
+int launch_attn_prefill_tc(const void* qkv, void* out, int B, int T, int H, int KV, int hd, float scale, int window,
+                           cudaStream_t s);
+int launch_attn_prefill_tc_paged(const void* qkv, void* out, const void* k_cache, const void* v_cache,
+                                 const int32_t* page_table, int max_pages, int num_pages, int B, int T, int prefix,
+                                 int H, int KV, int hd, int page_size, float scale, int window, cudaStream_t s);
+// The tcgen05 kernel takes ~5 us whatever it does (TMEM, barriers, a 128-row tile), the mma.sync kernel half of that; by the
+// longest key range of the call, us on B200 (mma.sync / tcgen05), one prompt, no prefix unless given:
+//   32 heads of 64:  T = 19: 2.7 / 5.3, 256: 5.3 / 6.6, 400: 9.0 / 8.3, 512: 10.4 / 8.7, 1777: 54 / 34, 4096: 249 / 132;
+//                    T = 16 after 512: 10.8 / 10.4, after 6000: 95 / 57
+//   12 heads of 64:  T = 256: 5.3 / 6.8, 400: 7.6 / 8.2, 512: 8.7 / 9.0, 800: 13.5 / 11.5, 1777: 34 / 19
+//   32 heads of 128: T = 19: 3.8 / 5.6, 64: 4.4 / 5.9, 128: 5.7 / 6.4 (eight prompts of 100: 12.0 / 9.9), 301: 11.6 / 7.9
+// DLI_PREFILL_ATTN=mma keeps the mma.sync kernel everywhere.
+static bool prefill_on_tc(int hd, int keys) {
+  static const bool tc = !(getenv("DLI_PREFILL_ATTN") && getenv("DLI_PREFILL_ATTN")[0] == 'm');
+  return tc && (hd == 64 ? keys >= 448 : keys > 64);
+}
+
 }  // namespace dli
 
 extern "C" int dli_attn_prefill_bf16(const void* qkv, void* out, int B, int T, int H, int KV, int hd,
@@ -229,13 +247,8 @@ extern "C" int dli_attn_prefill_bf16(const void* qkv, void* out, int B, int T, i
   if (B == 0 || T == 0) return DLI_OK;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (hd == 128) return launch_prefill<128, false>(qkv, out, B, T, H, KV, scale, window, s);
+  if (prefill_on_tc(hd, T)) return launch_attn_prefill_tc(qkv, out, B, T, H, KV, hd, scale, window, s);
   return launch_prefill<64, false>(qkv, out, B, T, H, KV, scale, window, s);
-}
-
-namespace dli {
-int launch_attn_prefill_tc_paged(const void* qkv, void* out, const void* k_cache, const void* v_cache,
-                                 const int32_t* page_table, int max_pages, int num_pages, int B, int T, int prefix,
-                                 int H, int KV, int page_size, float scale, int window, cudaStream_t s);
 }
 
 extern "C" int dli_attn_prefill_paged_bf16(const void* qkv, void* out, const void* k_cache, const void* v_cache,
@@ -259,12 +272,10 @@ extern "C" int dli_attn_prefill_paged_bf16(const void* qkv, void* out, const voi
   int shift = 0;
   while ((1 << shift) < page_size) ++shift;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  // head_dim 128: both attention GEMMs on tcgen05, K/V pages brought in by TMA (num_pages > 0 says how large the
-  // pools are); DLI_PREFILL_ATTN=mma keeps the mma.sync kernel
-  static const bool use_tc = !(getenv("DLI_PREFILL_ATTN") && getenv("DLI_PREFILL_ATTN")[0] == 'm');
-  if (hd == 128 && use_tc && num_pages > 0 && page_size <= 128)
+  // both attention GEMMs on tcgen05, K/V pages brought in by TMA (num_pages > 0 says how large the pools are)
+  if (prefill_on_tc(hd, prefix + T) && num_pages > 0 && page_size <= 128)
     return launch_attn_prefill_tc_paged(qkv, out, k_cache, v_cache, page_table, max_pages, num_pages, B, T, prefix, H,
-                                        KV, page_size, scale, window, s);
+                                        KV, hd, page_size, scale, window, s);
   if (hd == 128)
     return launch_prefill<128, true>(qkv, out, B, T, H, KV, scale, window, s, k_cache, v_cache, page_table, max_pages,
                                      shift, prefix);

@@ -1,4 +1,4 @@
-// Causal prefill attention on the 5th-generation tensor cores (head_dim 128).
+// Causal prefill attention on the 5th-generation tensor cores (head_dim 128 and 64).
 //
 // Work item = 128 query rows of one head; KV tiles of 128 tokens; one persistent CTA per SM walks a
 // length-sorted list of items (see TcItem below).  Both GEMMs of flash attention are tcgen05.mma
@@ -7,7 +7,7 @@
 //   O += P V    : A = P (bf16, two per 32-bit column, written to TENSOR memory by the softmax warps with
 //                 tcgen05.st; the TS form of the MMA reads it there), B = V tile as an MN-major operand
 //                 (hd contiguous, tokens along K), exactly as TMA lands the [tokens, hd] rows
-// TMEM: S0 | S1 (two score buffers, 128 columns each) | O (128 columns) | P0 | P1 (64 columns each).
+// TMEM: S0 | S1 (two score buffers, 128 columns each) | O (128 columns, hd of them used) | P0 | P1 (64 columns each).
 // Roles (576 threads): warp 0 = TMA producer, warp 1 = MMA issuer + TMEM owner, warps 2-17 =
 // softmax + output pass: four threads per query row (TMEM lane), 32 columns each, fp32 online softmax.
 // The MMA warp issues S(j+1) before it waits for the softmax of tile j, so the tensor pipe
@@ -20,17 +20,22 @@ namespace dli {
 
 constexpr int kRowThreads = 4;                 // softmax threads per query row (each owns 128 / kRowThreads columns)
 constexpr int kSmWarps = 4 * kRowThreads;      // softmax warps: kRowThreads per TMEM lane quadrant
-constexpr int kSmCols = 128 / kRowThreads;     // score / output columns per softmax thread
+constexpr int kSmCols = 128 / kRowThreads;     // score columns per softmax thread
 constexpr int kTcThreads = 64 + 32 * kSmWarps;  // TMA warp + MMA warp + softmax warps
 static_assert(kRowThreads == 4, "the P store writes 16 packed columns per thread; the TMEM map assumes 4 x 32 columns");
 constexpr int kTcTile = 128;      // query rows per item and tokens per KV tile
-constexpr int kTcHd = 128;
 constexpr int kSpanBytes = 128 * 64 * 2;  // one [128 rows x 64 elements] swizzled sub-tile: 16 KB
-constexpr int kTileBytes2 = 2 * kSpanBytes;  // a [128 x 128] bf16 operand tile: 32 KB
 
-// smem: Q | K0 K1 | V0 V1 | barriers
-// + alignment slack, barriers, row max exchange [2][kRowThreads][128], row sum exchange [kRowThreads][128]
-constexpr int kTcSmem = 5 * kTileBytes2 + 1024 + 256 + 3 * kRowThreads * 128 * 4;
+template <int HD>
+struct TcCfg {
+  static_assert(HD == 64 || HD == 128, "whole 64-element swizzle spans");
+  static constexpr int kSpans = HD / 64;
+  static constexpr int kTileBytes = kSpans * kSpanBytes;  // a [128 x HD] bf16 operand tile
+  static constexpr int kOutCols = HD / kRowThreads;       // output columns per softmax thread
+  // smem: Q | K0 K1 | V0 V1 | barriers
+  // + alignment slack, barriers, row max exchange [2][kRowThreads][128], row sum exchange [kRowThreads][128]
+  static constexpr int kSmem = 5 * kTileBytes + 1024 + 256 + 3 * kRowThreads * 128 * 4;
+};
 
 __device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t (&r)[32]) {
   asm volatile(
@@ -51,6 +56,11 @@ __device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t (&r
       "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
       : "memory");
 }
+// a thread's output columns: 32 (head size 128) or 16 (64)
+__device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&r)[32]) { tmem_ld_32x32(taddr, r); }
+__device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&r)[16]) { tmem_ld_32x16(taddr, r); }
+__device__ __forceinline__ void tmem_st_cols(uint32_t taddr, const uint32_t (&r)[32]) { tmem_st_32x32(taddr, r); }
+__device__ __forceinline__ void tmem_st_cols(uint32_t taddr, const uint32_t (&r)[16]) { tmem_st_32x16(taddr, r); }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // MN-major SWIZZLE_128B operand (V as B: N = hd contiguous, K = tokens): 64-element MN groups are
@@ -64,9 +74,9 @@ __device__ __forceinline__ uint64_t make_smem_desc_mn(uint32_t saddr) {
   d |= (uint64_t)2 << 61;
   return d;
 }
-// D=f32, A=bf16 K-major, B=bf16 (K-major or MN-major), M=128, N=128
-__host__ __device__ constexpr uint32_t make_idesc_attn(bool b_mn_major) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((b_mn_major ? 1u : 0u) << 16) | ((uint32_t)(128 >> 3) << 17) |
+// D=f32, A=bf16 K-major, B=bf16 (K-major or MN-major), M=128, N=n
+__host__ __device__ constexpr uint32_t make_idesc_attn(bool b_mn_major, int n) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((b_mn_major ? 1u : 0u) << 16) | ((uint32_t)(n >> 3) << 17) |
          ((uint32_t)(128 >> 4) << 24);
 }
 
@@ -85,12 +95,16 @@ struct TcItem {
 // from the paged cache through two more tensor maps (the cache seen as [pages*KV*page_size, hd] rows, box = one
 // page x 64 columns): the 32 lanes of the producer warp each issue one page-sized box of a 128-token tile.
 // A box whose first token lies beyond the context is requested out of bounds, i.e. zero-filled.
-template <bool kPaged>
+//
+// Head size 64 (TinyLlama, GPT-2): half the MMA work and operand bytes per tile, the same softmax, which is what bounds
+// the kernel at either size: 33.8 us for 1 777 tokens of 32 heads (54.1 on the mma.sync kernel), 132 for 4 096 (249).
+template <int HD, bool kPaged>
 __global__ void __launch_bounds__(kTcThreads, 1)
 attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant__ CUtensorMap tmK,
                        const __grid_constant__ CUtensorMap tmV, bf16* __restrict__ out, int T, int H, int KV,
                        float scale_log2, int window, const int32_t* __restrict__ page_table, int max_pages,
                        int page_shift, int prefix, int cache_rows, int B, int n_qtiles) {
+  constexpr int kTcHd = HD, kTileBytes2 = TcCfg<HD>::kTileBytes, kOutCols = TcCfg<HD>::kOutCols;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const uint32_t sQ = smem_addr(smem);
@@ -165,7 +179,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm, const __grid_cons
       tma_prefetch_desc(&tmV);
     }
     const int page_size = 1 << page_shift;
-    const int nb = kTcTile >> page_shift;  // boxes per 64-column half of a tile (<= 16)
+    const int nb = kTcTile >> page_shift;  // boxes per 64-column span of a tile (<= 16)
+    constexpr int kSpans = TcCfg<HD>::kSpans;
     const int half = lane / nb, bi = lane - half * nb;
     const int total = prefix + T;
     int g = 0;
@@ -175,14 +190,14 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm, const __grid_cons
         mbar_wait(q_empty, (n & 1) ^ 1);  // the last S = Q K^T of the previous item has read Q
         mbar_expect_tx(q_full, kTileBytes2);
         tma_load_2d(sQ, &tm, q_full, w.h * kTcHd, w.row_base + w.q0);
-        tma_load_2d(sQ + kSpanBytes, &tm, q_full, w.h * kTcHd + 64, w.row_base + w.q0);
+        if (HD > 64) tma_load_2d(sQ + kSpanBytes, &tm, q_full, w.h * kTcHd + 64, w.row_base + w.q0);
       }
       for (int j = w.t_begin; j < w.t_end; ++j, ++g) {
         const int st = g & 1;
         const uint32_t ph = (g >> 1) & 1;
         const int tok0 = j * kTcTile + bi * page_size;
         int row = cache_rows;  // out of bounds: the box is zero-filled
-        if (lane < 2 * nb && tok0 < total)
+        if (lane < kSpans * nb && tok0 < total)
           row = (page_table[(size_t)w.b * max_pages + (tok0 >> page_shift)] * KV + w.kvh) << page_shift;
         const uint32_t dst = (uint32_t)(st * kTileBytes2 + half * kSpanBytes + bi * page_size * 128);
         if (lane == 0) {
@@ -190,13 +205,13 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm, const __grid_cons
           mbar_expect_tx(k_full + 8 * st, kTileBytes2);
         }
         __syncwarp();
-        if (lane < 2 * nb) tma_load_2d(sK + dst, &tmK, k_full + 8 * st, half * 64, row);
+        if (lane < kSpans * nb) tma_load_2d(sK + dst, &tmK, k_full + 8 * st, half * 64, row);
         if (lane == 0) {
           mbar_wait(v_empty + 8 * st, ph ^ 1);
           mbar_expect_tx(v_full + 8 * st, kTileBytes2);
         }
         __syncwarp();
-        if (lane < 2 * nb) tma_load_2d(sV + dst, &tmV, v_full + 8 * st, half * 64, row);
+        if (lane < kSpans * nb) tma_load_2d(sV + dst, &tmV, v_full + 8 * st, half * 64, row);
       }
     }
   } else if (warp == 0) {
@@ -208,7 +223,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm, const __grid_cons
         mbar_wait(q_empty, (n & 1) ^ 1);
         mbar_expect_tx(q_full, kTileBytes2);
         tma_load_2d(sQ, &tm, q_full, w.h * kTcHd, w.row_base + w.q0);
-        tma_load_2d(sQ + kSpanBytes, &tm, q_full, w.h * kTcHd + 64, w.row_base + w.q0);
+        if (HD > 64) tma_load_2d(sQ + kSpanBytes, &tm, q_full, w.h * kTcHd + 64, w.row_base + w.q0);
         for (int j = w.t_begin; j < w.t_end; ++j, ++g) {
           const int st = g & 1;
           const uint32_t ph = (g >> 1) & 1;
@@ -216,11 +231,11 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm, const __grid_cons
           mbar_wait(k_empty + 8 * st, ph ^ 1);
           mbar_expect_tx(k_full + 8 * st, kTileBytes2);
           tma_load_2d(sK + st * kTileBytes2, &tm, k_full + 8 * st, (H + w.kvh) * kTcHd, krow);
-          tma_load_2d(sK + st * kTileBytes2 + kSpanBytes, &tm, k_full + 8 * st, (H + w.kvh) * kTcHd + 64, krow);
+          if (HD > 64) tma_load_2d(sK + st * kTileBytes2 + kSpanBytes, &tm, k_full + 8 * st, (H + w.kvh) * kTcHd + 64, krow);
           mbar_wait(v_empty + 8 * st, ph ^ 1);
           mbar_expect_tx(v_full + 8 * st, kTileBytes2);
           tma_load_2d(sV + st * kTileBytes2, &tm, v_full + 8 * st, (H + KV + w.kvh) * kTcHd, krow);
-          tma_load_2d(sV + st * kTileBytes2 + kSpanBytes, &tm, v_full + 8 * st, (H + KV + w.kvh) * kTcHd + 64, krow);
+          if (HD > 64) tma_load_2d(sV + st * kTileBytes2 + kSpanBytes, &tm, v_full + 8 * st, (H + KV + w.kvh) * kTcHd + 64, krow);
         }
       }
     }
@@ -228,7 +243,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm, const __grid_cons
     {
       // ---------------- MMA issuer: the whole warp runs the loop (uniform values stay in uniform registers), one
       // elected lane issues each tcgen05 instruction ----------------
-      constexpr uint32_t idesc_s = make_idesc_attn(false), idesc_o = make_idesc_attn(true);
+      constexpr uint32_t idesc_s = make_idesc_attn(false, kTcTile), idesc_o = make_idesc_attn(true, HD);
       // operand descriptors: the 14-bit start-address field (bytes >> 4) advances with the k-step, so a k-step is
       // an add on the low word.  Q/K: 16 elements = 32 B inside a 64-element span, spans kSpanBytes apart;
       // V (MN-major): 16 tokens = two 8-row groups = 2048 B
@@ -386,15 +401,12 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm, const __grid_cons
           // barrier (g-1) & 1 is in the phase of P.V(g-1) or just past it, never further.
           mbar_wait(pv_done + 8 * ((g - 1) & 1), ((g - 1) >> 1) & 1);
           tcgen05_fence_after();
+          uint32_t r[kOutCols];
+          tmem_ld_cols(tO + lane_off + part * kOutCols, r);
+          tmem_ld_wait();
 #pragma unroll
-          for (int c = 0; c < kSmCols / 32; ++c) {
-            uint32_t r[32];
-            tmem_ld_32x32(tO + lane_off + col0 + c * 32, r);
-            tmem_ld_wait();
-#pragma unroll
-            for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * corr);
-            tmem_st_32x32(tO + lane_off + col0 + c * 32, r);
-          }
+          for (int i = 0; i < kOutCols; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * corr);
+          tmem_st_cols(tO + lane_off + part * kOutCols, r);
         }
         tmem_st_wait();            // P (and O) are in tensor memory before the MMA warp is told
         tcgen05_fence_before();
@@ -410,22 +422,19 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm, const __grid_cons
       mbar_wait(pv_done + 8 * ((g - 1) & 1), ((g - 1) >> 1) & 1);  // the item's last P.V (same argument as above)
       tcgen05_fence_after();
       const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
-      bf16* dst = out + ((size_t)(w.row_base + qrel)) * ((size_t)H * kTcHd) + (size_t)w.h * kTcHd + col0;
+      bf16* dst = out + ((size_t)(w.row_base + qrel)) * ((size_t)H * kTcHd) + (size_t)w.h * kTcHd + part * kOutCols;
       {
-        uint32_t r[kSmCols / 32][32];
-#pragma unroll
-        for (int c = 0; c < kSmCols / 32; ++c) tmem_ld_32x32(tO + lane_off + col0 + c * 32, r[c]);
+        uint32_t r[kOutCols];
+        tmem_ld_cols(tO + lane_off + part * kOutCols, r);
         tmem_ld_wait();
         if (qrel < T) {
 #pragma unroll
-          for (int c = 0; c < kSmCols / 32; ++c)
+          for (int gq = 0; gq < kOutCols / 8; ++gq) {
+            float v[8];
 #pragma unroll
-            for (int gq = 0; gq < 4; ++gq) {
-              float v[8];
-#pragma unroll
-              for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[c][gq * 8 + i]) * inv;
-              st_16B(dst + c * 32 + gq * 8, pack8(v));
-            }
+            for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[gq * 8 + i]) * inv;
+            st_16B(dst + gq * 8, pack8(v));
+          }
         }
       }
       tcgen05_fence_before();  // O has been read: the next item's first P.V (after its P) may overwrite it
@@ -436,6 +445,69 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm, const __grid_cons
     tcgen05_fence_after();
     tmem_dealloc(tmem_base, 512);
   }
+}
+
+// ---- host side: the packed qkv matrix [B*T, cols], box = 128 rows x 64 columns (one swizzle span) --------------------
+template <int HD>
+static int launch_tc(const void* qkv, void* out, int B, int T, int H, int KV, float scale, int window, cudaStream_t s) {
+  static PerDeviceOnce once;
+  DLI_ONCE_PER_DEVICE(once, dev,
+                      DLI_CUDA_CALL(cudaFuncSetAttribute(attn_prefill_tc_kernel<HD, false>,
+                                                         cudaFuncAttributeMaxDynamicSharedMemorySize, TcCfg<HD>::kSmem)));
+  CUtensorMap tm;
+  const int rc = make_tmap(&tm, qkv, B * T, (H + 2 * KV) * HD, 128);
+  if (rc != DLI_OK) return rc;
+  const int n_qtiles = (T + kTcTile - 1) / kTcTile;
+  const long long n_items = (long long)n_qtiles * H * B;
+  dim3 grid((unsigned)(n_items < sm_count_cached() ? n_items : sm_count_cached()));  // persistent: one CTA per SM
+  DLI_LAUNCH("attn_prefill_tc_kernel", (attn_prefill_tc_kernel<HD, false>), grid, dim3(kTcThreads),
+             (size_t)TcCfg<HD>::kSmem, s, tm, tm, tm, (bf16*)out, T, H, KV, scale * 1.4426950408889634f, window,
+             (const int32_t*)nullptr, 0, 0, 0, 0, B, n_qtiles);
+  return DLI_OK;
+}
+
+int launch_attn_prefill_tc(const void* qkv, void* out, int B, int T, int H, int KV, int hd, float scale, int window,
+                           cudaStream_t s) {
+  return hd == 64 ? launch_tc<64>(qkv, out, B, T, H, KV, scale, window, s)
+                  : launch_tc<128>(qkv, out, B, T, H, KV, scale, window, s);
+}
+
+template <int HD>
+static int launch_tc_paged(const void* qkv, void* out, const void* k_cache, const void* v_cache,
+                           const int32_t* page_table, int max_pages, int num_pages, int B, int T, int prefix, int H,
+                           int KV, int page_size, float scale, int window, cudaStream_t s) {
+  static PerDeviceOnce once;
+  DLI_ONCE_PER_DEVICE(once, dev,
+                      DLI_CUDA_CALL(cudaFuncSetAttribute(attn_prefill_tc_kernel<HD, true>,
+                                                         cudaFuncAttributeMaxDynamicSharedMemorySize, TcCfg<HD>::kSmem)));
+  CUtensorMap tm, tmK, tmV;
+  int rc = make_tmap(&tm, qkv, B * T, (H + 2 * KV) * HD, 128);
+  if (rc != DLI_OK) return rc;
+  // the cache pools as [num_pages * KV * page_size, HD] rows; box = one page x 64 columns
+  const long long rows = (long long)num_pages * KV * page_size;
+  if (rows <= 0 || rows > 0x7fffffffLL) return fail(DLI_ERR_INVALID, "dli_attn_prefill_paged_bf16: cache too large for one tensor map");
+  rc = make_tmap(&tmK, k_cache, (int)rows, HD, page_size);
+  if (rc != DLI_OK) return rc;
+  rc = make_tmap(&tmV, v_cache, (int)rows, HD, page_size);
+  if (rc != DLI_OK) return rc;
+  int shift = 0;
+  while ((1 << shift) < page_size) ++shift;
+  const int n_qtiles = (T + kTcTile - 1) / kTcTile;
+  const long long n_items = (long long)n_qtiles * H * B;
+  dim3 grid((unsigned)(n_items < sm_count_cached() ? n_items : sm_count_cached()));
+  DLI_LAUNCH("attn_prefill_tc_kernel", (attn_prefill_tc_kernel<HD, true>), grid, dim3(kTcThreads),
+             (size_t)TcCfg<HD>::kSmem, s, tm, tmK, tmV, (bf16*)out, T, H, KV, scale * 1.4426950408889634f, window,
+             page_table, max_pages, shift, prefix, (int)rows, B, n_qtiles);
+  return DLI_OK;
+}
+
+// tcgen05 form of dli_attn_prefill_paged_bf16 (8 <= page_size <= 128); called from attn_prefill.cu.
+int launch_attn_prefill_tc_paged(const void* qkv, void* out, const void* k_cache, const void* v_cache,
+                                 const int32_t* page_table, int max_pages, int num_pages, int B, int T, int prefix,
+                                 int H, int KV, int hd, int page_size, float scale, int window, cudaStream_t s) {
+  const auto launch = hd == 64 ? launch_tc_paged<64> : launch_tc_paged<128>;
+  return launch(qkv, out, k_cache, v_cache, page_table, max_pages, num_pages, B, T, prefix, H, KV, page_size, scale,
+                window, s);
 }
 
 }  // namespace dli
@@ -450,52 +522,5 @@ extern "C" int dli_attn_prefill_tc_bf16(const void* qkv, void* out, int B, int T
   DLI_CHECK_ARG((long long)((T + 127) / 128) * H * B <= 0x7fffffffLL, "dli_attn_prefill_tc_bf16: too many query tiles");
   DLI_CHECK_ARG(aligned16(qkv) && aligned16(out), "dli_attn_prefill_tc_bf16: pointers must be 16-byte aligned");
   if (B == 0 || T == 0) return DLI_OK;
-  static PerDeviceOnce once;
-  DLI_ONCE_PER_DEVICE(once, dev, DLI_CUDA_CALL(cudaFuncSetAttribute(
-                                     attn_prefill_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem)));
-  CUtensorMap tm;
-  const int cols = (H + 2 * KV) * hd;
-  // the packed qkv matrix [B*T, cols]; box = 128 rows x 64 columns (one swizzle span)
-  int rc = make_tmap(&tm, qkv, B * T, cols, 128);
-  if (rc != DLI_OK) return rc;
-  const int n_qtiles = (T + kTcTile - 1) / kTcTile;
-  const long long n_items = (long long)n_qtiles * H * B;
-  dim3 grid((unsigned)(n_items < sm_count_cached() ? n_items : sm_count_cached()));  // persistent: one CTA per SM
-  DLI_LAUNCH("attn_prefill_tc_kernel", attn_prefill_tc_kernel<false>, grid, dim3(kTcThreads), (size_t)kTcSmem,
-             static_cast<cudaStream_t>(stream), tm, tm, tm, (bf16*)out, T, H, KV, scale * 1.4426950408889634f, window,
-             (const int32_t*)nullptr, 0, 0, 0, 0, B, n_qtiles);
-  return DLI_OK;
+  return launch_attn_prefill_tc(qkv, out, B, T, H, KV, hd, scale, window, static_cast<cudaStream_t>(stream));
 }
-
-namespace dli {
-
-// tcgen05 form of dli_attn_prefill_paged_bf16 (head_dim 128, 8 <= page_size <= 128); called from attn_prefill.cu.
-int launch_attn_prefill_tc_paged(const void* qkv, void* out, const void* k_cache, const void* v_cache,
-                                 const int32_t* page_table, int max_pages, int num_pages, int B, int T, int prefix,
-                                 int H, int KV, int page_size, float scale, int window, cudaStream_t s) {
-  static PerDeviceOnce once;
-  DLI_ONCE_PER_DEVICE(once, dev, DLI_CUDA_CALL(cudaFuncSetAttribute(
-                                     attn_prefill_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem)));
-  CUtensorMap tm, tmK, tmV;
-  const int cols = (H + 2 * KV) * kTcHd;
-  int rc = make_tmap(&tm, qkv, B * T, cols, 128);
-  if (rc != DLI_OK) return rc;
-  // the cache pools as [num_pages * KV * page_size, 128] rows; box = one page x 64 columns
-  const long long rows = (long long)num_pages * KV * page_size;
-  if (rows <= 0 || rows > 0x7fffffffLL) return fail(DLI_ERR_INVALID, "dli_attn_prefill_paged_bf16: cache too large for one tensor map");
-  rc = make_tmap(&tmK, k_cache, (int)rows, kTcHd, page_size);
-  if (rc != DLI_OK) return rc;
-  rc = make_tmap(&tmV, v_cache, (int)rows, kTcHd, page_size);
-  if (rc != DLI_OK) return rc;
-  int shift = 0;
-  while ((1 << shift) < page_size) ++shift;
-  const int n_qtiles = (T + kTcTile - 1) / kTcTile;
-  const long long n_items = (long long)n_qtiles * H * B;
-  dim3 grid((unsigned)(n_items < sm_count_cached() ? n_items : sm_count_cached()));
-  DLI_LAUNCH("attn_prefill_tc_kernel", attn_prefill_tc_kernel<true>, grid, dim3(kTcThreads), (size_t)kTcSmem, s, tm,
-             tmK, tmV, (bf16*)out, T, H, KV, scale * 1.4426950408889634f, window, page_table, max_pages, shift, prefix,
-             (int)rows, B, n_qtiles);
-  return DLI_OK;
-}
-
-}  // namespace dli

@@ -1,0 +1,61 @@
+"""Prompt attention at head size 64 on the tcgen05 kernel (and both head sizes on either side of the kernel rule) against
+float64.  Bound: the probabilities are rounded to bf16 (2^-9 each, relative), sums are fp32, the result is rounded to bf16
+once: 2^-9 sum |p v| / l + 2^-9 |out|, the exponential's 2^-20 beside it."""
+import pytest
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+BF = torch.bfloat16
+
+
+def _ref(q, k, v, scale, prefix, window):
+    T, S = q.shape[0], k.shape[0]
+    i = torch.arange(T, device=q.device)[:, None] + prefix
+    j = torch.arange(S, device=q.device)[None]
+    hide = (j > i) | ((j <= i - window) if window else torch.zeros_like(j > i))
+    p = torch.softmax((q @ k.T * scale).masked_fill(hide, -float("inf")), dim=-1)
+    return p @ v, p @ v.abs()
+
+
+def _check(out, q, k, v, H, KV, hd, prefix, window):
+    for h in range(H):
+        ref, mag = _ref(q[:, h], k[:, h * KV // H], v[:, h * KV // H], hd ** -0.5, prefix, window)
+        bound = 2.0 ** -8 * (mag + ref.abs()) + 1e-6
+        assert ((out[:, h] - ref).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("hd,B,T,H,KV,window", [(64, 1, 447, 4, 2, 0), (64, 1, 448, 4, 1, 0), (64, 2, 513, 3, 3, 0),
+                                                (64, 1, 1777, 2, 1, 300), (64, 3, 640, 12, 12, 0), (128, 2, 64, 4, 2, 0),
+                                                (128, 2, 65, 4, 2, 0), (64, 1, 2, 2, 2, 0)])
+def test_whole_prompts(cuda, hd, B, T, H, KV, window):
+    from dli_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(T + hd)
+    qkv = (1.3 * torch.randn(B * T, (H + 2 * KV) * hd, device=cuda, generator=g)).to(BF)
+    out = torch.full((B * T, H * hd), float("nan"), device=cuda, dtype=BF)
+    ops.attn_prefill(qkv, out, B, T, H, KV, hd, hd ** -0.5, window=window)
+    q, k, v = (x.double().view(B, T, -1, hd) for x in qkv.split([H * hd, KV * hd, KV * hd], dim=1))
+    for b in range(B):
+        _check(out.double().view(B, T, H, hd)[b], q[b], k[b], v[b], H, KV, hd, 0, window)
+
+
+@pytest.mark.parametrize("hd,B,T,prefix,H,KV,page,window", [(64, 2, 100, 400, 4, 2, 16, 0), (64, 1, 3, 1000, 2, 1, 8, 0),
+                                                             (64, 1, 300, 148, 3, 3, 64, 0), (64, 2, 130, 900, 4, 1, 16, 257),
+                                                             (64, 1, 40, 407, 2, 2, 16, 0), (128, 1, 20, 44, 4, 2, 16, 0),
+                                                             (128, 1, 20, 45, 4, 2, 16, 0)])
+def test_chunks_on_the_paged_cache(cuda, hd, B, T, prefix, H, KV, page, window):
+    from dli_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(T + prefix)
+    S = prefix + T
+    n = (S + page - 1) // page
+    kc = (1.3 * torch.randn(B * n + 2, KV, page, hd, device=cuda, generator=g)).to(BF)
+    vc = torch.randn(B * n + 2, KV, page, hd, device=cuda, generator=g).to(BF)
+    table = torch.randperm(B * n + 2, device=cuda, generator=g)[:B * n].int().view(B, n).contiguous()
+    qkv = (1.3 * torch.randn(B * T, (H + 2 * KV) * hd, device=cuda, generator=g)).to(BF)
+    out = torch.full((B * T, H * hd), float("nan"), device=cuda, dtype=BF)
+    ops.attn_prefill_paged(qkv, out, kc, vc, table, B, T, prefix, H, KV, hd, hd ** -0.5, window=window)
+    q = qkv[:, :H * hd].double().view(B, T, H, hd)
+    for b in range(B):
+        k, v = (c[table[b].long()].double().transpose(1, 2).reshape(n * page, KV, hd)[:S] for c in (kc, vc))
+        _check(out.double().view(B, T, H, hd)[b], q[b], k, v, H, KV, hd, prefix, window)
