@@ -280,6 +280,26 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm, const __grid_cons
           const int st = g & 1;
           mbar_wait(p_full, g & 1);                 // P(g) in tensor memory, O rescaled (or, it == 0, read out)
           mbar_wait(v_full + 8 * st, (g >> 1) & 1);
+          // Rows of the last key tile past the context hold whatever follows in memory: the rest of the last cache page,
+          // or the next sequence's rows.  Their probabilities are 0, but 0 x inf is not: zero them before P V.
+          {
+            const int tile0 = (w.t_begin + it) * kTcTile, ctx = (kPaged ? prefix : 0) + T;
+            int dirty_end = 0;
+            if (ctx < tile0 + kTcTile) {
+              const int page_end = kPaged ? (((ctx - 1) >> page_shift) + 1) << page_shift : 0;
+              dirty_end = kPaged ? min(page_end - tile0, kTcTile) : w.b + 1 < B ? kTcTile : 0;
+            }
+            if (dirty_end > ctx - tile0) {
+              // a row is 128 bytes per span whatever the swizzle does inside it: eight lanes a row
+#pragma unroll
+              for (int sp = 0; sp < TcCfg<HD>::kSpans; ++sp)
+                for (int r = ctx - tile0 + (lane >> 3); r < dirty_end; r += 4)
+                  *reinterpret_cast<uint4*>(smem + (sV - sQ) + st * kTileBytes2 + sp * kSpanBytes + r * 128 + (lane & 7) * 16) =
+                      make_uint4(0u, 0u, 0u, 0u);
+              fence_proxy_async();
+              __syncwarp();
+            }
+          }
           tcgen05_fence_after();
           const uint64_t vdesc = vdesc0 + (uint64_t)(st * (kTileBytes2 >> 4));
           if (elect_one()) {

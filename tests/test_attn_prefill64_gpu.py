@@ -52,6 +52,9 @@ def test_chunks_on_the_paged_cache(cuda, hd, B, T, prefix, H, KV, page, window):
     kc = (1.3 * torch.randn(B * n + 2, KV, page, hd, device=cuda, generator=g)).to(BF)
     vc = torch.randn(B * n + 2, KV, page, hd, device=cuda, generator=g).to(BF)
     table = torch.randperm(B * n + 2, device=cuda, generator=g)[:B * n].int().view(B, n).contiguous()
+    for b in range(B):  # what lies past the context in its last page must not matter
+        if S % page:
+            kc[table[b, -1], :, S % page:], vc[table[b, -1], :, S % page:] = float("nan"), float("inf")
     qkv = (1.3 * torch.randn(B * T, (H + 2 * KV) * hd, device=cuda, generator=g)).to(BF)
     out = torch.full((B * T, H * hd), float("nan"), device=cuda, dtype=BF)
     ops.attn_prefill_paged(qkv, out, kc, vc, table, B, T, prefix, H, KV, hd, hd ** -0.5, window=window)
@@ -59,3 +62,18 @@ def test_chunks_on_the_paged_cache(cuda, hd, B, T, prefix, H, KV, page, window):
     for b in range(B):
         k, v = (c[table[b].long()].double().transpose(1, 2).reshape(n * page, KV, hd)[:S] for c in (kc, vc))
         _check(out.double().view(B, T, H, hd)[b], q[b], k, v, H, KV, hd, prefix, window)
+
+
+@pytest.mark.parametrize("hd,T", [(64, 450), (128, 130), (64, 40), (128, 40)])
+def test_a_sequence_does_not_see_its_neighbour(cuda, hd, T):
+    """The tile after a sequence's last row holds the next sequence's keys and values: infinities there stay there."""
+    from dli_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(T)
+    H = KV = 2
+    qkv = torch.randn(2 * T, 3 * H * hd, device=cuda, generator=g).to(BF)
+    alone, both = torch.empty(T, H * hd, device=cuda, dtype=BF), torch.empty(2 * T, H * hd, device=cuda, dtype=BF)
+    ops.attn_prefill(qkv[:T].contiguous(), alone, 1, T, H, KV, hd, hd ** -0.5)
+    qkv[T:, H * hd:] = float("inf")
+    ops.attn_prefill(qkv, both, 2, T, H, KV, hd, hd ** -0.5)
+    assert torch.equal(both[:T], alone)
