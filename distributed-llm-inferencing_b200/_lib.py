@@ -17,12 +17,33 @@ EPI_NONE, EPI_BIAS, EPI_RESIDUAL, EPI_GELU_NEW = 0, 1, 2, 4
 
 _vp, _i, _f, _sz, _ll = C.c_void_p, C.c_int, C.c_float, C.c_size_t, C.c_longlong
 
+
+
+class LayerWeights(C.Structure):
+    """dli_layer_weights of include/dli.h."""
+
+    _fields_ = [(n, C.c_void_p) for n in ("norm1", "norm1_b", "w_qkv", "b_qkv", "w_o", "b_o", "norm2", "norm2_b", "w_ff",
+                                          "b_ff", "w_down", "b_down", "k_cache", "v_cache")]
+
+
+class PromptPass(C.Structure):
+    """dli_prompt_pass of include/dli.h."""
+
+    _fields_ = ([(n, C.c_int) for n in ("n_layers", "B", "T", "prefix", "d", "ff", "H", "KV", "hd", "window", "page_size",
+                                        "max_pages", "num_pages", "tensor_core")] +
+                [("eps", C.c_float), ("scale", C.c_float)] +
+                [(n, C.c_void_p) for n in ("h_in", "h", "x", "qkv", "attn", "act", "cos", "sin", "positions", "seq_ids",
+                                           "page_table", "page_rows")])
+
+
 # name -> (restype, argtypes); mirrors include/dli.h one to one
 SIGNATURES = {
     "dli_last_error": (C.c_char_p, []),
     "dli_version": (_i, []),
     "dli_sm_count": (_i, []),
     "dli_embedding_bf16": (_i, [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _vp]),
+    "dli_prompt_layers_bf16": (_i, [C.POINTER(LayerWeights), C.POINTER(PromptPass), C.POINTER(_i), _vp]),
+    "dli_prompt_rows": (_i, [_vp, _vp, _vp, _i, _i, _i, _i, _vp]),
     "dli_add_rmsnorm_bf16": (_i, [_vp, _vp, _vp, _vp, _vp, _i, _i, _f, _vp]),
     "dli_add_layernorm_bf16": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _f, _vp]),
     "dli_rope_kv_append_bf16": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _i, _vp, _vp, _i, _i, _i, _i, _i, _vp]),

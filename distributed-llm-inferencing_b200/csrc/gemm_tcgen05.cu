@@ -384,6 +384,29 @@ static bool use_rows(int M, int N, int K, bool gated, RowsShape* shape, int* rc)
   return M <= 128 || 1.1 * us < pick_prefill(M, N, K, gated, &p) + 9.5;
 }
 
+// qkv = x w^T (+ bias), q and k rotated, k and v appended to the cache pages: one kernel where a projection kernel has that
+// epilogue, the projection and the rotation kernel otherwise (the same bits).
+int linear_qkv_append(const void* x, const void* w, const void* bias, void* qkv, int M, int K, const RopeArgs& rope, int hd,
+                      cudaStream_t s, int* launches) {
+  const int N = (rope.H + 2 * rope.KV) * hd;
+  *launches += 1;
+  if (M > 2 && K % 64 == 0 && aligned16(x) && aligned16(w) && aligned16(qkv) && aligned16(bias) && aligned16(rope.k_cache) &&
+      aligned16(rope.v_cache)) {
+    RowsShape sh;
+    int rc;
+    if (use_rows(M, N, K, false, &sh, &rc))
+      return launch_gemm_rows(kRowsRope, x, w, bias, nullptr, qkv, M, N, K, bias ? DLI_EPI_BIAS : 0, sh, s, rope, hd);
+    if (rc != DLI_OK) return rc;
+    if (hd == 128 && rope.H % 2 == 0 && rope.KV % 2 == 0 && !bias && rope.cos_t)
+      return launch_prefill_gemm<256, false, 1, true>(x, w, nullptr, nullptr, qkv, M, N, K, 0, s, rope);
+  }
+  const int rc = dli_linear_bf16(x, w, bias, nullptr, qkv, M, N, K, bias ? DLI_EPI_BIAS : 0, s);
+  if (rc != DLI_OK) return rc;
+  *launches += 1;
+  return dli_rope_kv_append_bf16(qkv, rope.cos_t, rope.sin_t, rope.positions, rope.seq_ids, rope.page_table, rope.max_pages,
+                                 rope.k_cache, rope.v_cache, M, rope.H, rope.KV, hd, 1 << rope.page_shift, s);
+}
+
 }  // namespace dli
 
 extern "C" {

@@ -244,8 +244,6 @@ class ShardEngine:
         torch.cuda.set_device(self.device)
         self.sms = ops.sm_count()
         self.l2_prefetch = os.environ.get("DLI_L2_PREFETCH", "0") == "1"
-        # prompt passes: qkv projection + RoPE + cache append as one kernel (DLI_FUSE_QKV_ROPE=0: three steps as before)
-        self.fuse_qkv_rope = os.environ.get("DLI_FUSE_QKV_ROPE", "1") == "1"
         # kernels may start (and prefetch weights) while their predecessor drains
         ops.set_pdl(os.environ.get("DLI_PDL", "1") == "1")
         self.w: Dict[str, torch.Tensor] = {}
@@ -407,7 +405,7 @@ class ShardEngine:
         self.kv.k.clear()
         self.kv.v.clear()
         self._ws_rows = 0
-        for name in ("_h", "_x", "_qkv", "_attn", "_act"):
+        for name in ("_h", "_x", "_qkv", "_attn", "_act", "_row_meta"):
             if hasattr(self, name):
                 delattr(self, name)
         torch.cuda.empty_cache()
@@ -422,6 +420,8 @@ class ShardEngine:
         self._qkv = torch.empty(rows, (s.n_heads + 2 * s.n_kv_heads) * s.head_dim, dtype=BF, device=dev)
         self._attn = torch.empty(rows, s.n_heads * s.head_dim, dtype=BF, device=dev)
         self._act = torch.empty(rows, s.d_ff, dtype=BF, device=dev)
+        # position, sequence id and (of each prompt) last row of a prompt pass
+        self._row_meta = torch.empty(3, rows, dtype=torch.int32, device=dev)
         self._ws_rows = rows
         self._graphs.clear()  # captured graphs hold the old workspace pointers
 
@@ -438,8 +438,8 @@ class ShardEngine:
         return max(1, min((tiles + 3) // 4, want, 64))
 
     # ------------------------------------------------------------------ one layer range
-    def _layers_forward(self, h, rows, positions, seq_ids, seq_lens, prefill_shape, st, h_in=None, h_out=None):
-        """h: [rows, d] residual stream (updated in place).  prefill_shape=(B,T) or None for decode.
+    def _layers_forward(self, h, rows, positions, seq_ids, seq_lens, st, h_in=None, h_out=None):
+        """A decode step's layers.  h: [rows, d] residual stream (updated in place).
         h_in: where the stage's INPUT lives when that is not h (read only: the first norm and the first
         residual add read it, e.g. a neighbour's hidden state inside a pipeline mailbox); h_out: where the
         LAST projection writes the stage's output when that is not h."""
@@ -448,11 +448,10 @@ class ShardEngine:
         last_li = len(self.layers) - 1
         x, qkv, attn, act = self._x[:rows], self._qkv[:rows], self._attn[:rows], self._act[:rows]
         H, KV, hd = s.n_heads, s.n_kv_heads, s.head_dim
-        decode = prefill_shape is None
         # rows <= 2: CUDA-core GEMV with the RMSNorm fused in (6.0-7.3 TB/s); 3..128 rows: split-K tcgen05
         # weight stream on every SM (the GEMV's FMA work grows with the rows: 4.1-5.0 TB/s at 3-4 rows)
-        fuse_norm = decode and rows <= _GEMV_MAX_ROWS and s.arch == "llama"
-        split_k = decode and _GEMV_MAX_ROWS < rows <= 128
+        fuse_norm = rows <= _GEMV_MAX_ROWS and s.arch == "llama"
+        split_k = _GEMV_MAX_ROWS < rows <= 128
         if split_k and self._sk is None:
             n_max = max(s.vocab, 2 * s.d_ff, (H + 2 * KV) * hd, s.d_model)
             self._sk = torch.zeros(ops.gemm_splitk_scratch_bytes(128, n_max), dtype=torch.uint8, device=self.device)
@@ -471,37 +470,18 @@ class ShardEngine:
                 ops.rmsnorm_linear(res, L["ln1"], s.eps, L["wqkv"], out=qkv)
             elif s.arch == "llama":
                 ops.add_rmsnorm(res, L["ln1"], s.eps, out=x)
-                # a prompt pass: RoPE and the cache append ride in the projection's epilogue (same bits)
-                fused_rope = (not decode and self.fuse_qkv_rope
-                              and ops.qkv_rope_append_supported(rows, x.shape[1], H, KV, hd, None))
-                if fused_rope:
-                    ops.linear_qkv_rope_append(x, L["wqkv"], qkv, self.cos, self.sin, positions, seq_ids,
-                                               self.kv.page_table, self.kv.k[li], self.kv.v[li], H, KV, hd)
-                else:
-                    lin(x, L["wqkv"], out=qkv)
+                lin(x, L["wqkv"], out=qkv)
             else:
                 ops.add_layernorm(res, L["ln1"], L["ln1b"], s.eps, out=x)
                 lin(x, L["wqkv"], bias=L["bqkv"], out=qkv)
-            if decode:
-                # RoPE + KV append of the new token + split-KV attention in one kernel; the
-                # kernel indexes page-table rows by batch row, so it gets the slot's rows
-                ops.paged_attn_decode_fused(qkv, self.cos, self.sin, self.kv.k[li], self.kv.v[li], st["page_rows"],
-                                            seq_lens, attn, H, KV, hd, self.scale, num_splits=st["splits"],
-                                            scratch=st["scratch"], window=s.sliding_window,
-                                            # spare SMs pull the next projections' weights into L2 meanwhile
-                                            prefetch_a=L["wo"] if self.l2_prefetch else None,
-                                            prefetch_b=L.get("wgu_head") if self.l2_prefetch else None)
-            else:
-                if not (s.arch == "llama" and fused_rope):
-                    ops.rope_kv_append(qkv, self.cos, self.sin, positions, seq_ids, self.kv.page_table,
-                                       self.kv.k[li], self.kv.v[li], H, KV, hd)
-                if len(prefill_shape) > 2:  # a chunk at positions prefix..: keys/values from the paged cache
-                    ops.attn_prefill_paged(qkv, attn, self.kv.k[li], self.kv.v[li], st["page_rows"], prefill_shape[0],
-                                           prefill_shape[1], prefill_shape[2], H, KV, hd, self.scale,
-                                           window=s.sliding_window)
-                else:
-                    ops.attn_prefill(qkv, attn, prefill_shape[0], prefill_shape[1], H, KV, hd, self.scale,
-                                     window=s.sliding_window)
+            # RoPE + KV append of the new token + split-KV attention in one kernel; the
+            # kernel indexes page-table rows by batch row, so it gets the slot's rows
+            ops.paged_attn_decode_fused(qkv, self.cos, self.sin, self.kv.k[li], self.kv.v[li], st["page_rows"],
+                                        seq_lens, attn, H, KV, hd, self.scale, num_splits=st["splits"],
+                                        scratch=st["scratch"], window=s.sliding_window,
+                                        # spare SMs pull the next projections' weights into L2 meanwhile
+                                        prefetch_a=L["wo"] if self.l2_prefetch else None,
+                                        prefetch_b=L.get("wgu_head") if self.l2_prefetch else None)
             if s.arch == "llama":
                 lin(attn, L["wo"], residual=res, out=h)
                 res = h
@@ -638,21 +618,25 @@ class ShardEngine:
         rows = B * T
         self._workspace(max(rows, B))
         st = self._dec[(B, mb)]
-        dev = self.device
-        positions = (torch.arange(T, dtype=torch.int32, device=dev) + (prefix or 0)).repeat(B)
-        seq_ids = st["seq_ids"].repeat_interleave(T)
+        s = self.spec
+        positions, seq_ids, last_rows = self._row_meta[0, :rows], self._row_meta[1, :rows], self._row_meta[2, :B]
+        ops.prompt_rows(positions, seq_ids, last_rows, B, T, prefix or 0, mb * B)
         h = self._h[:rows]
         if self.is_first:
-            if self.spec.arch == "gpt2":
+            if s.arch == "gpt2":
                 ops.embedding(ids, self.w["embed"], out=h, positions=positions, pos_table=self.w["wpe"])
             else:
                 ops.embedding(ids, self.w["embed"], out=h)
-        elif hidden.data_ptr() != h.data_ptr():
-            h.copy_(hidden)
-        self._layers_forward(h, rows, positions, seq_ids, None, (B, T) if prefix is None else (B, T, prefix), st)
+        # later stages: the first layer reads the stage's input where it lies
+        h_in = h if self.is_first else hidden
+        if h_in.shape != h.shape or h_in.dtype != BF or h_in.device != h.device or not h_in.is_contiguous() or \
+                h_in.data_ptr() % 16:
+            h_in = h.copy_(hidden)
+        ops.prompt_layers(self.layers, self.kv.k, self.kv.v, self.kv.page_table, st["page_rows"], h_in, h, self._x[:rows],
+                          self._qkv[:rows], self._attn[:rows], self._act[:rows], self.cos, self.sin, positions, seq_ids,
+                          B, T, prefix, s.n_heads, s.n_kv_heads, s.head_dim, s.eps, self.scale, window=s.sliding_window)
         if not self.is_last or not final:
             return h
-        last_rows = (torch.arange(B, dtype=torch.int32, device=dev) + 1) * T - 1
         if self.head_shard is not None:
             return ops.embedding(last_rows, h, out=st["hf"])  # final hidden of the last positions -> all stages
         h_last = ops.embedding(last_rows, h, out=st["h"])  # row gather of the last positions
@@ -687,7 +671,7 @@ class ShardEngine:
                 ops.embedding(st["tokens"], self.w["embed"], out=h, positions=st["positions"], pos_table=self.w["wpe"])
             else:
                 ops.embedding(st["tokens"], self.w["embed"], out=h)
-        self._layers_forward(h, B, st["positions"], st["seq_ids"], st["seq_lens"], None, st)
+        self._layers_forward(h, B, st["positions"], st["seq_ids"], st["seq_lens"], st)
         if self.has_head:
             self._head(h, st["logits"], st["tokens"], st)
         # head-shard mode: stage 0 logs the token it just consumed (the previous step's choice)
@@ -882,7 +866,7 @@ class ShardEngine:
             else:
                 h_in = m["in_h"][rd][m["rank"] - 1]
             h_out = None if self.has_head else m["out_h"][ph]
-            self._layers_forward(h, B, st["positions"], st["seq_ids"], st["seq_lens"], None, st, h_in=h_in, h_out=h_out)
+            self._layers_forward(h, B, st["positions"], st["seq_ids"], st["seq_lens"], st, h_in=h_in, h_out=h_out)
             tokens = st["tokens"]
             if self.has_head:
                 tokens = m["out_tok"][ph]

@@ -6,6 +6,7 @@ stream.  Tensors must be CUDA, contiguous where noted, bf16 unless stated.
 """
 from __future__ import annotations
 
+import ctypes as _ct
 import os as _os
 
 import torch
@@ -22,7 +23,8 @@ def _p(t):
 
 
 def _stream():
-    return torch.cuda.current_stream().cuda_stream
+    """Handle of torch's current stream on the current device (without the Stream object: 0.2 instead of 3 us a call)."""
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def _req(t, dtype=torch.bfloat16):
@@ -115,6 +117,64 @@ def linear_qkv_rope_append(x, w_qkv, qkv, cos, sin, positions, seq_ids, page_tab
     return qkv
 
 
+def prompt_rows(positions, seq_ids, last_rows, B, T, prefix, seq0):
+    """Position and sequence id of every row of a prompt pass of B prompts of T tokens (int32 [>= B*T]), and the row of
+    each prompt's last token (int32 [B] or None)."""
+    global launch_count
+    _req(positions, torch.int32), _req(seq_ids, torch.int32), _req(last_rows, torch.int32)
+    if min(positions.numel(), seq_ids.numel()) < B * T or (last_rows is not None and last_rows.numel() < B):
+        raise ValueError("prompt_rows: buffers are too small")
+    _lib.check("dli_prompt_rows", _lib.load().dli_prompt_rows(_p(positions), _p(seq_ids), _p(last_rows), B, T, prefix, seq0,
+                                                              _stream()))
+    launch_count += 1
+
+
+# layer tensors of an engine under the names of dli_layer_weights
+_LAYER_KEYS = (("norm1", "ln1"), ("norm1_b", "ln1b"), ("w_qkv", "wqkv"), ("b_qkv", "bqkv"), ("w_o", "wo"), ("b_o", "bo"),
+               ("norm2", "ln2"), ("norm2_b", "ln2b"), ("w_down", "wdown"), ("b_down", "bdown"), ("b_ff", "bfc"))
+
+
+def prompt_layers(layers, k_pools, v_pools, page_table, page_rows, h_in, h, x, qkv, attn, act, cos, sin, positions, seq_ids,
+                  B, T, prefix, H, KV, hd, eps, scale, window=0):
+    """A prompt pass through all `layers` (dicts of an engine's layer tensors) in one native call: B prompts of T tokens,
+    whole (prefix None) or a chunk at positions prefix ..; h_in [B*T, d] is read, h receives the result, x / qkv / attn /
+    act are workspaces of B*T rows."""
+    global launch_count
+    rows, d = h.shape
+    if rows != B * T or h_in.shape != h.shape or x.shape != h.shape or qkv.shape != (rows, (H + 2 * KV) * hd) or \
+            attn.shape != (rows, H * hd) or act.shape[0] != rows:
+        raise ValueError("prompt_layers: workspaces do not match B, T and the layers")
+    for t in (h_in, h, x, qkv, attn, act, cos, sin):
+        _req(t)
+    for t in (page_table, page_rows, positions, seq_ids):
+        _req(t, torch.int32)
+    ff = act.shape[1]
+    table = (_lib.LayerWeights * len(layers))()
+    for L, c, k, v in zip(layers, table, k_pools, v_pools):
+        for name, key in _LAYER_KEYS:
+            t = L.get(key)
+            if t is not None:
+                _req(t)
+                setattr(c, name, t.data_ptr())
+        w_ff = L["wgu"] if "wgu" in L else L["wfc"]
+        _req(w_ff), _req(k), _req(v)
+        if L["wqkv"].shape != (qkv.shape[1], d) or L["wo"].shape != (d, H * hd) or L["wdown"].shape != (d, ff) or \
+                w_ff.shape != ((2 if "wgu" in L else 1) * ff, d) or k.shape != v.shape or k.shape[1] != KV or k.shape[3] != hd:
+            raise ValueError("prompt_layers: a layer's weights or caches do not match the sizes")
+        c.w_ff, c.k_cache, c.v_cache = w_ff.data_ptr(), k.data_ptr(), v.data_ptr()
+    p = _lib.PromptPass(
+        n_layers=len(layers), B=B, T=T, prefix=-1 if prefix is None else prefix, d=d, ff=ff, H=H, KV=KV, hd=hd, window=window,
+        page_size=k_pools[0].shape[2] if layers else 8, max_pages=page_table.shape[1],
+        num_pages=k_pools[0].shape[0] if layers else 0, tensor_core=int(_prefill_tensor_core(hd, T)), eps=eps, scale=scale,
+        h_in=_p(h_in), h=_p(h), x=_p(x), qkv=_p(qkv), attn=_p(attn), act=_p(act), cos=_p(cos), sin=_p(sin),
+        positions=_p(positions), seq_ids=_p(seq_ids), page_table=_p(page_table), page_rows=_p(page_rows))
+    n = _ct.c_int(0)
+    rc = _lib.load().dli_prompt_layers_bf16(table, _ct.byref(p), _ct.byref(n), _stream())
+    launch_count += n.value
+    _lib.check("dli_prompt_layers_bf16", rc)
+    return h
+
+
 def attn_decode_scratch_bytes(B, H, hd, num_splits) -> int:
     return int(_lib.load().dli_paged_attn_decode_scratch_bytes(B, H, hd, num_splits))
 
@@ -136,6 +196,10 @@ def paged_attn_decode(q, q_stride, k_cache, v_cache, page_table, seq_lens, out, 
     return out
 
 
+def _prefill_tensor_core(hd, T) -> bool:
+    return hd == 128 and T > 64 and _os.environ.get("DLI_PREFILL_ATTN", "tc") != "mma"
+
+
 def attn_prefill(qkv, out, B, T, H, KV, hd, scale, window=0, tensor_core=None):
     """Causal prefill attention.  head_dim 128 runs on tcgen05 (dli_attn_prefill_tc_bf16) from 65 tokens, where it
     overtakes the mma.sync kernel (64 tokens of 32 heads: 5.9 against 4.4 us), unless tensor_core=False or
@@ -143,7 +207,7 @@ def attn_prefill(qkv, out, B, T, H, KV, hd, scale, window=0, tensor_core=None):
     global launch_count
     _req(qkv), _req(out)
     if tensor_core is None:
-        tensor_core = hd == 128 and T > 64 and _os.environ.get("DLI_PREFILL_ATTN", "tc") != "mma"
+        tensor_core = _prefill_tensor_core(hd, T)
     if tensor_core:
         _lib.check("dli_attn_prefill_tc_bf16", _lib.load().dli_attn_prefill_tc_bf16(
             _p(qkv), _p(out), B, T, H, KV, hd, float(scale), window, _stream()))

@@ -206,15 +206,45 @@ int dli_attn_prefill_tc_bf16(const void* qkv, void* out, int B, int T, int H, in
  * dli_rope_kv_append_bf16 must have appended the chunk first.  page_table:
  * int32 [B, max_pages], row b = sequence b of this call.  prefix == 0 gives
  * the result of dli_attn_prefill_bf16.  num_pages = pages in the k_cache /
- * v_cache pools: with head_dim 128 the tcgen05 kernel reads whole pages by TMA
- * and needs the pool extent (0 = use the mma.sync kernel); cache rows beyond a
- * sequence's end inside its last page must hold finite values (a pool that was
- * zero-filled once is fine: they are multiplied by a probability of exactly 0). */
+ * v_cache pools: the tcgen05 kernel reads whole pages by TMA and needs the pool
+ * extent (0 = use the mma.sync kernel); cache rows beyond a sequence's end inside
+ * its last page may hold anything. */
 int dli_attn_prefill_paged_bf16(const void* qkv, void* out, const void* k_cache,
                                 const void* v_cache, const int32_t* page_table,
                                 int max_pages, int num_pages, int B, int T, int prefix,
                                 int H, int KV, int hd, int page_size, float scale,
                                 int window, dli_stream_t stream);
+
+/* A prompt pass through consecutive decoder layers in one call: per layer the launches
+ * of norm, qkv projection + RoPE + cache append, causal attention, output projection,
+ * norm and feed-forward, in order on `stream` (reference: LlamaDecoderLayer /
+ * GPT2Block.forward at T > 1, TF:models/llama/modeling_llama.py:305-345).
+ * norm1_b / norm2_b NULL: RMSNorm and the gated SiLU feed-forward, w_ff = the
+ * interleaved [2 ff, d] gate/up matrix; given: LayerNorm and GELU(tanh) of x w_ff^T + b_ff
+ * (GPT-2).  Any other bias may be NULL.  Weights are [out, in] bf16. */
+typedef struct {
+  const void *norm1, *norm1_b, *w_qkv, *b_qkv, *w_o, *b_o, *norm2, *norm2_b, *w_ff, *b_ff, *w_down, *b_down;
+  void *k_cache, *v_cache; /* [num_pages, KV, page_size, hd] */
+} dli_layer_weights;
+typedef struct {
+  int n_layers, B, T;
+  int prefix; /* -1: whole prompts; >= 0: chunks at positions prefix .. prefix + T - 1 */
+  int d, ff, H, KV, hd, window, page_size, max_pages, num_pages;
+  int tensor_core; /* whole prompts: dli_attn_prefill_tc_bf16 instead of dli_attn_prefill_bf16 */
+  float eps, scale;
+  const void* h_in; /* [B*T, d] input, read only unless it is h */
+  void *h, *x, *qkv, *attn, *act; /* [B*T, .]: result, normed rows, (H+2KV)*hd, H*hd, ff */
+  const void *cos, *sin; /* bf16 [max_pos, hd/2] or NULL: no rotation */
+  const int32_t *positions, *seq_ids; /* [B*T] */
+  const int32_t* page_table; /* [n_seqs, max_pages], indexed by seq_ids */
+  const int32_t* page_rows;  /* its rows of the B sequences of this call */
+} dli_prompt_pass;
+/* *launches: kernels enqueued (also where a later launch failed). */
+int dli_prompt_layers_bf16(const dli_layer_weights* layers, const dli_prompt_pass* pass, int* launches,
+                           dli_stream_t stream);
+/* positions[b*T + t] = prefix + t, seq_ids[b*T + t] = seq0 + b, and (unless NULL) last_rows[b] = (b+1)*T - 1. */
+int dli_prompt_rows(int32_t* positions, int32_t* seq_ids, int32_t* last_rows, int B, int T, int prefix, int seq0,
+                    dli_stream_t stream);
 
 /* ---- projections -----------------------------------------------------------
  * y[M,N] = epi(x[M,K] . w[N,K]^T)   — w is the HF nn.Linear layout [out,in].
