@@ -8,10 +8,10 @@
 // HBM-bound by design: every weight byte is read exactly once per pass with
 // 128-bit streaming loads (ld.global.nc.L1::no_allocate); algorithmic bytes per
 // launch = N*K*2 (+ M*K*2 for x, + M*N*2 for y; both negligible).  A CTA works
-// on kRows weight rows at a time; its 8 warps split K between them so that one
-// CTA iteration reads kRows contiguous 4 KB row segments (256 lanes x 16 B),
+// on R weight rows at a time; its 8 warps split K between them so that one
+// CTA iteration reads R contiguous 4 KB row segments (256 lanes x 16 B),
 // then partial sums are combined through shared memory (one warp per output).
-// Groups of kRows rows are dealt round-robin to a grid sized as a multiple of the SM count,
+// Groups of R rows are dealt round-robin to a grid sized as a multiple of the SM count,
 // so at any moment the grid streams one contiguous band of the matrix (two balanced
 // dealings were measured and lost, see `deal` in the kernel; so did a software-pipelined
 // 2-row variant for the small matrices, profiles/r2_notes.md).
@@ -29,7 +29,6 @@ namespace dli {
 
 constexpr int kGemvThreads = 256;
 constexpr int kGemvWarps = kGemvThreads / 32;
-constexpr int kGemvRows = 4;  // weight rows per task
 
 // Row index of logical row `n` of the gated [gate|up] matrix, interleaved in
 // blocks of 128 rows (see dli.h: dli_gemv_gated_silu_bf16).
@@ -37,20 +36,21 @@ __device__ __forceinline__ size_t gated_row(int n, int is_up) {
   return (size_t)(n >> 7) * 256 + (n & 127) + (is_up ? 128 : 0);
 }
 
-template <int M, bool kGated, bool kNorm>
+template <int M, bool kGated, bool kNorm, int R>
 __global__ void __launch_bounds__(kGemvThreads, M <= 2 ? 3 : 2)
 gemv_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, const bf16* __restrict__ bias,
             const bf16* residual, bf16* y, int N, int K, int epilogue,
             const bf16* __restrict__ ln_w, float eps, int pf_l2, float* __restrict__ cand, int deal) {
   // partial sums: [parity][value][thread]; value = row * M + m
-  __shared__ float part[2][kGemvRows * M][kGemvThreads];
+  __shared__ float part[2][R * M][kGemvThreads];
   __shared__ float red[kGemvWarps][M];
   extern __shared__ __align__(16) uint8_t xnorm_raw[];  // kNorm: normalised x, [M][K] bf16
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int kvec = K >> 3;
   const int iters = (kvec + kGemvThreads - 1) / kGemvThreads;
   // gated: a task is 2 output columns (2 gate rows + their 2 up rows)
-  constexpr int kOutPerTask = kGated ? kGemvRows / 2 : kGemvRows;
+  constexpr int kOutPerTask = kGated ? R / 2 : R;
+  constexpr int V = R > 4 ? 1 : 2;  // vectors of a row a thread asks for at a time
   const uint4 zero = make_uint4(0, 0, 0, 0);
 
   // How the N outputs are dealt to the CTAs (`deal`):
@@ -90,9 +90,9 @@ gemv_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, const bf16* 
   };
 
   // rows of group [n0, n0 + cnt): row r is live when its output index r % kOutPerTask < cnt
-  auto row_ptrs = [&](int n0, int cnt, const uint4* (&wrow)[kGemvRows]) {
+  auto row_ptrs = [&](int n0, int cnt, const uint4* (&wrow)[R]) {
 #pragma unroll
-    for (int r = 0; r < kGemvRows; ++r) {
+    for (int r = 0; r < R; ++r) {
       size_t row;
       if (kGated) {
         const int n = n0 + min(r % kOutPerTask, cnt - 1);
@@ -104,8 +104,8 @@ gemv_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, const bf16* 
     }
   };
 
-  const uint4* wrow[kGemvRows];
-  if (pf_l2 && ngroups > 0 && tid < kGemvRows) {
+  const uint4* wrow[R];
+  if (pf_l2 && ngroups > 0 && tid < R) {
     // Before waiting for the previous kernel: pull the head of this CTA's first weight rows into L2
     // with one bulk prefetch per row (no registers, shared memory or L1 footprint), so HBM keeps
     // streaming through the kernel boundary.  Worth ~1.5 us per layer on the 4-GEMV chain.
@@ -115,7 +115,7 @@ gemv_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, const bf16* 
     const uint32_t bytes = (uint32_t)min((size_t)K * 2, (size_t)pf_l2) & ~15u;
     const uint4* mine = wrow[0];
 #pragma unroll
-    for (int r = 1; r < kGemvRows; ++r)
+    for (int r = 1; r < R; ++r)
       if (tid == r) mine = wrow[r];  // (no dynamic indexing: keeps wrow in registers)
     if (tid % kOutPerTask < cnt0)
       asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(mine), "r"(bytes) : "memory");
@@ -183,39 +183,38 @@ gemv_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, const bf16* 
     int n0, cnt;
     group(g, n0, cnt);
     row_ptrs(n0, cnt, wrow);
-    bool live[kGemvRows];
+    bool live[R];
 #pragma unroll
-    for (int r = 0; r < kGemvRows; ++r) live[r] = (r % kOutPerTask) < cnt;
-    float acc[kGemvRows][M];
+    for (int r = 0; r < R; ++r) live[r] = (r % kOutPerTask) < cnt;
+    float acc[R][M];
 #pragma unroll
-    for (int r = 0; r < kGemvRows; ++r)
+    for (int r = 0; r < R; ++r)
 #pragma unroll
       for (int m = 0; m < M; ++m) acc[r][m] = 0.f;
 
-    for (int j = 0; j < iters; j += 2) {
-      const int i0 = tid + j * kGemvThreads, i1 = i0 + kGemvThreads;
-      const bool p0 = i0 < kvec, p1 = i1 < kvec;
-      uint4 wv0[kGemvRows], wv1[kGemvRows];
+    for (int j = 0; j < iters; j += V) {
+      uint4 wv[V][R], xa[V][M];
 #pragma unroll
-      for (int r = 0; r < kGemvRows; ++r) {
-        wv0[r] = (p0 && live[r]) ? ld_stream_16B(wrow[r] + i0) : zero;
-        wv1[r] = (p1 && live[r]) ? ld_stream_16B(wrow[r] + i1) : zero;
-      }
-      uint4 xa[M], xb[M];
+      for (int h = 0; h < V; ++h) {
+        const int i = tid + (j + h) * kGemvThreads;
 #pragma unroll
-      for (int m = 0; m < M; ++m) {
-        xa[m] = p0 ? ld_16B(xv + (size_t)m * kvec + i0) : zero;
-        xb[m] = p1 ? ld_16B(xv + (size_t)m * kvec + i1) : zero;
+        for (int r = 0; r < R; ++r) wv[h][r] = (i < kvec && live[r]) ? ld_stream_16B(wrow[r] + i) : zero;
       }
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
+      for (int h = 0; h < V; ++h) {
+        const int i = tid + (j + h) * kGemvThreads;
+#pragma unroll
+        for (int m = 0; m < M; ++m) xa[h][m] = i < kvec ? ld_16B(xv + (size_t)m * kvec + i) : zero;
+      }
+#pragma unroll
+      for (int h = 0; h < V; ++h) {
         float xf[M][8];
 #pragma unroll
-        for (int m = 0; m < M; ++m) unpack8(h ? xb[m] : xa[m], xf[m]);
+        for (int m = 0; m < M; ++m) unpack8(xa[h][m], xf[m]);
 #pragma unroll
-        for (int r = 0; r < kGemvRows; ++r) {
+        for (int r = 0; r < R; ++r) {
           float wf[8];
-          unpack8(h ? wv1[r] : wv0[r], wf);
+          unpack8(wv[h][r], wf);
 #pragma unroll
           for (int m = 0; m < M; ++m)
 #pragma unroll
@@ -225,7 +224,7 @@ gemv_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, const bf16* 
     }
 
 #pragma unroll
-    for (int r = 0; r < kGemvRows; ++r)
+    for (int r = 0; r < R; ++r)
 #pragma unroll
       for (int m = 0; m < M; ++m) part[parity][r * M + m][tid] = acc[r][m];
     __syncthreads();
@@ -289,11 +288,11 @@ gemv_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, const bf16* 
   }
 }
 
-template <int M, bool kGated, bool kNorm>
-static int launch_gemv(const bf16* x, const bf16* w, const bf16* bias, const bf16* residual, bf16* y, int N, int K,
+template <int M, bool kGated, bool kNorm, int R>
+static int launch_gemv_r(const bf16* x, const bf16* w, const bf16* bias, const bf16* residual, bf16* y, int N, int K,
                        int epilogue, const bf16* ln_w, float eps, cudaStream_t s, float* cand = nullptr,
                        int* grid_out = nullptr) {
-  constexpr int kOutPerTask = kGated ? kGemvRows / 2 : kGemvRows;
+  constexpr int kOutPerTask = kGated ? R / 2 : R;
   const int ngroups_total = (N + kOutPerTask - 1) / kOutPerTask;
   const int sms = sm_count_cached();
   if (sms <= 0) return fail(DLI_ERR_CUDA, "gemv: no CUDA device");
@@ -307,10 +306,10 @@ static int launch_gemv(const bf16* x, const bf16* w, const bf16* bias, const bf1
     if (dyn > once.bytes[d]) once.done[d] = false;
   }
   DLI_ONCE_PER_DEVICE(once, dev, {
-    DLI_CUDA_CALL(cudaFuncSetAttribute(gemv_kernel<M, kGated, kNorm>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    DLI_CUDA_CALL(cudaFuncSetAttribute(gemv_kernel<M, kGated, kNorm, R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)(dyn > 131072 ? dyn : 131072)));
     int o = 0;
-    DLI_CUDA_CALL(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, gemv_kernel<M, kGated, kNorm>, kGemvThreads, dyn));
+    DLI_CUDA_CALL(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, gemv_kernel<M, kGated, kNorm, R>, kGemvThreads, dyn));
     once.value[dev] = o > 0 ? o : 1;
     once.bytes[dev] = dyn;
   });
@@ -320,9 +319,60 @@ static int launch_gemv(const bf16* x, const bf16* w, const bf16* bias, const bf1
   // bytes per row prefetched into L2 across the kernel boundary (the whole row, or 8 KB)
   static const int pf_l2 = getenv("DLI_GEMV_PF_L2") ? atoi(getenv("DLI_GEMV_PF_L2")) : 8192;
   static const int deal = getenv("DLI_GEMV_DEAL") ? atoi(getenv("DLI_GEMV_DEAL")) : 0;  // measurement knob, see kernel
-  DLI_LAUNCH("gemv_kernel", gemv_kernel<M, kGated, kNorm>, dim3(grid), dim3(kGemvThreads), dyn, s, x, w, bias, residual,
+  DLI_LAUNCH("gemv_kernel", (gemv_kernel<M, kGated, kNorm, R>), dim3(grid), dim3(kGemvThreads), dyn, s, x, w, bias, residual,
              y, N, K, epilogue, ln_w, eps, pf_l2, cand, deal);
   return DLI_OK;
+}
+
+// Weight rows per task: the R whose waves of tasks are fullest.  The grid is one resident wave of 3 CTAs per SM that walks
+// ceil(tasks / CTAs) tasks each, so N / R just above a multiple of it costs a whole task: 4096 rows make 2.3 waves of 4 and
+// 1.85 of 5.  Rows of at most 2048 elements are one vector per thread, where 4 rows leave half of the loads unasked for.
+// cost = waves of tasks / (tasks / CTAs) x a factor of R for what it has in flight (measured on matrices of many waves:
+// 32000 x 2048: 29.4, 25.1, 23.3, 21.7, 20.5 us with 4 ... 8 rows; 128256 x 4096: 145.5, 158.8, 151.4, 148.0, 148.0).
+// One row of x, us per launch in a chain over rotating weights, 4 rows -> this rule (B200):
+//   2560 x 2048: 4.35 -> 2.78 (6)    2048 x 2048: 3.81 -> 2.52 (5)    2048 x 5632: 6.45 -> 4.65 (5)    32000 x 2048: 29.4 -> 20.5 (8)
+//   6144 x 4096: 9.18 -> 8.05 (7)    4096 x 4096: 6.95 -> 6.36 (5)    4096 x 14336: 20.3 -> 18.7 (5)   128256 x 4096: 145.5 (4)
+// Two rows of x take it up to 2048 elements only (more registers: longer rows measured slower).  The sums do not depend
+// on R: a thread always adds its vectors of a row in order.
+static int gemv_rows(int M, int N, int K, bool gated) {
+  if (M > 2 || (M == 2 && K > 2048)) return 4;
+  static const double kShort[] = {1.35, 1.20, 1.10, 1.04, 1.00}, kLong[] = {1.00, 1.09, 1.08, 1.02, 1.03};
+  static const double kShortGated[] = {1.35, 0.0, 1.03, 0.0, 1.05};  // 6 rows: 8.2 us for 8192 x 2048, 8 rows: 9.1
+  const double* factor = K > 2048 ? kLong : gated ? kShortGated : kShort;
+  const long long ctas = 3LL * (sm_count_cached() > 0 ? sm_count_cached() : 148);
+  int pick = 4;
+  double best = 1e30;
+  for (int r = 4; r <= 8; r += gated ? 2 : 1) {
+    const int outs = gated ? r / 2 : r;
+    const long long tasks = (N + outs - 1) / outs, waves = (tasks + ctas - 1) / ctas;
+    const double cost = (double)(waves * ctas) * outs / N * factor[r - 4];
+    if (cost < best) best = cost, pick = r;
+  }
+  return pick;
+}
+
+template <int M, bool kGated, bool kNorm>
+static int launch_gemv(const bf16* x, const bf16* w, const bf16* bias, const bf16* residual, bf16* y, int N, int K,
+                       int epilogue, const bf16* ln_w, float eps, cudaStream_t s, float* cand = nullptr,
+                       int* grid_out = nullptr) {
+#define DLI_GO(r) return launch_gemv_r<M, kGated, kNorm, r>(x, w, bias, residual, y, N, K, epilogue, ln_w, eps, s, cand, grid_out)
+  switch (gemv_rows(M, N, K, kGated)) {
+    case 5:
+      if constexpr (M <= 2 && !kGated) DLI_GO(5);
+      break;
+    case 6:
+      if constexpr (M <= 2) DLI_GO(6);
+      break;
+    case 7:
+      if constexpr (M <= 2 && !kGated) DLI_GO(7);
+      break;
+    case 8:
+      if constexpr (M <= 2) DLI_GO(8);
+      break;
+    default: break;
+  }
+  DLI_GO(4);
+#undef DLI_GO
 }
 
 template <bool kGated, bool kNorm>
