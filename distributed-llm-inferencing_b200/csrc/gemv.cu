@@ -335,7 +335,7 @@ static int launch_gemv_r(const bf16* x, const bf16* w, const bf16* bias, const b
 // Two rows of x take it up to 2048 elements only (more registers: longer rows measured slower).  The sums do not depend
 // on R: a thread always adds its vectors of a row in order.
 static int gemv_rows(int M, int N, int K, bool gated) {
-  if (M > 2 || (M == 2 && K > 2048)) return 4;
+  if (M > 2) return 4;
   static const double kShort[] = {1.35, 1.20, 1.10, 1.04, 1.00}, kLong[] = {1.00, 1.09, 1.08, 1.02, 1.03};
   static const double kShortGated[] = {1.35, 0.0, 1.03, 0.0, 1.05};  // 6 rows: 8.2 us for 8192 x 2048, 8 rows: 9.1
   const double* factor = K > 2048 ? kLong : gated ? kShortGated : kShort;
