@@ -7,7 +7,7 @@
 // page by page into shared memory with 16-byte cp.async (each page row segment
 // is a contiguous hd*2-byte run, fully coalesced), double-buffered; scores and
 // P.V use warp-level m16n8k16 MMAs, the softmax is an online (running max/sum)
-// softmax in fp32 with quad shuffles.  The 4 warps split each tile's tokens and
+// softmax in fp32 with quad shuffles.  The warps split each tile's tokens and
 // are merged through shared memory at the end; with num_splits > 1 the CTA
 // writes an un-normalised partial (O, max, sum) to scratch and a second tiny
 // kernel merges the splits.
@@ -73,9 +73,16 @@ __device__ __forceinline__ float ld_dsmem_f32(uint32_t local_smem_addr, uint32_t
   return v;
 }
 
-// NS = cp.async stages, NW = warps.  Three configurations are used:
-//  * NW = 4, NS = 3 (two CTAs per SM, two 64-token tiles each in flight): the large-batch,
-//    bandwidth-bound case — 5.5-5.6 TB/s at 32-64 sequences x 2k tokens with ONE split.
+// NS = cp.async stages, NW = warps, each with 16 tokens of a tile.  The configurations:
+//  * many CTAs (large batches).  A CTA is bound by the chain of its warps (a tile of 16 tokens per warp: wait, ldmatrix ->
+//    mma, softmax, mma, next request), and with sequences of different lengths the longest one's chain is the kernel's
+//    time however few CTAs are left.  So the chain is kept short — a warp requests and multiplies its own rows
+//    without block barriers, rows of one page with one lookup and constant offsets, masks only at the ends, O rescaled only
+//    when a row maximum moved (647 -> ~330 instructions per tile and warp) — and the shared memory of a CTA is cut into
+//    more warps with two stages rather than four warps with three.  us on B200, start -> now, 8 heads of 128 x 4 query
+//    heads: 32 sequences of 256 ... 2048 tokens 41.8 -> 31.4 (4.9 TB/s), all of 2048 45.8 -> 44.6; 64 of 256 ... 2048 70.6 ->
+//    57.9; 48 of 2048 88.8 -> 62.5 (2 stages x 4 warps: three CTAs per SM make one wave of them).  4 heads of 64 x 8: 64
+//    sequences of 256 ... 2048 31.4 -> 18.8 (2 stages x 8 warps), 128 of 64 ... 512 12.1 -> 11.1 (3 x 4: one wave).
 //  * NW = 16, NS = 1 / NW = 8, NS = 2 (one CTA per SM at most, a whole 256-token split in flight):
 //    the few-CTA case, i.e. a batch-1 step.  That case is not bandwidth- but ISSUE-bound: ncu on
 //    the former 4-warp form showed one warp per scheduler, stalled on fixed-latency dependencies
@@ -137,21 +144,46 @@ paged_attn_decode_kernel(const bf16* __restrict__ q, int q_stride,
   const int page_mask = (1 << page_shift) - 1;
   const int32_t* pt = page_table + (size_t)b * max_pages;
 
-  auto load_tile = [&](int tile, int stage) {
-    const uint32_t dK = sK + stage * L::kTileBytes, dV = sV + stage * L::kTileBytes;
+  // A warp brings in the 16 rows of a tile that it multiplies itself, so nothing but Q is shared between the warps and
+  // they run through the tiles on their own: no block barrier per tile.  Where the 16 rows lie in one page (page sizes from
+  // 16) they are one contiguous run: one page lookup, made a tile ahead, and constant offsets from one address.
+  constexpr int kLoads = 16 * CH / 32;       // 16-byte pieces of the rows per lane
+  constexpr int kRowStep = 32 / CH;          // rows between a lane's pieces
+  constexpr int kSwzSteps = 8 / kRowStep;    // pieces after which the swizzle pattern repeats
+  const int lrow = lane / CH, lc = lane % CH;
+  uint32_t soff[kSwzSteps];
 #pragma unroll
-    for (int i = 0; i < kAttnTile * CH / kAttnThreads; ++i) {
-      const int id = tid + i * kAttnThreads;
-      const int row = id / CH, c = id - row * CH;
-      const int tok = tile * kAttnTile + row;
+  for (int i = 0; i < kSwzSteps; ++i) soff[i] = swz<RB>(warp * 16 + lrow + i * kRowStep, lc);
+  const bool one_page = page_shift >= 4;
+  auto page_of = [&](int tile) -> int {  // of the warp's rows of a tile; rows past the end: any page that is the sequence's
+    return pt[min(tile * kAttnTile + warp * 16, seq_len - 1) >> page_shift];
+  };
+  auto load_tile = [&](int tile, int stage, int page) {
+    const uint32_t dK = sK + stage * L::kTileBytes, dV = sV + stage * L::kTileBytes;
+    const int tok0 = tile * kAttnTile + warp * 16;
+    const int left = seq_len - tok0;  // rows of the warp's 16 that exist
+    if (one_page) {
+      size_t off = ((((size_t)page * KV + kvh) << page_shift) + (tok0 & page_mask)) * HD + lane * 8;
+      if (left <= 0) off = 0;  // nothing is read, but the addresses stay in the pools
+      const bf16 *kp = k_cache + off, *vp = v_cache + off;
+#pragma unroll
+      for (int i = 0; i < kLoads; ++i) {
+        const int bytes = lrow + i * kRowStep < left ? 16 : 0;
+        const uint32_t so = soff[i % kSwzSteps] + (i / kSwzSteps) * (8 * RB);
+        cp_async_16B(dK + so, kp + (bytes ? i * 256 : 0), bytes);
+        cp_async_16B(dV + so, vp + (bytes ? i * 256 : 0), bytes);
+      }
+      return;
+    }
+#pragma unroll
+    for (int i = 0; i < kLoads; ++i) {
+      const int tok = tok0 + lrow + i * kRowStep;
       const bool valid = tok < seq_len;
       size_t off = 0;
-      if (valid) {
-        const int page = pt[tok >> page_shift];
-        off = ((((size_t)page * KV + kvh) << page_shift) + (tok & page_mask)) * HD + c * 8;
-      }
-      cp_async_16B(dK + swz<RB>(row, c), k_cache + off, valid ? 16 : 0);
-      cp_async_16B(dV + swz<RB>(row, c), v_cache + off, valid ? 16 : 0);
+      if (valid) off = ((((size_t)pt[tok >> page_shift] * KV + kvh) << page_shift) + (tok & page_mask)) * HD + lc * 8;
+      const uint32_t so = soff[i % kSwzSteps] + (i / kSwzSteps) * (8 * RB);
+      cp_async_16B(dK + so, k_cache + off, valid ? 16 : 0);
+      cp_async_16B(dV + so, v_cache + off, valid ? 16 : 0);
     }
   };
 
@@ -165,9 +197,10 @@ paged_attn_decode_kernel(const bf16* __restrict__ q, int q_stride,
   // one commit group per stage (empty groups keep the count uniform)
 #pragma unroll
   for (int st = 0; st < NS; ++st) {
-    if (t_begin + st < t_end) load_tile(t_begin + st, st);
+    if (t_begin + st < t_end) load_tile(t_begin + st, st, page_of(t_begin + st));
     cp_async_commit();
   }
+  int page_next = t_begin + NS < t_end ? page_of(t_begin + NS) : 0;
   if (fused) {
     pdl_wait();  // q and the new token's k, v
     pdl_trigger();
@@ -181,47 +214,75 @@ paged_attn_decode_kernel(const bf16* __restrict__ q, int q_stride,
   }
   cp_async_commit();
 
-  // Fused form: cos/sin of the new position, and on the CTA that owns the last tile the new token's k, v and cache
-  // page, are needed only once the first K/V tile has landed.  Requested here, their round trips hide under that
-  // wait instead of following it (the kernel is bound by its chain of dependent loads, not by bandwidth).
-  // Every thread rotates elements i = tid % (HD/2) only (the block size is a multiple of HD/2), so one pair does.
-  float pre_c = 1.f, pre_s = 0.f, pre_k1 = 0.f, pre_k2 = 0.f;
-  uint4 pre_v = make_uint4(0u, 0u, 0u, 0u);
-  int pre_page = 0;
-  if (fused && t_begin < t_end) {
-    const int pos = seq_len - 1, half = HD / 2;
-    if (cos_t) {
-      pre_c = __bfloat162float(cos_t[(size_t)pos * half + (tid % half)]);
-      pre_s = __bfloat162float(sin_t[(size_t)pos * half + (tid % half)]);
+  // Fused form: cos/sin of the new position, and in the warp that owns the new token's row its k, v and cache page, are
+  // needed only once the first K/V rows have landed.  Requested here, their round trips hide under that wait instead of
+  // following it (the kernel is bound by its chain of dependent loads, not by bandwidth).
+  // Every thread rotates elements i = tid % (HD/2) of Q only (the block size is a multiple of HD/2), so one pair does.
+  constexpr int half = HD / 2;
+  const int pos = seq_len - 1;
+  const bool owner = fused && t_begin < t_end && t_end == tile_hi && warp == (pos - (tile_hi - 1) * kAttnTile) >> 4;
+  float pre_c = 1.f, pre_s = 0.f, own_k1[half / 32], own_k2[half / 32], own_c[half / 32], own_s[half / 32];
+  uint4 own_v = make_uint4(0u, 0u, 0u, 0u);
+  int own_page = 0;
+  if (fused && t_begin < t_end && cos_t) {
+    pre_c = __bfloat162float(cos_t[(size_t)pos * half + (tid % half)]);
+    pre_s = __bfloat162float(sin_t[(size_t)pos * half + (tid % half)]);
+  }
+  if (owner) {
+    own_page = pt[pos >> page_shift];
+    const bf16* knew = q + (size_t)b * q_stride + (size_t)(H + kvh) * HD;
+#pragma unroll
+    for (int u = 0; u < half / 32; ++u) {
+      const int i = lane + 32 * u;
+      own_k1[u] = __bfloat162float(knew[i]);
+      own_k2[u] = __bfloat162float(knew[i + half]);
+      own_c[u] = cos_t ? __bfloat162float(cos_t[(size_t)pos * half + i]) : 1.f;
+      own_s[u] = cos_t ? __bfloat162float(sin_t[(size_t)pos * half + i]) : 0.f;
     }
-    if (t_end == tile_hi && tid < half + CH) {
-      pre_page = pt[pos >> page_shift];
-      if (tid < half) {
-        const bf16* knew = q + (size_t)b * q_stride + (size_t)(H + kvh) * HD;
-        pre_k1 = __bfloat162float(knew[tid]);
-        pre_k2 = __bfloat162float(knew[tid + half]);
-      } else {
-        pre_v = ld_16B(q + (size_t)b * q_stride + (size_t)(H + KV + kvh) * HD + (tid - half) * 8);
+    if (lane < CH) own_v = ld_16B(q + (size_t)b * q_stride + (size_t)(H + KV + kvh) * HD + lane * 8);
+  }
+
+  if (t_begin < t_end) {
+    cp_async_wait<0>();  // Q (the newest group) and every stage requested so far
+    __syncthreads();
+    if (fused && cos_t) {
+      // rotate the G query rows in shared memory (rotate-half, bf16 op by op)
+      for (int idx = tid; idx < G * half; idx += kAttnThreads) {
+        const int g = idx / half, i = idx - g * half;
+        bf16* p1 = reinterpret_cast<bf16*>(smem + swz<RB>(g, i >> 3) + (i & 7) * 2);
+        bf16* p2 = reinterpret_cast<bf16*>(smem + swz<RB>(g, (i + half) >> 3) + (i & 7) * 2);
+        const float x1 = __bfloat162float(*p1), x2 = __bfloat162float(*p2);
+        const float c = pre_c, sn = pre_s;  // i == tid % half on every iteration
+        *p1 = __float2bfloat16_rn(round_bf16(x1 * c) + round_bf16(-x2 * sn));
+        *p2 = __float2bfloat16_rn(round_bf16(x2 * c) + round_bf16(x1 * sn));
+      }
+      __syncthreads();
+    }
+    if (!kStreamQ) {
+#pragma unroll
+      for (int kk = 0; kk < HD / 16; ++kk) {
+        const int mi = lane >> 3;
+        ldmatrix_x4(qf[kStreamQ ? 0 : kk], sQ + swz<RB>((mi & 1) * 8 + (lane & 7), kk * 2 + (mi >> 1)));
       }
     }
   }
 
   for (int tile = t_begin; tile < t_end; ++tile) {
     const int stage = (tile - t_begin) % NS;
-    if (tile == t_begin) cp_async_wait<0>();  // Q (the newest group) and every stage requested so far
-    else cp_async_wait<NS - 1>();             // all but the newest NS-1 groups have landed: this tile is in
-    __syncthreads();
+    if (tile != t_begin) cp_async_wait<NS - 1>();  // all but the newest NS-1 groups have landed: this tile's rows are in
+    __syncwarp();
     const uint32_t cK = sK + stage * L::kTileBytes, cV = sV + stage * L::kTileBytes;
-    if (fused && tile == tile_hi - 1) {
-      // this CTA owns the tile of the new token (position seq_len-1): rotate its k, store
-      // k and v to the cache page and patch them into the staged tile
-      const int pos = seq_len - 1, row = pos - tile * kAttnTile, half = HD / 2;
-      const size_t coff = ((((size_t)pre_page * KV + kvh) << page_shift) + (pos & page_mask)) * HD;
-      if (tid < half) {
-        const int i = tid;
-        float x1 = pre_k1, x2 = pre_k2;
+    if (owner && tile == tile_hi - 1) {
+      // this warp owns the row of the new token (position seq_len-1): rotate its k, store k and v to the cache page and
+      // patch them into the staged row
+      const int row = pos - tile * kAttnTile;
+      const size_t coff = ((((size_t)own_page * KV + kvh) << page_shift) + (pos & page_mask)) * HD;
+#pragma unroll
+      for (int u = 0; u < half / 32; ++u) {
+        const int i = lane + 32 * u;
+        float x1 = own_k1[u], x2 = own_k2[u];
         if (cos_t) {
-          const float c = pre_c, sn = pre_s;
+          const float c = own_c[u], sn = own_s[u];
           const float o1 = round_bf16(x1 * c) + round_bf16(-x2 * sn);
           const float o2 = round_bf16(x2 * c) + round_bf16(x1 * sn);
           x1 = o1; x2 = o2;
@@ -231,36 +292,12 @@ paged_attn_decode_kernel(const bf16* __restrict__ q, int q_stride,
         k_cache_w[coff + i + half] = b2;
         *reinterpret_cast<bf16*>(smem + (cK - sQ) + swz<RB>(row, i >> 3) + (i & 7) * 2) = b1;
         *reinterpret_cast<bf16*>(smem + (cK - sQ) + swz<RB>(row, (i + half) >> 3) + (i & 7) * 2) = b2;
-      } else if (tid < half + CH) {
-        const int c = tid - half;
-        const uint4 u = pre_v;
-        st_16B(v_cache_w + coff + c * 8, u);
-        *reinterpret_cast<uint4*>(smem + (cV - sQ) + swz<RB>(row, c)) = u;
       }
-      __syncthreads();
-    }
-    if (tile == t_begin) {
-      if (fused && cos_t) {
-        // rotate the G query rows in shared memory (rotate-half, bf16 op by op)
-        const int half = HD / 2;
-        for (int idx = tid; idx < G * half; idx += kAttnThreads) {
-          const int g = idx / half, i = idx - g * half;
-          bf16* p1 = reinterpret_cast<bf16*>(smem + swz<RB>(g, i >> 3) + (i & 7) * 2);
-          bf16* p2 = reinterpret_cast<bf16*>(smem + swz<RB>(g, (i + half) >> 3) + (i & 7) * 2);
-          const float x1 = __bfloat162float(*p1), x2 = __bfloat162float(*p2);
-          const float c = pre_c, sn = pre_s;  // i == tid % half on every iteration
-          *p1 = __float2bfloat16_rn(round_bf16(x1 * c) + round_bf16(-x2 * sn));
-          *p2 = __float2bfloat16_rn(round_bf16(x2 * c) + round_bf16(x1 * sn));
-        }
-        __syncthreads();
+      if (lane < CH) {
+        st_16B(v_cache_w + coff + lane * 8, own_v);
+        *reinterpret_cast<uint4*>(smem + (cV - sQ) + swz<RB>(row, lane)) = own_v;
       }
-      if (!kStreamQ) {
-#pragma unroll
-        for (int kk = 0; kk < HD / 16; ++kk) {
-          const int mi = lane >> 3;
-          ldmatrix_x4(qf[kStreamQ ? 0 : kk], sQ + swz<RB>((mi & 1) * 8 + (lane & 7), kk * 2 + (mi >> 1)));
-        }
-      }
+      __syncwarp();
     }
 
     // ---- S = Q K^T for this warp's 16 tokens ---------------------------------------
@@ -277,14 +314,17 @@ paged_attn_decode_kernel(const bf16* __restrict__ q, int q_stride,
       mma_16816(s[1], qf[kStreamQ ? 0 : kk], kf[2], kf[3]);
     }
     // ---- mask + online softmax --------------------------------------------------------
-    const int tok0 = tile * kAttnTile + warp * 16 + 2 * (lane & 3);
+    const int row0 = tile * kAttnTile + warp * 16;
+    if (row0 + 16 > seq_len || row0 < first_tok) {  // rows past the end or before the window
+      const int tok0 = row0 + 2 * (lane & 3);
 #pragma unroll
-    for (int j = 0; j < 2; ++j)
+      for (int j = 0; j < 2; ++j)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int tok = tok0 + j * 8 + (e & 1);
-        if (tok >= seq_len || tok < first_tok) s[j][e] = -INFINITY;
-      }
+        for (int e = 0; e < 4; ++e) {
+          const int tok = tok0 + j * 8 + (e & 1);
+          if (tok >= seq_len || tok < first_tok) s[j][e] = -INFINITY;
+        }
+    }
     uint32_t pa[4];
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
@@ -303,10 +343,12 @@ paged_attn_decode_kernel(const bf16* __restrict__ q, int q_stride,
       l_run[r] = l_run[r] * corr + (p[0] + p[1] + p[2] + p[3]);
       pa[r] = pack_bf16(p[0], p[1]);      // a0 (row g) / a1 (row g+8): tokens 2t,2t+1
       pa[2 + r] = pack_bf16(p[2], p[3]);  // a2 / a3: tokens 8+2t, 8+2t+1
+      if (__any_sync(0xffffffffu, corr != 1.f)) {  // most tiles leave the running maximum alone
 #pragma unroll
-      for (int i = 0; i < HD / 8; ++i) {
-        o[i][2 * r] *= corr;
-        o[i][2 * r + 1] *= corr;
+        for (int i = 0; i < HD / 8; ++i) {
+          o[i][2 * r] *= corr;
+          o[i][2 * r + 1] *= corr;
+        }
       }
     }
     // ---- O += P V ------------------------------------------------------------------------
@@ -318,9 +360,10 @@ paged_attn_decode_kernel(const bf16* __restrict__ q, int q_stride,
       mma_16816(o[2 * jp], pa, vf[0], vf[1]);
       mma_16816(o[2 * jp + 1], pa, vf[2], vf[3]);
     }
-    __syncthreads();  // every warp is done with this stage: refill it
-    if (tile + NS < t_end) load_tile(tile + NS, stage);
+    __syncwarp();  // the warp is done with its rows of this stage: refill them
+    if (tile + NS < t_end) load_tile(tile + NS, stage, page_next);
     cp_async_commit();
+    if (tile + NS + 1 < t_end) page_next = page_of(tile + NS + 1);
   }
   cp_async_wait<0>();
   __syncthreads();
@@ -550,6 +593,21 @@ static int attn_wide_env() {
   return v;
 }
 
+// CTAs of a form that run at once on the current device.
+template <int HD, int NS, int NW>
+static int decode_at_once(int* n) {
+  using L = DecodeSmem<HD, NS, NW>;
+  static PerDeviceOnce once;
+  DLI_ONCE_PER_DEVICE(once, dev, {
+    DLI_CUDA_CALL(cudaFuncSetAttribute(paged_attn_decode_kernel<HD, NS, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal));
+    int o = 0;
+    DLI_CUDA_CALL(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, paged_attn_decode_kernel<HD, NS, NW>, L::kThreads, L::kTotal));
+    once.value[dev] = (o > 0 ? o : 1) * (sm_count_cached() > 0 ? sm_count_cached() : 1);
+  });
+  *n = once.value[dev];
+  return DLI_OK;
+}
+
 template <int HD>
 static int launch_decode(const void* q, int q_stride, const void* k_cache, const void* v_cache,
                          const int32_t* page_table, int max_pages, const int32_t* seq_lens,
@@ -560,8 +618,24 @@ static int launch_decode(const void* q, int q_stride, const void* k_cache, const
 #define DLI_DECODE_ARGS                                                                                            \
   q, q_stride, k_cache, v_cache, page_table, max_pages, seq_lens, out, scratch, B, H, KV, page_shift, num_splits, \
       scale, window, s, fused, cos_t, sin_t, pf_a, pf_a_bytes, pf_b, pf_b_bytes
-  // many CTAs: occupancy (two 4-warp CTAs per SM, 3 stages)
-  if ((size_t)num_splits * KV * B > (size_t)sm_count_cached()) return launch_decode_ns<HD, 3, 4>(DLI_DECODE_ARGS);
+  // many CTAs: several per SM
+  if ((size_t)num_splits * KV * B > (size_t)sm_count_cached()) {
+    // The form whose CTAs need fewer waves; the first one on a tie (its CTA is the faster one).
+    const size_t n = (size_t)num_splits * KV * B;
+    int at_once[2];
+    const int rc = HD == 128 ? decode_at_once<HD, 2, 6>(&at_once[0]) : decode_at_once<HD, 2, 8>(&at_once[0]);
+    if (rc != DLI_OK) return rc;
+    const int rc2 = HD == 128 ? decode_at_once<HD, 2, 4>(&at_once[1]) : decode_at_once<HD, 3, 4>(&at_once[1]);
+    if (rc2 != DLI_OK) return rc2;
+    const bool second = (n + at_once[1] - 1) / at_once[1] < (n + at_once[0] - 1) / at_once[0];
+    if constexpr (HD == 128) {
+      if (second) return launch_decode_ns<HD, 2, 4>(DLI_DECODE_ARGS);
+      return launch_decode_ns<HD, 2, 6>(DLI_DECODE_ARGS);
+    } else {
+      if (second) return launch_decode_ns<HD, 3, 4>(DLI_DECODE_ARGS);
+      return launch_decode_ns<HD, 2, 8>(DLI_DECODE_ARGS);
+    }
+  }
   // few CTAs (batch-1 style): at most one CTA per SM, the whole split in flight, many warps
   const bool cluster = num_splits > 1 && num_splits <= 8 && scratch == nullptr;
   int wide = attn_wide_env();

@@ -332,8 +332,7 @@ static int launch_gemv_r(const bf16* x, const bf16* w, const bf16* bias, const b
 // One row of x, us per launch in a chain over rotating weights, 4 rows -> this rule (B200):
 //   2560 x 2048: 4.35 -> 2.78 (6)    2048 x 2048: 3.81 -> 2.52 (5)    2048 x 5632: 6.45 -> 4.65 (5)    32000 x 2048: 29.4 -> 20.5 (8)
 //   6144 x 4096: 9.18 -> 8.05 (7)    4096 x 4096: 6.95 -> 6.36 (5)    4096 x 14336: 20.3 -> 18.7 (5)   128256 x 4096: 145.5 (4)
-// Two rows of x take it up to 2048 elements only (more registers: longer rows measured slower).  The sums do not depend
-// on R: a thread always adds its vectors of a row in order.
+// The sums do not depend on R: a thread always adds its vectors of a row in order.
 static int gemv_rows(int M, int N, int K, bool gated) {
   if (M > 2) return 4;
   static const double kShort[] = {1.35, 1.20, 1.10, 1.04, 1.00}, kLong[] = {1.00, 1.09, 1.08, 1.02, 1.03};
