@@ -249,14 +249,45 @@ postnorm_add_norm_kernel(const E* __restrict__ y, float* __restrict__ x, float* 
   pdl_wait();
   pdl_trigger();
   const size_t o = (size_t)blockIdx.x * d;
-  float ss = 0.f;
+  float ss = 0.f, s2 = 0.f;
+  constexpr int kHeld = 8;
+  if (d <= kHeld * (int)blockDim.x) {
+    // the row of y and of x in registers, asked for together: one pass over memory instead of three (the same sums).
+    // Latency-bound: 7.4 -> 5.4 us averaged over prompt (547 x 2048) and decode rows
+    float yv[kHeld], xv[kHeld];
+#pragma unroll
+    for (int i = 0; i < kHeld; ++i) {
+      const int c = threadIdx.x + i * blockDim.x;
+      yv[i] = c < d ? to_f(y[o + c]) : 0.f;
+      xv[i] = c < d ? x[o + c] : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < kHeld; ++i) ss += yv[i] * yv[i];
+    ss = block_sum(ss, red);
+    const float r = g_post / sqrtf(ss / d + eps);
+#pragma unroll
+    for (int i = 0; i < kHeld; ++i) {
+      const int c = threadIdx.x + i * blockDim.x;
+      xv[i] += yv[i] * r;
+      if (c < d) x[o + c] = xv[i];
+      s2 += xv[i] * xv[i];
+    }
+    if (hn == nullptr) return;
+    s2 = block_sum(s2, red);
+    const float r2 = g_next / sqrtf(s2 / d + eps);
+#pragma unroll
+    for (int i = 0; i < kHeld; ++i) {
+      const int c = threadIdx.x + i * blockDim.x;
+      if (c < d) hn[o + c] = xv[i] * r2;
+    }
+    return;
+  }
   for (int c = threadIdx.x; c < d; c += blockDim.x) {
     const float v = to_f(y[o + c]);
     ss += v * v;
   }
   ss = block_sum(ss, red);
   const float r = g_post / sqrtf(ss / d + eps);
-  float s2 = 0.f;
   for (int c = threadIdx.x; c < d; c += blockDim.x) {
     const float v = x[o + c] + to_f(y[o + c]) * r;
     x[o + c] = v;
@@ -295,6 +326,47 @@ causal_conv_kernel(const float* __restrict__ h, const float* __restrict__ tail, 
   }
 }
 
+// The same with four channels per thread (d % 4 == 0) and four taps: every input of a thread — the row, the three before
+// it, the weights — is one 16-byte load, all asked for before any is used.  The sums run over the taps in the same order.
+// The scalar form above walks 8 channels per thread with a branch per tap: 547 rows of 2048 12.2 -> 7.0 us.
+template <typename E>
+__global__ void __launch_bounds__(256)
+causal_conv4_kernel(const float* __restrict__ h, const float* __restrict__ tail, const float* __restrict__ w,
+                    const int32_t* __restrict__ row_ent, const int32_t* __restrict__ ent, E* __restrict__ out, int d) {
+  const int c = (blockIdx.y * 256 + threadIdx.x) * 4;
+  float4 wv[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) wv[i] = c < d ? reinterpret_cast<const float4*>(w)[c + i] : make_float4(0.f, 0.f, 0.f, 0.f);
+  pdl_wait();
+  pdl_trigger();
+  if (c >= d) return;
+  const int row = blockIdx.x;
+  const int4 e = reinterpret_cast<const int4*>(ent)[row_ent[row]];  // slot, row0, n, start
+  const int back = row - e.y, pos = e.w + back;
+  float4 v[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int dist = 3 - j;
+    const float* src = dist <= back ? h + (size_t)(row - dist) * d + c : tail + ((size_t)e.x * 3 + (3 - (dist - back))) * d + c;
+    v[j] = pos - dist >= 0 ? *reinterpret_cast<const float4*>(src) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  const float vv[4][4] = {{v[0].x, v[0].y, v[0].z, v[0].w}, {v[1].x, v[1].y, v[1].z, v[1].w},
+                          {v[2].x, v[2].y, v[2].z, v[2].w}, {v[3].x, v[3].y, v[3].z, v[3].w}};
+  float r[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float wj[4] = {wv[i].x, wv[i].y, wv[i].z, wv[i].w};
+    float acc = 0.f;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (pos - (3 - j) >= 0) acc += wj[j] * vv[j][i];
+    r[i] = vv[3][i] + acc;
+  }
+  E* o = out + (size_t)row * d + c;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) o[i] = from_f<E>(r[i]);
+}
+
 // The same for a step in which every entry brings ONE row (decode): the row's CTA is the only reader and writer of
 // its slot's tail, so the convolution and the tail's shift are one kernel.
 template <typename E>
@@ -329,11 +401,84 @@ postnorm_add_norm_conv_single_kernel(const E* __restrict__ y, float* __restrict_
                                      const float* __restrict__ w, const int32_t* __restrict__ ent, E* __restrict__ out,
                                      int d, int taps, float eps, float g_post, float g_next) {
   __shared__ float red[32];
-  pdl_wait();
-  pdl_trigger();
   const int row = blockIdx.x;
   const size_t o = (size_t)row * d;
   float s2 = 0.f;
+  constexpr int kHeld = 4, kTaps = 4;
+  if (taps <= kTaps && d <= kHeld * (int)blockDim.x) {
+    // Everything a thread's channels need in registers, and what the kernel just before this one did not write — the
+    // weights and the slot's tail; with a post-norm also the row of x, whose last writer is two kernels back — asked
+    // for before the dependency wait (every kernel of the library waits for its predecessor before it lets its
+    // successor start).  After it only y is left.  The sums are those of the general form below.
+    // Latency-bound: three rows of 2048 7.5 -> 6.0 us without the overlap, 0.2 ms of a 2.9 ms pass with it.
+    const int4 e = reinterpret_cast<const int4*>(ent)[row];
+    const int keep = taps - 1;
+    float xv[kHeld], tv[kHeld][kTaps - 1], wv[kHeld][kTaps];
+#pragma unroll
+    for (int i = 0; i < kHeld; ++i) {
+      const int c = threadIdx.x + i * blockDim.x;
+      const bool on = c < d;
+#pragma unroll
+      for (int j = 0; j < kTaps; ++j) wv[i][j] = on && j < taps ? w[(size_t)c * taps + j] : 0.f;
+#pragma unroll
+      for (int j = 0; j < kTaps - 1; ++j)
+        tv[i][j] = on && j < keep && e.w - keep + j >= 0 ? tail[((size_t)e.x * keep + j) * d + c] : 0.f;
+      xv[i] = on && y != nullptr ? x[o + c] : 0.f;
+    }
+    pdl_wait();
+    pdl_trigger();
+    if (y != nullptr) {
+      float yv[kHeld], ss = 0.f;
+#pragma unroll
+      for (int i = 0; i < kHeld; ++i) {
+        const int c = threadIdx.x + i * blockDim.x;
+        yv[i] = c < d ? to_f(y[o + c]) : 0.f;
+      }
+#pragma unroll
+      for (int i = 0; i < kHeld; ++i) ss += yv[i] * yv[i];
+      ss = block_sum(ss, red);
+      const float r = g_post / sqrtf(ss / d + eps);
+#pragma unroll
+      for (int i = 0; i < kHeld; ++i) {
+        const int c = threadIdx.x + i * blockDim.x;
+        xv[i] += yv[i] * r;
+        if (c < d) x[o + c] = xv[i];
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < kHeld; ++i) {
+        const int c = threadIdx.x + i * blockDim.x;
+        xv[i] = c < d ? x[o + c] : 0.f;
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < kHeld; ++i) s2 += xv[i] * xv[i];
+    s2 = block_sum(s2, red);
+    const float r2 = g_next / sqrtf(s2 / d + eps);
+#pragma unroll
+    for (int i = 0; i < kHeld; ++i) {
+      const int c = threadIdx.x + i * blockDim.x;
+      if (c >= d) break;
+      const float cur = xv[i] * r2;
+      float* t = tail + (size_t)e.x * keep * d + c;
+      float acc = 0.f;
+#pragma unroll
+      for (int j = 0; j < kTaps; ++j)
+        if (j == keep) acc = wv[i][j] * cur;
+#pragma unroll
+      for (int j = 0; j < kTaps - 1; ++j) {
+        if (j < keep) {
+          acc += wv[i][j] * tv[i][j];
+          if (j > 0) t[(size_t)(j - 1) * d] = tv[i][j];
+        }
+      }
+      if (keep > 0) t[(size_t)(keep - 1) * d] = cur;
+      out[o + c] = from_f<E>(cur + acc);
+    }
+    return;
+  }
+  pdl_wait();
+  pdl_trigger();
   if (y != nullptr) {
     float ss = 0.f;
     for (int c = threadIdx.x; c < d; c += blockDim.x) {
@@ -396,7 +541,7 @@ conv_tail_update_kernel(const float* __restrict__ h, float* __restrict__ tail, c
   pdl_trigger();
   const int4 e = reinterpret_cast<const int4*>(ent)[blockIdx.x];
   const int keep = taps - 1, end = e.w + e.z;
-  for (int c = threadIdx.x; c < d; c += blockDim.x) {
+  for (int c = blockIdx.y * blockDim.x + threadIdx.x; c < d; c += gridDim.y * blockDim.x) {  // a thread per channel
     float* t = tail + (size_t)e.x * keep * d + c;
     for (int i = 0; i < keep; ++i) {  // ascending: slot i reads old slot i + n (n >= 1), never one already written
       const int p = end - keep + i;
@@ -742,9 +887,17 @@ int dli_causal_conv_ragged(const float* h, float* tail, const float* w, const in
     else DLI_LAUNCH("causal_conv_single", causal_conv_single_kernel<float>, dim3(rows), dim3(256), 0, s, h, tail, w, ent, (float*)out, d, taps);
     return DLI_OK;
   }
-  if (dt == 0) DLI_LAUNCH("causal_conv", causal_conv_kernel<bf16>, dim3(rows), dim3(256), 0, s, h, (const float*)tail, w, row_ent, ent, (bf16*)out, d, taps);
-  else DLI_LAUNCH("causal_conv", causal_conv_kernel<float>, dim3(rows), dim3(256), 0, s, h, (const float*)tail, w, row_ent, ent, (float*)out, d, taps);
-  if (taps > 1) DLI_LAUNCH("conv_tail_update", conv_tail_update_kernel, dim3(n_ent), dim3(256), 0, s, h, tail, ent, d, taps);
+  const auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
+  if (taps == 4 && d % 4 == 0 && d <= 65535 * 1024 && al16(h) && al16(tail) && al16(w)) {
+    const dim3 grid(rows, (d + 1023) / 1024);
+    if (dt == 0) DLI_LAUNCH("causal_conv", causal_conv4_kernel<bf16>, grid, dim3(256), 0, s, h, (const float*)tail, w, row_ent, ent, (bf16*)out, d);
+    else DLI_LAUNCH("causal_conv", causal_conv4_kernel<float>, grid, dim3(256), 0, s, h, (const float*)tail, w, row_ent, ent, (float*)out, d);
+  } else if (dt == 0) {
+    DLI_LAUNCH("causal_conv", causal_conv_kernel<bf16>, dim3(rows), dim3(256), 0, s, h, (const float*)tail, w, row_ent, ent, (bf16*)out, d, taps);
+  } else {
+    DLI_LAUNCH("causal_conv", causal_conv_kernel<float>, dim3(rows), dim3(256), 0, s, h, (const float*)tail, w, row_ent, ent, (float*)out, d, taps);
+  }
+  if (taps > 1) DLI_LAUNCH("conv_tail_update", conv_tail_update_kernel, dim3(n_ent, (d + 255) / 256 < 65535 ? (d + 255) / 256 : 65535), dim3(256), 0, s, h, tail, ent, d, taps);
   return DLI_OK;
 }
 
