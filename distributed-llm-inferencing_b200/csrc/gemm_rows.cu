@@ -194,91 +194,126 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
 
   // ---- epilogue over this CTA's columns: an item is 8 consecutive outputs of one activation row (two groups of 8 where
   // two belong together: gate and up, or the halves of a rotation pair) ----
+  // A thread keeps its group of outputs (the block is a multiple of kGroups) and takes kBatch rows at a time: what it needs
+  // from global memory for all of them — residual, position, rotation, page — is asked for before any is used.
   constexpr int kGroups = kMode == kRowsPlain ? 16 : 8;
+  constexpr int kBatch = 4;
+  static_assert(kRowsThreads % kGroups == 0, "a thread keeps its group");
   const int n_out = kGated ? N / 2 : N;
   const int col0 = rank * per;
   const int items = max(0, min(per, rows - col0)) * kGroups;
   const float* sums = reinterpret_cast<const float*>(smem);
-  for (int id = threadIdx.x; id < items; id += kRowsThreads) {
-    const int c = id / kGroups, g = id - c * kGroups;
-    const int m = m0 + col0 + c;
-    // first weight row of the item inside the tile, and how much further its second group starts
-    const int half = hd >> 1;
-    const int r0 = kMode == kRowsRope && hd == 64 ? (g >> 2) * 64 + (g & 3) * 8 : g * 8;
-    const int r1 = kMode == kRowsRope ? half : 64;
-    const int n = kGated ? n_tile * 64 + r0 : n_tile * 128 + r0;
-    if (n >= n_out) continue;  // n_out is a multiple of 16 (of hd with heads): a group is whole or absent
-    const size_t at = (size_t)m * n_out + n;
-    uint4 res = make_uint4(0u, 0u, 0u, 0u), bv = res, bv2 = res;
-    if (kMode == kRowsPlain && (epilogue & DLI_EPI_RESIDUAL)) res = ld_16B(residual + at);
-    if (!kGated && (epilogue & DLI_EPI_BIAS)) {
-      bv = ld_16B(bias + n);
-      if (kMode == kRowsRope) bv2 = ld_16B(bias + n + half);
-    }
-    float a[8], b[8];
-#pragma unroll
-    for (int e = 0; e < 8; ++e) a[e] = 0.f, b[e] = 0.f;
-    for (int sp = 0; sp < splits; ++sp) {  // in split order: deterministic
-      const float4* p = reinterpret_cast<const float4*>(sums + (size_t)(sp * per + c) * 128 + r0);
-      const float4 u = p[0], v = p[1];
-      a[0] += u.x; a[1] += u.y; a[2] += u.z; a[3] += u.w;
-      a[4] += v.x; a[5] += v.y; a[6] += v.z; a[7] += v.w;
-      if (kMode != kRowsPlain) {
-        const float4 u2 = p[r1 / 4], v2 = p[r1 / 4 + 1];
-        b[0] += u2.x; b[1] += u2.y; b[2] += u2.z; b[3] += u2.w;
-        b[4] += v2.x; b[5] += v2.y; b[6] += v2.z; b[7] += v2.w;
+  const int g = threadIdx.x % kGroups;
+  // first weight row of the group inside the tile, and how much further its second group starts
+  const int half = hd >> 1;
+  const int r0 = kMode == kRowsRope && hd == 64 ? (g >> 2) * 64 + (g & 3) * 8 : g * 8;
+  const int r1 = kMode == kRowsRope ? half : 64;
+  const int n = kGated ? n_tile * 64 + r0 : n_tile * 128 + r0;
+  if (n < n_out) {  // n_out is a multiple of 16 (of hd with heads): a group is whole or absent
+    float bb[8], bb2[8];
+    {
+      uint4 bv = make_uint4(0u, 0u, 0u, 0u), bv2 = bv;
+      if (!kGated && (epilogue & DLI_EPI_BIAS)) {
+        bv = ld_16B(bias + n);
+        if (kMode == kRowsRope) bv2 = ld_16B(bias + n + half);
       }
+      unpack8(bv, bb);
+      unpack8(bv2, bb2);
     }
-    if (kGated) {
+    const int head = hd == 64 ? n_tile * 2 + (g >> 2) : n_tile;  // kRowsRope: q heads, then k heads, then v heads
+    const int he = hd == 64 ? (g & 3) * 8 : g * 8;               // element of the head's first half
+    const bool turned = kMode == kRowsRope && rope.cos_t && head < rope.H + rope.KV;
+    for (int id0 = threadIdx.x; id0 < items; id0 += kBatch * kRowsThreads) {
+      uint4 pre1[kBatch], pre2[kBatch];  // residual; or cosines and sines
+      int pos[kBatch], page[kBatch];
 #pragma unroll
-      for (int e = 0; e < 8; ++e) a[e] = round_bf16(a[e]), b[e] = round_bf16(b[e]);
-      gated_combine_n(a, b, reinterpret_cast<const float*>(bias));
-      st_16B(y + at, pack8(a));
-      continue;
-    }
-    float bb[8];
-    unpack8(bv, bb);
-#pragma unroll
-    for (int e = 0; e < 8; ++e) a[e] = round_bf16(a[e] + bb[e]);
-    if (kMode == kRowsPlain) {
-      float rr[8];
-      unpack8(res, rr);
-      if (epilogue & DLI_EPI_GELU_NEW) {
-#pragma unroll
-        for (int e = 0; e < 8; ++e) a[e] = round_bf16(gelu_new_f(a[e]));
-      }
-#pragma unroll
-      for (int e = 0; e < 8; ++e) a[e] += rr[e];
-      st_16B(y + at, pack8(a));
-    } else {
-      unpack8(bv2, bb);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) b[e] = round_bf16(b[e] + bb[e]);
-      const int head = hd == 64 ? n_tile * 2 + (g >> 2) : n_tile;  // q heads, then k heads, then v heads
-      const int i = hd == 64 ? (g & 3) * 8 : g * 8;                // element of the head's first half
-      const int pos = rope.positions[m];
-      if (rope.cos_t && head < rope.H + rope.KV) {
-        float cs[8], sn[8];
-        unpack8(ld_16B(rope.cos_t + (size_t)pos * half + i), cs);
-        unpack8(ld_16B(rope.sin_t + (size_t)pos * half + i), sn);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          const float x1 = a[e], x2 = b[e];
-          a[e] = round_bf16(x1 * cs[e]) + round_bf16(-x2 * sn[e]);
-          b[e] = round_bf16(x2 * cs[e]) + round_bf16(x1 * sn[e]);
+      for (int q = 0; q < kBatch; ++q) {
+        const int m = m0 + col0 + (id0 + q * kRowsThreads) / kGroups;
+        const bool on = id0 + q * kRowsThreads < items;
+        pre1[q] = pre2[q] = make_uint4(0u, 0u, 0u, 0u);
+        pos[q] = page[q] = 0;
+        if (kMode == kRowsPlain && on && (epilogue & DLI_EPI_RESIDUAL)) pre1[q] = ld_16B(residual + (size_t)m * n_out + n);
+        if (kMode == kRowsRope && on) {
+          pos[q] = rope.positions[m];
+          if (head >= rope.H) page[q] = rope.seq_ids[m];
         }
       }
-      const uint4 u1 = pack8(a), u2 = pack8(b);
-      st_16B(y + at, u1);
-      st_16B(y + at + half, u2);
-      if (head >= rope.H) {
-        const bool is_k = head < rope.H + rope.KV;
-        const int kvh = head - rope.H - (is_k ? 0 : rope.KV);
-        const int page = rope.page_table[(size_t)rope.seq_ids[m] * rope.max_pages + (pos >> rope.page_shift)];
-        const size_t row = (((size_t)page * rope.KV + kvh) << rope.page_shift) + (pos & ((1 << rope.page_shift) - 1));
-        bf16* dst = (is_k ? rope.k_cache : rope.v_cache) + row * hd + i;
-        st_16B(dst, u1);
-        st_16B(dst + half, u2);
+      if (kMode == kRowsRope) {
+#pragma unroll
+        for (int q = 0; q < kBatch; ++q) {
+          if (id0 + q * kRowsThreads >= items) continue;
+          if (turned) {
+            pre1[q] = ld_16B(rope.cos_t + (size_t)pos[q] * half + he);
+            pre2[q] = ld_16B(rope.sin_t + (size_t)pos[q] * half + he);
+          }
+          if (head >= rope.H) page[q] = rope.page_table[(size_t)page[q] * rope.max_pages + (pos[q] >> rope.page_shift)];
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < kBatch; ++q) {
+        const int id = id0 + q * kRowsThreads;
+        if (id >= items) continue;
+        const int c = id / kGroups;
+        const size_t at = (size_t)(m0 + col0 + c) * n_out + n;
+        float a[8], b[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) a[e] = 0.f, b[e] = 0.f;
+        for (int sp = 0; sp < splits; ++sp) {  // in split order: deterministic
+          const float4* p = reinterpret_cast<const float4*>(sums + (size_t)(sp * per + c) * 128 + r0);
+          const float4 u = p[0], v = p[1];
+          a[0] += u.x; a[1] += u.y; a[2] += u.z; a[3] += u.w;
+          a[4] += v.x; a[5] += v.y; a[6] += v.z; a[7] += v.w;
+          if (kMode != kRowsPlain) {
+            const float4 u2 = p[r1 / 4], v2 = p[r1 / 4 + 1];
+            b[0] += u2.x; b[1] += u2.y; b[2] += u2.z; b[3] += u2.w;
+            b[4] += v2.x; b[5] += v2.y; b[6] += v2.z; b[7] += v2.w;
+          }
+        }
+        if (kGated) {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) a[e] = round_bf16(a[e]), b[e] = round_bf16(b[e]);
+          gated_combine_n(a, b, reinterpret_cast<const float*>(bias));
+          st_16B(y + at, pack8(a));
+          continue;
+        }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) a[e] = round_bf16(a[e] + bb[e]);
+        if (kMode == kRowsPlain) {
+          float rr[8];
+          unpack8(pre1[q], rr);
+          if (epilogue & DLI_EPI_GELU_NEW) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) a[e] = round_bf16(gelu_new_f(a[e]));
+          }
+#pragma unroll
+          for (int e = 0; e < 8; ++e) a[e] += rr[e];
+          st_16B(y + at, pack8(a));
+        } else {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) b[e] = round_bf16(b[e] + bb2[e]);
+          if (turned) {
+            float cs[8], sn[8];
+            unpack8(pre1[q], cs);
+            unpack8(pre2[q], sn);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              const float x1 = a[e], x2 = b[e];
+              a[e] = round_bf16(x1 * cs[e]) + round_bf16(-x2 * sn[e]);
+              b[e] = round_bf16(x2 * cs[e]) + round_bf16(x1 * sn[e]);
+            }
+          }
+          const uint4 u1 = pack8(a), u2 = pack8(b);
+          st_16B(y + at, u1);
+          st_16B(y + at + half, u2);
+          if (head >= rope.H) {
+            const bool is_k = head < rope.H + rope.KV;
+            const int kvh = head - rope.H - (is_k ? 0 : rope.KV);
+            const size_t row = (((size_t)page[q] * rope.KV + kvh) << rope.page_shift) + (pos[q] & ((1 << rope.page_shift) - 1));
+            bf16* dst = (is_k ? rope.k_cache : rope.v_cache) + row * hd + he;
+            st_16B(dst, u1);
+            st_16B(dst + half, u2);
+          }
+        }
       }
     }
   }
