@@ -380,8 +380,15 @@ static double rows_cost(int M, int N, int K, const RowsShape& sh, const int* cap
   const long long waves = (ctas + at_once - 1) / at_once, rest = ctas - (waves - 1) * at_once;
   const long long last = (rest + cap[sh.splits] - 1) / cap[sh.splits];
   const double rounds = (double)(waves - 1) * r + (double)(last < r ? last : r);
-  const double mma = rounds * kbp * (0.104 + 0.00127 * sh.bn), chain = (double)waves * kbp * 0.234;
-  const double mem = (double)N * K * 2 / 5.54e6;
+  double mma = rounds * kbp * (0.104 + 0.00127 * sh.bn);
+  // One CTA on an SM: nothing hides its epilogue, and a ring meant for two leaves the feed short.  4096 x 14336 at 301 rows in
+  // 160-row tiles, 2 splits: 50.6 us with 3 stages, 40.0 with 6, 4 splits (two CTAs per SM) 39.3; 6144 x 4096 at 301 rows,
+  // 112-row tiles: 28.9 (1 split, 3 stages), 24.6 (7 stages), 21.3 (2 splits).
+  if (ctas <= cap[sh.splits]) mma *= (size_t)sh.stages * (128 + sh.bn) * kBlockK * 2 >= 160 * 1024 ? 1.12 : 1.35;
+  const double chain = (double)waves * kbp * 0.234;
+  double mem = (double)N * K * 2 / 5.54e6;
+  // fewer than ~240 CTAs ask for less than HBM delivers: 4096 x 14336 at 24 rows 25.8 us with 96 CTAs, 22.5 with 256
+  if (ctas < 240) mem *= 1.0 + 0.2 * (double)(240 - ctas) / 240.0;
   double t = mma > chain ? mma : chain;
   if (mem > t) t = mem;
   return t + 2.55 + 0.0323 * sh.bn + 5.0 * (double)(waves - 1);
