@@ -260,23 +260,12 @@ gemm_prefill_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             }
           }
         }
-      } else {
-      const int h = (warp - 2) >> 2;  // warps 2-5: rows 0-127 of the tile, warps 6-9 (MT = 2): rows 128-255
-      const uint32_t lane_base = tmem_base + as * Cfg::kAccCols + h * BN + ((uint32_t)(quad * 32) << 16);
-      const int m = m_blk * kMRows + h * 128 + quad * 32 + lane;
-      // the residual runs a chunk of 16 columns ahead: its latency under the chunk before it, not in front of its own
-      const bool with_res = !kGated && (epilogue & DLI_EPI_RESIDUAL) && m < M;
-      uint4 ahead[2];
-      auto ask = [&](int n0) {
-#pragma unroll
-        for (int h2 = 0; h2 < 2; ++h2)
-          ahead[h2] = with_res && n0 + h2 * 8 < n_out ? ld_16B(residual + (size_t)m * n_out + n0 + h2 * 8) : make_uint4(0u, 0u, 0u, 0u);
-      };
-      ask(n_tile0);
+      } else
 #pragma unroll 1
       for (int c0 = 0; c0 < Cfg::kOutCols; c0 += 16) {
-        const uint4 res[2] = {ahead[0], ahead[1]};
-        if (c0 + 16 < Cfg::kOutCols) ask(n_tile0 + c0 + 16);
+        const int h = (warp - 2) >> 2;  // warps 2-5: rows 0-127 of the tile, warps 6-9 (MT = 2): rows 128-255
+        const uint32_t lane_base = tmem_base + as * Cfg::kAccCols + h * BN + ((uint32_t)(quad * 32) << 16);
+        const int m = m_blk * kMRows + h * 128 + quad * 32 + lane;
         uint32_t r[16], r2[16];
         tmem_ld_32x16(lane_base + c0, r);
         if (kGated) tmem_ld_32x16(lane_base + 128 + c0, r2);
@@ -307,9 +296,9 @@ gemm_prefill_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             if (n0 + h * 8 < n_out) {
-              if (with_res) {
+              if (!kGated && (epilogue & DLI_EPI_RESIDUAL)) {
                 float rr[8];
-                unpack8(res[h], rr);
+                unpack8(ld_16B(residual + (size_t)m * n_out + n0 + h * 8), rr);
 #pragma unroll
                 for (int j = 0; j < 8; ++j) v[h * 8 + j] += rr[j];
               }
@@ -317,7 +306,6 @@ gemm_prefill_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             }
           }
         }
-      }
       }
       // this warp is done reading the accumulator stage: hand it back to the MMA warp
       tcgen05_fence_before();
