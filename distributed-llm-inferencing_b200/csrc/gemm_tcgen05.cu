@@ -190,6 +190,11 @@ gemm_prefill_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       mbar_wait(tfull_bar + 8 * as, Cfg::kAccStages == 2 ? ((tl >> 1) & 1) : (tl & 1));
       tcgen05_fence_after();
       const int n_tile0 = n_blk * Cfg::kOutCols;
+      // The residual comes a 128-byte line of the row at a time, all of it before the line's first store: its latency is waited
+      // for once per 64 columns, and no load meets a store to its own line.  Tiles of 256 and 240 columns, residual = y, us:
+      // 4096 x 4096 at 4 096 rows 127 -> 119, 2048 x 5632 at 1 777 rows 42 -> 35, 4096 x 4096 at 1 024 rows 37 -> 29 (loaded
+      // per 16 columns before).  A chunk of 16 columns ahead instead: 127 -> 198, the store and the load share the line.
+      constexpr int kLine = kGated ? 16 : 64;
       const int n_out = kGated ? N / 2 : N;
       if constexpr (kRope) {
         const uint32_t lane_base = tmem_base + as * Cfg::kAccCols + ((uint32_t)(quad * 32) << 16);
@@ -260,12 +265,22 @@ gemm_prefill_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             }
           }
         }
-      } else
+      } else {
+      const int h = (warp - 2) >> 2;  // warps 2-5: rows 0-127 of the tile, warps 6-9 (MT = 2): rows 128-255
+      const uint32_t lane_base = tmem_base + as * Cfg::kAccCols + h * BN + ((uint32_t)(quad * 32) << 16);
+      const int m = m_blk * kMRows + h * 128 + quad * 32 + lane;
+      const bool with_res = !kGated && (epilogue & DLI_EPI_RESIDUAL) && m < M;
 #pragma unroll 1
-      for (int c0 = 0; c0 < Cfg::kOutCols; c0 += 16) {
-        const int h = (warp - 2) >> 2;  // warps 2-5: rows 0-127 of the tile, warps 6-9 (MT = 2): rows 128-255
-        const uint32_t lane_base = tmem_base + as * Cfg::kAccCols + h * BN + ((uint32_t)(quad * 32) << 16);
-        const int m = m_blk * kMRows + h * 128 + quad * 32 + lane;
+      for (int cb = 0; cb < Cfg::kOutCols; cb += kLine) {
+      uint4 res[kLine / 8];
+#pragma unroll
+      for (int i = 0; i < kLine / 8; ++i)
+        res[i] = with_res && cb + i * 8 < Cfg::kOutCols && n_tile0 + cb + i * 8 < n_out ? ld_16B(residual + (size_t)m * n_out + n_tile0 + cb + i * 8)
+                                                          : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+      for (int ci = 0; ci < kLine / 16; ++ci) {
+        const int c0 = cb + ci * 16;
+        if (Cfg::kOutCols % kLine != 0 && c0 >= Cfg::kOutCols) break;
         uint32_t r[16], r2[16];
         tmem_ld_32x16(lane_base + c0, r);
         if (kGated) tmem_ld_32x16(lane_base + 128 + c0, r2);
@@ -296,9 +311,9 @@ gemm_prefill_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             if (n0 + h * 8 < n_out) {
-              if (!kGated && (epilogue & DLI_EPI_RESIDUAL)) {
+              if (with_res) {
                 float rr[8];
-                unpack8(ld_16B(residual + (size_t)m * n_out + n0 + h * 8), rr);
+                unpack8(res[ci * 2 + h], rr);
 #pragma unroll
                 for (int j = 0; j < 8; ++j) v[h * 8 + j] += rr[j];
               }
@@ -306,6 +321,8 @@ gemm_prefill_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             }
           }
         }
+      }
+      }
       }
       // this warp is done reading the accumulator stage: hand it back to the MMA warp
       tcgen05_fence_before();

@@ -87,3 +87,17 @@ def test_qkv_projection_with_rope_equals_the_separate_steps(cuda, rows, H, KV, K
             ops.rope_kv_append(qkv, cos, sin, positions, seq_ids, table, k, v, H, KV, hd)
         out.append((qkv, k, v))
     assert all(torch.equal(a, b) for a, b in zip(*out))
+
+
+@pytest.mark.parametrize("M", [300, 1024, 1777])
+@pytest.mark.parametrize("N,K", [(72, 512), (240, 768), (488, 1024), (2048, 2048), (4096, 512)])
+def test_residual_read_by_the_line(cuda, M, N, K):
+    """The persistent tiles (all widths, a last tile cut in a line): the residual added, also where it is the output."""
+    from dli_b200 import ops
+    g, x, w, acc, slack = _inputs(M, N, K, M + N)
+    r = torch.randn(M, N, device="cuda", generator=g).to(BF)
+    y = ops.linear(x, w, residual=r)
+    _within(y, acc + r.double(), slack + HALF_ULP * (acc.abs() + slack) + HALF_ULP * (acc + r.double()).abs() * 1.01)
+    z = r.clone()
+    ops.linear(x, w, residual=z, out=z)
+    assert torch.equal(y, z)
