@@ -266,63 +266,63 @@ gemm_prefill_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
           }
         }
       } else {
-      const int h = (warp - 2) >> 2;  // warps 2-5: rows 0-127 of the tile, warps 6-9 (MT = 2): rows 128-255
-      const uint32_t lane_base = tmem_base + as * Cfg::kAccCols + h * BN + ((uint32_t)(quad * 32) << 16);
-      const int m = m_blk * kMRows + h * 128 + quad * 32 + lane;
-      const bool with_res = !kGated && (epilogue & DLI_EPI_RESIDUAL) && m < M;
+        const int h = (warp - 2) >> 2;  // warps 2-5: rows 0-127 of the tile, warps 6-9 (MT = 2): rows 128-255
+        const uint32_t lane_base = tmem_base + as * Cfg::kAccCols + h * BN + ((uint32_t)(quad * 32) << 16);
+        const int m = m_blk * kMRows + h * 128 + quad * 32 + lane;
+        const bool with_res = !kGated && (epilogue & DLI_EPI_RESIDUAL) && m < M;
 #pragma unroll 1
-      for (int cb = 0; cb < Cfg::kOutCols; cb += kLine) {
-      uint4 res[kLine / 8];
+        for (int cb = 0; cb < Cfg::kOutCols; cb += kLine) {
+          uint4 res[kLine / 8];
 #pragma unroll
-      for (int i = 0; i < kLine / 8; ++i)
-        res[i] = with_res && cb + i * 8 < Cfg::kOutCols && n_tile0 + cb + i * 8 < n_out ? ld_16B(residual + (size_t)m * n_out + n_tile0 + cb + i * 8)
-                                                          : make_uint4(0u, 0u, 0u, 0u);
+          for (int i = 0; i < kLine / 8; ++i)
+            res[i] = with_res && cb + i * 8 < Cfg::kOutCols && n_tile0 + cb + i * 8 < n_out
+                         ? ld_16B(residual + (size_t)m * n_out + n_tile0 + cb + i * 8) : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
-      for (int ci = 0; ci < kLine / 16; ++ci) {
-        const int c0 = cb + ci * 16;
-        if (Cfg::kOutCols % kLine != 0 && c0 >= Cfg::kOutCols) break;
-        uint32_t r[16], r2[16];
-        tmem_ld_32x16(lane_base + c0, r);
-        if (kGated) tmem_ld_32x16(lane_base + 128 + c0, r2);
-        tmem_ld_wait();
-        const int n0 = n_tile0 + c0;
-        if (m < M && n0 < n_out) {
-          float v[16];
+          for (int ci = 0; ci < kLine / 16; ++ci) {
+            const int c0 = cb + ci * 16;
+            if (Cfg::kOutCols % kLine != 0 && c0 >= Cfg::kOutCols) break;
+            uint32_t r[16], r2[16];
+            tmem_ld_32x16(lane_base + c0, r);
+            if (kGated) tmem_ld_32x16(lane_base + 128 + c0, r2);
+            tmem_ld_wait();
+            const int n0 = n_tile0 + c0;
+            if (m < M && n0 < n_out) {
+              float v[16];
 #pragma unroll
-          for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
-          if (kGated) {
-            float up[16];
+              for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
+              if (kGated) {
+                float up[16];
 #pragma unroll
-            for (int j = 0; j < 16; ++j) { v[j] = round_bf16(v[j]); up[j] = round_bf16(__uint_as_float(r2[j])); }
-            gated_combine_n(v, up, reinterpret_cast<const float*>(bias));
-          } else {
-            if (epilogue & DLI_EPI_BIAS) {
+                for (int j = 0; j < 16; ++j) { v[j] = round_bf16(v[j]); up[j] = round_bf16(__uint_as_float(r2[j])); }
+                gated_combine_n(v, up, reinterpret_cast<const float*>(bias));
+              } else {
+                if (epilogue & DLI_EPI_BIAS) {
 #pragma unroll
-              for (int j = 0; j < 16; ++j) v[j] += (n0 + j < N) ? __bfloat162float(bias[n0 + j]) : 0.f;
-            }
+                  for (int j = 0; j < 16; ++j) v[j] += (n0 + j < N) ? __bfloat162float(bias[n0 + j]) : 0.f;
+                }
 #pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] = round_bf16(v[j]);
-            if (epilogue & DLI_EPI_GELU_NEW) {
+                for (int j = 0; j < 16; ++j) v[j] = round_bf16(v[j]);
+                if (epilogue & DLI_EPI_GELU_NEW) {
 #pragma unroll
-              for (int j = 0; j < 16; ++j) v[j] = round_bf16(gelu_new_f(v[j]));
-            }
-          }
-          bf16* dst = y + (size_t)m * n_out + n0;
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            if (n0 + h * 8 < n_out) {
-              if (with_res) {
-                float rr[8];
-                unpack8(res[ci * 2 + h], rr);
-#pragma unroll
-                for (int j = 0; j < 8; ++j) v[h * 8 + j] += rr[j];
+                  for (int j = 0; j < 16; ++j) v[j] = round_bf16(gelu_new_f(v[j]));
+                }
               }
-              st_16B(dst + h * 8, pack8(v + h * 8));
+              bf16* dst = y + (size_t)m * n_out + n0;
+#pragma unroll
+              for (int h = 0; h < 2; ++h) {
+                if (n0 + h * 8 < n_out) {
+                  if (with_res) {
+                    float rr[8];
+                    unpack8(res[ci * 2 + h], rr);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) v[h * 8 + j] += rr[j];
+                  }
+                  st_16B(dst + h * 8, pack8(v + h * 8));
+                }
+              }
             }
           }
         }
-      }
-      }
       }
       // this warp is done reading the accumulator stage: hand it back to the MMA warp
       tcgen05_fence_before();
