@@ -399,34 +399,45 @@ template <typename E>
 __global__ void __launch_bounds__(1024)
 postnorm_add_norm_conv_single_kernel(const E* __restrict__ y, float* __restrict__ x, float* __restrict__ tail,
                                      const float* __restrict__ w, const int32_t* __restrict__ ent, E* __restrict__ out,
-                                     int d, int taps, float eps, float g_post, float g_next) {
+                                     int d, int taps, float eps, float g_post, float g_next, int ahead) {
   __shared__ float red[32];
   const int row = blockIdx.x;
   const size_t o = (size_t)row * d;
   float s2 = 0.f;
   constexpr int kHeld = 4, kTaps = 4;
   if (taps <= kTaps && d <= kHeld * (int)blockDim.x) {
-    // Everything a thread's channels need in registers, and what the kernel just before this one did not write — the
-    // weights and the slot's tail; with a post-norm also the row of x, whose last writer is two kernels back — asked
-    // for before the dependency wait (every kernel of the library waits for its predecessor before it lets its
-    // successor start).  After it only y is left.  The sums are those of the general form below.
+    // Everything a thread's channels need in registers, asked for together.  Before the dependency wait only the weights, which
+    // no kernel writes; with `ahead` also the slots, their tails and (with a post-norm) the row of x, for a caller whose
+    // launch just before this one writes none of them (the writer two launches back is complete by then: every kernel of
+    // the library waits for its predecessor before it lets its successor start).  After the wait only y is left then.
+    // The sums are those of the general form below.
     // Latency-bound: three rows of 2048 7.5 -> 6.0 us without the overlap, 0.2 ms of a 2.9 ms pass with it.
-    const int4 e = reinterpret_cast<const int4*>(ent)[row];
     const int keep = taps - 1;
     float xv[kHeld], tv[kHeld][kTaps - 1], wv[kHeld][kTaps];
 #pragma unroll
     for (int i = 0; i < kHeld; ++i) {
       const int c = threadIdx.x + i * blockDim.x;
-      const bool on = c < d;
 #pragma unroll
-      for (int j = 0; j < kTaps; ++j) wv[i][j] = on && j < taps ? w[(size_t)c * taps + j] : 0.f;
+      for (int j = 0; j < kTaps; ++j) wv[i][j] = c < d && j < taps ? w[(size_t)c * taps + j] : 0.f;
+    }
+    if (!ahead) {
+      pdl_wait();
+      pdl_trigger();
+    }
+    const int4 e = reinterpret_cast<const int4*>(ent)[row];
+#pragma unroll
+    for (int i = 0; i < kHeld; ++i) {
+      const int c = threadIdx.x + i * blockDim.x;
+      const bool on = c < d;
 #pragma unroll
       for (int j = 0; j < kTaps - 1; ++j)
         tv[i][j] = on && j < keep && e.w - keep + j >= 0 ? tail[((size_t)e.x * keep + j) * d + c] : 0.f;
       xv[i] = on && y != nullptr ? x[o + c] : 0.f;
     }
-    pdl_wait();
-    pdl_trigger();
+    if (ahead) {
+      pdl_wait();
+      pdl_trigger();
+    }
     if (y != nullptr) {
       float yv[kHeld], ss = 0.f;
 #pragma unroll
@@ -901,17 +912,29 @@ int dli_causal_conv_ragged(const float* h, float* tail, const float* w, const in
   return DLI_OK;
 }
 
-int dli_postnorm_add_norm_conv_single(const void* y, float* x, float* tail, const float* w, const int32_t* ent, void* out,
-                                      int rows, int d, int taps, float eps, float g_post, float g_next, int dt,
-                                      dli_stream_t stream) {
+static int postnorm_add_norm_conv_single(const void* y, float* x, float* tail, const float* w, const int32_t* ent, void* out,
+                                         int rows, int d, int taps, float eps, float g_post, float g_next, int dt, int ahead,
+                                         dli_stream_t stream) {
   DLI_CHECK_ARG(x && w && ent && out && d > 0 && taps >= 1 && (tail || taps == 1), "dli_postnorm_add_norm_conv_single: null pointer or empty shape");
   DLI_CHECK_ARG((reinterpret_cast<uintptr_t>(ent) & 15u) == 0, "dli_postnorm_add_norm_conv_single: ent must be 16-byte aligned");
   DT_CHECK(dt);
   if (rows <= 0) return DLI_OK;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (dt == 0) DLI_LAUNCH("postnorm_add_norm_conv_single", postnorm_add_norm_conv_single_kernel<bf16>, dim3(rows), dim3(row_threads(rows, d)), 0, s, (const bf16*)y, x, tail, w, ent, (bf16*)out, d, taps, eps, g_post, g_next);
-  else DLI_LAUNCH("postnorm_add_norm_conv_single", postnorm_add_norm_conv_single_kernel<float>, dim3(rows), dim3(row_threads(rows, d)), 0, s, (const float*)y, x, tail, w, ent, (float*)out, d, taps, eps, g_post, g_next);
+  if (dt == 0) DLI_LAUNCH("postnorm_add_norm_conv_single", postnorm_add_norm_conv_single_kernel<bf16>, dim3(rows), dim3(row_threads(rows, d)), 0, s, (const bf16*)y, x, tail, w, ent, (bf16*)out, d, taps, eps, g_post, g_next, ahead);
+  else DLI_LAUNCH("postnorm_add_norm_conv_single", postnorm_add_norm_conv_single_kernel<float>, dim3(rows), dim3(row_threads(rows, d)), 0, s, (const float*)y, x, tail, w, ent, (float*)out, d, taps, eps, g_post, g_next, ahead);
   return DLI_OK;
+}
+
+int dli_postnorm_add_norm_conv_single(const void* y, float* x, float* tail, const float* w, const int32_t* ent, void* out,
+                                      int rows, int d, int taps, float eps, float g_post, float g_next, int dt,
+                                      dli_stream_t stream) {
+  return postnorm_add_norm_conv_single(y, x, tail, w, ent, out, rows, d, taps, eps, g_post, g_next, dt, 0, stream);
+}
+
+int dli_postnorm_add_norm_conv_single_ahead(const void* y, float* x, float* tail, const float* w, const int32_t* ent,
+                                            void* out, int rows, int d, int taps, float eps, float g_post, float g_next,
+                                            int dt, dli_stream_t stream) {
+  return postnorm_add_norm_conv_single(y, x, tail, w, ent, out, rows, d, taps, eps, g_post, g_next, dt, 1, stream);
 }
 
 int dli_gather_cast(const float* src, const int32_t* rows, void* out, int n, int d, int dt, dli_stream_t stream) {

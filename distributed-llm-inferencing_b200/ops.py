@@ -748,14 +748,15 @@ def mlstm_ragged_parallel(proj, o_scratch, out, ent, tiles, scratch, H, D, V, q_
     return out
 
 
-def postnorm_add_norm_conv_single(y, x, tail, w, ent, out, g_post: float, g_next: float, eps: float):
+def postnorm_add_norm_conv_single(y, x, tail, w, ent, out, g_post: float, g_next: float, eps: float, ahead: bool = False):
     """Decode rows (one per entry): x += y / rms(y) * g_post (skipped when y is None), h = x / rms(x) * g_next,
     out = h + conv(h) with the slot's tail shifted — postnorm_add_norm and the next sublayer's causal_conv_ragged
-    as one kernel."""
+    as one kernel.  ahead: the launch just before this one writes none of ent, tail and (with y) x, which may then be
+    read while it still runs."""
     _f32(x, tail, w), _i32(ent), _req(out, out.dtype)
     if y is not None:
         _req(y, out.dtype)
-    _call("dli_postnorm_add_norm_conv_single", 1, _p(y), _p(x), _p(tail), _p(w), _p(ent), _p(out), x.shape[0], x.shape[1],
+    _call("dli_postnorm_add_norm_conv_single" + ("_ahead" if ahead else ""), 1, _p(y), _p(x), _p(tail), _p(w), _p(ent), _p(out), x.shape[0], x.shape[1],
           w.shape[1], float(eps), float(g_post), float(g_next), _dt(out), _stream())
     return out
 

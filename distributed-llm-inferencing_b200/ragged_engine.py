@@ -814,7 +814,9 @@ class RaggedEngine:
             """Close the previous sublayer (x += postnorm(y_prev)) and open the next one: hc = its normed and convolved
             input.  One kernel for decode rows, norm kernel + convolution (+ tail shift) otherwise."""
             if single:
-                ops.postnorm_add_norm_conv_single(y_prev, x, tail, taps_w, d_ent, hc, g_post, g_next, s.eps)
+                # the launch before it is the projection that wrote y_prev, or (no y_prev) one that may write x: never the
+                # entries or this tail, and with y_prev not x
+                ops.postnorm_add_norm_conv_single(y_prev, x, tail, taps_w, d_ent, hc, g_post, g_next, s.eps, ahead=True)
                 return
             if y_prev is None:
                 ops.scalar_rmsnorm(x, g_next, s.eps, hn)

@@ -479,6 +479,11 @@ int dli_causal_conv_ragged(const float* h, float* tail, const float* w, const in
 int dli_postnorm_add_norm_conv_single(const void* y, float* x, float* tail, const float* w, const int32_t* ent, void* out,
                                       int rows, int d, int taps, float eps, float g_post, float g_next, int dt,
                                       dli_stream_t stream);
+/* The same for callers that know their launch order: under programmatic dependent launch it reads ent, tail and (with y) x
+ * while the launch just before it on the stream may still run, so that launch must write none of the three. */
+int dli_postnorm_add_norm_conv_single_ahead(const void* y, float* x, float* tail, const float* w, const int32_t* ent,
+                                            void* out, int rows, int d, int taps, float eps, float g_post, float g_next,
+                                            int dt, dli_stream_t stream);
 int dli_gather_cast(const float* src, const int32_t* rows, void* out, int n, int d, int dt, dli_stream_t stream);
 /* y[M,N] = x[M,K] . w[N,K]^T on the CUDA cores with fp32 accumulation: any shape, both element types. */
 int dli_linear_any(const void* x, const void* w, void* y, int M, int N, int K, int ldx, int ldy, int dt,
