@@ -81,12 +81,14 @@ __device__ __forceinline__ uint32_t cluster_add(uint32_t addr, uint32_t v) {
   asm volatile("atom.shared::cluster.add.u32 %0, [%1], %2;" : "=r"(old) : "r"(addr), "r"(v) : "memory");
   return old;
 }
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  cluster_arrive();
+  cluster_wait();
 }
 
-// Larger of the two 16-bit halves' keys, and the keys of a vector's elements.
+// Element e of a vector's eight, as raw bits.
 __device__ __forceinline__ uint32_t vec_elem(const uint4& u, int e) {
   const uint32_t w = e < 2 ? u.x : e < 4 ? u.y : e < 6 ? u.z : u.w;
   return (e & 1) ? w >> 16 : w & 0xffffu;
@@ -184,9 +186,11 @@ sample_kernel(const bf16* __restrict__ logits, int ld, int32_t* __restrict__ out
   uint32_t bound = 0;
   const bool narrow = k <= kSampleThreads;
   if (narrow) {
+    cluster_arrive();
 #pragma unroll 1
     for (uint32_t bit = 0x8000u; bit; bit >>= 1)
       if (__syncthreads_count(top >= (bound | bit)) >= k) bound |= bit;
+    cluster_wait();  // every CTA of the cluster runs: from here on its shared memory may be written
     if (tid < ctas) cluster_st(cluster_addr(&bounds[rank], tid), bound);
     cluster_sync_all();
     for (int c = 0; c < ctas; ++c) bound = max(bound, bounds[c]);

@@ -105,3 +105,23 @@ def test_rows_keep_their_draws_in_any_batch(cuda):
         one = torch.full((1,), -5, dtype=torch.int32, device=cuda)
         ops.sample_rows(x[b:b + 1], one, seeds[b:b + 1], steps[b:b + 1], mask[b:b + 1])
         assert int(one) == int(out[b])
+
+
+@pytest.mark.parametrize("V", [16400, 50257, 128256])
+def test_ctas_of_a_row_that_start_apart(cuda, V):
+    """The CTAs of a cluster write into each other's shared memory: the same kept sets and tokens on a device whose SMs free up
+    one by one (another stream keeps them busy with kernels of uneven length)."""
+    from dli_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(V)
+    x = (2.5 * torch.randn(40, V, device=cuda, generator=g)).to(BF)
+    seed = torch.tensor([5], dtype=torch.int64, device=cuda)
+    want = ops.sample(x, seed=seed, debug_cap=64)
+    other, load = torch.cuda.Stream(), [torch.randn(n, n, device=cuda) for n in (300, 900, 1700)]
+    torch.cuda.synchronize()
+    for _ in range(10):
+        with torch.cuda.stream(other):
+            for m in load:
+                m @ m
+        got = [ops.sample(x, seed=seed, debug_cap=64) for _ in range(4)]
+        assert all(torch.equal(a, b) for r in got for a, b in zip(r, want))
