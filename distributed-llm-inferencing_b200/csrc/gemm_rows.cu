@@ -213,12 +213,21 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     float bb[8], bb2[8];
     {
       uint4 bv = make_uint4(0u, 0u, 0u, 0u), bv2 = bv;
-      if (!kGated && (epilogue & DLI_EPI_BIAS)) {
+      const bool biased = !kGated && (epilogue & DLI_EPI_BIAS);
+      const bool whole = (reinterpret_cast<uintptr_t>(bias) & 15u) == 0;
+      if (biased && whole) {
         bv = ld_16B(bias + n);
         if (kMode == kRowsRope) bv2 = ld_16B(bias + n + half);
       }
       unpack8(bv, bb);
       unpack8(bv2, bb2);
+      if (biased && !whole) {  // a slice of a longer vector may start anywhere
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          bb[e] = __bfloat162float(bias[n + e]);
+          if (kMode == kRowsRope) bb2[e] = __bfloat162float(bias[n + half + e]);
+        }
+      }
     }
     const int head = hd == 64 ? n_tile * 2 + (g >> 2) : n_tile;  // kRowsRope: q heads, then k heads, then v heads
     const int he = hd == 64 ? (g & 3) * 8 : g * 8;               // element of the head's first half

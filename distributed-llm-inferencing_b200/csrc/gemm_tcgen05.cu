@@ -407,8 +407,7 @@ int linear_qkv_append(const void* x, const void* w, const void* bias, void* qkv,
                       cudaStream_t s, int* launches) {
   const int N = (rope.H + 2 * rope.KV) * hd;
   *launches += 1;
-  if (M > 2 && K % 64 == 0 && aligned16(x) && aligned16(w) && aligned16(qkv) && aligned16(bias) && aligned16(rope.k_cache) &&
-      aligned16(rope.v_cache)) {
+  if (M > 2 && K % 64 == 0 && aligned16(x) && aligned16(w) && aligned16(qkv) && aligned16(rope.k_cache) && aligned16(rope.v_cache)) {
     RowsShape sh;
     int rc;
     if (use_rows(M, N, K, false, &sh, &rc))

@@ -101,3 +101,19 @@ def test_residual_read_by_the_line(cuda, M, N, K):
     z = r.clone()
     ops.linear(x, w, residual=z, out=z)
     assert torch.equal(y, z)
+
+
+@pytest.mark.parametrize("off", [1, 2, 4, 7])
+@pytest.mark.parametrize("M,N,K", [(3, 48, 64), (17, 208, 1088), (128, 768, 768), (200, 2304, 4096), (9, 8192, 4096)])
+def test_bias_that_starts_anywhere(cuda, M, N, K, off):
+    """A slice of a packed bias vector: the same bits as an aligned copy of it, and right against float64."""
+    from dli_b200 import ops
+
+    g, x, w, acc, slack = _inputs(M, N, K, M + N + off)
+    bias = torch.randn(N + 8, device=cuda, generator=g).to(BF)[off:off + N]
+    assert bias.data_ptr() % 16
+    z = acc + bias.double()
+    for call in (ops.gemm, ops.linear, lambda *a, **k: ops.linear_splitk(*a, None, **k)):
+        y = call(x, w, bias=bias)
+        _within(y, z, slack + HALF_ULP * (z.abs() + slack))
+        assert torch.equal(y, call(x, w, bias=bias.clone()))
