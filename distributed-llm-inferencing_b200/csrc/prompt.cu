@@ -63,6 +63,8 @@ int dli_prompt_layers_bf16(const dli_layer_weights* layers, const dli_prompt_pas
   const int rows = p.B * p.T;
   if (rows == 0) return DLI_OK;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (p.n_layers == 0 && p.h_in != p.h)  // no projection writes the result
+    DLI_CUDA_CALL(cudaMemcpyAsync(p.h, p.h_in, (size_t)rows * p.d * sizeof(bf16), cudaMemcpyDeviceToDevice, s));
   RopeArgs ra;
   ra.cos_t = (const bf16*)p.cos;
   ra.sin_t = (const bf16*)p.sin;
