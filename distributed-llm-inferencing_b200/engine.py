@@ -627,10 +627,12 @@ class ShardEngine:
                 ops.embedding(ids, self.w["embed"], out=h, positions=positions, pos_table=self.w["wpe"])
             else:
                 ops.embedding(ids, self.w["embed"], out=h)
-        # later stages: the first layer reads the stage's input where it lies
-        h_in = h if self.is_first else hidden
-        if h_in.shape != h.shape or h_in.dtype != BF or h_in.device != h.device or not h_in.is_contiguous() or \
-                h_in.data_ptr() % 16:
+        # later stages: the first layer reads the stage's input where it lies (in the workspace already, under any shape, or
+        # in a buffer of the caller's; one that overlaps the workspace cannot be read while the layers write there)
+        h_in = h if self.is_first or hidden.data_ptr() == h.data_ptr() else hidden
+        if h_in is not h and (h_in.shape != h.shape or h_in.dtype != BF or h_in.device != h.device or
+                              not h_in.is_contiguous() or h_in.data_ptr() % 16 or
+                              abs(h_in.data_ptr() - h.data_ptr()) < h.nbytes):
             h_in = h.copy_(hidden)
         ops.prompt_layers(self.layers, self.kv.k, self.kv.v, self.kv.page_table, st["page_rows"], h_in, h, self._x[:rows],
                           self._qkv[:rows], self._attn[:rows], self._act[:rows], self.cos, self.sin, positions, seq_ids,

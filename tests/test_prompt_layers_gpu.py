@@ -20,3 +20,48 @@ def test_no_layers_hand_the_input_on(cuda):
         out = ops.prompt_layers([], [], [], table, table, src, h, x, qkv, attn, act, None, None, positions, seq_ids, B, T,
                                 None, H, H, hd, 1e-5, hd ** -0.5)
         assert out is h and torch.equal(h, h_in)
+
+
+@pytest.fixture(scope="module")
+def stages():
+    from dli_b200.engine import ModelSpec, ShardEngine
+    from oracle import decoder_ref as R
+
+    spec = ModelSpec("llama", 3, 256, 4, 2, 64, 512, 512, 1e-5, 10000.0, 0, 128)
+    sd = R.seeded_state_dict(R.ModelSpec(**spec.__dict__), seed=7, std=0.06)
+    first, last = ShardEngine(spec, 0, 0, device="cuda:0", max_batch=2, max_seq_len=64), ShardEngine(
+        spec, 1, 2, device="cuda:0", max_batch=2, max_seq_len=64)
+    for e in (first, last):
+        e.load_state_dict(sd)
+    return first, last
+
+
+def test_hidden_states_in_any_form(cuda, stages):
+    """What a later stage is given: a buffer of its own, strided, unaligned, of another type, or the stage's own workspace
+    under another shape — the same logits; a buffer that overlaps the workspace is refused as a copy of it always was."""
+    first, last = stages
+    B, T, d = 2, 11, 256
+    for e in stages:
+        e.start_batch(B, T, T + 4)
+    ids = torch.randint(0, 512, (B * T,), device=cuda, dtype=torch.int32)
+    hidden = first.prefill(B, T, ids=ids).clone()
+
+    def logits(h):
+        last.prefill(B, T, hidden=h)
+        return last._state(B, 0)["logits"].clone()
+
+    want, kept = logits(hidden), hidden.clone()
+    assert torch.equal(hidden, kept)  # read only
+    flat = torch.empty(B * T * d + 1, device=cuda, dtype=BF)
+    flat[1:] = hidden.view(-1)
+    wide = torch.zeros(B * T, 2 * d, device=cuda, dtype=BF)
+    wide[:, ::2] = hidden
+    forms = [flat[1:].view(B * T, d), wide[:, ::2], hidden.float()]
+    own = last._h[:B * T]
+    for h in forms + [own, own.view(B, T, d)]:
+        if h.data_ptr() == own.data_ptr():
+            own.copy_(hidden)
+        assert torch.equal(logits(h), want)
+    last._workspace(B * T + 1)
+    with pytest.raises(RuntimeError):
+        last.prefill(B, T, hidden=last._h[1:B * T + 1])
