@@ -13,6 +13,7 @@
 // (the earlier chunks and this one, appended by dli_rope_kv_append_bf16 just before) come from the
 // paged KV cache, page by page like the decode kernel does it.  Same arithmetic otherwise.
 #include <stdlib.h>
+#include <string.h>
 
 #include "mma_utils.cuh"
 
@@ -227,16 +228,18 @@ int launch_attn_prefill_tc_paged(const void* qkv, void* out, const void* k_cache
 //                    T = 16 after 512: 10.8 / 10.4, after 6000: 95 / 57
 //   12 heads of 64:  T = 256: 5.3 / 6.8, 400: 7.6 / 8.2, 512: 8.7 / 9.0, 800: 13.5 / 11.5, 1777: 34 / 19
 //   32 heads of 128: T = 19: 3.8 / 5.6, 64: 4.4 / 5.9, 128: 5.7 / 6.4 (eight prompts of 100: 12.0 / 9.9), 301: 11.6 / 7.9
-// DLI_PREFILL_ATTN=mma keeps the mma.sync kernel everywhere.
+// DLI_PREFILL_ATTN=mma, looked up at every call, keeps the mma.sync kernel everywhere.
 static bool prefill_on_tc(int hd, int keys) {
-  static const bool tc = !(getenv("DLI_PREFILL_ATTN") && getenv("DLI_PREFILL_ATTN")[0] == 'm');
+  const char* choice = getenv("DLI_PREFILL_ATTN");
+  const bool tc = !(choice && strcmp(choice, "mma") == 0);
   return tc && (hd == 64 ? keys >= 448 : keys > 64);
 }
 
 }  // namespace dli
 
-extern "C" int dli_attn_prefill_bf16(const void* qkv, void* out, int B, int T, int H, int KV, int hd,
-                                     float scale, int window, dli_stream_t stream) {
+// by_rule: head size 64 may go to the tcgen05 kernel
+static int attn_prefill(const void* qkv, void* out, int B, int T, int H, int KV, int hd, float scale, int window, bool by_rule,
+                        dli_stream_t stream) {
   using namespace dli;
   DLI_CHECK_ARG(qkv && out, "dli_attn_prefill_bf16: null pointer");
   DLI_CHECK_ARG(hd == 64 || hd == 128, "dli_attn_prefill_bf16: hd must be 64 or 128 (got %d)", hd);
@@ -247,8 +250,18 @@ extern "C" int dli_attn_prefill_bf16(const void* qkv, void* out, int B, int T, i
   if (B == 0 || T == 0) return DLI_OK;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (hd == 128) return launch_prefill<128, false>(qkv, out, B, T, H, KV, scale, window, s);
-  if (prefill_on_tc(hd, T)) return launch_attn_prefill_tc(qkv, out, B, T, H, KV, hd, scale, window, s);
+  if (by_rule && prefill_on_tc(hd, T)) return launch_attn_prefill_tc(qkv, out, B, T, H, KV, hd, scale, window, s);
   return launch_prefill<64, false>(qkv, out, B, T, H, KV, scale, window, s);
+}
+
+extern "C" int dli_attn_prefill_bf16(const void* qkv, void* out, int B, int T, int H, int KV, int hd,
+                                     float scale, int window, dli_stream_t stream) {
+  return attn_prefill(qkv, out, B, T, H, KV, hd, scale, window, true, stream);
+}
+
+extern "C" int dli_attn_prefill_mma_bf16(const void* qkv, void* out, int B, int T, int H, int KV, int hd,
+                                         float scale, int window, dli_stream_t stream) {
+  return attn_prefill(qkv, out, B, T, H, KV, hd, scale, window, false, stream);
 }
 
 extern "C" int dli_attn_prefill_paged_bf16(const void* qkv, void* out, const void* k_cache, const void* v_cache,

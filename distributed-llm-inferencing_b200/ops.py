@@ -201,20 +201,16 @@ def _prefill_tensor_core(hd, T) -> bool:
 
 
 def attn_prefill(qkv, out, B, T, H, KV, hd, scale, window=0, tensor_core=None):
-    """Causal prefill attention.  head_dim 128 runs on tcgen05 (dli_attn_prefill_tc_bf16) from 65 tokens, where it
-    overtakes the mma.sync kernel (64 tokens of 32 heads: 5.9 against 4.4 us), unless tensor_core=False or
-    DLI_PREFILL_ATTN=mma; head_dim 64 chooses by the same kind of rule inside dli_attn_prefill_bf16."""
+    """Causal prefill attention.  tensor_core=True: the tcgen05 kernel (head_dim 128), False: the mma.sync kernel, None: by
+    rule — head_dim 128 runs on tcgen05 (dli_attn_prefill_tc_bf16) from 65 tokens, where it overtakes the mma.sync kernel
+    (64 tokens of 32 heads: 5.9 against 4.4 us), head_dim 64 chooses by the same kind of rule inside
+    dli_attn_prefill_bf16, and with DLI_PREFILL_ATTN=mma both stay on mma.sync."""
     global launch_count
     _req(qkv), _req(out)
-    if tensor_core is None:
-        tensor_core = _prefill_tensor_core(hd, T)
-    if tensor_core:
-        _lib.check("dli_attn_prefill_tc_bf16", _lib.load().dli_attn_prefill_tc_bf16(
-            _p(qkv), _p(out), B, T, H, KV, hd, float(scale), window, _stream()))
-        launch_count += 1
-        return out
-    _lib.check("dli_attn_prefill_bf16", _lib.load().dli_attn_prefill_bf16(
-        _p(qkv), _p(out), B, T, H, KV, hd, float(scale), window, _stream()))
+    name = "dli_attn_prefill_mma_bf16" if tensor_core is not None else "dli_attn_prefill_bf16"
+    if tensor_core or (tensor_core is None and _prefill_tensor_core(hd, T)):
+        name = "dli_attn_prefill_tc_bf16"
+    _lib.check(name, getattr(_lib.load(), name)(_p(qkv), _p(out), B, T, H, KV, hd, float(scale), window, _stream()))
     launch_count += 1
     return out
 

@@ -77,3 +77,35 @@ def test_a_sequence_does_not_see_its_neighbour(cuda, hd, T):
     qkv[T:, H * hd:] = float("inf")
     ops.attn_prefill(qkv, both, 2, T, H, KV, hd, hd ** -0.5)
     assert torch.equal(both[:T], alone)
+
+
+@pytest.mark.parametrize("hd,T", [(64, 512), (64, 1777), (128, 130)])
+def test_the_caller_chooses_the_kernel(cuda, monkeypatch, hd, T):
+    """tensor_core=False is the mma.sync kernel at either head size, whatever the rule says, and DLI_PREFILL_ATTN is looked up
+    at every call.  The kernels tile the keys differently, so their bits differ: that tells them apart."""
+    from dli_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(T)
+    H, KV, page = 4, 2, 16
+    n = (T + page - 1) // page
+    qkv = (1.3 * torch.randn(T, (H + 2 * KV) * hd, device=cuda, generator=g)).to(BF)
+    kc, vc = (c.reshape(T, KV, hd) for c in qkv[:, H * hd:].split([KV * hd, KV * hd], dim=1))
+    kc, vc = (torch.nn.functional.pad(c, (0, 0, 0, 0, 0, n * page - T)).view(n, page, KV, hd).transpose(1, 2).contiguous()
+              for c in (kc, vc))
+    table = torch.arange(n, device=cuda).int().view(1, n)
+
+    def whole(choice):
+        return ops.attn_prefill(qkv, torch.empty(T, H * hd, device=cuda, dtype=BF), 1, T, H, KV, hd, hd ** -0.5,
+                                tensor_core=choice).clone()
+
+    def chunk():
+        return ops.attn_prefill_paged(qkv, torch.empty(T, H * hd, device=cuda, dtype=BF), kc, vc, table, 1, T, 0, H, KV, hd,
+                                      hd ** -0.5).clone()
+
+    monkeypatch.delenv("DLI_PREFILL_ATTN", raising=False)
+    by_rule, mma, paged = whole(None), whole(False), chunk()
+    assert not torch.equal(by_rule, mma) and torch.equal(by_rule, paged)
+    monkeypatch.setenv("DLI_PREFILL_ATTN", "mma")
+    assert torch.equal(whole(None), mma) and torch.equal(chunk(), mma)
+    monkeypatch.delenv("DLI_PREFILL_ATTN")
+    assert torch.equal(whole(None), by_rule) and torch.equal(chunk(), paged)
