@@ -30,7 +30,7 @@ class PromptPass(C.Structure):
     """dli_prompt_pass of include/dli.h."""
 
     _fields_ = ([(n, C.c_int) for n in ("n_layers", "B", "T", "prefix", "d", "ff", "H", "KV", "hd", "window", "page_size",
-                                        "max_pages", "num_pages", "tensor_core")] +
+                                        "max_pages", "num_pages", "tensor_core", "split_rope")] +
                 [("eps", C.c_float), ("scale", C.c_float)] +
                 [(n, C.c_void_p) for n in ("h_in", "h", "x", "qkv", "attn", "act", "cos", "sin", "positions", "seq_ids",
                                            "page_table", "page_rows")])

@@ -402,12 +402,14 @@ static bool use_rows(int M, int N, int K, bool gated, RowsShape* shape, int* rc)
 }
 
 // qkv = x w^T (+ bias), q and k rotated, k and v appended to the cache pages: one kernel where a projection kernel has that
-// epilogue, the projection and the rotation kernel otherwise (the same bits).
+// epilogue (and one_kernel), the projection and the rotation kernel otherwise: the same bits where dli_linear_bf16 takes that
+// projection kernel too (3-8 rows of a small matrix go to another one).
 int linear_qkv_append(const void* x, const void* w, const void* bias, void* qkv, int M, int K, const RopeArgs& rope, int hd,
-                      cudaStream_t s, int* launches) {
+                      bool one_kernel, cudaStream_t s, int* launches) {
   const int N = (rope.H + 2 * rope.KV) * hd;
   *launches += 1;
-  if (M > 2 && K % 64 == 0 && aligned16(x) && aligned16(w) && aligned16(qkv) && aligned16(rope.k_cache) && aligned16(rope.v_cache)) {
+  if (one_kernel && M > 2 && K % 64 == 0 && aligned16(x) && aligned16(w) && aligned16(qkv) && aligned16(rope.k_cache) &&
+      aligned16(rope.v_cache)) {
     RowsShape sh;
     int rc;
     if (use_rows(M, N, K, false, &sh, &rc))

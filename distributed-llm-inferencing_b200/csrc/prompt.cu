@@ -10,7 +10,7 @@ namespace dli {
 
 // gemm_tcgen05.cu; *launches grows by the kernels enqueued
 int linear_qkv_append(const void* x, const void* w, const void* bias, void* qkv, int M, int K, const RopeArgs& rope, int hd,
-                      cudaStream_t s, int* launches);
+                      bool one_kernel, cudaStream_t s, int* launches);
 
 __global__ void __launch_bounds__(256)
 prompt_rows_kernel(int32_t* __restrict__ positions, int32_t* __restrict__ seq_ids, int32_t* __restrict__ last_rows, int B,
@@ -99,7 +99,7 @@ int dli_prompt_layers_bf16(const dli_layer_weights* layers, const dli_prompt_pas
     DLI_STEP(norm(res, L.norm1, L.norm1_b));
     ra.k_cache = (bf16*)L.k_cache;
     ra.v_cache = (bf16*)L.v_cache;
-    if ((rc = linear_qkv_append(p.x, L.w_qkv, L.b_qkv, p.qkv, rows, p.d, ra, p.hd, s, &n)) != DLI_OK) return rc;
+    if ((rc = linear_qkv_append(p.x, L.w_qkv, L.b_qkv, p.qkv, rows, p.d, ra, p.hd, !p.split_rope, s, &n)) != DLI_OK) return rc;
     if (p.prefix >= 0)  // a chunk at positions prefix ..: keys and values from the paged cache
       DLI_STEP(dli_attn_prefill_paged_bf16(p.qkv, p.attn, L.k_cache, L.v_cache, p.page_rows, p.max_pages, p.num_pages, p.B,
                                            p.T, p.prefix, p.H, p.KV, p.hd, p.page_size, p.scale, p.window, stream));

@@ -244,6 +244,8 @@ class ShardEngine:
         torch.cuda.set_device(self.device)
         self.sms = ops.sm_count()
         self.l2_prefetch = os.environ.get("DLI_L2_PREFETCH", "0") == "1"
+        # prompt passes: RoPE and the cache append in the qkv projection's epilogue (DLI_FUSE_QKV_ROPE=0: a kernel of their own)
+        self.fuse_qkv_rope = os.environ.get("DLI_FUSE_QKV_ROPE", "1") == "1"
         # kernels may start (and prefetch weights) while their predecessor drains
         ops.set_pdl(os.environ.get("DLI_PDL", "1") == "1")
         self.w: Dict[str, torch.Tensor] = {}
@@ -636,7 +638,8 @@ class ShardEngine:
             h_in = h.copy_(hidden)
         ops.prompt_layers(self.layers, self.kv.k, self.kv.v, self.kv.page_table, st["page_rows"], h_in, h, self._x[:rows],
                           self._qkv[:rows], self._attn[:rows], self._act[:rows], self.cos, self.sin, positions, seq_ids,
-                          B, T, prefix, s.n_heads, s.n_kv_heads, s.head_dim, s.eps, self.scale, window=s.sliding_window)
+                          B, T, prefix, s.n_heads, s.n_kv_heads, s.head_dim, s.eps, self.scale, window=s.sliding_window,
+                          fuse_rope=self.fuse_qkv_rope)
         if not self.is_last or not final:
             return h
         if self.head_shard is not None:

@@ -135,10 +135,10 @@ _LAYER_KEYS = (("norm1", "ln1"), ("norm1_b", "ln1b"), ("w_qkv", "wqkv"), ("b_qkv
 
 
 def prompt_layers(layers, k_pools, v_pools, page_table, page_rows, h_in, h, x, qkv, attn, act, cos, sin, positions, seq_ids,
-                  B, T, prefix, H, KV, hd, eps, scale, window=0):
+                  B, T, prefix, H, KV, hd, eps, scale, window=0, fuse_rope=True):
     """A prompt pass through all `layers` (dicts of an engine's layer tensors) in one native call: B prompts of T tokens,
     whole (prefix None) or a chunk at positions prefix ..; h_in [B*T, d] is read, h receives the result, x / qkv / attn /
-    act are workspaces of B*T rows."""
+    act are workspaces of B*T rows.  fuse_rope=False: rotation and cache append as a kernel of their own."""
     global launch_count
     rows, d = h.shape
     if rows != B * T or h_in.shape != h.shape or x.shape != h.shape or qkv.shape != (rows, (H + 2 * KV) * hd) or \
@@ -165,7 +165,8 @@ def prompt_layers(layers, k_pools, v_pools, page_table, page_rows, h_in, h, x, q
     p = _lib.PromptPass(
         n_layers=len(layers), B=B, T=T, prefix=-1 if prefix is None else prefix, d=d, ff=ff, H=H, KV=KV, hd=hd, window=window,
         page_size=k_pools[0].shape[2] if layers else 8, max_pages=page_table.shape[1],
-        num_pages=k_pools[0].shape[0] if layers else 0, tensor_core=int(_prefill_tensor_core(hd, T)), eps=eps, scale=scale,
+        num_pages=k_pools[0].shape[0] if layers else 0, tensor_core=int(_prefill_tensor_core(hd, T)),
+        split_rope=int(not fuse_rope), eps=eps, scale=scale,
         h_in=_p(h_in), h=_p(h), x=_p(x), qkv=_p(qkv), attn=_p(attn), act=_p(act), cos=_p(cos), sin=_p(sin),
         positions=_p(positions), seq_ids=_p(seq_ids), page_table=_p(page_table), page_rows=_p(page_rows))
     n = _ct.c_int(0)

@@ -234,6 +234,7 @@ typedef struct {
   int prefix; /* -1: whole prompts; >= 0: chunks at positions prefix .. prefix + T - 1 */
   int d, ff, H, KV, hd, window, page_size, max_pages, num_pages;
   int tensor_core; /* whole prompts: dli_attn_prefill_tc_bf16 instead of dli_attn_prefill_bf16 */
+  int split_rope;  /* 1: rotation and cache append as a kernel of their own behind the qkv projection */
   float eps, scale;
   const void* h_in; /* [B*T, d] input, read only unless it is h */
   void *h, *x, *qkv, *attn, *act; /* [B*T, .]: result, normed rows, (H+2KV)*hd, H*hd, ff */

@@ -65,3 +65,28 @@ def test_hidden_states_in_any_form(cuda, stages):
     last._workspace(B * T + 1)
     with pytest.raises(RuntimeError):
         last.prefill(B, T, hidden=last._h[1:B * T + 1])
+
+
+@pytest.mark.parametrize("name", ["llama", "gpt2"])
+def test_rotation_as_a_kernel_of_its_own(cuda, monkeypatch, name):
+    """DLI_FUSE_QKV_ROPE=0: one launch more per layer, the same caches and logits."""
+    from dli_b200 import ops
+    from dli_b200.engine import ModelSpec, ShardEngine
+    from oracle import decoder_ref as R
+
+    spec = ModelSpec("llama", 2, 256, 4, 2, 64, 512, 512, 1e-5, 10000.0, 0, 128) if name == "llama" else ModelSpec(
+        "gpt2", 2, 256, 4, 4, 64, 1024, 512, 1e-5, 0.0, 0, 128, True)
+    sd = R.seeded_state_dict(R.ModelSpec(**spec.__dict__), seed=3, std=0.06)
+    B, T = 2, 21
+    ids = torch.randint(0, 512, (B * T,), device=cuda, dtype=torch.int32)
+    runs = []
+    for switch in ("1", "0"):
+        monkeypatch.setenv("DLI_FUSE_QKV_ROPE", switch)
+        e = ShardEngine(spec, device="cuda:0", max_batch=B, max_seq_len=64)
+        e.load_state_dict(sd)
+        e.start_batch(B, T, T + 4)
+        n0 = ops.launch_count
+        e.prefill(B, T, ids=ids)
+        runs.append((ops.launch_count - n0, [e._state(B, 0)["logits"].clone()] + [t.clone() for t in e.kv.k + e.kv.v]))
+    assert runs[1][0] == runs[0][0] + spec.n_layers
+    assert all(torch.equal(a, b) for a, b in zip(runs[0][1], runs[1][1]))
