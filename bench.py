@@ -886,8 +886,7 @@ def fubepel_kernel_times(eng, spec, T, peaks):
         L, P = spec.layers[li_d], eng.layers[li_d]
         act = torch.empty(rows, L.ff, dtype=E, device=dev)
         if P["packed"]:
-            sk = eng._splitk() if 2 < rows <= 128 else None
-            ms = timeit(lambda: ops.linear_gated_act(he, P["w_gu"], P["ff_act"], sk, out=act), n=3, reps=3)
+            ms = timeit(lambda: ops.linear_gated_act(he, P["w_gu"], P["ff_act"], out=act), n=3, reps=3)
             if rows > 1:
                 put(f"{tag}_ff_gate_up_act", ms, flops=4 * rows * W * L.ff)
             else:

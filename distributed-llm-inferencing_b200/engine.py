@@ -266,7 +266,6 @@ class ShardEngine:
         # generate(): prompts longer than this are prefilled in chunks of this many tokens (bounded activation
         # workspace; None = whole prompt at once)
         self.prefill_chunk: Optional[int] = None
-        self._sk = None  # split-K workspace of the batched-decode projections (zeroed once, self-resetting)
         self._graphs: Dict[tuple, tuple] = {}
         self._dec: Dict[tuple, dict] = {}
 
@@ -450,21 +449,11 @@ class ShardEngine:
         last_li = len(self.layers) - 1
         x, qkv, attn, act = self._x[:rows], self._qkv[:rows], self._attn[:rows], self._act[:rows]
         H, KV, hd = s.n_heads, s.n_kv_heads, s.head_dim
-        # rows <= 2: CUDA-core GEMV with the RMSNorm fused in (6.0-7.3 TB/s); 3..128 rows: split-K tcgen05
-        # weight stream on every SM (the GEMV's FMA work grows with the rows: 4.1-5.0 TB/s at 3-4 rows)
+        # rows <= 2: CUDA-core GEMV with the RMSNorm fused in (6.0-7.3 TB/s); 3..128 rows: the tcgen05 weight stream, K split
+        # over clusters so that every SM has a share (the GEMV's FMA work grows with the rows: 4.1-5.0 TB/s at 3-4 rows)
         fuse_norm = rows <= _GEMV_MAX_ROWS and s.arch == "llama"
-        split_k = _GEMV_MAX_ROWS < rows <= 128
-        if split_k and self._sk is None:
-            n_max = max(s.vocab, 2 * s.d_ff, (H + 2 * KV) * hd, s.d_model)
-            self._sk = torch.zeros(ops.gemm_splitk_scratch_bytes(128, n_max), dtype=torch.uint8, device=self.device)
-
-        def lin(x_, w_, **kw):
-            return ops.linear_splitk(x_, w_, self._sk, **kw) if split_k else ops.linear(x_, w_, **kw)
-
-        def gated(x_, w_, out):
-            if split_k:
-                return ops.linear_splitk_gated_silu(x_, w_, self._sk, out=out)
-            return ops.linear_gated_silu(x_, w_, out=out)
+        few = _GEMV_MAX_ROWS < rows <= 128
+        lin, gated = (ops.gemm, ops.gemm_gated_silu) if few else (ops.linear, ops.linear_gated_silu)
 
         for li, L in enumerate(self.layers):
             dst = h_out if (li == last_li and h_out is not None) else h
@@ -491,7 +480,7 @@ class ShardEngine:
                     ops.rmsnorm_linear_gated_silu(h, L["ln2"], s.eps, L["wgu"], out=act)
                 else:
                     ops.add_rmsnorm(h, L["ln2"], s.eps, out=x)
-                    gated(x, L["wgu"], act)
+                    gated(x, L["wgu"], out=act)
                 lin(act, L["wdown"], residual=h, out=dst)
             else:
                 lin(attn, L["wo"], bias=L["bo"], residual=res, out=h)

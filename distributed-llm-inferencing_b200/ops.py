@@ -294,7 +294,7 @@ def gemm_gated_silu(x, w_gu, out=None):
 
 def linear_gated_act(x, w_gu, act, scratch=None, out=None):
     """min(g, l) * sigmoid(a min(g, l)) * (clamp(u, -l, l) + 1) with g = x @ Wg.T, u = x @ Wu.T as the projection's epilogue;
-    w_gu = pack_gate_up(Wg, Wu), act float32 [2] = (l, a) on the device; scratch: the split-K buffer (3..128 rows)."""
+    w_gu = pack_gate_up(Wg, Wu), act float32 [2] = (l, a) on the device.  `scratch` is accepted and not used."""
     global launch_count
     _req(x), _req(w_gu), _req(out), _req(act, torch.float32)
     M, K = x.shape
@@ -402,8 +402,8 @@ def gemm_splitk_scratch_bytes(M, N) -> int:
 
 
 def linear_splitk(x, w, scratch, bias=None, residual=None, out=None, epilogue=EPI_NONE):
-    """Batched-decode projection: the split-K tcgen05 weight stream gemm() takes for few rows.  `scratch` (a tensor of
-    gemm_splitk_scratch_bytes(M, N) bytes) is accepted and not used: partial sums meet in shared memory."""
+    """Batched-decode projection: gemm() as callers with a scratch buffer know it.  `scratch` (a tensor of
+    gemm_splitk_scratch_bytes(M, N) bytes, or None) is accepted and not used: partial sums meet in shared memory."""
     global launch_count
     _req(x), _req(w), _req(bias), _req(residual), _req(out)
     M, K = x.shape

@@ -563,7 +563,6 @@ class RaggedEngine:
 
     def unload(self) -> None:
         self._graphs.clear()
-        self._sk = None
         self.w.clear()
         self.layers.clear()
         self.kv.release_all()
@@ -667,20 +666,11 @@ class RaggedEngine:
         if self.dtype == BF and x.shape[1] % 8 == 0 and w.shape[0] % 8 == 0 and x.is_contiguous() and \
                 not (x.shape[0] > 16 and (x.shape[1] % 64 or w.shape[0] % 16)):  # those would run row by row on the GEMV
             if 2 < x.shape[0] <= 128 and x.shape[1] % 64 == 0 and w.shape[0] % 16 == 0:
-                # few rows (batched decode, short portions): the split-K weight stream on every SM, as the uniform
+                # few rows (batched decode, short portions): the weight stream with K split over clusters, as the uniform
                 # stacks' batched decode does
-                return ops.linear_splitk(x, w, self._splitk(), out=out)
+                return ops.gemm(x, w, out=out)
             return ops.linear(x, w, out=out)
         return ops.linear_any(x, w, out)
-
-    def _splitk(self) -> torch.Tensor:
-        """Zero-filled scratch of the split-K projections (self-resetting; calls are ordered on one stream)."""
-        if getattr(self, "_sk", None) is None:
-            n_max = max([self.w["head"].shape[0], self.spec.width] +
-                        [v.shape[0] for d in self.layers.values() for k, v in d.items() if k.startswith("w") and
-                         isinstance(v, torch.Tensor) and v.dim() == 2])
-            self._sk = torch.zeros(ops.gemm_splitk_scratch_bytes(128, n_max), dtype=torch.uint8, device=self.device)
-        return self._sk
 
     # ------------------------------------------------------------------ one step
     def step(self, batch: Sequence[Tuple[int, Sequence[int]]], want: Optional[Sequence[Sequence[int]]] = None):
@@ -908,7 +898,7 @@ class RaggedEngine:
                 enter_sublayer(y, g_post, P["norm2"], self.slots.tensors.get(("tail2", li)), P.get("canon2"))
                 act = self._act[:rows * L.ff].view(rows, L.ff)
                 if P["packed"] and 2 < rows <= 128 and W % 64 == 0:
-                    ops.linear_splitk_gated_silu(hc, P["w_gu"], self._splitk(), out=act)
+                    ops.gemm_gated_silu(hc, P["w_gu"], out=act)
                 elif P["packed"]:
                     ops.linear_gated_silu(hc, P["w_gu"], out=act)
                 else:
@@ -986,8 +976,7 @@ class RaggedEngine:
         if L.ff:
             act = self._act[:rows * L.ff].view(rows, L.ff)
             if P["packed"]:
-                ops.linear_gated_act(h, P["w_gu"], P["ff_act"], self._splitk() if 2 < rows <= 128 and s.width % 64 == 0 else None,
-                                     out=act)
+                ops.linear_gated_act(h, P["w_gu"], P["ff_act"], out=act)
             else:
                 n_gu = P["w_gu"].shape[0]
                 gu = self._gu[:rows * n_gu].view(rows, n_gu)
@@ -1083,9 +1072,9 @@ class RaggedEngine:
         gelu = L.ff_fn == "gelu_tanh"
         few = 2 < rows <= 128 and W % 64 == 0
         if P["packed"] and gelu:
-            ops.linear_gated_act(he, P["w_gu"], P["ff_act"], self._splitk() if few else None, out=act)
+            ops.linear_gated_act(he, P["w_gu"], P["ff_act"], out=act)
         elif P["packed"] and few:
-            ops.linear_splitk_gated_silu(he, P["w_gu"], self._splitk(), out=act)
+            ops.gemm_gated_silu(he, P["w_gu"], out=act)
         elif P["packed"]:
             ops.linear_gated_silu(he, P["w_gu"], out=act)
         else:

@@ -299,8 +299,7 @@ int dli_linear_gated_silu_bf16(const void* x, const void* w_gu, void* y, int M,
 /* The same gated projection pair with the clamped activation g * sigmoid(alpha g) * (u + 1), g = min(gate, limit),
  * u = clamp(up, -limit, limit), in the epilogue; act points at {limit, alpha} (two floats) on the device.  w_gu in
  * the interleaved layout of dli_gemv_gated_silu_bf16.  dli_linear_gated_act_bf16 picks the weight stream (M <= 2 or
- * K % 64 != 0), the split-K tensor-core stream (M <= 128 with scratch of dli_gemm_splitk_scratch_bytes) or the
- * tensor-core GEMM. */
+ * K % 64 != 0) or the tensor-core GEMM; scratch is accepted and not used. */
 int dli_gemv_gated_act_bf16(const void* x, const void* w_gu, void* y, int M, int F, int K, const float* act,
                             dli_stream_t stream);
 int dli_linear_gated_act_bf16(const void* x, const void* w_gu, void* y, int M, int F, int K, const float* act, void* scratch,
