@@ -21,13 +21,16 @@
 // an element at least that large), the largest such bound of the cluster leaves a few hundred candidates, and these meet
 // in the first CTA's shared memory, where the exact threshold is a binary search over keys.  (The two 256-bin
 // histograms with shared-memory atomics and their serial scans, three passes of 2-byte loads by one CTA per row, took
-// 62 us for one row as for 48, V = 128 256.)
+// 62 us for one row as for 48, V = 128 256.  They are left for large k, see launch_sample.)
+#include <math.h>
+
 #include "common.cuh"
 
 namespace dli {
 
 constexpr int kSampleThreads = 512;
 constexpr int kMaxCand = 2048;  // candidates kept in shared memory (k plus ties)
+constexpr int kMaxRanked = 128;  // candidates that are put in order by counting
 
 // monotone key: larger bf16 value <-> larger 16-bit key
 __device__ __forceinline__ uint32_t bf16_key(uint16_t b) { return (b & 0x8000u) ? (uint16_t)~b : (uint16_t)(b | 0x8000u); }
@@ -94,6 +97,21 @@ __device__ __forceinline__ uint32_t vec_elem(const uint4& u, int e) {
   return (e & 1) ? w >> 16 : w & 0xffffu;
 }
 
+// f(key, index) for every element of the row by the threads of one CTA, eight loads of a thread in flight at a time.
+template <typename F>
+__device__ __forceinline__ void for_each_key(const uint16_t* __restrict__ row, int V, F f) {
+  constexpr int kBatch = 8;
+  int i = threadIdx.x;
+  for (; i + (kBatch - 1) * kSampleThreads < V; i += kBatch * kSampleThreads) {
+    uint16_t raw[kBatch];
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) raw[u] = row[i + u * kSampleThreads];
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) f(bf16_key(raw[u]), i + u * kSampleThreads);
+  }
+  for (; i < V; i += kSampleThreads) f(bf16_key(row[i]), i);
+}
+
 // Largest key t such that at least `k` elements of the row have key >= t (two 8-bit radix passes over global memory): the
 // general form, for k above the number of threads and rows with more candidates than fit.
 __device__ uint32_t kth_largest_key(const uint16_t* __restrict__ row, int V, int k, uint32_t* hist /*256*/,
@@ -104,11 +122,10 @@ __device__ uint32_t kth_largest_key(const uint16_t* __restrict__ row, int V, int
   for (int pass = 0; pass < 2; ++pass) {
     for (int i = tid; i < 256; i += kSampleThreads) hist[i] = 0;
     __syncthreads();
-    for (int i = tid; i < V; i += kSampleThreads) {
-      const uint32_t key = bf16_key(row[i]);
+    for_each_key(row, V, [&](uint32_t key, int) {
       if (pass == 0) atomicAdd(&hist[key >> 8], 1u);
       else if ((key >> 8) == prefix) atomicAdd(&hist[key & 0xff], 1u);
-    }
+    });
     __syncthreads();
     if (tid == 0) {
       int acc = 0, bin = 255;
@@ -127,15 +144,28 @@ __device__ uint32_t kth_largest_key(const uint16_t* __restrict__ row, int V, int
   return prefix;
 }
 
-// grid: rows x CTAs of a row (a cluster)
+// The candidates' order as whole numbers: larger value <-> larger number, -0 = 0, a NaN above every number; 0 lies below all.
+__device__ __forceinline__ uint32_t order_key(float v) {
+  const uint32_t u = __float_as_uint(v + 0.f);
+  return v != v ? 0xffffffffu : (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+__device__ __forceinline__ float order_value(uint32_t u) {
+  return __uint_as_float((u & 0x80000000u) ? (u & 0x7fffffffu) : ~u);
+}
+// Descending by value, equal values by ascending token id.
+__device__ __forceinline__ bool comes_before(uint32_t a, int ia, uint32_t b, int ib) {
+  return a > b || (a == b && (unsigned)ia < (unsigned)ib);
+}
+
+// grid: rows x CTAs of a row (a cluster).  narrow: see launch_sample; otherwise one CTA per row
 __global__ void __launch_bounds__(kSampleThreads)
 sample_kernel(const bf16* __restrict__ logits, int ld, int32_t* __restrict__ out, int V, float inv_temperature,
               int top_k, float top_p, const uint64_t* __restrict__ seed, const int32_t* __restrict__ step,
               float* __restrict__ dbg_probs, int32_t* __restrict__ dbg_ids, int dbg_cap, int per_row,
-              const int32_t* __restrict__ row_mask, int ctas) {
+              const int32_t* __restrict__ row_mask, int ctas, int narrow) {
   __shared__ uint32_t hist[256];
   __shared__ uint32_t sh[2];
-  __shared__ float cval[kMaxCand];
+  __shared__ float cval[kMaxCand];  // candidates: keys, then values, then probabilities
   __shared__ int cidx[kMaxCand];
   __shared__ uint32_t gkey[kMaxCand];  // first CTA: the row's candidates
   __shared__ int gidx[kMaxCand];
@@ -143,53 +173,57 @@ sample_kernel(const bf16* __restrict__ logits, int ld, int32_t* __restrict__ out
   __shared__ uint32_t gcount;
   __shared__ uint32_t gbase;
   __shared__ int ncand;
+  __shared__ int nties;
   __shared__ float red[kSampleThreads / 32];
+  uint32_t* ckey = reinterpret_cast<uint32_t*>(cval);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int b = blockIdx.x / ctas, rank = blockIdx.x - b * ctas;
-  if (tid == 0) gcount = 0, ncand = 0;
+  if (tid == 0) gcount = 0, ncand = 0, nties = 0;
   pdl_wait();
   pdl_trigger();
   if (row_mask != nullptr && row_mask[b] == 0) return;  // this row keeps the token already in out[]
   const uint16_t* row = reinterpret_cast<const uint16_t*>(logits + (size_t)b * ld);
   const int k = top_k > 0 ? min(top_k, V) : V;
 
-  // ---- this CTA's share of the row: whole 16-byte vectors; what lies before and after them goes to the first CTA --------
-  const int head = min(V, (int)(((16u - (uint32_t)(reinterpret_cast<uintptr_t>(row) & 15u)) & 15u) >> 1));
-  const int n_vec = (V - head) >> 3, tail0 = head + n_vec * 8;
-  const int v0 = (int)((long long)n_vec * rank / ctas), v1 = (int)((long long)n_vec * (rank + 1) / ctas);
-  const uint4* vecs = reinterpret_cast<const uint4*>(row + head);
-  uint4 held[kSliceVecs];
-#pragma unroll
-  for (int i = 0; i < kSliceVecs; ++i) {
-    const int v = v0 + i * kSampleThreads + tid;
-    // beyond the slice: the lowest key (a negative NaN), never at or above a bound
-    held[i] = v < v1 ? vecs[v] : make_uint4(0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu);
-  }
-  int edge = -1;  // an element of the unaligned ends
-  if (rank == 0) {
-    if (tid < head) edge = tid;
-    else if (tail0 + tid - head < V) edge = tail0 + tid - head;
-  }
-  uint32_t top = 0;
-#pragma unroll
-  for (int i = 0; i < kSliceVecs; ++i)
-#pragma unroll
-    for (int e = 0; e < 8; ++e) top = max(top, bf16_key((uint16_t)vec_elem(held[i], e)));
-  for (int v = v0 + kSliceVecs * kSampleThreads + tid; v < v1; v += kSampleThreads) {
-    const uint4 u = vecs[v];
-#pragma unroll
-    for (int e = 0; e < 8; ++e) top = max(top, bf16_key((uint16_t)vec_elem(u, e)));
-  }
-  if (edge >= 0) top = max(top, bf16_key(row[edge]));
-
-  // ---- lower bound of the k-th largest key: the k-th largest of the per-thread maxima, bit by bit ---------------------
-  uint32_t bound = 0;
-  const bool narrow = k <= kSampleThreads;
   if (narrow) {
+    // ---- this CTA's share of the row: whole 16-byte vectors; what lies before and after them goes to the first CTA --------
+    const int head = min(V, (int)(((16u - (uint32_t)(reinterpret_cast<uintptr_t>(row) & 15u)) & 15u) >> 1));
+    const int n_vec = (V - head) >> 3, tail0 = head + n_vec * 8;
+    const int v0 = (int)((long long)n_vec * rank / ctas), v1 = (int)((long long)n_vec * (rank + 1) / ctas);
+    const uint4* vecs = reinterpret_cast<const uint4*>(row + head);
+    uint4 held[kSliceVecs];
+#pragma unroll
+    for (int i = 0; i < kSliceVecs; ++i) {
+      const int v = v0 + i * kSampleThreads + tid;
+      // beyond the slice: the lowest key (a negative NaN), never at or above a bound
+      held[i] = v < v1 ? vecs[v] : make_uint4(0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu);
+    }
+    int edge = -1;  // an element of the unaligned ends
+    if (rank == 0) {
+      if (tid < head) edge = tid;
+      else if (tail0 + tid - head < V) edge = tail0 + tid - head;
+    }
+    uint32_t top = 0;
+#pragma unroll
+    for (int i = 0; i < kSliceVecs; ++i)
+#pragma unroll
+      for (int e = 0; e < 8; ++e) top = max(top, bf16_key((uint16_t)vec_elem(held[i], e)));
+    for (int v = v0 + kSliceVecs * kSampleThreads + tid; v < v1; v += kSampleThreads) {
+      const uint4 u = vecs[v];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) top = max(top, bf16_key((uint16_t)vec_elem(u, e)));
+    }
+    if (edge >= 0) top = max(top, bf16_key(row[edge]));
+
+    // ---- lower bound of the k-th largest key: the k-th largest of the per-thread maxima, bit by bit (a row of at most a
+    // thread per logit needs none: all of it are candidates) ----
+    uint32_t bound = 0;
     cluster_arrive();
+    if (V > kSampleThreads) {
 #pragma unroll 1
-    for (uint32_t bit = 0x8000u; bit; bit >>= 1)
-      if (__syncthreads_count(top >= (bound | bit)) >= k) bound |= bit;
+      for (uint32_t bit = 0x8000u; bit; bit >>= 1)
+        if (__syncthreads_count(top >= (bound | bit)) >= k) bound |= bit;
+    }
     cluster_wait();  // every CTA of the cluster runs: from here on its shared memory may be written
     if (tid < ctas) cluster_st(cluster_addr(&bounds[rank], tid), bound);
     cluster_sync_all();
@@ -199,7 +233,7 @@ sample_kernel(const bf16* __restrict__ logits, int ld, int32_t* __restrict__ out
       const uint32_t key = bf16_key((uint16_t)raw);
       if (key >= bound) {
         const int slot = atomicAdd(&ncand, 1);
-        if (slot < kMaxCand) { cval[slot] = __uint_as_float(key); cidx[slot] = i; }
+        if (slot < kMaxCand) { ckey[slot] = key; cidx[slot] = i; }
       }
     };
 #pragma unroll
@@ -223,7 +257,7 @@ sample_kernel(const bf16* __restrict__ logits, int ld, int32_t* __restrict__ out
     const uint32_t base = gbase, kb = cluster_addr(gkey, 0), ib = cluster_addr(gidx, 0);
     if (mine <= (uint32_t)kMaxCand && base + mine <= (uint32_t)kMaxCand) {
       for (uint32_t i = tid; i < mine; i += kSampleThreads) {
-        cluster_st(kb + (base + i) * 4, __float_as_uint(cval[i]));
+        cluster_st(kb + (base + i) * 4, ckey[i]);
         cluster_st(ib + (base + i) * 4, (uint32_t)cidx[i]);
       }
     }
@@ -254,48 +288,54 @@ sample_kernel(const bf16* __restrict__ logits, int ld, int32_t* __restrict__ out
       const int i = q * kSampleThreads + tid;
       if (i < n_c && keys[q] >= thr) {
         const int slot = atomicAdd(&ncand, 1);
-        cval[slot] = key_value(keys[q]) * inv_temperature;
+        ckey[slot] = order_key(key_value(keys[q]) * inv_temperature);
         cidx[slot] = gidx[i];
       }
     }
   } else {
     const uint32_t thr = kth_largest_key(row, V, min(k, kMaxCand), hist, sh);
-    // what lies above the threshold first (fewer than k elements): ties beyond the capacity are dropped, never those
-    for (int ties = 0; ties < 2; ++ties) {
-      for (int i = tid; i < V; i += kSampleThreads) {
-        const uint32_t key = bf16_key(row[i]);
-        if (ties ? key == thr : key > thr) {
-          const int slot = atomicAdd(&ncand, 1);
-          if (slot < kMaxCand) { cval[slot] = key_value(key) * inv_temperature; cidx[slot] = i; }
-        }
+    // what lies above the threshold (fewer than k elements) first: ties beyond the capacity are dropped, never those
+    for_each_key(row, V, [&](uint32_t key, int i) {
+      if (key > thr) {
+        const int slot = atomicAdd(&ncand, 1);
+        ckey[slot] = order_key(key_value(key) * inv_temperature);
+        cidx[slot] = i;
+      } else if (key == thr) {
+        const int slot = atomicAdd(&nties, 1);
+        if (slot < kMaxCand) gidx[slot] = i;
       }
-      __syncthreads();
+    });
+    __syncthreads();
+    const int above = ncand, ties = min(nties, kMaxCand - above);
+    __syncthreads();
+    for (int i = tid; i < ties; i += kSampleThreads) {
+      ckey[above + i] = order_key(key_value(thr) * inv_temperature);
+      cidx[above + i] = gidx[i];
     }
+    if (tid == 0) ncand = above + ties;
   }
   __syncthreads();
-  const int n = min(ncand, kMaxCand);
+  const int n = ncand;  // at most kMaxCand
   // Descending by value, equal values by ascending token id.  Which of several EQUAL-probability tokens survive at the
   // nucleus boundary depends on torch.sort's tie order in the reference (not specified); here the lower token ids stay.
-  if (n <= kSampleThreads) {
-    // every candidate counts those before it (a NaN goes before every number)
-    float a = 0.f;
-    int ia = 0, place = 0;
-    if (tid < n) {
-      a = cval[tid];
-      ia = cidx[tid];
-      for (int j = 0; j < n; ++j) {
-        const float c = cval[j];
-        const bool tie = c == a || (c != c && a != a);
-        place += (c > a || (c != c && a == a) || (tie && cidx[j] < ia)) ? 1 : 0;
-      }
-    }
+  int npow = 1;
+  while (npow < n) npow <<= 1;
+  if (n == 1) {
+    // in order already
+  } else if (npow <= kMaxRanked) {
+    // every candidate's place is the number of those before it, counted by `lanes` threads of a warp (500 candidates counted
+    // by one thread each took 30 us, the sorting network takes 4)
+    const int lanes = min(32, kSampleThreads / npow), me = tid / lanes;
+    const uint32_t a = ckey[min(me, n - 1)];
+    const int ia = cidx[min(me, n - 1)];
+    int place = 0;
+    for (int j = tid % lanes; j < n; j += lanes) place += comes_before(ckey[j], cidx[j], a, ia) ? 1 : 0;
+    for (int o = lanes >> 1; o > 0; o >>= 1) place += __shfl_xor_sync(0xffffffffu, place, o);
     __syncthreads();
-    if (tid < n) { cval[place] = a; cidx[place] = ia; }
+    if (me < n && tid % lanes == 0) { ckey[place] = a; cidx[place] = ia; }
     __syncthreads();
   } else {
-    int npow = 1;
-    while (npow < n) npow <<= 1;
-    for (int i = n + tid; i < npow; i += kSampleThreads) { cval[i] = -INFINITY; cidx[i] = -1; }
+    for (int i = n + tid; i < npow; i += kSampleThreads) { ckey[i] = 0u; cidx[i] = -1; }
     __syncthreads();
     // bitonic sort
     for (int size = 2; size <= npow; size <<= 1) {
@@ -304,10 +344,9 @@ sample_kernel(const bf16* __restrict__ logits, int ld, int32_t* __restrict__ out
           const int j = i ^ stride;
           if (j > i) {
             const bool desc = (i & size) == 0;
-            const float a = cval[i], b = cval[j];
+            const uint32_t a = ckey[i], b = ckey[j];
             const int ia = cidx[i], ib = cidx[j];
-            const bool a_first = (a > b) || (a == b && (unsigned)ia < (unsigned)ib);
-            if (a_first != desc) { cval[i] = b; cval[j] = a; cidx[i] = ib; cidx[j] = ia; }
+            if (comes_before(a, ia, b, ib) != desc) { ckey[i] = b; ckey[j] = a; cidx[i] = ib; cidx[j] = ia; }
           }
         }
         __syncthreads();
@@ -315,16 +354,16 @@ sample_kernel(const bf16* __restrict__ logits, int ld, int32_t* __restrict__ out
     }
   }
   // ---- softmax over the top-k set, nucleus cut, renormalise, draw (n <= 2048: one warp scans) ----
-  const float vmax = cval[0];
+  const float vmax = order_value(ckey[0]);
   float part = 0.f;
-  for (int i = tid; i < n; i += kSampleThreads) part += __expf(cval[i] - vmax);
+  for (int i = tid; i < n; i += kSampleThreads) part += __expf(order_value(ckey[i]) - vmax);
   part = warp_sum(part);
   if (lane == 0) red[warp] = part;
   __syncthreads();
   float denom = 0.f;
 #pragma unroll
   for (int w = 0; w < kSampleThreads / 32; ++w) denom += red[w];
-  for (int i = tid; i < n; i += kSampleThreads) cval[i] = __expf(cval[i] - vmax) / denom;  // probabilities, descending
+  for (int i = tid; i < n; i += kSampleThreads) cval[i] = __expf(order_value(ckey[i]) - vmax) / denom;  // probabilities, descending
   __syncthreads();
   if (warp == 0) {
     // exclusive prefix sums in descending order; keep while prefix < top_p (always the first)
@@ -381,16 +420,28 @@ sample_kernel(const bf16* __restrict__ logits, int ld, int32_t* __restrict__ out
 }
 
 // A cluster of as many CTAs as the row has slices of 16 384 logits, at most the portable 8 (beyond 131 072 logits a
-// thread reads the rest of its slice twice).
+// thread reads the rest of its slice twice).  That way (`narrow`) is for k small enough that few logits lie above the
+// bound: with `per` logits a thread, k of 512 maxima above it means a share of 1 - (1 - k/512)^(1/per) of all logits, and a
+// bf16 step at the bound adds up to some V / 4096 ties.  Larger k would overflow the first CTA's shared memory after all the
+// work; it takes the histograms of one CTA per row at once.
+//   one row, us, one CTA for every k / clusters up to k = 512 / this rule: 128 256 logits, k = 50: 57.8 / 13.9 / 11.6,
+//   k = 128: 62.3 / 21.0 / 17.3, k = 256: 65.5 / 109 / 65.1, k = 512: 76.2 / 107 / 74.5, k = 1000: 97.3 / 105 / 79.2;
+//   500 logits, k = 500: 16.3 / 47.9 / 15.7
 static int launch_sample(const char* what, const void* logits, int ld, int32_t* out, int B, int V, float temperature,
                          int top_k, float top_p, const uint64_t* seed, const int32_t* step, float* dbg_probs,
                          int32_t* dbg_ids, int dbg_cap, int per_row, const int32_t* row_mask, cudaStream_t s) {
   int ctas = (V - 1) / kSliceElems + 1;
   if (ctas > kMaxRowCtas) ctas = kMaxRowCtas;
   if ((long long)B * ctas > 0x7fffffffLL) ctas = 1;
+  const int k = top_k > 0 && top_k < V ? top_k : V;
+  const double per = (double)V / (kSampleThreads * ctas);
+  const bool narrow = k <= kSampleThreads &&
+                      (V <= kMaxCand || V * (1.0 - pow(1.0 - (double)k / kSampleThreads, 1.0 / per)) <= kMaxCand - V / 4096);
+  if (!narrow) ctas = 1;
   const cudaError_t e = launch_kernel_cluster(sample_kernel, dim3((unsigned)B * ctas), dim3(kSampleThreads), (size_t)0, s,
                                               (unsigned)ctas, (const bf16*)logits, ld, out, V, 1.0f / temperature, top_k,
-                                              top_p, seed, step, dbg_probs, dbg_ids, dbg_cap, per_row, row_mask, ctas);
+                                              top_p, seed, step, dbg_probs, dbg_ids, dbg_cap, per_row, row_mask, ctas,
+                                              narrow ? 1 : 0);
   if (e != cudaSuccess) return fail(DLI_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
   return DLI_OK;
 }

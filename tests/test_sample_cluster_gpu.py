@@ -125,3 +125,27 @@ def test_ctas_of_a_row_that_start_apart(cuda, V):
                 m @ m
         got = [ops.sample(x, seed=seed, debug_cap=64) for _ in range(4)]
         assert all(torch.equal(a, b) for r in got for a, b in zip(r, want))
+
+
+@pytest.mark.parametrize("V,k", [(300, 300), (512, 512), (513, 512), (2048, 400), (2100, 128), (5000, 65), (5000, 129), (40000, 400),
+                                 (128256, 200), (128256, 256), (262151, 200), (262151, 128)])
+def test_either_side_of_the_rules(cuda, V, k):
+    """k where candidates are put in order by counting, by the network, and where a row stays with one CTA."""
+    g = torch.Generator(device="cuda").manual_seed(V + k)
+    _check((2.5 * torch.randn(2, V, device=cuda, generator=g)).to(BF), top_k=k, top_p=1.0)
+
+
+@pytest.mark.parametrize("zeros", [40, 150, 700])
+def test_signed_zeros_and_nan(cuda, zeros):
+    """-0 and 0 stand by token id (put in order by counting, by the network, with one CTA); a NaN before every number."""
+    from dli_b200 import ops
+
+    x = torch.full((1, 5000), -3.0, device=cuda, dtype=BF)
+    x[0, 7:7 + zeros] = 0.0
+    x[0, 8:7 + zeros:2] = -0.0
+    x[0, [4000, 2, 3000]] = torch.tensor([-1.0, -1.5, 2.0], device=cuda, dtype=BF)
+    _check(x, top_k=zeros + 3, top_p=1.0)
+    x[0, 3] = float("nan")
+    seed = torch.tensor([1], dtype=torch.int64, device=cuda)
+    _, _, ids = ops.sample(x, top_k=zeros + 3, top_p=1.0, seed=seed, debug_cap=8)
+    assert int(ids[0, 0]) == 3
