@@ -12,8 +12,12 @@
 // Queries still come from the packed qkv buffer of the chunk, keys and values of the WHOLE context
 // (the earlier chunks and this one, appended by dli_rope_kv_append_bf16 just before) come from the
 // paged KV cache, page by page like the decode kernel does it.  Same arithmetic otherwise.
+#include <math.h>
 #include <stdlib.h>
 #include <string.h>
+
+#include <algorithm>
+#include <functional>
 
 #include "mma_utils.cuh"
 
@@ -222,17 +226,68 @@ int launch_attn_prefill_tc(const void* qkv, void* out, int B, int T, int H, int 
 int launch_attn_prefill_tc_paged(const void* qkv, void* out, const void* k_cache, const void* v_cache,
                                  const int32_t* page_table, int max_pages, int num_pages, int B, int T, int prefix,
                                  int H, int KV, int hd, int page_size, float scale, int window, cudaStream_t s);
-// The tcgen05 kernel takes ~5 us whatever it does (TMEM, barriers, a 128-row tile), the mma.sync kernel half of that; by the
-// longest key range of the call, us on B200 (mma.sync / tcgen05), one prompt, no prefix unless given:
-//   32 heads of 64:  T = 19: 2.7 / 5.3, 256: 5.3 / 6.6, 400: 9.0 / 8.3, 512: 10.4 / 8.7, 1777: 54 / 34, 4096: 249 / 132;
-//                    T = 16 after 512: 10.8 / 10.4, after 6000: 95 / 57
-//   12 heads of 64:  T = 256: 5.3 / 6.8, 400: 7.6 / 8.2, 512: 8.7 / 9.0, 800: 13.5 / 11.5, 1777: 34 / 19
-//   32 heads of 128: T = 19: 3.8 / 5.6, 64: 4.4 / 5.9, 128: 5.7 / 6.4 (eight prompts of 100: 12.0 / 9.9), 301: 11.6 / 7.9
+// Which kernel?  Head size 128: tcgen05 above 64 keys (us on B200, mma.sync / tcgen05, one prompt of 32 heads: T = 19: 3.8 / 5.6,
+// 64: 4.4 / 5.9, 128: 5.7 / 6.4, 301: 11.6 / 7.9).  Head size 64, where a tile is half the MMA work and the same softmax: by
+// estimated time, because how many items a call has, how long the longest is and how many of its keys a window leaves all
+// shift the line: 32 heads, T = 512: 10.8 / 9.4, 2 heads 8.8 / 9.0; T = 1777 of 12 heads 35 / 20, in a window of 100 8.8 / 12.8.
+//   mma.sync, CTA per 64 queries: c0 + hypot(c1 x longest, (c2 x tiles + c3 x CTAs) / SMs), tiles of 64 keys
+//   tcgen05, 128 queries an item: d0 + d1 x tiles + d2 x items of the fullest CTA of the serpentine deal, tiles of 128 keys
+// fitted to 2 700 calls (2 ... 64 heads, 1 ... 16 sequences, 1 ... 2048 queries, up to 8 000 keys, windows), within 4 and 6 %.
+// Taken where it is estimated 5 % faster: over those calls 0.4 % slower than the better kernel on average, and at most 13 %
+// than mma.sync.  (448 keys as the line: 9.8 % on average, up to 58 %.)
 // DLI_PREFILL_ATTN=mma, looked up at every call, keeps the mma.sync kernel everywhere.
-static bool prefill_on_tc(int hd, int keys) {
+constexpr int kMaxListed = 1024;
+struct KeyTiles {
+  int count, total, longest;  // query tiles, key tiles of all of them, of the longest
+  int of[kMaxListed];         // per query tile, as far as they fit
+};
+static void key_tiles(KeyTiles& n, int T, int prefix, int window, int q_tile, int k_tile) {
+  n.count = n.total = n.longest = 0;
+  for (int q0 = 0; q0 < T; q0 += q_tile) {
+    const int end = prefix + (T - q0 < q_tile ? T : q0 + q_tile);
+    const int first = window > 0 && prefix + q0 - window + 1 > 0 ? prefix + q0 - window + 1 : 0;
+    const int t = (end + k_tile - 1) / k_tile - first / k_tile;
+    if (n.count < kMaxListed) n.of[n.count] = t;
+    ++n.count;
+    n.total += t;
+    if (t > n.longest) n.longest = t;
+  }
+}
+static bool prefill64_on_tc(int B, int T, int prefix, int H, int window, bool paged) {
+  const int sms = sm_count_cached() > 0 ? sm_count_cached() : 148;
+  const double copies = (double)H * B;
+  KeyTiles n;
+  key_tiles(n, T, prefix, window, 64, 64);
+  const double even = copies * (paged ? 0.65 * n.total + 0.6 * n.count : 0.5 * n.total + 0.8 * n.count) / sms;
+  const double mma = paged ? 2.0 + hypot(1.0 * n.longest, even) : 2.5 + hypot(0.8 * n.longest, even);
+  key_tiles(n, T, prefix, window, 128, 128);
+  const long long items = (long long)(copies * n.count), rounds = (items + sms - 1) / sms;
+  double tiles = 0, count = 0;
+  if (rounds > 16 || n.count > kMaxListed) {
+    tiles = copies * n.total / sms;
+    count = (double)rounds;
+  } else {
+    std::sort(n.of, n.of + n.count, std::greater<int>());
+    // the first and the last CTA, and those at either side of where the last round ends
+    const int last = (int)(items - (rounds - 1) * sms);
+    const int side = rounds % 2 ? last - 1 : sms - last, other = rounds % 2 ? (last < sms ? last : sms - 1) : (side > 0 ? side - 1 : 0);
+    double most = -1;
+    for (const int c : {0, sms - 1, side, other}) {
+      double t = 0, k = 0;
+      for (long long r = 0; r < rounds; ++r) {
+        const long long at = r * sms + (r % 2 ? sms - 1 - c : c);
+        if (at < items) t += n.of[at / (long long)copies], k += 1;
+      }
+      if (t + 2 * k > most) most = t + 2 * k, tiles = t, count = k;
+    }
+  }
+  const double tc = paged ? 3.4 + 1.08 * tiles + 3.4 * count : 3.2 + 1.11 * tiles + 2.1 * count;
+  return 1.05 * tc < mma;
+}
+static bool prefill_on_tc(int B, int T, int prefix, int H, int hd, int window, bool paged) {
   const char* choice = getenv("DLI_PREFILL_ATTN");
-  const bool tc = !(choice && strcmp(choice, "mma") == 0);
-  return tc && (hd == 64 ? keys >= 448 : keys > 64);
+  if (choice && strcmp(choice, "mma") == 0) return false;
+  return hd == 64 ? prefill64_on_tc(B, T, prefix, H, window, paged) : prefix + T > 64;
 }
 
 }  // namespace dli
@@ -250,7 +305,7 @@ static int attn_prefill(const void* qkv, void* out, int B, int T, int H, int KV,
   if (B == 0 || T == 0) return DLI_OK;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (hd == 128) return launch_prefill<128, false>(qkv, out, B, T, H, KV, scale, window, s);
-  if (by_rule && prefill_on_tc(hd, T)) return launch_attn_prefill_tc(qkv, out, B, T, H, KV, hd, scale, window, s);
+  if (by_rule && prefill_on_tc(B, T, 0, H, hd, window, false)) return launch_attn_prefill_tc(qkv, out, B, T, H, KV, hd, scale, window, s);
   return launch_prefill<64, false>(qkv, out, B, T, H, KV, scale, window, s);
 }
 
@@ -286,7 +341,7 @@ extern "C" int dli_attn_prefill_paged_bf16(const void* qkv, void* out, const voi
   while ((1 << shift) < page_size) ++shift;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   // both attention GEMMs on tcgen05, K/V pages brought in by TMA (num_pages > 0 says how large the pools are)
-  if (prefill_on_tc(hd, prefix + T) && num_pages > 0 && page_size <= 128)
+  if (num_pages > 0 && page_size <= 128 && prefill_on_tc(B, T, prefix, H, hd, window, true))
     return launch_attn_prefill_tc_paged(qkv, out, k_cache, v_cache, page_table, max_pages, num_pages, B, T, prefix, H,
                                         KV, hd, page_size, scale, window, s);
   if (hd == 128)

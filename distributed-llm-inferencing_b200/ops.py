@@ -204,7 +204,7 @@ def _prefill_tensor_core(hd, T) -> bool:
 def attn_prefill(qkv, out, B, T, H, KV, hd, scale, window=0, tensor_core=None):
     """Causal prefill attention.  tensor_core=True: the tcgen05 kernel (head_dim 128), False: the mma.sync kernel, None: by
     rule — head_dim 128 runs on tcgen05 (dli_attn_prefill_tc_bf16) from 65 tokens, where it overtakes the mma.sync kernel
-    (64 tokens of 32 heads: 5.9 against 4.4 us), head_dim 64 chooses by the same kind of rule inside
+    (64 tokens of 32 heads: 5.9 against 4.4 us), head_dim 64 chooses by estimated time inside
     dli_attn_prefill_bf16, and with DLI_PREFILL_ATTN=mma both stay on mma.sync."""
     global launch_count
     _req(qkv), _req(out)

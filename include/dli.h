@@ -187,8 +187,9 @@ int dli_paged_attn_decode_static_bf16(const void* q, int q_stride, const void* k
  * Replaces the same reference code as above at T>1 with a causal mask
  * (TF:masking_utils create_causal_mask, called at
  * TF:models/llama/modeling_llama.py:398-405).  window as above.
- * out: [B*T, H*hd] bf16.  head_dim 64 from 448 tokens on runs on the tcgen05 kernel below unless the
- * environment says DLI_PREFILL_ATTN=mma; everything else here on mma.sync.  _mma_: mma.sync whatever the size. */
+ * out: [B*T, H*hd] bf16.  head_dim 64 runs on the tcgen05 kernel below where that is estimated to be faster (longer
+ * prompts), unless the environment says DLI_PREFILL_ATTN=mma; everything else here on mma.sync.  _mma_: mma.sync
+ * whatever the size. */
 int dli_attn_prefill_bf16(const void* qkv, void* out, int B, int T, int H, int KV,
                           int hd, float scale, int window, dli_stream_t stream);
 int dli_attn_prefill_mma_bf16(const void* qkv, void* out, int B, int T, int H, int KV,

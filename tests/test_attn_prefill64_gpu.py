@@ -79,7 +79,7 @@ def test_a_sequence_does_not_see_its_neighbour(cuda, hd, T):
     assert torch.equal(both[:T], alone)
 
 
-@pytest.mark.parametrize("hd,T", [(64, 512), (64, 1777), (128, 130)])
+@pytest.mark.parametrize("hd,T", [(64, 1100), (64, 1777), (128, 130)])
 def test_the_caller_chooses_the_kernel(cuda, monkeypatch, hd, T):
     """tensor_core=False is the mma.sync kernel at either head size, whatever the rule says, and DLI_PREFILL_ATTN is looked up
     at every call.  The kernels tile the keys differently, so their bits differ: that tells them apart."""
@@ -109,3 +109,55 @@ def test_the_caller_chooses_the_kernel(cuda, monkeypatch, hd, T):
     assert torch.equal(whole(None), mma) and torch.equal(chunk(), mma)
     monkeypatch.delenv("DLI_PREFILL_ATTN")
     assert torch.equal(whole(None), by_rule) and torch.equal(chunk(), paged)
+
+
+@pytest.mark.parametrize("B,T,H,KV,window", [(1, 1025, 2, 1, 0), (1, 1151, 4, 2, 0), (2, 1280, 3, 3, 0), (8, 1025, 2, 2, 257),
+                                             (1, 1777, 2, 1, 1000), (3, 450, 12, 12, 0), (16, 512, 8, 8, 0)])
+def test_whole_prompts_of_head_size_64_on_tcgen05(cuda, B, T, H, KV, window):
+    """Sizes that the rule gives to the tcgen05 kernel (its bits are not those of the mma.sync kernel)."""
+    from dli_b200 import ops
+
+    hd, g = 64, torch.Generator(device="cuda").manual_seed(T + B)
+    qkv = (1.3 * torch.randn(B * T, (H + 2 * KV) * hd, device=cuda, generator=g)).to(BF)
+    out, mma = (torch.full((B * T, H * hd), float("nan"), device=cuda, dtype=BF) for _ in range(2))
+    ops.attn_prefill(qkv, out, B, T, H, KV, hd, hd ** -0.5, window=window)
+    ops.attn_prefill(qkv, mma, B, T, H, KV, hd, hd ** -0.5, window=window, tensor_core=False)
+    assert not torch.equal(out, mma)
+    q, k, v = (x.double().view(B, T, -1, hd) for x in qkv.split([H * hd, KV * hd, KV * hd], dim=1))
+    for b in range(B):
+        for o in (out, mma):
+            _check(o.double().view(B, T, H, hd)[b], q[b], k[b], v[b], H, KV, hd, 0, window)
+
+
+@pytest.mark.parametrize("B,T,prefix,H,KV,page,window", [(1, 1, 1000, 2, 1, 8, 0), (2, 100, 900, 2, 2, 16, 0), (1, 100, 900, 2, 2, 64, 600),
+                                                         (2, 40, 900, 3, 3, 16, 0), (2, 513, 407, 2, 2, 32, 0), (1, 130, 2000, 4, 2, 16, 0),
+                                                         (4, 100, 407, 32, 8, 16, 600), (1, 3, 2000, 2, 2, 128, 0)])
+def test_chunks_of_head_size_64_on_tcgen05(cuda, monkeypatch, B, T, prefix, H, KV, page, window):
+    from dli_b200 import ops
+
+    hd, g = 64, torch.Generator(device="cuda").manual_seed(T + prefix)
+    S = prefix + T
+    n = (S + page - 1) // page
+    kc = (1.3 * torch.randn(B * n + 2, KV, page, hd, device=cuda, generator=g)).to(BF)
+    vc = torch.randn(B * n + 2, KV, page, hd, device=cuda, generator=g).to(BF)
+    table = torch.randperm(B * n + 2, device=cuda, generator=g)[:B * n].int().view(B, n).contiguous()
+    for b in range(B):
+        if S % page:
+            kc[table[b, -1], :, S % page:], vc[table[b, -1], :, S % page:] = float("nan"), float("inf")
+    qkv = (1.3 * torch.randn(B * T, (H + 2 * KV) * hd, device=cuda, generator=g)).to(BF)
+    outs = []
+    for choice in ("tc", "mma"):
+        monkeypatch.setenv("DLI_PREFILL_ATTN", choice)
+        outs.append(torch.full((B * T, H * hd), float("nan"), device=cuda, dtype=BF))
+        ops.attn_prefill_paged(qkv, outs[-1], kc, vc, table, B, T, prefix, H, KV, hd, hd ** -0.5, window=window)
+    assert not torch.equal(*outs)
+    q = qkv[:, :H * hd].double().view(B, T, H, hd)
+    for b in range(B):
+        k, v = (c[table[b].long()].double().transpose(1, 2).reshape(n * page, KV, hd)[:S] for c in (kc, vc))
+        for o in outs:
+            _check(o.double().view(B, T, H, hd)[b], q[b], k, v, H, KV, hd, prefix, window)
+
+
+@pytest.mark.parametrize("T", [1030, 1800])
+def test_long_prompts_of_head_size_64_do_not_see_their_neighbours(cuda, T):
+    test_a_sequence_does_not_see_its_neighbour(cuda, 64, T)
