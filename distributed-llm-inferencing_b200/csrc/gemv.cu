@@ -333,19 +333,27 @@ static int launch_gemv_r(const bf16* x, const bf16* w, const bf16* bias, const b
 //   2560 x 2048: 4.35 -> 2.78 (6)    2048 x 2048: 3.81 -> 2.52 (5)    2048 x 5632: 6.45 -> 4.65 (5)    32000 x 2048: 29.4 -> 20.5 (8)
 //   6144 x 4096: 9.18 -> 8.05 (7)    4096 x 4096: 6.95 -> 6.36 (5)    4096 x 14336: 20.3 -> 18.7 (5)   128256 x 4096: 145.5 (4)
 // The sums do not depend on R: a thread always adds its vectors of a row in order.
-static int gemv_rows(int M, int N, int K, bool gated) {
-  if (M > 2) return 4;
+// Two rows of x and long rows: 4 rows go two vectors at a time, and where a thread's vectors come out even that is the
+// faster loop (4096 x 8192: 15.9 us, 5 rows 16.4; x 10240, five vectors: 20.6, 19.1).
+// With the norm in front the rows of x stand in shared memory beside the partial sums (2 KB per row of x and weight row of a
+// task): counted with the CTAs that are left, and more rows per task must not cost one of them — two rows of x of 12288
+// elements, 18432 outputs: three CTAs an SM with 4 rows per task, 73 us, two with 8, 101 us.
+static int gemv_rows(int M, int N, int K, bool gated, bool norm) {
+  if (M > 2 || (M == 2 && K > 6144 && ((K + 2047) >> 11) % 2 == 0)) return 4;
+  const auto per_sm = [&](int r) { return (228 << 10) / ((norm ? 2 * M * K : 0) + 2048 * r * M + 1280); };  // 1280: red, system
+  const int most = per_sm(4) < 3 ? per_sm(4) : 3;
   static const double kShort[] = {1.35, 1.20, 1.10, 1.04, 1.00}, kLong[] = {1.00, 1.09, 1.08, 1.02, 1.03};
   static const double kShortGated[] = {1.35, 0.0, 1.03, 0.0, 1.05};  // 6 rows: 8.2 us for 8192 x 2048, 8 rows: 9.1
   const double* factor = K > 2048 ? kLong : gated ? kShortGated : kShort;
-  const long long ctas = 3LL * (sm_count_cached() > 0 ? sm_count_cached() : 148);
+  const long long ctas = (long long)most * (sm_count_cached() > 0 ? sm_count_cached() : 148);
   int pick = 4;
   double best = 1e30;
   for (int r = 4; r <= 8; r += gated ? 2 : 1) {
+    if (per_sm(r) < most) break;
     const int outs = gated ? r / 2 : r;
     const long long tasks = (N + outs - 1) / outs, waves = (tasks + ctas - 1) / ctas;
     const double cost = (double)(waves * ctas) * outs / N * factor[r - 4];
-    if (cost < best) best = cost, pick = r;
+    if (cost < (pick == 4 ? 0.985 : 1.0) * best) best = cost, pick = r;  // a tie stays at 4
   }
   return pick;
 }
@@ -355,7 +363,7 @@ static int launch_gemv(const bf16* x, const bf16* w, const bf16* bias, const bf1
                        int epilogue, const bf16* ln_w, float eps, cudaStream_t s, float* cand = nullptr,
                        int* grid_out = nullptr) {
 #define DLI_GO(r) return launch_gemv_r<M, kGated, kNorm, r>(x, w, bias, residual, y, N, K, epilogue, ln_w, eps, s, cand, grid_out)
-  switch (gemv_rows(M, N, K, kGated)) {
+  switch (gemv_rows(M, N, K, kGated, kNorm)) {
     case 5:
       if constexpr (M <= 2 && !kGated) DLI_GO(5);
       break;

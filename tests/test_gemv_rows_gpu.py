@@ -48,3 +48,17 @@ def test_gated(cuda, M, F, K):
     a, b = ops.gemv(x, wg).float(), ops.gemv(x, wu).float()  # the same sums
     ref = torch.nn.functional.silu(a).to(BF).float() * b
     torch.testing.assert_close(y.float(), ref, rtol=2.0 ** -7, atol=1e-6)  # one ulp: expf against torch's
+
+
+@pytest.mark.parametrize("M", [1, 2])
+@pytest.mark.parametrize("N,K", [(3000, 10752), (18432, 12288), (2221, 14336), (1500, 16384)])
+def test_norm_of_long_rows(cuda, M, N, K):
+    """Rows of x that take so much shared memory that it bounds the rows per task: the same bits as in pieces."""
+    from dli_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(N + K)
+    x, ln = torch.randn(M, K, device=cuda, generator=g).to(BF), torch.randn(K, device=cuda, generator=g).to(BF)
+    w = (torch.randn(N, K, device=cuda, generator=g) * K ** -0.5).to(BF)
+    y = ops.rmsnorm_linear(x, ln, 1e-5, w)
+    parts = [ops.rmsnorm_linear(x, ln, 1e-5, w[i:i + 997].contiguous()) for i in range(0, N, 997)]
+    assert torch.equal(y, torch.cat(parts, dim=1))
