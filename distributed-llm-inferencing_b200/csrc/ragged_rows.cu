@@ -241,7 +241,8 @@ scalar_rmsnorm_kernel(const float* __restrict__ x, float* __restrict__ hn, int d
 
 // x += y / sqrt(mean(y^2) + eps) * g_post; then (hn != NULL) hn = x / sqrt(mean(x^2) + eps) * g_next:
 // the post-norm of one sublayer, the fp32 residual add and the pre-norm of the next sublayer in one pass.
-template <typename E>
+// kHeld: elements of the row a thread keeps in registers (kHeld * blockDim >= d), 0: none.
+template <typename E, int kHeld>
 __global__ void __launch_bounds__(1024)
 postnorm_add_norm_kernel(const E* __restrict__ y, float* __restrict__ x, float* __restrict__ hn, int d, float eps,
                          float g_post, float g_next) {
@@ -250,10 +251,11 @@ postnorm_add_norm_kernel(const E* __restrict__ y, float* __restrict__ x, float* 
   pdl_trigger();
   const size_t o = (size_t)blockIdx.x * d;
   float ss = 0.f, s2 = 0.f;
-  constexpr int kHeld = 8;
-  if (d <= kHeld * (int)blockDim.x) {
-    // the row of y and of x in registers, asked for together: one pass over memory instead of three (the same sums).
-    // Latency-bound: 7.4 -> 5.4 us averaged over prompt (547 x 2048) and decode rows
+  if constexpr (kHeld > 0) {
+    // the row of y and of x asked for together: one pass over memory instead of three (the same sums).  Latency-bound, then
+    // bound by the rows in flight, which the registers held decide; us (three passes / 8 elements held by every row they
+    // hold / as many as the row has): 3 x 2048 3.3 / 3.6 / 2.7, 547 x 72 2.6 / 3.2 / 2.2, 547 x 2048 6.5 / 3.7 / 3.7,
+    // 1300 x 256 4.1 / 5.8 / 3.4, 1300 x 4096 18.7 / 25.4 / 18.8
     float yv[kHeld], xv[kHeld];
 #pragma unroll
     for (int i = 0; i < kHeld; ++i) {
@@ -280,23 +282,23 @@ postnorm_add_norm_kernel(const E* __restrict__ y, float* __restrict__ x, float* 
       const int c = threadIdx.x + i * blockDim.x;
       if (c < d) hn[o + c] = xv[i] * r2;
     }
-    return;
+  } else {
+    for (int c = threadIdx.x; c < d; c += blockDim.x) {
+      const float v = to_f(y[o + c]);
+      ss += v * v;
+    }
+    ss = block_sum(ss, red);
+    const float r = g_post / sqrtf(ss / d + eps);
+    for (int c = threadIdx.x; c < d; c += blockDim.x) {
+      const float v = x[o + c] + to_f(y[o + c]) * r;
+      x[o + c] = v;
+      s2 += v * v;
+    }
+    if (hn == nullptr) return;
+    s2 = block_sum(s2, red);
+    const float r2 = g_next / sqrtf(s2 / d + eps);
+    for (int c = threadIdx.x; c < d; c += blockDim.x) hn[o + c] = x[o + c] * r2;
   }
-  for (int c = threadIdx.x; c < d; c += blockDim.x) {
-    const float v = to_f(y[o + c]);
-    ss += v * v;
-  }
-  ss = block_sum(ss, red);
-  const float r = g_post / sqrtf(ss / d + eps);
-  for (int c = threadIdx.x; c < d; c += blockDim.x) {
-    const float v = x[o + c] + to_f(y[o + c]) * r;
-    x[o + c] = v;
-    s2 += v * v;
-  }
-  if (hn == nullptr) return;
-  s2 = block_sum(s2, red);
-  const float r2 = g_next / sqrtf(s2 / d + eps);
-  for (int c = threadIdx.x; c < d; c += blockDim.x) hn[o + c] = x[o + c] * r2;
 }
 
 // out[t] = h[t] + sum_j w[:, j] * h[t - taps + 1 + j]: a causal convolution over time on each channel.  Rows
@@ -781,6 +783,19 @@ using namespace dli;
 // few rows of a wide model: one CTA per row needs many threads to cover the row's latency; many rows: 256 are enough
 static inline int row_threads(int rows, int d) { return (rows <= 64 && d >= 2048) ? 1024 : 256; }
 
+template <typename E>
+static int launch_postnorm_add_norm(const E* y, float* x, float* hn, int rows, int d, float eps, float g_post, float g_next,
+                                    cudaStream_t s) {
+  const int threads = row_threads(rows, d), held = (d + threads - 1) / threads;
+  const auto kernel = held <= 1   ? postnorm_add_norm_kernel<E, 1>
+                      : held <= 2 ? postnorm_add_norm_kernel<E, 2>
+                      : held <= 4 ? postnorm_add_norm_kernel<E, 4>
+                      : held <= 8 ? postnorm_add_norm_kernel<E, 8>
+                                  : postnorm_add_norm_kernel<E, 0>;
+  DLI_LAUNCH("postnorm_add_norm", kernel, dim3(rows), dim3(threads), (size_t)0, s, y, x, hn, d, eps, g_post, g_next);
+  return DLI_OK;
+}
+
 extern "C" {
 
 int dli_embedding_f32(const int32_t* ids, const void* table, float* x, float* x2, void* xe, int rows, int d, int vocab,
@@ -880,9 +895,8 @@ int dli_postnorm_add_norm(const void* y, float* x, float* hn, int rows, int d, f
   DT_CHECK(dt);
   if (rows <= 0) return DLI_OK;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (dt == 0) DLI_LAUNCH("postnorm_add_norm", postnorm_add_norm_kernel<bf16>, dim3(rows), dim3(row_threads(rows, d)), 0, s, (const bf16*)y, x, hn, d, eps, g_post, g_next);
-  else DLI_LAUNCH("postnorm_add_norm", postnorm_add_norm_kernel<float>, dim3(rows), dim3(row_threads(rows, d)), 0, s, (const float*)y, x, hn, d, eps, g_post, g_next);
-  return DLI_OK;
+  return dt == 0 ? launch_postnorm_add_norm((const bf16*)y, x, hn, rows, d, eps, g_post, g_next, s)
+                 : launch_postnorm_add_norm((const float*)y, x, hn, rows, d, eps, g_post, g_next, s);
 }
 
 int dli_causal_conv_ragged(const float* h, float* tail, const float* w, const int32_t* row_ent, const int32_t* ent,
