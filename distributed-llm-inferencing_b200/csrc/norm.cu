@@ -179,7 +179,7 @@ rmsnorm_rows_kernel(const bf16* __restrict__ x, const bf16* __restrict__ residua
 // The same for rows of at most 2 048 elements of any multiple of 8 (GPT-2: 768), LayerNorm or RMSNorm: lane l plays the
 // threads l, l + 32, ... of the CTA-per-row kernel, one vector each, and the sums take that kernel's trees, so the bits are
 // the same.  That kernel keeps 160 of its 256 threads idle at 768 elements and pays four block barriers per row; bound
-// by latency either way (4.1 MB at 1 350 x 768): 10.2 -> 4.8 us for LayerNorm of 1 350 rows.
+// by latency either way (4.1 MB at 1 350 x 768): 10.2 -> 4.8 us for LayerNorm of 1 350 rows.  For many rows, see launch_norm.
 template <bool kLayerNorm>
 __global__ void __launch_bounds__(kNormThreads)
 norm_small_rows_kernel(const bf16* __restrict__ x, const bf16* __restrict__ residual, const bf16* __restrict__ weight,
@@ -297,8 +297,13 @@ static int launch_norm(bool ln, const void* x, const void* residual, const void*
                  (const bf16*)weight, (bf16*)resid_out, (bf16*)y, rows, eps);
     return DLI_OK;
   }
-  // 64 rows: below, a CTA per row spreads over more SMs than eight rows per CTA
-  if (rows >= 64 && d <= 8 * kNormThreads) {
+  // A warp per row takes one time whatever the rows (up to some 1 200), more with d, whose sums it forms alone; a CTA per row
+  // takes a round per two (LayerNorm) or three CTAs an SM.  us, CTA / warp: LayerNorm 296 x 768 2.65 / 3.47, 301 x 768 4.04 /
+  // 3.44, 301 x 1024 4.06 / 3.88, 592 x 2048 4.85 / 5.86, 600 x 2048 6.03 / 5.87; RMSNorm 200 x 256 1.98 / 1.98, 400 x 768
+  // 2.18 / 2.68, 450 x 1024 3.07 / 3.05, 888 x 1536 3.79 / 3.82, 900 x 1536 4.46 / 3.78.
+  const int sms = sm_count_cached() > 0 ? sm_count_cached() : 148;
+  const int from = ln ? (d <= 1024 ? 2 : 4) : d <= 256 ? 1 : d <= 1024 ? 3 : 6;
+  if (rows > from * sms && d <= 8 * kNormThreads) {
     const dim3 grid((rows + kRowsPerCta - 1) / kRowsPerCta);
     const auto kernel = ln ? norm_small_rows_kernel<true> : norm_small_rows_kernel<false>;
     DLI_LAUNCH(name, kernel, grid, dim3(kNormThreads), (size_t)0, s, (const bf16*)x, (const bf16*)residual,
