@@ -148,6 +148,11 @@ def prompt_layers(layers, k_pools, v_pools, page_table, page_rows, h_in, h, x, q
         _req(t)
     for t in (page_table, page_rows, positions, seq_ids):
         _req(t, torch.int32)
+    if min(positions.numel(), seq_ids.numel()) < rows or page_rows.dim() != 2 or page_rows.shape[0] < B or \
+            page_rows.shape[1] != page_table.shape[1]:
+        raise ValueError("prompt_layers: positions, sequence ids or page rows do not cover the prompts")
+    if len(k_pools) < len(layers) or len(v_pools) < len(layers):
+        raise ValueError("prompt_layers: a layer lacks its caches")
     ff = act.shape[1]
     table = (_lib.LayerWeights * len(layers))()
     for L, c, k, v in zip(layers, table, k_pools, v_pools):

@@ -90,3 +90,41 @@ def test_rotation_as_a_kernel_of_its_own(cuda, monkeypatch, name):
         runs.append((ops.launch_count - n0, [e._state(B, 0)["logits"].clone()] + [t.clone() for t in e.kv.k + e.kv.v]))
     assert runs[1][0] == runs[0][0] + spec.n_layers
     assert all(torch.equal(a, b) for a, b in zip(runs[0][1], runs[1][1]))
+
+
+def test_buffers_that_are_too_small(cuda):
+    """Refused on the host: nothing is launched on buffers that do not cover the prompts."""
+    from dli_b200 import ops
+
+    B, T, d, H, hd = 2, 5, 128, 2, 64
+    rows = B * T
+    mat = lambda n, w: torch.zeros(n, w, device=cuda, dtype=BF)  # noqa: E731
+    ints = lambda *n: torch.zeros(*n, device=cuda, dtype=torch.int32)  # noqa: E731
+    good = dict(layers=[], k_pools=[], v_pools=[], page_table=ints(B, 3), page_rows=ints(B, 3), h_in=mat(rows, d), h=mat(rows, d),
+                x=mat(rows, d), qkv=mat(rows, 3 * H * hd), attn=mat(rows, H * hd), act=mat(rows, d), cos=None, sin=None,
+                positions=ints(rows), seq_ids=ints(rows), B=B, T=T, prefix=None, H=H, KV=H, hd=hd, eps=1e-5, scale=0.125)
+    ops.prompt_layers(**good)
+    for bad in (dict(positions=ints(rows - 1)), dict(seq_ids=ints(rows - 1)), dict(page_rows=ints(B - 1, 3)),
+                dict(page_rows=ints(B, 2)), dict(page_rows=ints(B * 3)), dict(layers=[{}]), dict(h_in=mat(rows + 1, d)),
+                dict(qkv=mat(rows, 64)), dict(attn=mat(rows - 1, H * hd))):
+        n0 = ops.launch_count
+        with pytest.raises(ValueError):
+            ops.prompt_layers(**{**good, **bad})
+        assert ops.launch_count == n0
+    with pytest.raises(ValueError):
+        ops.prompt_rows(ints(rows), ints(rows - 1), None, B, T, 0, 0)
+    with pytest.raises(ValueError):
+        ops.prompt_rows(ints(rows), ints(rows), ints(B - 1), B, T, 0, 0)
+
+
+@pytest.mark.parametrize("B,T,prefix,seq0", [(1, 1, 0, 0), (3, 7, 5, 6), (2, 200, 1000, 2)])
+def test_prompt_rows(cuda, B, T, prefix, seq0):
+    from dli_b200 import ops
+
+    n = B * T
+    pos, seq, last = (torch.full((n + 3,), -7, device=cuda, dtype=torch.int32) for _ in range(3))
+    ops.prompt_rows(pos, seq, last, B, T, prefix, seq0)
+    b, t = torch.arange(n, device=cuda) // T, torch.arange(n, device=cuda) % T
+    assert torch.equal(pos[:n].long(), prefix + t) and torch.equal(seq[:n].long(), seq0 + b)
+    assert torch.equal(last[:B].long(), (torch.arange(B, device=cuda) + 1) * T - 1)
+    assert (pos[n:] == -7).all() and (seq[n:] == -7).all() and (last[B:] == -7).all()
