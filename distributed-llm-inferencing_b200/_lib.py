@@ -66,6 +66,7 @@ SIGNATURES = {
     "dli_sample_rows_bf16": (_i, [_vp, _i, _vp, _i, _i, _f, _i, _f, _vp, _vp, _vp, _vp]),
     "dli_set_pdl": (_i, [_i]),
     "dli_gemm_splitk_scratch_bytes": (_sz, [_i, _i]),
+    "dli_gemm_plan": (_i, [_i, _i, _i, _i, C.POINTER(_i)]),
     "dli_gemm_splitk_bf16": (_i, [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp, _sz, _vp]),
     "dli_gemm_splitk_gated_silu_bf16": (_i, [_vp, _vp, _vp, _i, _i, _i, _vp, _sz, _vp]),
     "dli_rmsnorm_gemv_bf16": (_i, [_vp, _vp, _f, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp]),

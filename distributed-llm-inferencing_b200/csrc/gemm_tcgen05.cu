@@ -386,6 +386,20 @@ static double pick_prefill(int M, int N, int K, bool gated, PrefillShape* pick) 
   return best;
 }
 
+// The persistent kernel's tile: by cost where the matrix is wide, else the width that holds it.
+static PrefillShape prefill_tile(int M, int N, int K, bool gated) {
+  static const int force = getenv("DLI_GEMM_TILE") ? atoi(getenv("DLI_GEMM_TILE")) : 0;  // measurement knob: mt * 1000 + bn
+  PrefillShape p = kPrefillShapes[0];
+  if (gated) return p;
+  if (N % 256 == 0 || N >= 2048) {
+    pick_prefill(M, N, K, false, &p);
+    if (force) p.mt = force / 1000, p.bn = force % 1000;
+    return p;
+  }
+  p.bn = N % 128 == 0 || N > 128 ? 128 : N > 32 ? 64 : 32;
+  return p;
+}
+
 // Clusters that split K (gemm_rows.cu) or the persistent kernel?  By estimated time, over 12 matrices x 12 row counts
 // above 128: the persistent kernel takes 9.5 us beyond its rounds (its set-up, and the epilogue of the last round, which
 // nothing hides); the clusters' estimate is taken 10 % high, because where it errs it errs low (one full wave of wide
@@ -446,21 +460,39 @@ int dli_gemm_bf16(const void* x, const void* w, const void* bias, const void* re
   if (use_rows(M, N, K, false, &sh, &rc))
     return launch_gemm_rows(kRowsPlain, x, w, bias, residual, y, M, N, K, epilogue, sh, s);
   if (rc != DLI_OK) return rc;
-  if (N % 256 == 0 || N >= 2048) {
-    static const int force = getenv("DLI_GEMM_TILE") ? atoi(getenv("DLI_GEMM_TILE")) : 0;  // measurement knob: mt * 1000 + bn
-    PrefillShape p;
-    pick_prefill(M, N, K, false, &p);
-    if (force) p.mt = force / 1000, p.bn = force % 1000;
-    if (p.mt == 2) {
-      if (p.bn == 240) return launch_prefill_gemm<240, false, 2>(x, w, bias, residual, y, M, N, K, epilogue, s);
-      return launch_prefill_gemm<256, false, 2>(x, w, bias, residual, y, M, N, K, epilogue, s);
-    }
-    if (p.bn == 240) return launch_prefill_gemm<240, false>(x, w, bias, residual, y, M, N, K, epilogue, s);
-    return launch_prefill_gemm<256, false>(x, w, bias, residual, y, M, N, K, epilogue, s);
+  const PrefillShape p = prefill_tile(M, N, K, false);
+  if (p.mt == 2) {
+    if (p.bn == 240) return launch_prefill_gemm<240, false, 2>(x, w, bias, residual, y, M, N, K, epilogue, s);
+    return launch_prefill_gemm<256, false, 2>(x, w, bias, residual, y, M, N, K, epilogue, s);
   }
-  if (N % 128 == 0 || N > 128) return launch_prefill_gemm<128, false>(x, w, bias, residual, y, M, N, K, epilogue, s);
-  if (N > 32) return launch_prefill_gemm<64, false>(x, w, bias, residual, y, M, N, K, epilogue, s);
-  return launch_prefill_gemm<32, false>(x, w, bias, residual, y, M, N, K, epilogue, s);
+  switch (p.bn) {
+    case 240: return launch_prefill_gemm<240, false>(x, w, bias, residual, y, M, N, K, epilogue, s);
+    case 128: return launch_prefill_gemm<128, false>(x, w, bias, residual, y, M, N, K, epilogue, s);
+    case 64: return launch_prefill_gemm<64, false>(x, w, bias, residual, y, M, N, K, epilogue, s);
+    case 32: return launch_prefill_gemm<32, false>(x, w, bias, residual, y, M, N, K, epilogue, s);
+    default: return launch_prefill_gemm<256, false>(x, w, bias, residual, y, M, N, K, epilogue, s);
+  }
+}
+
+int dli_gemm_plan(int M, int N, int K, int gated, int* plan) {
+  using namespace dli;
+  DLI_CHECK_ARG(plan, "dli_gemm_plan: null pointer");
+  DLI_CHECK_ARG(M > 0 && N > 0 && K > 0 && K % 64 == 0 && N % (gated ? 256 : 16) == 0,
+                "dli_gemm_plan: need K %% 64 == 0 and N %% 16 == 0 (gated: N %% 256 == 0) (got M=%d N=%d K=%d)", M, N, K);
+  RowsShape sh;
+  int rc;
+  if (use_rows(M, N, K, gated != 0, &sh, &rc)) {
+    plan[0] = 1;
+    plan[1] = sh.bn;
+    plan[2] = sh.splits;
+    return DLI_OK;
+  }
+  if (rc != DLI_OK) return rc;
+  const PrefillShape p = prefill_tile(M, N, K, gated != 0);
+  plan[0] = 0;
+  plan[1] = p.bn;
+  plan[2] = p.mt;
+  return DLI_OK;
 }
 
 int dli_gemm_qkv_rope_append_bf16(const void* x, const void* w_qkv, void* qkv, int M, int K, const void* cos,

@@ -333,6 +333,10 @@ int dli_gemm_qkv_rope_append_bf16(const void* x, const void* w_qkv, void* qkv, i
  * aligned buffer or NULL, and dli_gemm_bf16 / dli_gemm_gated_silu_bf16 run the same
  * kernel.  dli_gemm_splitk_scratch_bytes keeps the size it has always returned. */
 size_t dli_gemm_splitk_scratch_bytes(int M, int N);
+/* What dli_gemm_bf16 (gated: dli_gemm_gated_silu_bf16, N = 2 F) runs for these sizes on the current device, for tests and
+ * measurements, as three numbers: plan[0] = 1: K split over clusters, plan[1] activation rows per tile, plan[2] splits; plan[0] = 0: the
+ * persistent kernel, plan[1] weight rows per tile, plan[2] 128-row halves per tile. */
+int dli_gemm_plan(int M, int N, int K, int gated, int* plan);
 int dli_gemm_splitk_bf16(const void* x, const void* w, const void* bias,
                          const void* residual, void* y, int M, int N, int K,
                          int epilogue, void* scratch, size_t scratch_bytes,

@@ -103,3 +103,30 @@ def test_right_after_the_convolution_that_writes_its_tail(cuda, n):
             ops.postnorm_add_norm_conv_single(y, xa, ta, w, ent, out, 0.7, 1.3, 1e-5)
             runs.append([mid, out, xa, ta])
     assert all(torch.equal(a, b) for r in runs[1:] for a, b in zip(runs[0], r))
+
+
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("d", [4, 72, 1024, 1028, 2052])
+def test_four_channels_a_thread_as_one(cuda, d, dt):
+    """The 16-byte form of the input convolution and the scalar one (which a tail that starts off 16 bytes takes): the same
+    bits, in portions shorter and longer than the taps, at a sequence's start and later."""
+    from dli_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(d)
+    ns, starts = [1, 2, 9, 40, 3], [0, 1, 0, 77, 2]
+    rows, at, ent, row_ent = sum(ns), 0, [], []
+    for i, (n, s) in enumerate(zip(ns, starts)):
+        ent += [len(ns) - 1 - i, at, n, s]
+        row_ent += [i] * n
+        at += n
+    ent, row_ent = (torch.tensor(v, device=cuda, dtype=torch.int32) for v in (ent, row_ent))
+    h, w = torch.randn(rows, d, device=cuda, generator=g), torch.randn(d, 4, device=cuda, generator=g)
+    tail = torch.randn(len(ns), 3, d, device=cuda, generator=g)
+    flat = torch.empty(tail.numel() + 1, device=cuda)
+    flat[1:] = tail.view(-1)
+    outs = []
+    for t in (tail, flat[1:].view_as(tail)):
+        out = torch.full((rows, d), float("nan"), device=cuda, dtype=dt)
+        ops.causal_conv_ragged(h, t, w, row_ent, ent, out)
+        outs.append((out, t))
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])

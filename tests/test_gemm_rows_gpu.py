@@ -92,7 +92,7 @@ def test_qkv_projection_with_rope_equals_the_separate_steps(cuda, rows, H, KV, K
 @pytest.mark.parametrize("M", [300, 1024, 1777])
 @pytest.mark.parametrize("N,K", [(72, 512), (240, 768), (488, 1024), (2048, 2048), (4096, 512)])
 def test_residual_read_by_the_line(cuda, M, N, K):
-    """The persistent tiles (all widths, a last tile cut in a line): the residual added, also where it is the output."""
+    """The residual added, also where it is the output, whatever kernel the sizes take (clusters, GEMV, persistent tiles)."""
     from dli_b200 import ops
     g, x, w, acc, slack = _inputs(M, N, K, M + N)
     r = torch.randn(M, N, device="cuda", generator=g).to(BF)
@@ -101,6 +101,28 @@ def test_residual_read_by_the_line(cuda, M, N, K):
     z = r.clone()
     ops.linear(x, w, residual=z, out=z)
     assert torch.equal(y, z)
+
+
+@pytest.mark.parametrize("M,N,K,tile", [(130, 16, 512, (32, 1)), (300, 48, 64, (64, 1)), (301, 112, 1024, (64, 1)),
+                                        (4097, 1040, 512, (128, 1)), (4352, 2320, 1024, (256, 1)), (4352, 4112, 4096, (256, 2)),
+                                        (8192, 2064, 4096, (240, 2))])
+def test_residual_on_the_persistent_tiles(cuda, M, N, K, tile):
+    """Every width that sizes lead to, the last tile cut inside a 64-column line of the residual: the residual added, also
+    where it is the output, with a bias and without."""
+    from dli_b200 import ops
+
+    if ops.sm_count() == 148:  # the choice counts SMs
+        assert ops.gemm_plan(M, N, K) == ("persistent", *tile)
+    g, x, w, acc, slack = _inputs(M, N, K, M + N)
+    r = torch.randn(M, N, device=cuda, generator=g).to(BF)
+    bias = torch.randn(N, device=cuda, generator=g).to(BF)
+    for b in (None, bias):
+        z = acc if b is None else acc + b.double()
+        y = ops.gemm(x, w, bias=b, residual=r)
+        _within(y, z + r.double(), slack + HALF_ULP * (z.abs() + slack) + HALF_ULP * (z + r.double()).abs() * 1.01)
+        out = r.clone()
+        ops.gemm(x, w, bias=b, residual=out, out=out)
+        assert torch.equal(y, out)
 
 
 @pytest.mark.parametrize("off", [1, 2, 4, 7])

@@ -128,3 +128,52 @@ def test_prompt_rows(cuda, B, T, prefix, seq0):
     assert torch.equal(pos[:n].long(), prefix + t) and torch.equal(seq[:n].long(), seq0 + b)
     assert torch.equal(last[:B].long(), (torch.arange(B, device=cuda) + 1) * T - 1)
     assert (pos[n:] == -7).all() and (seq[n:] == -7).all() and (last[B:] == -7).all()
+
+
+def _shift(t, off):
+    """The same values starting `off` elements into a buffer."""
+    flat = torch.empty(t.numel() + off, device=t.device, dtype=t.dtype)
+    flat[off:] = t.view(-1)
+    return flat[off:].view(t.shape)
+
+
+@pytest.mark.parametrize("arch,hd,H,KV,d,bias", [("llama", 64, 4, 2, 256, None), ("llama", 64, 3, 3, 768, 0), ("llama", 64, 32, 4, 2048, 1),
+                                                 ("llama", 128, 3, 1, 512, None), ("llama", 128, 4, 2, 512, 0), ("llama", 128, 5, 1, 640, 3),
+                                                 ("gpt2", 64, 12, 12, 768, 0), ("gpt2", 64, 4, 4, 256, 5), ("gpt2", 128, 2, 2, 256, 0)])
+@pytest.mark.parametrize("B,T", [(1, 3), (1, 19), (2, 64), (2, 65), (1, 700), (3, 1400)])
+def test_qkv_epilogue_equals_the_separate_steps(cuda, arch, hd, H, KV, d, bias, B, T):
+    """Projection, rotation and cache append of a prompt pass against gemm + rope_kv_append: the same bits, with one and two
+    heads per tile, an odd number of heads, a bias (aligned or not) and none, with rotation and without."""
+    from dli_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(B * T + d)
+    rnd = lambda *s, std=1.0: (std * torch.randn(*s, device=cuda, generator=g)).to(BF)  # noqa: E731
+    rows, N, ff, page, prefix, pages = B * T, (H + 2 * KV) * hd, 256, 16, 5, (T + 5 + 15) // 16
+    L = {"ln1": rnd(d), "ln2": rnd(d), "wqkv": rnd(N, d, std=0.05), "wo": rnd(d, H * hd, std=0.05), "wdown": rnd(d, ff, std=0.05)}
+    if arch == "gpt2":
+        L.update(ln1b=rnd(d), ln2b=rnd(d), wfc=rnd(ff, d, std=0.05))
+    else:
+        L.update(wgu=ops.pack_gate_up(rnd(ff, d, std=0.05), rnd(ff, d, std=0.05)))
+    if bias is not None:
+        L["bqkv"] = _shift(rnd(N), bias)
+    cos = sin = None
+    if arch == "llama":
+        ang = torch.rand(T + prefix, hd // 2, device=cuda, generator=g) * 6.28
+        cos, sin = ang.cos().to(BF), ang.sin().to(BF)
+    table = torch.randperm((B + 1) * pages, device=cuda, generator=g).int().view(B + 1, pages)
+    positions, seq_ids, last = (torch.empty(rows, device=cuda, dtype=torch.int32) for _ in range(3))
+    ops.prompt_rows(positions, seq_ids, last, B, T, prefix, 1)
+    h_in = rnd(rows, d)
+    kc, vc = (torch.zeros((B + 1) * pages, KV, page, hd, device=cuda, dtype=BF) for _ in range(2))
+    h, x, qkv, attn, act = (torch.empty(rows, w, device=cuda, dtype=BF) for w in (d, d, N, H * hd, ff))
+    ops.prompt_layers([L], [kc], [vc], table, table[1:], h_in, h, x, qkv, attn, act, cos, sin, positions, seq_ids, B, T, prefix,
+                      H, KV, hd, 1e-5, hd ** -0.5)
+    if arch == "gpt2":
+        ops.add_layernorm(h_in, L["ln1"], L["ln1b"], 1e-5, out=x)
+    else:
+        ops.add_rmsnorm(h_in, L["ln1"], 1e-5, out=x)
+    want = ops.gemm(x, L["wqkv"], bias=L.get("bqkv"))
+    k2, v2 = torch.zeros_like(kc), torch.zeros_like(vc)
+    ops.rope_kv_append(want, cos, sin, positions, seq_ids, table, k2, v2, H, KV, hd)
+    assert torch.equal(qkv, want) and torch.equal(kc, k2) and torch.equal(vc, v2)
+    assert torch.isfinite(h.float()).all()
