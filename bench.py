@@ -6,8 +6,8 @@
 Prints ONE JSON line (rank 0).  A "step" is one decode step: one new token for
 every sequence of the batch, with the KV cache already holding `ctx` tokens.
 
-N = 1 : config[2] of BASELINE.json — Llama-3-8B shape, bf16, random-init weights,
-        batch 1, 2k-token context, paged KV (the north-star target).  Also reports
+N = 1 : Llama-3-8B shape, bf16, random-init weights,
+        batch 1, 2k-token context, paged KV.  Also reports
         the 2k-token prefill and (extra) batch-32 decode.
 N > 1 : the same model split into N contiguous layer ranges (reference sharder
         formula), one stage per GPU; decode hands hidden states, head candidates and
@@ -17,7 +17,7 @@ N > 1 : the same model split into N contiguous layer ranges (reference sharder
         batch fixed, per-GPU weights shrink).  Before timing, rank 0 checks the
         pipeline's first tokens against the single-GPU engine on the same weights and
         the run aborts on a mismatch (extra.parity_check); extra.named_config runs the
-        BASELINE.json configuration that is stated for exactly N GPUs.
+        configuration that is stated for exactly N GPUs.
 
 value  : decode tokens/s with everything resident in HBM (CUDA-graph replay).
 e2e    : the same metric through the plugin call the reference's master makes
@@ -213,7 +213,7 @@ def e2e_through_worker(eng, prompt_row, ctx, K):
 
 def hf_gpu_comparator(spec, ctx, n_new=32):
     """transformers generate (bf16, sdpa, greedy) on this GPU at the same shape: the stock-PyTorch GPU
-    comparator BASELINE.md 5 names — what the reference's worker runs with USE_GPU=1
+    comparator: what the reference's worker runs with USE_GPU=1
     (reference worker/app.py:23-26,121-124,297-305) on a torch that supports the B200."""
     import gc
 
@@ -269,7 +269,7 @@ def dominant_kernel_roofline(eng, spec, B, peaks):
     nbytes = 2 * spec.d_ff * spec.d_model * 2
     ach = nbytes / (ms / 1e3) / 1e9
     # dram__bytes_read.sum + dram__bytes_write.sum of ONE launch of this kernel from an `ncu --set full` capture
-    # (profiles/): a recorded measurement, not taken in this run — the capture's tree is named beside it
+    # (profiles/roofline_traffic.json): a recorded measurement, not taken in this run — the capture's tree is named beside it
     traffic, traffic_src = None, None
     tp = os.path.join(ROOT, "profiles", "roofline_traffic.json")
     if os.path.exists(tp):
@@ -277,7 +277,7 @@ def dominant_kernel_roofline(eng, spec, B, peaks):
         traffic = rec.get("gate_up_projection_dram_bytes_per_launch")
         traffic_src = rec.get("source")
     return {"bound": "hbm", "kernel": "gemv_kernel<M,gated> (gate/up projection)" if B <= 4 else
-            "gemm_tcgen05_kernel<swap,gated> (gate/up projection)", "achieved": ach, "peak": peaks["hbm_gbs"],
+            "gemm_rows_kernel<gated> (gate/up projection)", "achieved": ach, "peak": peaks["hbm_gbs"],
             "unit": "GB/s", "frac": ach / peaks["hbm_gbs"], "traffic": traffic, "traffic_source": traffic_src,
             "bytes_per_launch": nbytes,
             "us_per_launch": ms * 1e3, "peak_source": peaks["source"]}
@@ -336,7 +336,7 @@ def cpu_baseline(spec, args, new_tokens=4, prompt_len=16):
 
 
 def cpu_configs0():
-    """BASELINE.json configs[0]: GPT-2 small (124M) random-init, fp32 (the reference's default load dtype,
+    """GPT-2 small (124M) random-init, fp32 (the reference's default load dtype,
     worker/app.py:121), USE_GPU=0, 32-token prompt -> 64 new tokens (max_length 96) through the port of the
     reference's /inference body — greedy (the parity mode) and with the reference's own sampling call."""
     from dli_b200.engine import NAMED_SPECS

@@ -1,7 +1,7 @@
 """Continuous batching of concurrent /inference requests on one full-range ShardEngine.
 
 The reference serves strictly one request at a time (one sync gunicorn worker,
-worker/Dockerfile:45; SURVEY.md §8f rank 3).  Decode at batch 1 is a pure weight
+worker/Dockerfile:45).  Decode at batch 1 is a pure weight
 stream, so up to `max_batch` concurrent requests can share every weight read: each
 request is prefilled alone into its own sequence slot (its own KV pages), then all
 active slots decode together — one token per slot per step — and requests join and

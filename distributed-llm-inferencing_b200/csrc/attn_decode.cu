@@ -127,8 +127,8 @@ paged_attn_decode_kernel(const bf16* __restrict__ q, int q_stride,
   // the sequence length, the page table and the cache pages of the OLD tokens were written at least one kernel
   // earlier, and that kernel is complete once this one runs at all (every kernel of the library waits for its
   // predecessor before it lets its successor start).  So the dependency wait moves below the K/V requests: the
-  // sequence-length -> page-table -> K/V chain (2.7 us of the 6.5 us this kernel took after the wait at batch 1,
-  // scratch/trace_decode_run.py) runs while the projection drains.  The unfused form reads K/V that the rope
+  // sequence-length -> page-table -> K/V chain (2.7 us of the 6.5 us this kernel took after the wait at batch 1)
+  // runs while the projection drains.  The unfused form reads K/V that the rope
   // kernel just before it appended: it waits first.
   if (!fused) {
     pdl_wait();

@@ -5,7 +5,7 @@
 // consumed by warp-level m16n8k16 MMAs with an fp32 online softmax (flash-style:
 // the T x T score matrix is never written).  Heavier (later) query tiles are
 // scheduled first.  Tensor-bound in principle (4*T^2/2*hd FLOPs per head) but
-// only ~4 % of prefill FLOPs at T=2048 (SURVEY.md §8d); K/V re-reads by the
+// only ~4 % of prefill FLOPs at T=2048; K/V re-reads by the
 // G query heads of a KV head are served by L2.
 //
 // kPaged (chunked prefill): the T rows are a CHUNK of each prompt at positions prefix .. prefix+T-1.

@@ -147,8 +147,8 @@ gemm_prefill_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       }
     }
   } else if (warp == 1) {
-    // MMA issuer: the whole warp walks the loop with warp-uniform values (descriptors stay in uniform registers:
-    // no per-instruction R2UR chain as under a `lane == 0` branch), one elected lane issues
+    // MMA issuer: the whole warp walks the loop with warp-uniform values and one elected lane issues (measured faster than the
+    // loop under a `lane == 0` branch)
     constexpr uint32_t idesc = make_idesc(BN);
     const uint64_t adesc0 = make_smem_desc(smem_addr(smem));
     const uint64_t bdesc0 = make_smem_desc(smem_addr(smem) + Cfg::kABytes);
@@ -363,7 +363,7 @@ static int launch_prefill_gemm(const void* x, const void* w, const void* bias, c
 }
 
 // Tile shapes of the persistent kernel and what a round of them costs: cost (us) = rounds x (k-blocks x rows x width x c +
-// epilogue), c fitted per shape on B200 (scratch/exp_gemm_vs_cublas.py, profiles/r2_notes.md).  Two effects: (1) wave
+// epilogue), c fitted per shape on B200.  Two effects: (1) wave
 // quantisation — a 2k-token prefill has few tiles, so the tile WIDTH is chosen to fill whole rounds (UMMA N may be any
 // multiple of 16: 240-column tiles turn 256 / 384 tiles = 1.73 / 2.59 waves into 288 / 416 = 1.95 / 2.81); (2) operand
 // feed — a 256-row tile (two MMAs per weight sub-tile) needs less L2 bandwidth per MMA than a 128-row tile, but its two
@@ -607,7 +607,7 @@ static int gemm_splitk_gated_act(const void* x, const void* w_gu, void* y, int M
 
 int dli_linear_bf16(const void* x, const void* w, const void* bias, const void* residual, void* y, int M, int N,
                     int K, int epilogue, dli_stream_t stream) {
-  // measured on B200 (profiles/r1_notes.md): the CUDA-core GEMV streams at 6.0-7.3 TB/s for M <= 2 but
+  // measured on B200: the CUDA-core GEMV streams at 6.0-7.3 TB/s for M <= 2 but
   // drops to 4.1-5.0 TB/s at M = 3-4 (FMA issue bound); the tensor-core streams hold 5-6
   if (M <= 2 || K % 64 != 0 || N % 16 != 0)
     return dli_gemv_bf16(x, w, bias, residual, y, M, N, K, epilogue, stream);

@@ -14,13 +14,13 @@
 // Groups of R rows are dealt round-robin to a grid sized as a multiple of the SM count,
 // so at any moment the grid streams one contiguous band of the matrix (two balanced
 // dealings were measured and lost, see `deal` in the kernel; so did a software-pipelined
-// 2-row variant for the small matrices, profiles/r2_notes.md).
+// 2-row variant for the small matrices).
 //
 // Programmatic dependent launch: a CTA of the next kernel may move in while this
 // kernel drains; it waits (pdl_wait) before reading activations.  Prefetching the
 // first task's weights ahead of that wait (registers, or cp.async into shared
 // memory) was measured and gave nothing: the shared-memory variant costs L1
-// capacity that the streaming loads need (profiles/r1_notes.md).
+// capacity that the streaming loads need.
 #include <stdlib.h>
 
 #include "common.cuh"
@@ -61,7 +61,7 @@ gemv_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, const bf16* 
   //     (measured: 444 far-apart streams cost the gate/up matrix 10 % of its bandwidth, 35.2 -> 39.0 us);
   //  2  the full waves round-robin as in 0, then the outputs of the ragged last wave split evenly over ALL
   //     CTAs in groups of 1..kOutPerTask — the access pattern of 0 with the balance of 1.
-  // Measured on the Llama-3-8B batch-1 step (B200, profiles/r2_notes.md): 0 -> 2.985 ms, 2 -> 3.062 ms,
+  // Measured on the Llama-3-8B batch-1 step (B200): 0 -> 2.985 ms, 2 -> 3.062 ms,
   // 1 -> 3.171 ms.  The ragged wave costs less than short groups do (fewer loads in flight per thread), so
   // 0 stays the default; 1 and 2 remain selectable (DLI_GEMV_DEAL) to reproduce the comparison.
   const int full_waves = deal == 2 ? (N / kOutPerTask) / (int)gridDim.x : 0;  // waves of COMPLETE groups only

@@ -2,10 +2,9 @@
 // loop structure of the CUDA-core GEMV (gemv.cu) with the multiply-adds moved to mma.sync, so the
 // kernel stays an HBM stream where the scalar GEMV becomes FMA-issue bound (4.1-5.0 TB/s at 3-4
 // rows against 6.0-7.3 at 1-2).  Measured 4.2-5.5 TB/s (8B shapes) and 5.0-6.3 TB/s (70B shapes)
-// at 3-8 rows.  dli_linear_bf16 uses it when it has no split-K workspace and the matrix has too
-// few 128-row tiles to fill the GPU with the swap-AB tcgen05 kernel (that kernel: 1.8 TB/s on
-// 4096 x 14336).  Inside the decode step the engine passes a workspace and the split-K tcgen05
-// stream is faster (profiles/r1_notes.md), so this kernel is not on that path.
+// at 3-8 rows.  dli_linear_bf16 uses it for those rows of matrices up to 32 M elements, where its
+// shorter start beats the K-split clusters (the rule stands there).  The engines' decode steps call
+// dli_gemm_bf16 from 3 rows on, so this kernel is not on that path.
 //
 //   y[m, n] = epi( sum_k x[m,k] * w[n,k] ),   w in the HF Linear layout [N, K]
 //

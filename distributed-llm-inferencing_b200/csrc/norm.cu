@@ -2,7 +2,7 @@
 //
 // HBM-bound: algorithmic bytes per row = d*2 (x) [+ d*2 residual] read,
 // d*2 (y) [+ d*2 resid_out] written, + d*2 weight (L2-resident after row 0).
-// Rounding points follow HF exactly (SURVEY.md §7.2):
+// Rounding points follow HF exactly:
 //   h  = bf16(residual + x)                       modeling_llama.py:325,:331
 //   hn = bf16(float(h) * rsqrt(mean(h^2) + eps))  modeling_llama.py:64-66
 //   y  = bf16(weight * hn)                        modeling_llama.py:67

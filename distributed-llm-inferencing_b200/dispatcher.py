@@ -1,7 +1,7 @@
 """Client-side dispatch of an inference request to worker nodes — the caller of the worker
 boundary (reference master/dashboard/views.py:305-455 `process_inference_request`), without
 Django: plain functions over a `post(url, json, headers, timeout)` callable (requests.post by
-default).  SURVEY.md §8f rank 2.  Kept semantics: shards known -> /inference with `shard_ids`
+default).  Kept semantics: shards known -> /inference with `shard_ids`
 (max_length 100, timeout 60, HTTP timeout 120, views.py:345-355); no shards -> /load_model
 (HTTP timeout 300) then /inference on the first active node (views.py:391-421); a non-200
 answer or `status != success` is a failure with the worker's message.

@@ -1,11 +1,11 @@
 """ShardEngine — one contiguous layer range of a causal LM on one B200.
 
 This is the host-side mirror of what the reference worker does with a shard
-(reference worker/app.py:332-372 `run_shard_inference`, intended semantics per
-SURVEY.md §0: run layers [start_layer, end_layer] on hidden states and hand the
+(reference worker/app.py:332-372 `run_shard_inference`, intended semantics: run
+layers [start_layer, end_layer] on hidden states and hand the
 result to the next shard) and, with the full range, of the unsharded path
 (worker/app.py:289-308).  Stage 0 additionally owns the embedding, the last
-stage the final norm, lm_head and the greedy argmax (SURVEY.md §8b).
+stage the final norm, lm_head and the greedy argmax.
 
 PyTorch is plumbing here: device memory, streams, CUDA-graph capture.  All
 arithmetic goes through the C-ABI kernels (ops.py -> include/dli.h).
@@ -28,7 +28,7 @@ _GEMV_MAX_ROWS = int(os.environ.get("DLI_GEMV_MAX_ROWS", "2"))  # rows served by
 
 @dataclass
 class ModelSpec:
-    """Architecture numbers (same fields as the oracle's spec; SURVEY.md §A.2)."""
+    """Architecture numbers (same fields as the oracle's spec)."""
 
     arch: str  # "llama" (Llama / TinyLlama / Mistral) or "gpt2"
     n_layers: int
@@ -92,7 +92,7 @@ class ModelSpec:
         raise ValueError(f"unsupported model_type {mt!r} (llama, mistral, gpt2)")
 
     def layer_weight_bytes(self) -> int:
-        """bf16 bytes of one decoder layer's matrices (SURVEY.md §8d W_layer)."""
+        """bf16 bytes of one decoder layer's matrices."""
         d, hd = self.d_model, self.head_dim
         qkv_o = (self.n_heads + 2 * self.n_kv_heads) * hd * d + self.n_heads * hd * d
         mlp = (3 if self.arch == "llama" else 2) * d * self.d_ff
@@ -105,7 +105,7 @@ class ModelSpec:
         return 2 * 2 * self.n_kv_heads * self.head_dim * (self.n_layers if n_layers is None else n_layers)
 
 
-# SURVEY.md §A.2 shapes (random-init; there are no checkpoints offline)
+# the shapes of the reference's models and of larger ones of their kind (random-init; there are no checkpoints offline)
 NAMED_SPECS = {
     "gpt2": ModelSpec("gpt2", 12, 768, 12, 12, 64, 3072, 50257, 1e-5, 0.0, 0, 1024, True),
     "tinyllama-1.1b": ModelSpec("llama", 22, 2048, 32, 4, 64, 5632, 32000, 1e-5, 10000.0, 0, 2048),
@@ -274,7 +274,7 @@ class ShardEngine:
         """Take HF-named tensors (any dtype, any device), keep ONLY this stage's
         layer range (+ embedding on stage 0, final norm/lm_head on the last
         stage): out-of-range tensors of a reference shard directory are random
-         and are never read."""
+        and are never read."""
         s, dev = self.spec, self.device
 
         def t(name, transpose=False):
@@ -971,7 +971,7 @@ class ShardEngine:
         """on_tokens(ids [B, T + k] int64 on the host): called every 8 decode steps with everything generated so far
         (a streaming client's progress; the steps stay on the CUDA-graph path).
         Greedy generate (the parity mode of worker/app.py:297-305: the reference
-        samples, see SURVEY.md §0 F3).  input_ids: int [B, T] on any device;
+        samples by default).  input_ids: int [B, T] on any device;
         `max_length` is the TOTAL length like the reference's.  Returns int64
         [B, max_length] on the host, plus the per-step last-position logits
         (fp32, host) when return_logits.  `forced` [B, n_new] teacher-forces the
@@ -1014,7 +1014,7 @@ class ShardEngine:
             for i in range(n_new - 1):
                 if (deadline is not None or eos or on_tokens is not None) and (i & 7) == 0:
                     # the reference can only check its timeout around generate() (worker/app.py:293,:311);
-                    # here it is checked between decode steps (SURVEY.md A.3 Q6), together with the EOS rule
+                    # here it is checked between decode steps, together with the EOS rule
                     torch.cuda.current_stream().synchronize()
                     if deadline is not None and time.time() > deadline:
                         raise TimeoutError("Inference generation timed out")

@@ -1,5 +1,5 @@
 """Measurement helpers shared by bench.py and the pipeline bench (pipeline.run_pipeline_bench): the NVML clock
-sampler and the algorithmic byte / FLOP counts of SURVEY.md 8d.  No arithmetic of the path lives here."""
+sampler and the algorithmic byte / FLOP counts.  No arithmetic of the path lives here."""
 from __future__ import annotations
 
 import statistics
@@ -67,13 +67,13 @@ class ClockSampler:
 
 
 def decode_step_bytes(spec, n_layers, has_head, B, S):
-    """Algorithmic HBM bytes of one decode stage pass (SURVEY.md §8d)."""
+    """Algorithmic HBM bytes of one decode stage pass."""
     kv = spec.kv_bytes_per_token(n_layers)
     return n_layers * spec.layer_weight_bytes() + (spec.head_weight_bytes() if has_head else 0) + B * S * kv + B * kv
 
 
 def prefill_flops(spec, B, T):
-    """Algorithmic FLOPs of a prefill (SURVEY.md §8d): linear + causal attention + last-position head."""
+    """Algorithmic FLOPs of a prefill: linear + causal attention + last-position head."""
     p_layer = spec.layer_weight_bytes() // 2
     return 2 * spec.n_layers * p_layer * B * T + 2 * spec.d_model * spec.vocab * B \
         + 4 * B * (T * T // 2) * spec.n_heads * spec.head_dim * spec.n_layers

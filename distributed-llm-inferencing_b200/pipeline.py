@@ -3,7 +3,7 @@ the B200 box, gloo in the CPU tests).
 
 This is the reference's DECLARED design — a model split into N contiguous layer
 ranges on N nodes (shard_model.py:55-66) whose shards pass hidden states along
-(worker/app.py:332-335 comment, never implemented: SURVEY.md §0 F1) — with the
+(worker/app.py:332-335 comment, never implemented) — with the
 HTTP/JSON hop replaced by send/recv of the `[b, d]` bf16 hidden tile between
 neighbouring GPUs, and the sampled `[b]` int32 tokens returned from the last
 stage to stage 0.  There is no collective on this path (no tensor parallelism):
@@ -102,7 +102,7 @@ class PipelineRunner:
 
 
 def run_chunked_prefill(stage, rank: int, world: int, n_micro: int, n_chunks: int, group=None) -> None:
-    """Chunked prefill ("chunk the prefill to pipeline it").  A prompt pass through N
+    """Chunked prefill.  A prompt pass through N
     stages keeps only one stage busy at a time; cut into C chunks of tokens, stage s can work on chunk
     c+1 while stage s+1 works on chunk c (attention reads the earlier chunks' keys/values from the paged
     cache).  This runs chunks 0 .. C-2 of every slot — unit u = slot*(C-1) + chunk, stage s works on unit
@@ -599,7 +599,7 @@ def measure_pipeline(spec, model_name, rank, world, local, b, n_slots, ctx, K, W
     busy = min(M, P) / P  # share of ticks in which a stage has a slot to work on
     ach = torch.tensor([stage_bytes / (tick_ms / 1e3) / 1e9], device="cuda")
     dist.all_reduce(ach, op=dist.ReduceOp.MIN)
-    # what a pure layer pipeline can reach at this batch: every stage re-reads its weights once per slot (SURVEY 8d)
+    # what a pure layer pipeline can reach at this batch: every stage re-reads its weights once per slot
     ceiling = M * b / (P * (stage_bytes / (peaks["hbm_gbs"] * 1e9)))
     res = {"value": M * b * K / (ms / 1e3), "ms_per_step": ms / K, "gpu_launches": int(launches.item()),
            "clocks": clk.summary(), "tick_ms": tick_ms, "prefill_ms": pf_ms,
@@ -750,7 +750,7 @@ def serve_e2e(spec, model_name, rank, world, local, ctx, n_short, n_long, hop, p
     return out
 
 
-# BASELINE.json configs run on exactly N GPUs: (model, total batch, context, note)
+# workloads stated for exactly N GPUs: (model, total batch, context, note)
 NAMED_CONFIGS = {
     2: ("tinyllama-1.1b", 1, 1024, "configs[1]: TinyLlama-1.1B, 2 layer-range shards, batch 1 greedy decode"),
     4: ("mistral-7b", 64, 4096, "configs[3]: Mistral-7B, 4 shards, micro-batched decode, batch 64, 4k context"),
@@ -799,7 +799,7 @@ def run_pipeline_bench(args, spec, peaks):
                      "prefill_tokens_per_s": r["prefill_tokens_per_s"], "prefill_chunks": r["prefill_chunks"],
                      "parity_check": r["parity_check"], "clocks": r["clocks"], "workload": r["workload"],
                      "note": "a pure layer pipeline re-reads every stage's weights once per micro-batch, so its ceiling is "
-                             "batch / (period x stage-pass time at the HBM peak), not the once-per-step figure of BASELINE.md 4"}
+                             "batch / (period x stage-pass time at the HBM peak), not the figure of one read per step"}
         except RuntimeError as e:
             if "pipeline tokens differ" in str(e):
                 raise
@@ -812,7 +812,7 @@ def run_pipeline_bench(args, spec, peaks):
     roof = {"bound": "hbm", "kernel": "stage pass (all kernels of one micro-batch on one stage)",
             "achieved": main["stage_pass_gbs"], "peak": peaks["hbm_gbs"], "unit": "GB/s", "frac": main["stage_pass_frac"],
             "traffic": None, "bytes_per_launch": main["stage_bytes"], "micro_batches": main["slots"],
-            "note": "min over stages; every stage re-reads its weights once per micro-batch (SURVEY 8d)"}
+            "note": "min over stages; every stage re-reads its weights once per micro-batch"}
     Mb = main["slots"] * main["b"]
     return {"value": main["value"], "ms_per_step": main["ms_per_step"], "gpu_launches": main["gpu_launches"],
             "clocks": main["clocks"],

@@ -3,8 +3,8 @@ CONCURRENT requests.
 
 The reference deploys one worker per node, registers shard i on node i (`/load_shard`, worker/app.py:139-206; one
 node per (model, shard): master/dashboard/models.py:27-28) and sends `/inference` with the shards of the first node
-that has any (master/dashboard/views.py:318-355) — whose worker then runs only its own shard (worker/app.py:336,
-SURVEY.md A.3 Q2), one request at a time (one sync gunicorn worker, worker/Dockerfile:45).  Here
+that has any (master/dashboard/views.py:318-355) — whose worker then runs only its own shard (worker/app.py:336),
+one request at a time (one sync gunicorn worker, worker/Dockerfile:45).  Here
 
     python -m torch.distributed.run --nproc-per-node N -m dli_b200.pipeline_worker --port 5000
 

@@ -7,7 +7,7 @@ Keeps the reference's shard-assignment semantics
     sibling `tokenizer/` directory (consumed at worker/app.py:168,:177);
   * `metadata.json` = {model_name, shard_id, num_shards, start_layer,
     end_layer (inclusive), total_layers}.
-What it does NOT keep is the reference's storage defect (SURVEY.md §0 F2): the
+What it does NOT keep is the reference's storage defect: the
 reference saves a full-depth model per shard with random out-of-range layers.
 `write_shards` stores only the tensors of the shard's layer range (+ embedding on
 shard 0, final norm / lm_head on the last shard), and `load_hf_state_dict` reads
@@ -129,7 +129,7 @@ def load_named_tensors(path: str, names) -> Dict[str, torch.Tensor]:
 
 def write_shards(state_dict: Dict[str, torch.Tensor], config: Dict[str, object], model_name: str, n_shards: int,
                  output_dir: str = "model_shards") -> List[str]:
-    """Real shard materialiser (SURVEY.md §8f rank 1): the same CLI contract as
+    """Real shard materialiser: the same CLI contract as
     `manage.py shard_model --model_name --num_shards --output_dir`
     (shard_model.py:11-14), but each shard directory holds only its own tensors."""
     from safetensors.torch import save_file
@@ -181,7 +181,7 @@ def shard_model_dir(source_dir: str, model_name: str, n_shards: int, output_dir:
     at a time into output files of at most `max_file_bytes` (with a `model.safetensors.index.json`), so a 70B
     checkpoint (141 GB) is sharded with a few GB of RAM — the reference instantiates the full model once per shard
     (shard_model.py:37,71).  Works for every architecture whose layers are `model.layers.N.` or `transformer.h.N.`
-    (Llama, Mistral, TinyLlama, GPT-2): the reference's own Llama branch crashes (SURVEY.md A.3 Q5)."""
+    (Llama, Mistral, TinyLlama, GPT-2): the reference's own Llama branch crashes."""
     import shutil
 
     from safetensors.torch import save_file

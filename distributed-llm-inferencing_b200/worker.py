@@ -1,8 +1,7 @@
 """Drop-in for the reference worker service (reference worker/app.py).
 
 Same routes, methods, JSON keys, status codes and environment variables as the
-Flask app the master talks to (worker/app.py:49-330; contract table SURVEY.md
-§A.1; behaviour recorded from the reference itself in
+Flask app the master talks to (worker/app.py:49-330; behaviour recorded from the reference itself in
 tests/golden/worker_contract.json):
 
     GET  /health          worker/app.py:49-92
@@ -15,7 +14,7 @@ tests/golden/worker_contract.json):
 the model object is a ShardEngine on the B200 instead of a transformers model on
 the CPU.  Built on werkzeug (Flask is not installed; werkzeug is what Flask wraps).
 
-Deliberate deviations from the reference (SURVEY.md §A.3), each a fixed defect:
+Deliberate deviations from the reference, each a fixed defect:
   Q1  `shard_id: 0` is accepted (the reference's `all([...])` rejects falsy ids);
   Q2  every shard id of the request is used (the reference silently uses only the
       first), as an in-process layer-range chain; the shards must cover all layers;

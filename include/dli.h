@@ -6,7 +6,7 @@
  * i.e. what `model.generate(...)` executes at worker/app.py:297-305 and
  * worker/app.py:359-367 (reference paths are relative to the reference repo;
  * `TF:` paths are relative to the `transformers` package the reference calls,
- * which is where the arithmetic lives — SURVEY.md §8c).
+ * which is where the arithmetic lives).
  *
  * Conventions
  *   - plain pointers and sizes only; every pointer is CALLER-OWNED DEVICE memory
@@ -203,7 +203,7 @@ int dli_attn_prefill_tc_bf16(const void* qkv, void* out, int B, int T, int H, in
 
 /* Causal attention of a CHUNK of each prompt against the whole context so far
  * (chunked prefill: the prompt is fed T tokens at a time so that pipeline
- * stages can work on different chunks at once, SURVEY.md 8e).  Same reference
+ * stages can work on different chunks at once).  Same reference
  * lines and arithmetic as dli_attn_prefill_bf16.  qkv holds the chunk's rows
  * (already rotated) at positions prefix .. prefix+T-1 of each sequence; keys
  * and values of positions 0 .. prefix+T-1 are read from the paged cache, so

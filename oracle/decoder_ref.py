@@ -5,7 +5,7 @@ reference worker executes through `model.generate(...)` at
 reference worker/app.py:297-305 and :359-367.  The arithmetic itself lives in the
 un-vendored third-party dependency `transformers` (pinned 4.30.2 in
 worker/requirements.txt:2; the pin predates GQA / rope_theta / Mistral and is not
-installable offline, so — per SURVEY.md §8c — the restatement follows the
+installable offline, so the restatement follows the
 installed transformers 5.5.0, cited as `TF:` paths below).
 
 Pinning: tests/test_oracle.py checks this file against (a) transformers itself,
@@ -13,7 +13,7 @@ imported in the test process, on the same seeded weights (logits, hidden states
 at shard boundaries, greedy tokens) and (b) the committed fixtures in
 tests/golden/ produced by oracle/gen_golden.py from transformers and from the
 reference's own worker/app.py.  The reference repository contains no tests or
-golden vectors of its own (SURVEY.md §4), so transformers is the only pin.
+golden vectors of its own, so transformers is the only pin.
 
 Only tests/, __graft_entry__.smoke() and bench.py's CPU-baseline legs may import
 this module.
@@ -37,7 +37,7 @@ import torch.nn.functional as F
 
 @dataclass
 class ModelSpec:
-    """Architecture numbers the forward needs (SURVEY.md §A.2)."""
+    """Architecture numbers the forward needs."""
 
     arch: str  # "llama" (Llama/TinyLlama/Mistral) or "gpt2"
     n_layers: int
@@ -234,7 +234,7 @@ def embed(ids: torch.Tensor, sd, spec: ModelSpec, pos0: int) -> torch.Tensor:
 
 def run_layers(h, sd, spec: ModelSpec, start: int, end: int, cache: KVCache, pos0: int) -> torch.Tensor:
     """Layers start..end inclusive on hidden states [B,T,d] — the intended shard
-    unit of reference worker/app.py:332-372 (SURVEY.md §0 F1)."""
+    unit of reference worker/app.py:332-372."""
     T = h.shape[1]
     if spec.arch == "llama":
         cos, sin = rope_cos_sin(spec, torch.arange(pos0, pos0 + T), h.dtype)

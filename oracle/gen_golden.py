@@ -244,7 +244,7 @@ def gen_worker_contract():
 # ------------------------------------------------------------------ reference sharder
 def gen_shard_ranges():
     """Run the reference's shard_model command on tiny GPT-2 models (its only working
-    branch, SURVEY.md §A.3 Q5) and record the metadata.json files it writes."""
+    branch) and record the metadata.json files it writes."""
     import transformers
 
     dj = types.ModuleType("django")
