@@ -54,7 +54,8 @@ __device__ __forceinline__ void cluster_barrier() {
 //   kRowsRope: the qkv projection of a prompt pass; the epilogue rotates q and k as rope_kv_append_kernel does on the
 //   stored bf16 values (a tile holds one 128-wide or two 64-wide heads, so a rotation pair meets in the tile's sums) and
 //   writes k and v to the cache pages too.
-template <int kMode>
+// kAnyBias: a bias that does not start on 16 bytes (a form of its own: the test in the kernel cost 0.04 us of every call).
+template <int kMode, bool kAnyBias = false>
 __global__ void __launch_bounds__(kRowsThreads, 2)
 gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX,
                  const bf16* __restrict__ bias, const bf16* residual, bf16* y, int M, int N, int K, int epilogue, int BN,
@@ -214,15 +215,13 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     float bb[8], bb2[8];
     {
       uint4 bv = make_uint4(0u, 0u, 0u, 0u), bv2 = bv;
-      const bool biased = !kGated && (epilogue & DLI_EPI_BIAS);
-      const bool whole = (reinterpret_cast<uintptr_t>(bias) & 15u) == 0;
-      if (biased && whole) {
+      if (!kAnyBias && !kGated && (epilogue & DLI_EPI_BIAS)) {
         bv = ld_16B(bias + n);
         if (kMode == kRowsRope) bv2 = ld_16B(bias + n + half);
       }
       unpack8(bv, bb);
       unpack8(bv2, bb2);
-      if (biased && !whole) {  // a slice of a longer vector may start anywhere
+      if (kAnyBias) {  // a slice of a longer vector may start anywhere
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
           bb[e] = __bfloat162float(bias[n + e]);
@@ -350,9 +349,14 @@ static int rows_setup(int* capacity /*[kRowsMaxCluster + 1]: CTAs that run at on
   static PerDeviceOnce once;
   static int cap[kMaxDevices][kRowsMaxCluster + 1];
   DLI_ONCE_PER_DEVICE(once, dev, {
-    DLI_CUDA_CALL(cudaFuncSetAttribute(gemm_rows_kernel<kRowsPlain>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowsMaxSmem));
-    DLI_CUDA_CALL(cudaFuncSetAttribute(gemm_rows_kernel<kRowsGated>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowsMaxSmem));
-    DLI_CUDA_CALL(cudaFuncSetAttribute(gemm_rows_kernel<kRowsRope>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowsMaxSmem));
+    const auto ring = [](const void* kernel) {
+      return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowsMaxSmem);
+    };
+    DLI_CUDA_CALL(ring((const void*)gemm_rows_kernel<kRowsPlain>));
+    DLI_CUDA_CALL(ring((const void*)gemm_rows_kernel<kRowsGated>));
+    DLI_CUDA_CALL(ring((const void*)gemm_rows_kernel<kRowsRope>));
+    DLI_CUDA_CALL(ring((const void*)gemm_rows_kernel<kRowsPlain, true>));
+    DLI_CUDA_CALL(ring((const void*)gemm_rows_kernel<kRowsRope, true>));
     for (int c = 1; c <= kRowsMaxCluster; ++c) {
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3(c, 64, 64);
@@ -455,12 +459,12 @@ int plan_gemm_rows(int M, int N, int K, RowsShape* shape, double* us) {
   return DLI_OK;
 }
 
-template <int kMode>
+template <int kMode, bool kAnyBias = false>
 static int launch_rows(const CUtensorMap& tmW, const CUtensorMap& tmX, const void* bias, const void* residual, void* y, int M,
                        int N, int K, int epilogue, const RowsShape& sh, cudaStream_t s, const RopeArgs& rope, int hd) {
   const int cols = sh.bn <= 32 ? 32 : sh.bn <= 64 ? 64 : sh.bn <= 128 ? 128 : 256;
   const dim3 grid(sh.splits, (M + sh.bn - 1) / sh.bn, (N + 127) / 128);
-  const cudaError_t e = launch_kernel_cluster(gemm_rows_kernel<kMode>, grid, dim3(kRowsThreads), rows_smem(sh.bn, sh.stages), s,
+  const cudaError_t e = launch_kernel_cluster(gemm_rows_kernel<kMode, kAnyBias>, grid, dim3(kRowsThreads), rows_smem(sh.bn, sh.stages), s,
                                               (unsigned)sh.splits, tmW, tmX, (const bf16*)bias, (const bf16*)residual,
                                               (bf16*)y, M, N, K, epilogue, sh.bn, sh.stages, cols, rope, hd);
   if (e != cudaSuccess) return fail(DLI_ERR_CUDA, "gemm_rows_kernel: %s", cudaGetErrorString(e));
@@ -479,9 +483,11 @@ int launch_gemm_rows(RowsMode mode, const void* x, const void* w, const void* bi
   CUtensorMap tmW, tmX;
   if ((rc = make_tmap(&tmW, w, N, K, mode == kRowsGated ? 64 : 128)) != DLI_OK) return rc;
   if ((rc = make_tmap(&tmX, x, M, K, sh.bn)) != DLI_OK) return rc;
-  if (mode == kRowsGated) return launch_rows<kRowsGated>(tmW, tmX, bias, residual, y, M, N, K, epilogue, sh, s, rope, hd);
-  if (mode == kRowsRope) return launch_rows<kRowsRope>(tmW, tmX, bias, residual, y, M, N, K, epilogue, sh, s, rope, hd);
-  return launch_rows<kRowsPlain>(tmW, tmX, bias, residual, y, M, N, K, epilogue, sh, s, rope, hd);
+  const bool any_bias = mode != kRowsGated && (epilogue & DLI_EPI_BIAS) && !aligned16(bias);
+  const auto launch = mode == kRowsGated ? launch_rows<kRowsGated>
+                      : mode == kRowsRope ? (any_bias ? launch_rows<kRowsRope, true> : launch_rows<kRowsRope>)
+                                          : (any_bias ? launch_rows<kRowsPlain, true> : launch_rows<kRowsPlain>);
+  return launch(tmW, tmX, bias, residual, y, M, N, K, epilogue, sh, s, rope, hd);
 }
 
 }  // namespace dli
