@@ -59,7 +59,9 @@ int dli_sm_count(void);
  * on (process-wide; returns the previous setting).  When on, a kernel may begin
  * (and the weight-streaming kernels prefetch their first weight chunk) while its
  * predecessor in the stream drains; each kernel waits for the predecessor's
- * results before reading activations, so results do not change.  Off by
+ * results before reading activations, so results do not change.  Two entry
+ * points read more than weights early and say so: the fused decode attention
+ * and dli_postnorm_add_norm_conv_single_ahead.  Off by
  * default; the host engine turns it on for the decode step. */
 int dli_set_pdl(int enable);
 
@@ -136,6 +138,10 @@ int dli_paged_attn_decode_bf16(const void* q, int q_stride, const void* k_cache,
  * q is rotated on the fly, the new k is rotated and written with v into the
  * sequence's cache page (k_cache / v_cache are written), then attended with
  * the rest of the context.  cos == NULL: no rotation (GPT-2).
+ * Under programmatic dependent launch seq_lens, page_table and the cache rows of
+ * the OLD tokens are read while the launch just before it on the stream may
+ * still run: that launch must write none of them (normally it is the qkv
+ * projection).
  * l2_prefetch_a / _b (optional, may be NULL): device ranges — normally the
  * weights of the projections that follow — pulled into L2 with
  * cp.async.bulk.prefetch by spare CTAs while the attention kernel (a) and the
