@@ -183,32 +183,62 @@ __device__ __forceinline__ uint4 pack8(const float* f) {
 // Activations, evaluated the way torch evaluates them on a bf16 tensor:
 // upcast to fp32, compute, round once to bf16 (the caller rounds).
 __device__ __forceinline__ float silu_f(float x) { return x / (1.0f + expf(-x)); }
+// Two values rounded to bf16 by ONE conversion: conversions, ex2 and reciprocals share a pipe of 16 lanes per clock and SM,
+// which is what bounds the epilogues of the projections.
+__device__ __forceinline__ void round2_bf16(float& a, float& b) {
+  const uint32_t u = pack_bf16(a, b);
+  a = bf_lo(u);
+  b = bf_hi(u);
+}
+// silu(x) for an x that is a bf16 value, to be rounded to bf16: then the bits of round_bf16(silu_f(x)) for all 65 536 of them
+// (tested one by one), from one ex2 and one reciprocal.  expf and the division are a dozen instructions and a branch per gate.
+__device__ __forceinline__ float silu_of_bf16(float x) {
+  const float sc = x < -64.f ? 0x1p-24f : 1.f;  // 1 + e^-x up to 2^127: its reciprocal must not be a denormal
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"((1.f + ex2_ftz(x * -1.4426950408889634f)) * sc));
+  return x * sc * r;
+}
 // gelu_new (tanh approximation), TF:activations.py:59-66
 __device__ __forceinline__ float gelu_new_f(float x) {
   const float k = 0.7978845608028654f;  // sqrt(2/pi)
   return 0.5f * x * (1.0f + tanhf(k * (x + 0.044715f * x * x * x)));
 }
+// gelu_new(x) for an x that is a bf16 value, to be rounded to bf16, from one ex2 and one reciprocal: 0.5 (1 + tanh z) =
+// 1 / (1 + e^(-2z)), which loses nothing where 1 + tanh z cancels.  Of all bf16 values 5 (below -10) do not come out as the
+// rounding of the exact result, with gelu_new_f 155 (below -2.9).
+__device__ __forceinline__ float gelu_of_bf16(float x) {
+  const float sc = x < -8.f ? 0x1p-24f : 1.f;  // as above
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"((1.f + ex2_ftz(-2.302208198144325f * (x + 0.044715f * x * x * x))) * sc));
+  return x * sc * r;
+}
 // The tanh form of gelu at silu's cost: 0.5 (1 + tanh z) = 1 / (1 + e^(-2z)).
 __device__ __forceinline__ float gelu_gate(float x) {
   return x / (1.0f + expf(-1.5957691216057308f * (x + 0.044715f * x * x * x)));
 }
-// Epilogue of a gated projection pair.  act == NULL: silu(gate) * up with the rounding points of a bf16 framework.
+// Epilogue of a gated projection pair.  act == NULL: silu(gate) * up with the rounding points of a bf16 framework (gate and up
+// come rounded to bf16).
 // act = {limit, alpha} (two floats on the device): the clamped form g * sigmoid(alpha g) * (u + 1) with
 // g = min(gate, limit), u = clamp(up, -limit, limit); limit <= 0: gelu (tanh form) of the gate, times up.
 __device__ __forceinline__ float gated_combine(float gte, float up, const float* __restrict__ act) {
-  if (act == nullptr) return round_bf16(silu_f(gte)) * up;
+  if (act == nullptr) return round_bf16(silu_of_bf16(gte)) * up;
   const float lim = act[0], alpha = act[1];
   if (lim <= 0.f) return gelu_gate(gte) * up;
   const float g = fminf(gte, lim), u = fminf(fmaxf(up, -lim), lim);
   return g / (1.0f + expf(-alpha * g)) * (u + 1.0f);
 }
 
-// The same on N gates (in place) and N ups: one test of the form for all of them.
+// The same on N gates (in place) and N ups, N even: one test of the form for all of them.
 template <int N>
 __device__ __forceinline__ void gated_combine_n(float (&g)[N], const float (&u)[N], const float* __restrict__ act) {
   if (act == nullptr) {
 #pragma unroll
-    for (int j = 0; j < N; ++j) g[j] = gated_combine(g[j], u[j], nullptr);
+    for (int j = 0; j < N; j += 2) {
+      float s0 = silu_of_bf16(g[j]), s1 = silu_of_bf16(g[j + 1]);
+      round2_bf16(s0, s1);
+      g[j] = s0 * u[j];
+      g[j + 1] = s1 * u[j + 1];
+    }
     return;
   }
   const float lim = act[0], alpha = act[1];

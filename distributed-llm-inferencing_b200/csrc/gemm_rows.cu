@@ -54,7 +54,8 @@ __device__ __forceinline__ void cluster_barrier() {
 //   kRowsRope: the qkv projection of a prompt pass; the epilogue rotates q and k as rope_kv_append_kernel does on the
 //   stored bf16 values (a tile holds one 128-wide or two 64-wide heads, so a rotation pair meets in the tile's sums) and
 //   writes k and v to the cache pages too.
-// kAnyBias: a bias that does not start on 16 bytes (a form of its own: the test in the kernel cost 0.04 us of every call).
+// kAnyBias: a bias that does not start on 16 bytes, or the parameters of a gated activation (forms of their own: the tests in
+// the kernel cost 0.04 us of every call, and more where the clamped activation stands beside silu).
 template <int kMode, bool kAnyBias = false>
 __global__ void __launch_bounds__(kRowsThreads, 2)
 gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX,
@@ -221,7 +222,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
       }
       unpack8(bv, bb);
       unpack8(bv2, bb2);
-      if (kAnyBias) {  // a slice of a longer vector may start anywhere
+      if (kAnyBias && !kGated) {  // a slice of a longer vector may start anywhere
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
           bb[e] = __bfloat162float(bias[n + e]);
@@ -280,26 +281,32 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
         }
         if (kGated) {
 #pragma unroll
-          for (int e = 0; e < 8; ++e) a[e] = round_bf16(a[e]), b[e] = round_bf16(b[e]);
-          gated_combine_n(a, b, reinterpret_cast<const float*>(bias));
+          for (int e = 0; e < 8; ++e) round2_bf16(a[e], b[e]);
+          gated_combine_n(a, b, kAnyBias ? reinterpret_cast<const float*>(bias) : nullptr);
           st_16B(y + at, pack8(a));
           continue;
         }
 #pragma unroll
-        for (int e = 0; e < 8; ++e) a[e] = round_bf16(a[e] + bb[e]);
+        for (int e = 0; e < 8; ++e) a[e] += bb[e];
+#pragma unroll
+        for (int e = 0; e < 8; e += 2) round2_bf16(a[e], a[e + 1]);
         if (kMode == kRowsPlain) {
           float rr[8];
           unpack8(pre1[q], rr);
           if (epilogue & DLI_EPI_GELU_NEW) {
 #pragma unroll
-            for (int e = 0; e < 8; ++e) a[e] = round_bf16(gelu_new_f(a[e]));
+            for (int e = 0; e < 8; ++e) a[e] = gelu_of_bf16(a[e]);
+#pragma unroll
+            for (int e = 0; e < 8; e += 2) round2_bf16(a[e], a[e + 1]);
           }
 #pragma unroll
           for (int e = 0; e < 8; ++e) a[e] += rr[e];
           st_16B(y + at, pack8(a));
         } else {
 #pragma unroll
-          for (int e = 0; e < 8; ++e) b[e] = round_bf16(b[e] + bb2[e]);
+          for (int e = 0; e < 8; ++e) b[e] += bb2[e];
+#pragma unroll
+          for (int e = 0; e < 8; e += 2) round2_bf16(b[e], b[e + 1]);
           if (turned) {
             float cs[8], sn[8];
             unpack8(pre1[q], cs);
@@ -307,8 +314,11 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
               const float x1 = a[e], x2 = b[e];
-              a[e] = round_bf16(x1 * cs[e]) + round_bf16(-x2 * sn[e]);
-              b[e] = round_bf16(x2 * cs[e]) + round_bf16(x1 * sn[e]);
+              float p = x1 * cs[e], q1 = -x2 * sn[e], q2 = x2 * cs[e], t = x1 * sn[e];
+              round2_bf16(p, q1);
+              round2_bf16(q2, t);
+              a[e] = p + q1;
+              b[e] = q2 + t;
             }
           }
           const uint4 u1 = pack8(a), u2 = pack8(b);
@@ -357,6 +367,7 @@ static int rows_setup(int* capacity /*[kRowsMaxCluster + 1]: CTAs that run at on
     DLI_CUDA_CALL(ring((const void*)gemm_rows_kernel<kRowsRope>));
     DLI_CUDA_CALL(ring((const void*)gemm_rows_kernel<kRowsPlain, true>));
     DLI_CUDA_CALL(ring((const void*)gemm_rows_kernel<kRowsRope, true>));
+    DLI_CUDA_CALL(ring((const void*)gemm_rows_kernel<kRowsGated, true>));
     for (int c = 1; c <= kRowsMaxCluster; ++c) {
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3(c, 64, 64);
@@ -483,8 +494,8 @@ int launch_gemm_rows(RowsMode mode, const void* x, const void* w, const void* bi
   CUtensorMap tmW, tmX;
   if ((rc = make_tmap(&tmW, w, N, K, mode == kRowsGated ? 64 : 128)) != DLI_OK) return rc;
   if ((rc = make_tmap(&tmX, x, M, K, sh.bn)) != DLI_OK) return rc;
-  const bool any_bias = mode != kRowsGated && (epilogue & DLI_EPI_BIAS) && !aligned16(bias);
-  const auto launch = mode == kRowsGated ? launch_rows<kRowsGated>
+  const bool any_bias = mode == kRowsGated ? bias != nullptr : (epilogue & DLI_EPI_BIAS) && !aligned16(bias);
+  const auto launch = mode == kRowsGated ? (any_bias ? launch_rows<kRowsGated, true> : launch_rows<kRowsGated>)
                       : mode == kRowsRope ? (any_bias ? launch_rows<kRowsRope, true> : launch_rows<kRowsRope>)
                                           : (any_bias ? launch_rows<kRowsPlain, true> : launch_rows<kRowsPlain>);
   return launch(tmW, tmX, bias, residual, y, M, N, K, epilogue, sh, s, rope, hd);

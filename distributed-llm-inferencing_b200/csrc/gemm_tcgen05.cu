@@ -293,7 +293,7 @@ gemm_prefill_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
               if (kGated) {
                 float up[16];
 #pragma unroll
-                for (int j = 0; j < 16; ++j) { v[j] = round_bf16(v[j]); up[j] = round_bf16(__uint_as_float(r2[j])); }
+                for (int j = 0; j < 16; ++j) { up[j] = __uint_as_float(r2[j]); round2_bf16(v[j], up[j]); }
                 gated_combine_n(v, up, reinterpret_cast<const float*>(bias));
               } else {
                 if (epilogue & DLI_EPI_BIAS) {
@@ -304,7 +304,7 @@ gemm_prefill_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                 for (int j = 0; j < 16; ++j) v[j] = round_bf16(v[j]);
                 if (epilogue & DLI_EPI_GELU_NEW) {
 #pragma unroll
-                  for (int j = 0; j < 16; ++j) v[j] = round_bf16(gelu_new_f(v[j]));
+                  for (int j = 0; j < 16; ++j) v[j] = round_bf16(gelu_of_bf16(v[j]));
                 }
               }
               bf16* dst = y + (size_t)m * n_out + n0;

@@ -249,7 +249,7 @@ gemv_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, const bf16* 
         } else {
           if (epilogue & DLI_EPI_BIAS) s += __bfloat162float(bias[n]);
           v = round_bf16(s);
-          if (epilogue & DLI_EPI_GELU_NEW) v = round_bf16(gelu_new_f(v));
+          if (epilogue & DLI_EPI_GELU_NEW) v = round_bf16(gelu_of_bf16(v));
           if (epilogue & DLI_EPI_RESIDUAL) v += __bfloat162float(residual[(size_t)m * N + n]);
         }
         const bf16 yb = __float2bfloat16_rn(v);

@@ -115,11 +115,11 @@ gemv_mma_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, const bf
         float v;
         if (kGated) {
           const float gte = round_bf16(s), up = round_bf16(s2);
-          v = round_bf16(silu_f(gte)) * up;
+          v = round_bf16(silu_of_bf16(gte)) * up;
         } else {
           if (epilogue & DLI_EPI_BIAS) s += __bfloat162float(bias[n]);
           v = round_bf16(s);
-          if (epilogue & DLI_EPI_GELU_NEW) v = round_bf16(gelu_new_f(v));
+          if (epilogue & DLI_EPI_GELU_NEW) v = round_bf16(gelu_of_bf16(v));
           if (epilogue & DLI_EPI_RESIDUAL) v += __bfloat162float(residual[(size_t)m * n_out + n]);
         }
         y[(size_t)m * n_out + n] = __float2bfloat16_rn(v);
