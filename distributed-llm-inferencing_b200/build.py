@@ -28,6 +28,7 @@ SOURCES = [
     "gemv_mma.cu",
     "gemm_tcgen05.cu",
     "gemm_rows.cu",
+    "gemm_pair.cu",
     "prompt.cu",
     "elementwise.cu",
     "sample.cu",

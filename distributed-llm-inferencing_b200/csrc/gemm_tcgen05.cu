@@ -6,14 +6,14 @@
 //                                              K contiguous) = HF Linear layout
 //
 // Persistent kernel for prompt passes of many rows; fewer rows (and every projection of a batched decode step) run as
-// K-split clusters with swapped operands (gemm_rows.cu), chosen per call by estimated time (use_rows below).
+// K-split clusters with swapped operands (gemm_rows.cu), chosen per call by estimated time (choose below).
 // Gated MLP (template kGated): w is the [gate128 | up128]-interleaved matrix, one BN = 256 tile holds gate columns 0-127
 //   and up columns 128-255; the epilogue computes bf16(silu(bf16(g))) * bf16(u) — the HF rounding points.
 //
 // Tensor-bound: 2*M*N*K FLOPs per launch.
 #include <stdlib.h>
 
-#include "gemm_rows.cuh"
+#include "gemm_pair.cuh"
 #include "tcgen05_utils.cuh"
 
 namespace dli {
@@ -68,19 +68,12 @@ __device__ __forceinline__ void prefill_tile_coords(int tile, int m_tiles, int n
   m_blk = m0 + r - n_blk * gsize;
 }
 
-// kRope (the qkv projection of a prompt pass, head_dim 128, 128 x 256 tiles = two whole heads per tile): the epilogue
-// rotates q and k (rotate-half RoPE with the rounding points of apply_rotary_pos_emb on bf16 tensors,
-// TF:models/llama/modeling_llama.py:138-168, applied to the bf16-rounded projection exactly as the separate
-// rope_kv_append_kernel applies it to the stored one) and appends k and v to the paged cache — the work of
-// dli_rope_kv_append_bf16 without a second pass over the qkv matrix.
-//
 // threads: TMA warp + MMA warp + four epilogue warps per 128-row half
-template <int BN, bool kGated, int MT, bool kRope = false>
+template <int BN, bool kGated, int MT>
 __global__ void __launch_bounds__(64 + 128 * MT, 1)
 gemm_prefill_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     const bf16* __restrict__ bias, const bf16* residual, bf16* y, int M, int N, int K,
-                    int epilogue, int m_tiles, int num_tiles, const __grid_constant__ RopeArgs rope) {
-  static_assert(!kRope || (BN == 256 && !kGated && MT == 1), "the RoPE epilogue works on two whole 128-wide heads");
+                    int epilogue, int m_tiles, int num_tiles) {
   using Cfg = PrefillCfg<BN, kGated, MT>;
   constexpr int S = Cfg::kStages;
   constexpr int kMRows = MT * 128;
@@ -196,76 +189,7 @@ gemm_prefill_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       // per 16 columns before).  A chunk of 16 columns ahead instead: 127 -> 198, the store and the load share the line.
       constexpr int kLine = kGated ? 16 : 64;
       const int n_out = kGated ? N / 2 : N;
-      if constexpr (kRope) {
-        const uint32_t lane_base = tmem_base + as * Cfg::kAccCols + ((uint32_t)(quad * 32) << 16);
-        const int m = m_blk * 128 + quad * 32 + lane;
-        const bool live = m < M;
-        int pos = 0;
-        size_t cache_row = 0;  // ((page * KV) * page_size + slot): + kvh * page_size gives the token's row of a kv head
-        if (live) {
-          pos = rope.positions[m];
-          const int page = rope.page_table[(size_t)rope.seq_ids[m] * rope.max_pages + (pos >> rope.page_shift)];
-          cache_row = ((size_t)page * rope.KV << rope.page_shift) + (pos & ((1 << rope.page_shift) - 1));
-        }
-#pragma unroll 1
-        for (int hh = 0; hh < 2; ++hh) {
-          const int head = (n_tile0 >> 7) + hh;  // q heads, then k heads, then v heads
-          if (head >= rope.H + 2 * rope.KV) break;
-          bf16* yrow = y + (size_t)m * N + (size_t)head * 128;
-          if (head < rope.H + rope.KV) {
-            bf16* crow = head >= rope.H ? rope.k_cache + (cache_row + ((size_t)(head - rope.H) << rope.page_shift)) * 128 : nullptr;
-#pragma unroll 1
-            for (int j = 0; j < 4; ++j) {  // 16 rotation pairs (i, i + 64) per step
-              uint32_t r1[16], r2[16];
-              tmem_ld_32x16(lane_base + hh * 128 + j * 16, r1);
-              tmem_ld_32x16(lane_base + hh * 128 + 64 + j * 16, r2);
-              tmem_ld_wait();
-              if (live) {
-                float c[16], sn[16], o1[16], o2[16];
-                unpack8(ld_16B(rope.cos_t + (size_t)pos * 64 + j * 16), c);
-                unpack8(ld_16B(rope.cos_t + (size_t)pos * 64 + j * 16 + 8), c + 8);
-                unpack8(ld_16B(rope.sin_t + (size_t)pos * 64 + j * 16), sn);
-                unpack8(ld_16B(rope.sin_t + (size_t)pos * 64 + j * 16 + 8), sn + 8);
-#pragma unroll
-                for (int e = 0; e < 16; ++e) {
-                  const float x1 = round_bf16(__uint_as_float(r1[e])), x2 = round_bf16(__uint_as_float(r2[e]));
-                  o1[e] = round_bf16(x1 * c[e]) + round_bf16(-x2 * sn[e]);
-                  o2[e] = round_bf16(x2 * c[e]) + round_bf16(x1 * sn[e]);
-                }
-#pragma unroll
-                for (int v8 = 0; v8 < 2; ++v8) {
-                  const uint4 u1 = pack8(o1 + v8 * 8), u2 = pack8(o2 + v8 * 8);
-                  st_16B(yrow + j * 16 + v8 * 8, u1);
-                  st_16B(yrow + 64 + j * 16 + v8 * 8, u2);
-                  if (crow) {
-                    st_16B(crow + j * 16 + v8 * 8, u1);
-                    st_16B(crow + 64 + j * 16 + v8 * 8, u2);
-                  }
-                }
-              }
-            }
-          } else {
-            bf16* crow = rope.v_cache + (cache_row + ((size_t)(head - rope.H - rope.KV) << rope.page_shift)) * 128;
-#pragma unroll 1
-            for (int j = 0; j < 8; ++j) {
-              uint32_t r1[16];
-              tmem_ld_32x16(lane_base + hh * 128 + j * 16, r1);
-              tmem_ld_wait();
-              if (live) {
-                float v[16];
-#pragma unroll
-                for (int e = 0; e < 16; ++e) v[e] = __uint_as_float(r1[e]);
-#pragma unroll
-                for (int v8 = 0; v8 < 2; ++v8) {
-                  const uint4 u = pack8(v + v8 * 8);
-                  st_16B(yrow + j * 16 + v8 * 8, u);
-                  st_16B(crow + j * 16 + v8 * 8, u);
-                }
-              }
-            }
-          }
-        }
-      } else {
+      {
         const int h = (warp - 2) >> 2;  // warps 2-5: rows 0-127 of the tile, warps 6-9 (MT = 2): rows 128-255
         const uint32_t lane_base = tmem_base + as * Cfg::kAccCols + h * BN + ((uint32_t)(quad * 32) << 16);
         const int m = m_blk * kMRows + h * 128 + quad * 32 + lane;
@@ -339,13 +263,12 @@ gemm_prefill_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 }
 
 // ---- host side ---------------------------------------------------------------------------
-template <int BN, bool kGated, int MT = 1, bool kRope = false>
+template <int BN, bool kGated, int MT = 1>
 static int launch_prefill_gemm(const void* x, const void* w, const void* bias, const void* residual, void* y, int M,
-                               int N /* rows of w */, int K, int epilogue, cudaStream_t s,
-                               const RopeArgs& rope = RopeArgs{}) {
+                               int N /* rows of w */, int K, int epilogue, cudaStream_t s) {
   using Cfg = PrefillCfg<BN, kGated, MT>;
   static PerDeviceOnce once;
-  DLI_ONCE_PER_DEVICE(once, dev, DLI_CUDA_CALL(cudaFuncSetAttribute(gemm_prefill_kernel<BN, kGated, MT, kRope>,
+  DLI_ONCE_PER_DEVICE(once, dev, DLI_CUDA_CALL(cudaFuncSetAttribute(gemm_prefill_kernel<BN, kGated, MT>,
                                                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                                     Cfg::kSmemBytes)));
   CUtensorMap tmA, tmB;
@@ -356,9 +279,9 @@ static int launch_prefill_gemm(const void* x, const void* w, const void* bias, c
   const int num_tiles = m_tiles * n_tiles;
   const int sms = sm_count_cached();
   const int grid = num_tiles < sms ? num_tiles : sms;
-  DLI_LAUNCH("gemm_prefill_kernel", (gemm_prefill_kernel<BN, kGated, MT, kRope>), dim3(grid), dim3(64 + 128 * MT),
+  DLI_LAUNCH("gemm_prefill_kernel", (gemm_prefill_kernel<BN, kGated, MT>), dim3(grid), dim3(64 + 128 * MT),
              (size_t)Cfg::kSmemBytes, s, tmA, tmB, (const bf16*)bias, (const bf16*)residual, (bf16*)y, M, N, K, epilogue,
-             m_tiles, num_tiles, rope);
+             m_tiles, num_tiles);
   return DLI_OK;
 }
 
@@ -400,19 +323,47 @@ static PrefillShape prefill_tile(int M, int N, int K, bool gated) {
   return p;
 }
 
-// Clusters that split K (gemm_rows.cu) or the persistent kernel?  By estimated time, over 12 matrices x 12 row counts
-// above 128: the persistent kernel takes 9.5 us beyond its rounds (its set-up, and the epilogue of the last round, which
-// nothing hides); the clusters' estimate is taken 10 % high, because where it errs it errs low (one full wave of wide
-// tiles, 6144 x 4096 at 1 024 rows: estimate 55, measured 65 us, persistent 56).  With these two the choice was never
-// the slower one on that set; measured gains in gemm_rows.cu.  4 096 rows bound what was measured.
-static bool use_rows(int M, int N, int K, bool gated, RowsShape* shape, int* rc) {
-  *rc = DLI_OK;
-  if (M > 4096 || (M > 128 && N < 128)) return false;
-  double us;
-  *rc = plan_gemm_rows(M, N, K, shape, &us);
-  if (*rc != DLI_OK) return false;
+// Which kernel takes a projection, by estimated time (over 16 matrices x 17 row counts from 130 on, what it picks is 1.2 %
+// slower than the faster of the first two on average):
+//  - clusters that split K (gemm_rows.cu), up to 4 096 rows, which bound what was measured, and always up to 128 rows;
+//  - pairs of SMs (gemm_pair.cu) in tiles of 256 rows, from some 400 rows on;
+//  - the persistent kernel above where 256-row tiles would be half padding and the matrix is large (57344 x 8192 at 301 ... 384
+//    rows: 285 us, pairs 320), and for widths that are no multiple of 128, which no matrix of the models has: the only ones it
+//    was measured against the clusters for, whose estimate is taken 10 % high there.  It costs 9.5 us beyond its rounds.
+enum Route { kRouteRows, kRoutePair, kRoutePersistent };
+struct Choice {
+  Route route;
+  RowsShape rows;
+  PairShape pair;
+};
+static int choose(int M, int N, int K, bool gated, Choice* c) {
+  int rc;
+  const bool pairs = N % 128 == 0;
+  c->route = kRoutePersistent;
+  if (M > 128 && N < 128) return DLI_OK;
   PrefillShape p;
-  return M <= 128 || 1.1 * us < pick_prefill(M, N, K, gated, &p) + 9.5;
+  double us, best = pick_prefill(M, N, K, gated, &p) + 9.5;
+  if (pairs && ((M + 127) / 128) % 2 == 0) best = 1e30;
+  if (M <= 4096) {
+    if ((rc = plan_gemm_rows(M, N, K, &c->rows, &us)) != DLI_OK) return rc;
+    if (M <= 128 || (pairs ? 1.0 : 1.1) * us < best) c->route = kRouteRows, best = us;
+    if (M <= 128) return DLI_OK;
+  }
+  if (pairs) {
+    if ((rc = plan_gemm_pair(gated ? kPairGated : kPairPlain, M, N, K, 128, &c->pair, &us)) != DLI_OK) return rc;
+    if (us < best) c->route = kRoutePair;
+  }
+  return DLI_OK;
+}
+
+// The persistent kernel and the pairs add K in the same order: the same bits whichever of them the projection by itself takes.
+static int launch_pair_rope(const void* x, const void* w, const void* bias, void* qkv, int M, int N, int K, const RopeArgs& rope,
+                            int hd, cudaStream_t s) {
+  PairShape sh;
+  double us;
+  const int rc = plan_gemm_pair(kPairRope, M, N, K, hd, &sh, &us);
+  if (rc != DLI_OK) return rc;
+  return launch_gemm_pair(kPairRope, x, w, bias, nullptr, qkv, M, N, K, bias ? DLI_EPI_BIAS : 0, sh, s, rope, hd);
 }
 
 // qkv = x w^T (+ bias), q and k rotated, k and v appended to the cache pages: one kernel where a projection kernel has that
@@ -424,13 +375,12 @@ int linear_qkv_append(const void* x, const void* w, const void* bias, void* qkv,
   *launches += 1;
   if (one_kernel && M > 2 && K % 64 == 0 && aligned16(x) && aligned16(w) && aligned16(qkv) && aligned16(rope.k_cache) &&
       aligned16(rope.v_cache)) {
-    RowsShape sh;
-    int rc;
-    if (use_rows(M, N, K, false, &sh, &rc))
-      return launch_gemm_rows(kRowsRope, x, w, bias, nullptr, qkv, M, N, K, bias ? DLI_EPI_BIAS : 0, sh, s, rope, hd);
+    Choice c;
+    const int rc = choose(M, N, K, false, &c);
     if (rc != DLI_OK) return rc;
-    if (hd == 128 && rope.H % 2 == 0 && rope.KV % 2 == 0 && !bias && rope.cos_t)
-      return launch_prefill_gemm<256, false, 1, true>(x, w, nullptr, nullptr, qkv, M, N, K, 0, s, rope);
+    if (c.route == kRouteRows)
+      return launch_gemm_rows(kRowsRope, x, w, bias, nullptr, qkv, M, N, K, bias ? DLI_EPI_BIAS : 0, c.rows, s, rope, hd);
+    if (N % 128 == 0) return launch_pair_rope(x, w, bias, qkv, M, N, K, rope, hd, s);
   }
   const int rc = dli_linear_bf16(x, w, bias, nullptr, qkv, M, N, K, bias ? DLI_EPI_BIAS : 0, s);
   if (rc != DLI_OK) return rc;
@@ -455,11 +405,11 @@ int dli_gemm_bf16(const void* x, const void* w, const void* bias, const void* re
                 "dli_gemm_bf16: pointers must be 16-byte aligned");
   if (M == 0) return DLI_OK;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  RowsShape sh;
-  int rc;
-  if (use_rows(M, N, K, false, &sh, &rc))
-    return launch_gemm_rows(kRowsPlain, x, w, bias, residual, y, M, N, K, epilogue, sh, s);
+  Choice c;
+  const int rc = choose(M, N, K, false, &c);
   if (rc != DLI_OK) return rc;
+  if (c.route == kRouteRows) return launch_gemm_rows(kRowsPlain, x, w, bias, residual, y, M, N, K, epilogue, c.rows, s);
+  if (c.route == kRoutePair) return launch_gemm_pair(kPairPlain, x, w, bias, residual, y, M, N, K, epilogue, c.pair, s);
   const PrefillShape p = prefill_tile(M, N, K, false);
   if (p.mt == 2) {
     if (p.bn == 240) return launch_prefill_gemm<240, false, 2>(x, w, bias, residual, y, M, N, K, epilogue, s);
@@ -479,15 +429,21 @@ int dli_gemm_plan(int M, int N, int K, int gated, int* plan) {
   DLI_CHECK_ARG(plan, "dli_gemm_plan: null pointer");
   DLI_CHECK_ARG(M > 0 && N > 0 && K > 0 && K % 64 == 0 && N % (gated ? 256 : 16) == 0,
                 "dli_gemm_plan: need K %% 64 == 0 and N %% 16 == 0 (gated: N %% 256 == 0) (got M=%d N=%d K=%d)", M, N, K);
-  RowsShape sh;
-  int rc;
-  if (use_rows(M, N, K, gated != 0, &sh, &rc)) {
+  Choice c;
+  const int rc = choose(M, N, K, gated != 0, &c);
+  if (rc != DLI_OK) return rc;
+  if (c.route == kRouteRows) {
     plan[0] = 1;
-    plan[1] = sh.bn;
-    plan[2] = sh.splits;
+    plan[1] = c.rows.bn;
+    plan[2] = c.rows.splits;
     return DLI_OK;
   }
-  if (rc != DLI_OK) return rc;
+  if (c.route == kRoutePair) {
+    plan[0] = 2;
+    plan[1] = c.pair.bn;
+    plan[2] = c.pair.n_main * c.pair.bn < N ? c.pair.bn_tail : 0;
+    return DLI_OK;
+  }
   const PrefillShape p = prefill_tile(M, N, K, gated != 0);
   plan[0] = 0;
   plan[1] = p.bn;
@@ -529,12 +485,12 @@ int dli_gemm_qkv_rope_append_bf16(const void* x, const void* w_qkv, void* qkv, i
   // the same kernel as dli_gemm_bf16 would take: the same K split, so the same bits as the projection by itself
   const int N = (H + 2 * KV) * hd;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  RowsShape sh;
-  int rc;
-  if (use_rows(M, N, K, false, &sh, &rc))
-    return launch_gemm_rows(kRowsRope, x, w_qkv, nullptr, nullptr, qkv, M, N, K, 0, sh, s, ra, hd);
+  Choice c;
+  const int rc = choose(M, N, K, false, &c);
   if (rc != DLI_OK) return rc;
-  return launch_prefill_gemm<256, false, 1, true>(x, w_qkv, nullptr, nullptr, qkv, M, N, K, 0, s, ra);
+  if (c.route == kRouteRows)
+    return launch_gemm_rows(kRowsRope, x, w_qkv, nullptr, nullptr, qkv, M, N, K, 0, c.rows, s, ra, hd);
+  return launch_pair_rope(x, w_qkv, nullptr, qkv, M, N, K, ra, hd, s);
 }
 
 static int gemm_gated_act(const void* x, const void* w_gu, void* y, int M, int F, int K, const float* act, dli_stream_t stream);
@@ -554,10 +510,11 @@ static int gemm_gated_act(const void* x, const void* w_gu, void* y, int M, int F
   if (M == 0) return DLI_OK;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int N2 = 2 * F;  // rows of w_gu
-  RowsShape sh;
-  int rc;
-  if (use_rows(M, N2, K, true, &sh, &rc)) return launch_gemm_rows(kRowsGated, x, w_gu, act, nullptr, y, M, N2, K, 0, sh, s);
+  Choice c;
+  const int rc = choose(M, N2, K, true, &c);
   if (rc != DLI_OK) return rc;
+  if (c.route == kRouteRows) return launch_gemm_rows(kRowsGated, x, w_gu, act, nullptr, y, M, N2, K, 0, c.rows, s);
+  if (c.route == kRoutePair) return launch_gemm_pair(act ? kPairGatedAct : kPairGated, x, w_gu, act, nullptr, y, M, N2, K, 0, c.pair, s);
   return launch_prefill_gemm<256, true>(x, w_gu, act, nullptr, y, M, N2, K, 0, s);
 }
 

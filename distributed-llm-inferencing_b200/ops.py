@@ -407,11 +407,11 @@ def gemm_splitk_scratch_bytes(M, N) -> int:
 
 
 def gemm_plan(M, N, K, gated=False):
-    """What gemm (gated: gemm_gated_silu, N = 2 F) runs: ("rows", rows per tile, K splits) or ("persistent", weight rows per
-    tile, 128-row halves)."""
+    """What gemm (gated: gemm_gated_silu, N = 2 F) runs: ("rows", rows per tile, K splits), ("pairs", weight rows per tile, per
+    tile of the tail or 0) or ("persistent", weight rows per tile, 128-row halves)."""
     plan = (_ct.c_int * 3)()
     _lib.check("dli_gemm_plan", _lib.load().dli_gemm_plan(M, N, K, int(gated), plan))
-    return ("rows" if plan[0] else "persistent", plan[1], plan[2])
+    return (("persistent", "rows", "pairs")[plan[0]], plan[1], plan[2])
 
 
 def linear_splitk(x, w, scratch, bias=None, residual=None, out=None, epilogue=EPI_NONE):
