@@ -41,6 +41,7 @@ attn_prefill_kernel(const bf16* __restrict__ qkv, bf16* __restrict__ out, int T,
   const uint32_t sV = sK + 2 * kTileBytes;
 
   pdl_wait();
+  pdl_trigger();  // the next projection's CTAs may come in and ask for their weights
   // z (dispatched slowest) walks the query tiles from the longest to the shortest, x and y the heads and sequences:
   // the longest CTAs of all heads start first (see attn_prefill_tc.cu)
   const int qtile = gridDim.z - 1 - blockIdx.z;

@@ -161,6 +161,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm, const __grid_cons
   }
   if (warp == 1) tmem_alloc(smem_addr(tmem_ptr_smem), 512);
   pdl_wait();
+  pdl_trigger();
   tcgen05_fence_before();
   __syncthreads();
   tcgen05_fence_after();

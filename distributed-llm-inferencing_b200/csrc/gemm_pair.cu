@@ -181,6 +181,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       const PairTile first = pair_tile(pre ? pair : 0, m_tiles, n_main, bn, bn_tail, n_tiles);
       for (int kb = 0; kb < pre; ++kb) load_b(first, kb, kb);
       pdl_wait();
+      pdl_trigger();  // every CTA is resident: the next kernel's may come in as these leave
       for (int kb = 0; kb < pre; ++kb) load_a(first, kb, kb);
       int s = pre == stages ? 0 : pre;
       uint32_t ph = pre == stages ? 0 : 1;  // parity of the empty barrier's phase this lap waits for
