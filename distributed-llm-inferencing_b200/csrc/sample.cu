@@ -16,12 +16,15 @@
 //         are what the parity test compares.
 //
 // What bounds it: latency.  A row is 64 ... 256 KB, a few us of one SM's load bandwidth, so it is cut over a cluster of up
-// to 8 CTAs (16 384 logits each) and read ONCE, with 16-byte loads, into registers.  The k-th largest logit is found
-// without a histogram of the row: the k-th largest of a CTA's 512 per-thread maxima is a lower bound of it (k threads hold
-// an element at least that large), the largest such bound of the cluster leaves a few hundred candidates, and these meet
-// in the first CTA's shared memory, where the exact threshold is a binary search over keys.  (The two 256-bin
-// histograms with shared-memory atomics and their serial scans, three passes of 2-byte loads by one CTA per row, took
-// 62 us for one row as for 48, V = 128 256.  They are left for large k, see launch_sample.)
+// to 8 CTAs (16 384 logits each) and read ONCE, with 16-byte loads, into registers, as keys that compare two at a time.  The k-th
+// largest logit is found without a histogram of the row: the k-th largest of a CTA's 512 per-thread maxima is a lower bound of it
+// (k threads hold an element at least that large), the largest such bound of the cluster leaves a few hundred candidates, each CTA
+// writes its own into its region of the first CTA's shared memory, and the exact threshold is a search over the bits in which
+// bound and maximum differ.  Up to 64 that remain are put in order by counting and finished by one warp in registers; the
+// uniform is drawn while the cluster meets.  One row of 128 256 logits, us: load and maxima 0.9, bound 1.5, exchange 0.5,
+// candidates 1.0, gathering 0.9, threshold 1.8, order 0.5, softmax and nucleus 0.9, draw 0.4.
+// (The two 256-bin histograms with shared-memory atomics and their serial scans, three passes of 2-byte loads by one CTA per
+// row, took 62 us for one row as for 48, V = 128 256.  They are left for large k, see launch_sample.)
 #include <math.h>
 
 #include "common.cuh"
@@ -31,6 +34,7 @@ namespace dli {
 constexpr int kSampleThreads = 512;
 constexpr int kMaxCand = 2048;  // candidates kept in shared memory (k plus ties)
 constexpr int kMaxRanked = 128;  // candidates that are put in order by counting
+constexpr int kOneWarp = 64;     // candidates that one warp finishes in registers
 
 // monotone key: larger bf16 value <-> larger 16-bit key
 __device__ __forceinline__ uint32_t bf16_key(uint16_t b) { return (b & 0x8000u) ? (uint16_t)~b : (uint16_t)(b | 0x8000u); }
@@ -70,6 +74,7 @@ __device__ __forceinline__ float philox_uniform(uint64_t seed, uint32_t step, ui
 constexpr int kSliceVecs = 4;                                  // 16-byte vectors a thread keeps in registers
 constexpr int kSliceElems = kSampleThreads * kSliceVecs * 8;   // logits of a CTA that are read once
 constexpr int kMaxRowCtas = 8;
+constexpr int kRegionSlots = 8 * kSampleThreads;               // eight candidates a thread of the first CTA
 
 __device__ __forceinline__ uint32_t cluster_addr(const void* p, uint32_t rank) {
   uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(p)), r;
@@ -79,10 +84,8 @@ __device__ __forceinline__ uint32_t cluster_addr(const void* p, uint32_t rank) {
 __device__ __forceinline__ void cluster_st(uint32_t addr, uint32_t v) {
   asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
-__device__ __forceinline__ uint32_t cluster_add(uint32_t addr, uint32_t v) {
-  uint32_t old;
-  asm volatile("atom.shared::cluster.add.u32 %0, [%1], %2;" : "=r"(old) : "r"(addr), "r"(v) : "memory");
-  return old;
+__device__ __forceinline__ void cluster_st16(uint32_t addr, uint32_t v) {
+  asm volatile("st.shared::cluster.b16 [%0], %1;" ::"r"(addr), "h"((uint16_t)v) : "memory");
 }
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
@@ -91,10 +94,31 @@ __device__ __forceinline__ void cluster_sync_all() {
   cluster_wait();
 }
 
-// Element e of a vector's eight, as raw bits.
-__device__ __forceinline__ uint32_t vec_elem(const uint4& u, int e) {
-  const uint32_t w = e < 2 ? u.x : e < 4 ? u.y : e < 6 ? u.z : u.w;
-  return (e & 1) ? w >> 16 : w & 0xffffu;
+// bf16_key of both halves of a word.
+__device__ __forceinline__ uint32_t bf16_keys2(uint32_t x) { return x ^ ((((x >> 15) & 0x00010001u) * 0x7fffu) | 0x80008000u); }
+__device__ __forceinline__ uint4 bf16_keys8(const uint4& u) {
+  return make_uint4(bf16_keys2(u.x), bf16_keys2(u.y), bf16_keys2(u.z), bf16_keys2(u.w));
+}
+__device__ __forceinline__ uint32_t max_keys2(uint32_t a, const uint4& u) {
+  return __vmaxu2(__vmaxu2(a, __vmaxu2(u.x, u.y)), __vmaxu2(u.z, u.w));
+}
+
+// The largest t in [base, base + 2^bits) with at least k of the block's keys >= t, where k of them are >= base: a bit a step, a
+// count of the block each (0.1 us).  Two bits a step take three counts, and every way to sum them over 16 warps (reductions, atomics)
+// was slower: 0.28 us a step.
+template <int NQ>
+__device__ __forceinline__ uint32_t kth_key(const uint32_t (&keys)[NQ], int nq, int k, uint32_t base, int bits) {
+  uint32_t t = base;
+#pragma unroll 1
+  for (int sh = bits - 1; sh >= 0; --sh) {
+    const uint32_t a = t + (1u << sh);
+    int count = 0;
+#pragma unroll
+    for (int q = 0; q < NQ; ++q)
+      if (q < nq) count += __syncthreads_count(keys[q] >= a);
+    if (count >= k) t = a;
+  }
+  return t;
 }
 
 // f(key, index) for every element of the row by the threads of one CTA, eight loads of a thread in flight at a time.
@@ -167,31 +191,43 @@ sample_kernel(const bf16* __restrict__ logits, int ld, int32_t* __restrict__ out
   __shared__ uint32_t sh[2];
   __shared__ float cval[kMaxCand];  // candidates: keys, then values, then probabilities
   __shared__ int cidx[kMaxCand];
-  __shared__ uint32_t gkey[kMaxCand];  // first CTA: the row's candidates
-  __shared__ int gidx[kMaxCand];
-  __shared__ uint32_t bounds[kMaxRowCtas];
-  __shared__ uint32_t gcount;
-  __shared__ uint32_t gbase;
+  __shared__ uint16_t gkey[kRegionSlots];  // first CTA: the row's candidates, a region per CTA of the cluster
+  __shared__ int gidx[kRegionSlots];
+  __shared__ uint32_t bounds[kMaxRowCtas];  // bound | largest key << 16 of each CTA
+  __shared__ uint32_t counts[kMaxRowCtas];  // first CTA: candidates of each CTA
+  __shared__ uint32_t tops[16], mths[16];   // of each warp: its largest key, its m-th largest maximum
   __shared__ int ncand;
   __shared__ int nties;
+  __shared__ float uniform;
   __shared__ float red[kSampleThreads / 32];
   uint32_t* ckey = reinterpret_cast<uint32_t*>(cval);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int b = blockIdx.x / ctas, rank = blockIdx.x - b * ctas;
-  if (tid == 0) gcount = 0, ncand = 0, nties = 0;
+  if (tid == 0) ncand = 0, nties = 0;
   pdl_wait();
   pdl_trigger();
   if (row_mask != nullptr && row_mask[b] == 0) return;  // this row keeps the token already in out[]
   const uint16_t* row = reinterpret_cast<const uint16_t*>(logits + (size_t)b * ld);
   const int k = top_k > 0 ? min(top_k, V) : V;
+  // per_row: every row has its own (seed, step) and the row index stays out of the key, so a sequence's draws do not depend on
+  // the batch row it happens to occupy.  One thread asks for the seed now and draws while the cluster meets.
+  const bool drawer = rank == 0 && tid == 32;
+  uint64_t my_seed = 0;
+  uint32_t my_step = 0;
+  if (drawer) {
+    if (seed) my_seed = seed[per_row ? b : 0];
+    if (step) my_step = (uint32_t)step[per_row ? b : 0];
+  }
 
+  int total = kMaxCand + 1;  // candidates of the row, if they fit
+  const int per_region = kSampleThreads / ctas, region_slots = 8 * per_region;
   if (narrow) {
     // ---- this CTA's share of the row: whole 16-byte vectors; what lies before and after them goes to the first CTA --------
     const int head = min(V, (int)(((16u - (uint32_t)(reinterpret_cast<uintptr_t>(row) & 15u)) & 15u) >> 1));
     const int n_vec = (V - head) >> 3, tail0 = head + n_vec * 8;
     const int v0 = (int)((long long)n_vec * rank / ctas), v1 = (int)((long long)n_vec * (rank + 1) / ctas);
     const uint4* vecs = reinterpret_cast<const uint4*>(row + head);
-    uint4 held[kSliceVecs];
+    uint4 held[kSliceVecs];  // keys
 #pragma unroll
     for (int i = 0; i < kSliceVecs; ++i) {
       const int v = v0 + i * kSampleThreads + tid;
@@ -203,96 +239,118 @@ sample_kernel(const bf16* __restrict__ logits, int ld, int32_t* __restrict__ out
       if (tid < head) edge = tid;
       else if (tail0 + tid - head < V) edge = tail0 + tid - head;
     }
-    uint32_t top = 0;
+    uint32_t top2 = 0;
+#pragma unroll 4
+    for (int v = v0 + kSliceVecs * kSampleThreads + tid; v < v1; v += kSampleThreads) top2 = max_keys2(top2, bf16_keys8(vecs[v]));
 #pragma unroll
-    for (int i = 0; i < kSliceVecs; ++i)
-#pragma unroll
-      for (int e = 0; e < 8; ++e) top = max(top, bf16_key((uint16_t)vec_elem(held[i], e)));
-    for (int v = v0 + kSliceVecs * kSampleThreads + tid; v < v1; v += kSampleThreads) {
-      const uint4 u = vecs[v];
-#pragma unroll
-      for (int e = 0; e < 8; ++e) top = max(top, bf16_key((uint16_t)vec_elem(u, e)));
+    for (int i = 0; i < kSliceVecs; ++i) {
+      held[i] = bf16_keys8(held[i]);
+      top2 = max_keys2(top2, held[i]);
     }
-    if (edge >= 0) top = max(top, bf16_key(row[edge]));
+    uint32_t top[1] = {max(top2 & 0xffffu, top2 >> 16)};
+    if (edge >= 0) top[0] = max(top[0], bf16_key(row[edge]));
 
-    // ---- lower bound of the k-th largest key: the k-th largest of the per-thread maxima, bit by bit (a row of at most a
-    // thread per logit needs none: all of it are candidates) ----
-    uint32_t bound = 0;
+    // ---- lower bound of the k-th largest key: the k-th largest of the per-thread maxima (a row of at most a thread per logit
+    // needs none: all of it are candidates) ----
+    uint32_t bound = 0, most = 0xffffu;
     cluster_arrive();
     if (V > kSampleThreads) {
-#pragma unroll 1
-      for (uint32_t bit = 0x8000u; bit; bit >>= 1)
-        if (__syncthreads_count(top >= (bound | bit)) >= k) bound |= bit;
+      // It lies between the smallest and the largest of the 16 warps' m-th largest, m = k / 16 rounded up: at least 16 m of the
+      // maxima reach the one, at most 16 (m - 1) < k exceed the other.  That leaves some 7 of the 16 bits.
+      uint32_t v = top[0], mth = 0;
+      for (int m = (k + 15) / 16, r = 1; r <= m; ++r) {
+        mth = __reduce_max_sync(0xffffffffu, v);
+        if (r == 1 && lane == 0) tops[warp] = mth;
+        const unsigned holders = __ballot_sync(0xffffffffu, v == mth);
+        if (lane == __ffs(holders) - 1) v = 0u;
+      }
+      if (lane == 0) mths[warp] = mth;
+      __syncthreads();
+      const uint32_t lo = __reduce_min_sync(0xffffffffu, mths[lane & 15]), hi = __reduce_max_sync(0xffffffffu, mths[lane & 15]);
+      bound = kth_key(top, 1, k, lo, 32 - __clz(hi - lo));
+      most = __reduce_max_sync(0xffffffffu, tops[lane & 15]);
     }
     cluster_wait();  // every CTA of the cluster runs: from here on its shared memory may be written
-    if (tid < ctas) cluster_st(cluster_addr(&bounds[rank], tid), bound);
+    if (tid < ctas) cluster_st(cluster_addr(&bounds[rank], tid), bound | most << 16);
     cluster_sync_all();
-    for (int c = 0; c < ctas; ++c) bound = max(bound, bounds[c]);
-    // ---- candidates: this CTA's elements at or above the bound, then all of the row's in the first CTA ----------------
-    auto take = [&](uint32_t raw, int i) {
-      const uint32_t key = bf16_key((uint16_t)raw);
+    most = 0;
+    for (int c = 0; c < ctas; ++c) bound = max(bound, bounds[c] & 0xffffu), most = max(most, bounds[c] >> 16);
+    // ---- candidates: this CTA's elements at or above the bound, straight into its region of the first CTA -------------------
+    const uint32_t kb = cluster_addr(gkey, 0) + rank * region_slots * 2, ib = cluster_addr(gidx, 0) + rank * region_slots * 4;
+    auto take = [&](uint32_t key, int i) {
       if (key >= bound) {
         const int slot = atomicAdd(&ncand, 1);
-        if (slot < kMaxCand) { ckey[slot] = key; cidx[slot] = i; }
+        if (slot < region_slots) {
+          cluster_st16(kb + slot * 2, key);
+          cluster_st(ib + slot * 4, (uint32_t)i);
+        }
+      }
+    };
+    const uint32_t bound2 = bound | bound << 16;
+    auto take8 = [&](const uint4& u, int i) {
+      const uint32_t top8 = max_keys2(0u, u);
+      if (max(top8 & 0xffffu, top8 >> 16) < bound) return;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const uint32_t w = e == 0 ? u.x : e == 1 ? u.y : e == 2 ? u.z : u.w;
+        if (__vmaxu2(w, bound2) == bound2 && (w & 0xffffu) != bound && (w >> 16) != bound) continue;
+        take(w & 0xffffu, i + 2 * e);
+        take(w >> 16, i + 2 * e + 1);
       }
     };
 #pragma unroll
     for (int i = 0; i < kSliceVecs; ++i) {
       const int v = v0 + i * kSampleThreads + tid;
-      if (v < v1) {
-#pragma unroll
-        for (int e = 0; e < 8; ++e) take(vec_elem(held[i], e), head + v * 8 + e);
-      }
+      if (v < v1) take8(held[i], head + v * 8);
     }
-    for (int v = v0 + kSliceVecs * kSampleThreads + tid; v < v1; v += kSampleThreads) {
-      const uint4 u = vecs[v];
-#pragma unroll
-      for (int e = 0; e < 8; ++e) take(vec_elem(u, e), head + v * 8 + e);
-    }
-    if (edge >= 0) take(row[edge], edge);
+#pragma unroll 4
+    for (int v = v0 + kSliceVecs * kSampleThreads + tid; v < v1; v += kSampleThreads) take8(bf16_keys8(vecs[v]), head + v * 8);
+    if (edge >= 0) take(bf16_key(row[edge]), edge);
     __syncthreads();
-    const uint32_t mine = (uint32_t)ncand;
-    if (tid == 0) gbase = cluster_add(cluster_addr(&gcount, 0), min(mine, (uint32_t)kMaxCand + 1));  // too many: too many there too
-    __syncthreads();
-    const uint32_t base = gbase, kb = cluster_addr(gkey, 0), ib = cluster_addr(gidx, 0);
-    if (mine <= (uint32_t)kMaxCand && base + mine <= (uint32_t)kMaxCand) {
-      for (uint32_t i = tid; i < mine; i += kSampleThreads) {
-        cluster_st(kb + (base + i) * 4, ckey[i]);
-        cluster_st(ib + (base + i) * 4, (uint32_t)cidx[i]);
-      }
-    }
-    cluster_sync_all();
-  }
-  if (rank != 0) return;
+    if (tid == 0) cluster_st(cluster_addr(&counts[rank], 0), (uint32_t)ncand);
+    cluster_arrive();
+    if (drawer) uniform = philox_uniform(my_seed, my_step, per_row ? 0u : b);
+    __syncwarp();
+    cluster_wait();
+    if (rank != 0) return;
 
-  // ---- first CTA: the exact threshold, and everything at or above it (ties are kept) ----------------------------------
-  if (tid == 0) ncand = 0;
-  if (narrow && gcount <= (uint32_t)kMaxCand) {
-    const int n_c = (int)gcount;
-    uint32_t keys[kMaxCand / kSampleThreads];
+    // ---- first CTA: the exact threshold, and everything at or above it (ties are kept) --------------------------------
+    uint32_t fullest = 0;
+    total = 0;
+    for (int c = 0; c < ctas; ++c) total += counts[c], fullest = max(fullest, counts[c]);
+    if (tid == 0) ncand = 0;
+    if (fullest <= (uint32_t)region_slots && total <= kMaxCand) {
+      const int region = tid / per_region, at = tid - region * per_region;
+      const int mine = region < ctas ? (int)counts[region] : 0;
+      const int nq = ((int)fullest + per_region - 1) / per_region;  // at most 8
+      uint32_t keys[8];
 #pragma unroll
-    for (int q = 0; q < kMaxCand / kSampleThreads; ++q)
-      keys[q] = q * kSampleThreads + tid < n_c ? gkey[q * kSampleThreads + tid] : 0u;
-    uint32_t thr = 0;
-#pragma unroll 1
-    for (uint32_t bit = 0x8000u; bit; bit >>= 1) {
-      int count = 0;
+      for (int q = 0; q < 8; ++q)
+        keys[q] = q < nq && q * per_region + at < mine ? gkey[region * region_slots + q * per_region + at] : 0u;
+      const uint32_t thr = kth_key(keys, nq, k, bound, 32 - __clz(most - bound));
+      __syncthreads();
 #pragma unroll
-      for (int q = 0; q < kMaxCand / kSampleThreads; ++q)
-        if (q * kSampleThreads < n_c) count += __syncthreads_count(keys[q] >= (thr | bit));
-      if (count >= k) thr |= bit;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < kMaxCand / kSampleThreads; ++q) {
-      const int i = q * kSampleThreads + tid;
-      if (i < n_c && keys[q] >= thr) {
-        const int slot = atomicAdd(&ncand, 1);
-        ckey[slot] = order_key(key_value(keys[q]) * inv_temperature);
-        cidx[slot] = gidx[i];
+      for (int q = 0; q < 8; ++q) {
+        if (q >= nq) break;
+        const bool in = q * per_region + at < mine && keys[q] >= thr;
+        const unsigned m = __ballot_sync(0xffffffffu, in);
+        int first = 0;
+        if (m && lane == 0) first = atomicAdd(&ncand, __popc(m));
+        first = __shfl_sync(0xffffffffu, first, 0);
+        if (in) {
+          const int slot = first + __popc(m & ((1u << lane) - 1));
+          ckey[slot] = order_key(key_value(keys[q]) * inv_temperature);
+          cidx[slot] = gidx[region * region_slots + q * per_region + at];
+        }
       }
+    } else {
+      total = kMaxCand + 1;
     }
-  } else {
+  } else if (drawer) {
+    uniform = philox_uniform(my_seed, my_step, per_row ? 0u : b);
+  }
+  if (total > kMaxCand) {
+    __syncthreads();
     const uint32_t thr = kth_largest_key(row, V, min(k, kMaxCand), hist, sh);
     // what lies above the threshold (fewer than k elements) first: ties beyond the capacity are dropped, never those
     for_each_key(row, V, [&](uint32_t key, int i) {
@@ -316,6 +374,74 @@ sample_kernel(const bf16* __restrict__ logits, int ld, int32_t* __restrict__ out
   }
   __syncthreads();
   const int n = ncand;  // at most kMaxCand
+  if (n <= kOneWarp) {
+    // A few: each one's place is the number of those before it, counted by eight threads; one warp does the rest in registers.
+    // The sums are formed in the order of the general form below.
+    const int me = tid >> 3;
+    const uint32_t a = ckey[min(me, n - 1)];
+    const int ia = cidx[min(me, n - 1)];
+    int place = 0;
+    for (int j = tid & 7; j < n; j += 8) place += comes_before(ckey[j], cidx[j], a, ia) ? 1 : 0;
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) place += __shfl_xor_sync(0xffffffffu, place, o);
+    uint32_t* const skey = ckey + kOneWarp;
+    int* const sidx = cidx + kOneWarp;
+    if (me < n && (tid & 7) == 0) skey[place] = a, sidx[place] = ia;
+    __syncthreads();
+    if (warp != 0) return;
+    const float vmax = order_value(skey[0]);
+    float p[2], sum[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      p[h] = h * 32 + lane < n ? __expf(order_value(skey[h * 32 + lane]) - vmax) : 0.f;
+      sum[h] = warp_sum(p[h]);
+    }
+    const float denom = sum[0] + sum[1];
+    int kept = 0;
+    float carry = 0.f;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      p[h] /= denom;
+      float incl = p[h];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const float t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += t;
+      }
+      const int i = h * 32 + lane;
+      const unsigned m = __ballot_sync(0xffffffffu, i < n && (i == 0 || carry + incl - p[h] < top_p));
+      if (kept == h * 32) kept += __popc(m);
+      carry += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    kept = max(kept, 1);
+    float mass = 0.f;
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      if (h * 32 + lane < kept) mass += p[h];
+    mass = warp_sum(mass);
+    if (dbg_probs) {
+      for (int i = lane; i < dbg_cap; i += 32) {
+        dbg_probs[(size_t)b * dbg_cap + i] = i < kept ? (i < 32 ? p[0] : p[1]) / mass : 0.f;
+        dbg_ids[(size_t)b * dbg_cap + i] = i < kept ? sidx[i] : -1;
+      }
+    }
+    // the inverse CDF, its sums in order: every lane walks them
+    const float u = uniform * mass;
+    float acc = 0.f;
+    int pick = kept - 1;
+#pragma unroll
+    for (int i0 = 0; i0 < 64; i0 += 8) {
+      if (i0 >= kept) break;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        acc += __shfl_sync(0xffffffffu, p[i0 >> 5], (i0 & 31) + e);
+        if (i0 + e < pick && u < acc) pick = i0 + e;
+      }
+      if (u < acc) break;
+    }
+    if (lane == 0) out[b] = sidx[pick];
+    return;
+  }
   // Descending by value, equal values by ascending token id.  Which of several EQUAL-probability tokens survive at the
   // nucleus boundary depends on torch.sort's tie order in the reference (not specified); here the lower token ids stay.
   int npow = 1;
@@ -396,10 +522,7 @@ sample_kernel(const bf16* __restrict__ logits, int ld, int32_t* __restrict__ out
       }
     }
     if (lane == 0) {
-      // per_row: every row has its own (seed, step) and the row index stays out of the key, so a sequence's
-      // draws do not depend on the batch row it happens to occupy
-      const int r = per_row ? b : 0;
-      const float u = philox_uniform(seed ? seed[r] : 0ull, step ? (uint32_t)step[r] : 0u, per_row ? 0u : b) * mass;
+      const float u = uniform * mass;
       float acc = 0.f;
       int pick = kept - 1;
       for (int i0 = 0; i0 < kept; i0 += 8) {  // eight loads in flight, the sums in order
@@ -419,20 +542,48 @@ sample_kernel(const bf16* __restrict__ logits, int ld, int32_t* __restrict__ out
   }
 }
 
-// A cluster of as many CTAs as the row has slices of 16 384 logits, at most the portable 8 (beyond 131 072 logits a
-// thread reads the rest of its slice twice).  That way (`narrow`) is for k small enough that few logits lie above the
-// bound: with `per` logits a thread, k of 512 maxima above it means a share of 1 - (1 - k/512)^(1/per) of all logits, and a
-// bf16 step at the bound adds up to some V / 4096 ties.  Larger k would overflow the first CTA's shared memory after all the
-// work; it takes the histograms of one CTA per row at once.
-//   one row, us, one CTA for every k / clusters up to k = 512 / this rule: 128 256 logits, k = 50: 57.8 / 13.9 / 11.6,
-//   k = 128: 62.3 / 21.0 / 17.3, k = 256: 65.5 / 109 / 65.1, k = 512: 76.2 / 107 / 74.5, k = 1000: 97.3 / 105 / 79.2;
-//   500 logits, k = 500: 16.3 / 47.9 / 15.7
+// CTAs that run at once as clusters of 1 ... 8 (asked of the driver once per device).
+static int sample_capacity(int* capacity /*[kMaxRowCtas + 1]*/) {
+  static PerDeviceOnce once;
+  static int cap[kMaxDevices][kMaxRowCtas + 1];
+  DLI_ONCE_PER_DEVICE(once, dev, {
+    for (int c = 1; c <= kMaxRowCtas; ++c) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3((unsigned)c * 1024);
+      cfg.blockDim = dim3(kSampleThreads);
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = c;
+      attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      int n = 0;
+      DLI_CUDA_CALL(cudaOccupancyMaxActiveClusters(&n, sample_kernel, &cfg));
+      cap[dev][c] = n * c;
+    }
+  });
+  for (int c = 1; c <= kMaxRowCtas; ++c) capacity[c] = cap[dev][c];
+  return DLI_OK;
+}
+
+// A cluster of as many CTAs as the row has slices of 16 384 logits, at most the portable 8, and no more than let all rows'
+// clusters run at once: a second wave is a second chain, a longer slice (read twice beyond 16 384 logits) a few loads.  128 256
+// logits, us with 8 / 4 / 2 / 1 CTAs a row: one row 10.3 / 12.4 / 14.9 / 18.9, 24 rows 13.3 / 13.7 / 15.8 / 20.0, 48 rows 20.6 /
+// 16.0 / 16.0 / 20.4, 128 rows 42 / 30 / 20.0 / 21.0 (48 rows before, always 8: 24.1).
+// That way (`narrow`) is for k small enough that few logits lie above the bound: with `per` logits a thread, k of 512 maxima above
+// it means a share of 1 - (1 - k/512)^(1/per) of all logits, and a bf16 step at the bound adds up to some V / 4096 ties.  Larger
+// k would overflow the first CTA's shared memory after all the work; it takes the histograms of one CTA per row at once.
+//   one row, us, one CTA for every k / clusters up to k = 512 / this rule: 128 256 logits, k = 128: 62.3 / 21.0 / 17.3,
+//   k = 256: 65.5 / 109 / 65.1, k = 512: 76.2 / 107 / 74.5, k = 1000: 97.3 / 105 / 79.2; 500 logits, k = 500: 16.3 / 47.9 / 15.7
 static int launch_sample(const char* what, const void* logits, int ld, int32_t* out, int B, int V, float temperature,
                          int top_k, float top_p, const uint64_t* seed, const int32_t* step, float* dbg_probs,
                          int32_t* dbg_ids, int dbg_cap, int per_row, const int32_t* row_mask, cudaStream_t s) {
   int ctas = (V - 1) / kSliceElems + 1;
   if (ctas > kMaxRowCtas) ctas = kMaxRowCtas;
-  if ((long long)B * ctas > 0x7fffffffLL) ctas = 1;
+  int cap[kMaxRowCtas + 1];
+  const int rc = sample_capacity(cap);
+  if (rc != DLI_OK) return rc;
+  while (ctas > 1 && (long long)B * ctas > cap[ctas]) --ctas;
   const int k = top_k > 0 && top_k < V ? top_k : V;
   const double per = (double)V / (kSampleThreads * ctas);
   const bool narrow = k <= kSampleThreads &&
