@@ -470,7 +470,7 @@ static int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUt
 
 // The cut is the cheapest by a model of the kernel's time, fitted to 240 shapes (768 x 768 ... 28672 x 4096, 257 ... 8 192 rows)
 // x up to 14 cuts each, B200: a cut it picks is 1.7 % slower than the best one on average.
-//   time = (5.7 us (launch, first loads, last epilogue) + what the busiest pair walks)
+//   time = (2.5 us (first loads, last epilogue) + what the busiest pair walks)
 //          x 1.24 at 10^12 operations and beyond (the power limit), in proportion below
 //   a tile = k-blocks x max(0.083 + 0.00091 width, 0.2) us + 0.0097 width us
 // The floor of 0.2 us is the latency of a load over the ring.  The tail pays where the last round of full tiles is far from
@@ -493,7 +493,7 @@ static double pair_cost(int M, int N, int K, const PairShape& sh, int pairs) {
     if (v > us) us = v;
   }
   const double tera = 2e-12 * M * N * K;
-  return (us + 5.7) * (1.0 + 0.24 * (tera < 1.0 ? tera : 1.0)) * (m_tiles <= 2 ? 1.05 : 1.0);  // (no neighbour's L2 lines)
+  return (us + 2.5) * (1.0 + 0.24 * (tera < 1.0 ? tera : 1.0)) * (m_tiles <= 2 ? 1.03 : 1.0);  // (no neighbour's L2 lines)
 }
 
 namespace {

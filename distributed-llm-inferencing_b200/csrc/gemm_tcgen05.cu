@@ -323,8 +323,9 @@ static PrefillShape prefill_tile(int M, int N, int K, bool gated) {
   return p;
 }
 
-// Which kernel takes a projection, by estimated time (over 16 matrices x 17 row counts from 130 on, what it picks is 1.2 %
-// slower than the faster of the first two on average):
+// Which kernel takes a projection, by estimated time.  The clusters' estimate errs high from some 250 rows on (28672 x 4096 gated
+// at 301 rows: 91 us, measured 74): 0.88 of it + 1.5 us.  Over 9 matrices x 12 row counts from 150 to 700 what is picked is 0.9 %
+// slower than the faster of the first two on average, 10 % at most.
 //  - clusters that split K (gemm_rows.cu), up to 4 096 rows, which bound what was measured, and always up to 128 rows;
 //  - pairs of SMs (gemm_pair.cu) in tiles of 256 rows, from some 400 rows on;
 //  - the persistent kernel above where 256-row tiles would be half padding and the matrix is large (57344 x 8192 at 301 ... 384
@@ -346,7 +347,8 @@ static int choose(int M, int N, int K, bool gated, Choice* c) {
   if (pairs && ((M + 127) / 128) % 2 == 0) best = 1e30;
   if (M <= 4096) {
     if ((rc = plan_gemm_rows(M, N, K, &c->rows, &us)) != DLI_OK) return rc;
-    if (M <= 128 || (pairs ? 1.0 : 1.1) * us < best) c->route = kRouteRows, best = us;
+    us = pairs ? 0.88 * us + 1.5 : 1.1 * us;
+    if (M <= 128 || us < best) c->route = kRouteRows, best = us;
     if (M <= 128) return DLI_OK;
   }
   if (pairs) {
