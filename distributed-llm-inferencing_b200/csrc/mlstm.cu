@@ -365,6 +365,7 @@ struct MlstmPar {
   float* cS;   // [blocks, H, D, V]
   float* cn;   // [blocks, H, D]
   float* csc;  // [blocks, H, 4] = (b_L, A_c, m_0 of the block, -)
+  int vec4;    // rows of the states are whole 16-byte vectors: D and V multiples of 4, all bases aligned
 };
 
 template <typename E>
@@ -402,9 +403,23 @@ __device__ __forceinline__ void mlstm_load_kv_gates(const E* base, const MlstmAr
       kT[d * kMcLp + t] = kv;
     }
   }
-  for (int i = tid; i < kMcL * kMcCols; i += kMcThreads) {
-    const int t = i / kMcCols, c = c0 + i % kMcCols;
-    vs[i] = (t < len && c < a.V) ? m_to_f(base[(size_t)t * a.ldp + a.v_off + h * a.V + c]) : 0.f;
+  if (sizeof(E) == 2 && a.V % 8 == 0 && (a.v_off + h * a.V) % 8 == 0 && a.ldp % 8 == 0) {
+#pragma unroll
+    for (int i = tid; i < kMcL * (kMcCols / 8); i += kMcThreads) {
+      const int t = i / (kMcCols / 8), c = c0 + i % (kMcCols / 8) * 8;
+      uint4 u = make_uint4(0, 0, 0, 0);
+      if (t < len && c < a.V) u = ld_16B(base + (size_t)t * a.ldp + a.v_off + h * a.V + c);
+      float f[8];
+      unpack8(u, f);
+      float4* dst = reinterpret_cast<float4*>(vs + t * kMcCols + i % (kMcCols / 8) * 8);
+      dst[0] = make_float4(f[0], f[1], f[2], f[3]);
+      dst[1] = make_float4(f[4], f[5], f[6], f[7]);
+    }
+  } else {
+    for (int i = tid; i < kMcL * kMcCols; i += kMcThreads) {
+      const int t = i / kMcCols, c = c0 + i % kMcCols;
+      vs[i] = (t < len && c < a.V) ? m_to_f(base[(size_t)t * a.ldp + a.v_off + h * a.V + c]) : 0.f;
+    }
   }
   if (tid < kMcL) {
     float ig = -INFINITY, fg = 0.f;
@@ -490,10 +505,15 @@ mlstm_par_local_kernel(const E* __restrict__ proj, MlstmArgs a, MlstmPar p) {
     for (int r = 0; r < 8; ++r) {
       const int d = dbase + ty + 16 * r;
       if (d >= D) continue;
+      if (p.vec4) {
+        if (c0 + 4 * tx < a.V)
+          *reinterpret_cast<float4*>(Ug + (size_t)d * a.V + c0 + 4 * tx) = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
+      } else {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int c = c0 + 4 * tx + j;
-        if (c < a.V) Ug[(size_t)d * a.V + c] = acc[r][j];
+        for (int j = 0; j < 4; ++j) {
+          const int c = c0 + 4 * tx + j;
+          if (c < a.V) Ug[(size_t)d * a.V + c] = acc[r][j];
+        }
       }
       if (tx == 0 && blockIdx.z == 0) nUg[d] = nacc[r];
     }
@@ -505,7 +525,10 @@ mlstm_par_local_kernel(const E* __restrict__ proj, MlstmArgs a, MlstmPar p) {
   }
 }
 
-// pass 2: one thread per state element (the D*V entries of S, then the D entries of n), blocks of the entry in order
+// pass 2: one thread per VEC state elements (the D*V elements of S, then the D of n), blocks of the entry in order.  Bound by a
+// thread's chain, so four elements share one where they are a vector: 20.6 -> 9.4 us for 3 sequences of 11 blocks, 8 heads of
+// 128 x 256.
+template <int VEC>
 __global__ void __launch_bounds__(256)
 mlstm_par_carry_kernel(MlstmArgs a, MlstmPar p, int n_tiles) {
   pdl_wait();
@@ -513,7 +536,7 @@ mlstm_par_carry_kernel(MlstmArgs a, MlstmPar p, int n_tiles) {
   const int ent_i = blockIdx.x, h = blockIdx.y;
   const int4 e = reinterpret_cast<const int4*>(a.ent)[ent_i];
   const size_t DV = (size_t)a.D * a.V, total = DV + a.D;
-  const size_t idx = (size_t)blockIdx.z * blockDim.x + threadIdx.x;
+  const size_t idx = ((size_t)blockIdx.z * blockDim.x + threadIdx.x) * VEC;
   int first = 0;
   while (first < n_tiles && p.tiles[2 * first] != ent_i) ++first;
   const int nblk = (e.z + kMcL - 1) / kMcL;
@@ -523,18 +546,33 @@ mlstm_par_carry_kernel(MlstmArgs a, MlstmPar p, int n_tiles) {
   float* state = nullptr;
   if (idx < DV) state = a.S + ((size_t)e.x * a.H + h) * DV + idx;
   else if (idx < total) state = a.n + ((size_t)e.x * a.H + h) * a.D + (idx - DV);
-  float sv = (state && !fresh) ? *state : 0.f;
+  const auto load = [](const float* src, float (&v)[VEC]) {
+    if constexpr (VEC == 4) {
+      const float4 t = *reinterpret_cast<const float4*>(src);
+      v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+    } else {
+      v[0] = *src;
+    }
+  };
+  const auto store = [](float* dst, const float (&v)[VEC]) {
+    if constexpr (VEC == 4) *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
+    else *dst = v[0];
+  };
+  const auto slot_of = [&](int blk) {
+    return idx < DV ? p.cS + ((size_t)blk * a.H + h) * DV + idx : p.cn + ((size_t)blk * a.H + h) * a.D + (idx - DV);
+  };
+  float sv[VEC] = {};
+  if (state && !fresh) load(state, sv);
   // eight blocks at a time: all their loads are issued before the first store, so the chain is the arithmetic only
   for (int b0 = 0; b0 < nblk; b0 += 8) {
-    float bL[8], A[8], u[8];
+    float bL[8], A[8], u[8][VEC] = {};
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const int blk = first + min(b0 + j, nblk - 1);
       const float* sc = p.csc + ((size_t)blk * a.H + h) * 4;
       bL[j] = sc[0];
       A[j] = sc[1];
-      u[j] = 0.f;
-      if (state) u[j] = idx < DV ? p.cS[((size_t)blk * a.H + h) * DV + idx] : p.cn[((size_t)blk * a.H + h) * a.D + (idx - DV)];
+      if (state) load(slot_of(blk), u[j]);
     }
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
@@ -542,28 +580,31 @@ mlstm_par_carry_kernel(MlstmArgs a, MlstmPar p, int n_tiles) {
       const int blk = first + b0 + j;
       const float M = fmaxf(m0, A[j]), g = expf(m0 - M), w = expf(A[j] - M);
       if (state) {
-        float* slot = idx < DV ? p.cS + ((size_t)blk * a.H + h) * DV + idx : p.cn + ((size_t)blk * a.H + h) * a.D + (idx - DV);
-        *slot = sv;
-        sv = g * sv + w * u[j];
+        store(slot_of(blk), sv);
+#pragma unroll
+        for (int k = 0; k < VEC; ++k) sv[k] = g * sv[k] + w * u[j][k];
       }
       if (idx == 0) p.csc[((size_t)blk * a.H + h) * 4 + 2] = m0;
       m0 = bL[j] + M;
     }
   }
-  if (state) *state = sv;
+  if (state) store(state, sv);
   // the slot's m is read by every CTA of this pass: its new value waits in the last block's scalars until pass 3
   if (idx == 0) p.csc[((size_t)(first + nblk - 1) * a.H + h) * 4 + 3] = m0;
 }
 
+// The state of a column slice takes the place of the keys once the scores are formed, so that two CTAs share an SM: with one, 370
+// CTAs of 136 KB were three waves of loads, products and exponentials one after the other (72 -> 59 us for 650 rows, 8 heads of
+// 128 x 256).
 template <typename E>
-__global__ void __launch_bounds__(kMcThreads)
+__global__ void __launch_bounds__(kMcThreads, 2)
 mlstm_par_readout_kernel(const E* __restrict__ proj, float* __restrict__ o, MlstmArgs a, MlstmPar p) {
   extern __shared__ __align__(16) float smc[];
   const int D = a.D;
   float* qT = smc;
   float* kT = qT + (size_t)D * kMcLp;
-  float* Ss = kT + (size_t)D * kMcLp;
-  float* AT = Ss + (size_t)D * kMcCols;
+  float* Ss = kT;  // [D][kMcCols], after the scores
+  float* AT = kT + (size_t)D * kMcLp;
   float* vs = AT + kMcL * kMcLp;
   float* ns = vs + kMcL * kMcCols;
   float* av = ns + D;
@@ -582,10 +623,6 @@ mlstm_par_readout_kernel(const E* __restrict__ proj, float* __restrict__ o, Mlst
   const float m0 = p.csc[((size_t)blk * a.H + h) * 4 + 2];
   if (tid == 0 && blockIdx.z == 0 && t0 + kMcL >= e.z)
     a.m[(size_t)e.x * a.H + h] = p.csc[((size_t)blk * a.H + h) * 4 + 3];
-  for (int i = tid; i < D * kMcCols; i += kMcThreads) {
-    const int d = i / kMcCols, c = c0 + i % kMcCols;
-    Ss[i] = c < a.V ? Sin[(size_t)d * a.V + c] : 0.f;
-  }
   for (int d = tid; d < D; d += kMcThreads) ns[d] = nin[d];
   mlstm_load_kv_gates(proj + (size_t)(e.y + t0) * a.ldp, a, h, len, c0, 1.f / sqrtf((float)D), ib, fb, qT, kT, vs, av, bv, true);
   __syncthreads();
@@ -611,10 +648,25 @@ mlstm_par_readout_kernel(const E* __restrict__ proj, float* __restrict__ o, Mlst
         AT[sidx * kMcLp + t] = (sidx <= t) ? acc[i][j] * expf(av[sidx] - Mv[t]) : 0.f;
       }
   }
-  if (tid < kMcL) {
+  __syncthreads();  // the keys have been read
+  if (p.vec4) {
+#pragma unroll 8
+    for (int i = tid; i < D * (kMcCols / 4); i += kMcThreads) {
+      const int d = i / (kMcCols / 4), c = c0 + i % (kMcCols / 4) * 4;
+      reinterpret_cast<float4*>(Ss)[i] = c < a.V ? *reinterpret_cast<const float4*>(Sin + (size_t)d * a.V + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  } else {
+    for (int i = tid; i < D * kMcCols; i += kMcThreads) {
+      const int d = i / kMcCols, c = c0 + i % kMcCols;
+      Ss[i] = c < a.V ? Sin[(size_t)d * a.V + c] : 0.f;
+    }
+  }
+  {  // q . n of a row by four threads
     float d0 = 0.f;
-    for (int d = 0; d < D; ++d) d0 = fmaf(ns[d], qT[d * kMcLp + tid], d0);
-    qn[tid] = d0;
+    for (int d = tid & 3; d < D; d += 4) d0 = fmaf(ns[d], qT[d * kMcLp + (tid >> 2)], d0);
+    d0 += __shfl_xor_sync(0xffffffffu, d0, 1);
+    d0 += __shfl_xor_sync(0xffffffffu, d0, 2);
+    if ((tid & 3) == 0) qn[tid >> 2] = d0;
   }
   __syncthreads();
   float inter[4][4] = {}, intra[4][4] = {};
@@ -653,6 +705,12 @@ mlstm_par_readout_kernel(const E* __restrict__ proj, float* __restrict__ o, Mlst
       if (c < a.V) o[((size_t)(e.y + t0 + t) * a.H + h) * a.V + c] = (g * inter[i][j] + intra[i][j]) / den;
     }
   }
+}
+
+static_assert(kMcThreads == 4 * kMcL, "four threads per row");
+
+static size_t mlstm_readout_smem(int D) {
+  return sizeof(float) * (2 * (size_t)D * kMcLp + kMcL * kMcLp + kMcL * kMcCols + D + 5 * kMcL);
 }
 
 static size_t mlstm_chunk_smem(int D) {
@@ -737,27 +795,30 @@ int dli_mlstm_ragged_parallel(const void* proj, float* o_scratch, void* y, const
   if (csmem > 220 * 1024) return dli::fail(DLI_ERR_UNSUPPORTED, "dli_mlstm_ragged_parallel: key size %d is too large for the block form", D);
   if (rows <= 0 || n_ent <= 0 || n_tiles <= 0) return DLI_OK;
   MlstmArgs a{ent, H, D, V, ldp, q_off, k_off, v_off, i_off, f_off, i_bias, f_bias, cap, S, n, m};
-  MlstmPar p{tiles, scratch, scratch + (size_t)n_tiles * H * D * V, scratch + (size_t)n_tiles * H * ((size_t)D * V + D)};
+  MlstmPar p{tiles, scratch, scratch + (size_t)n_tiles * H * D * V, scratch + (size_t)n_tiles * H * ((size_t)D * V + D),
+              D % 4 == 0 && V % 4 == 0 && aligned16(scratch) && aligned16(S) && aligned16(n)};
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const dim3 bgrid(n_tiles, H, (V + kMcCols - 1) / kMcCols);
   const size_t lsmem = sizeof(float) * ((size_t)D * kMcLp + kMcL * kMcCols + 4 * kMcL);
   const size_t total = (size_t)D * V + D;
-  const dim3 cgrid(n_ent, H, (unsigned)((total + 255) / 256));
+  const size_t rsmem = mlstm_readout_smem(D);
+  const dim3 cgrid(n_ent, H, (unsigned)((total + (p.vec4 ? 1023 : 255)) / (p.vec4 ? 1024 : 256)));
+  const auto carry = p.vec4 ? mlstm_par_carry_kernel<4> : mlstm_par_carry_kernel<1>;
   if (dt == 0) {
     static PerDeviceOnce once;
     DLI_ONCE_PER_DEVICE(once, dev, DLI_CUDA_CALL(cudaFuncSetAttribute(mlstm_par_local_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
                         DLI_CUDA_CALL(cudaFuncSetAttribute(mlstm_par_readout_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024)));
     DLI_LAUNCH("mlstm_par_local", mlstm_par_local_kernel<bf16>, bgrid, dim3(kMcThreads), lsmem, s, (const bf16*)proj, a, p);
-    DLI_LAUNCH("mlstm_par_carry", mlstm_par_carry_kernel, cgrid, dim3(256), 0, s, a, p, n_tiles);
-    DLI_LAUNCH("mlstm_par_readout", mlstm_par_readout_kernel<bf16>, bgrid, dim3(kMcThreads), csmem, s, (const bf16*)proj, o_scratch, a, p);
+    DLI_LAUNCH("mlstm_par_carry", carry, cgrid, dim3(256), 0, s, a, p, n_tiles);
+    DLI_LAUNCH("mlstm_par_readout", mlstm_par_readout_kernel<bf16>, bgrid, dim3(kMcThreads), rsmem, s, (const bf16*)proj, o_scratch, a, p);
     DLI_LAUNCH("mlstm_out", mlstm_out_kernel<bf16>, dim3((rows * H + 3) / 4), dim3(128), 0, s, (const float*)o_scratch, (const bf16*)proj, out_w, (bf16*)y, rows, H, V, ldp, g_off, eps);
   } else {
     static PerDeviceOnce once;
     DLI_ONCE_PER_DEVICE(once, dev, DLI_CUDA_CALL(cudaFuncSetAttribute(mlstm_par_local_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
                         DLI_CUDA_CALL(cudaFuncSetAttribute(mlstm_par_readout_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024)));
     DLI_LAUNCH("mlstm_par_local", mlstm_par_local_kernel<float>, bgrid, dim3(kMcThreads), lsmem, s, (const float*)proj, a, p);
-    DLI_LAUNCH("mlstm_par_carry", mlstm_par_carry_kernel, cgrid, dim3(256), 0, s, a, p, n_tiles);
-    DLI_LAUNCH("mlstm_par_readout", mlstm_par_readout_kernel<float>, bgrid, dim3(kMcThreads), csmem, s, (const float*)proj, o_scratch, a, p);
+    DLI_LAUNCH("mlstm_par_carry", carry, cgrid, dim3(256), 0, s, a, p, n_tiles);
+    DLI_LAUNCH("mlstm_par_readout", mlstm_par_readout_kernel<float>, bgrid, dim3(kMcThreads), rsmem, s, (const float*)proj, o_scratch, a, p);
     DLI_LAUNCH("mlstm_out", mlstm_out_kernel<float>, dim3((rows * H + 3) / 4), dim3(128), 0, s, (const float*)o_scratch, (const float*)proj, out_w, (float*)y, rows, H, V, ldp, g_off, eps);
   }
   return DLI_OK;
