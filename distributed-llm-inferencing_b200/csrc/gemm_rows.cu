@@ -19,7 +19,8 @@
 //   4096 x 14336   24.6 -> 21.7   35.2 -> 27.4   94.5 -> 40.1   97.4 -> 97.4 (persistent kernel)
 //   28672 gated    42.4 -> 39.8   62.8 -> 48.9   87.2 -> 79.2  181   -> 181  (persistent kernel)
 //   768 x 3072      9.7 ->  4.6   30.6 ->  6.0   29.2 ->  7.6   28.8 -> 11.8
-// (before: split-K through global memory up to 128 rows, the persistent kernel of 128-row tiles above.)
+// (before: split-K through global memory up to 128 rows, the persistent kernel of 128-row tiles above; from some 400 rows on pairs
+// of SMs take over, gemm_pair.cu: 4096 x 4096 at 1 024 rows 30 us, 4096 x 14336 85, 28672 gated 163.)
 #include "gemm_rows.cuh"
 #include "recent.h"
 

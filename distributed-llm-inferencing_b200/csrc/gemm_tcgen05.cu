@@ -5,8 +5,9 @@
 //   y[M,N] = epi( x[M,K] . w[N,K]^T )          both operands K-major (row-major,
 //                                              K contiguous) = HF Linear layout
 //
-// Persistent kernel for prompt passes of many rows; fewer rows (and every projection of a batched decode step) run as
-// K-split clusters with swapped operands (gemm_rows.cu), chosen per call by estimated time (choose below).
+// The GEMM entry points, which choose a kernel by estimated time (choose below), and one of the kernels: persistent, on single
+// SMs.  Few rows (every projection of a batched decode step among them) run as K-split clusters with swapped operands
+// (gemm_rows.cu), most prompt passes on pairs of SMs (gemm_pair.cu).
 // Gated MLP (template kGated): w is the [gate128 | up128]-interleaved matrix, one BN = 256 tile holds gate columns 0-127
 //   and up columns 128-255; the epilogue computes bf16(silu(bf16(g))) * bf16(u) — the HF rounding points.
 //
@@ -344,7 +345,7 @@ static int choose(int M, int N, int K, bool gated, Choice* c) {
   if (M > 128 && N < 128) return DLI_OK;
   PrefillShape p;
   double us, best = pick_prefill(M, N, K, gated, &p) + 9.5;
-  if (pairs && ((M + 127) / 128) % 2 == 0) best = 1e30;
+  if (pairs && (M > 1024 || ((M + 127) / 128) % 2 == 0)) best = 1e30;  // 256-row tiles are full, or nearly
   if (M <= 4096) {
     if ((rc = plan_gemm_rows(M, N, K, &c->rows, &us)) != DLI_OK) return rc;
     us = pairs ? 0.88 * us + 1.5 : 1.1 * us;
