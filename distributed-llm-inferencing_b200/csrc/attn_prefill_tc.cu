@@ -161,10 +161,12 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm, const __grid_cons
   }
   if (warp == 1) tmem_alloc(smem_addr(tmem_ptr_smem), 512);
   pdl_wait();
-  pdl_trigger();
   tcgen05_fence_before();
   __syncthreads();
   tcgen05_fence_after();
+  // Behind the barrier, that is with the tensor memory in hand: one thread's trigger counts for the CTA, and at head size 64 a
+  // projection's CTA fits beside this one.  It would take columns and wait for this grid, which would wait for the columns.
+  pdl_trigger();
   const uint32_t tmem_base = *tmem_ptr_smem;
   // S0 | S1 | O (128 columns each) | P0 | P1 (64 columns each: 128 bf16 probabilities per row, two per column)
   const uint32_t tS = tmem_base, tO = tmem_base + 256, tP = tmem_base + 384;
