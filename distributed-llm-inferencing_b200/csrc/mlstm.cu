@@ -115,6 +115,12 @@ mlstm_scan_kernel(const E* __restrict__ proj, float* __restrict__ o, MlstmArgs a
   }
 }
 
+// Columns off ... off + width - 1 of every row from `base` on as whole 16-byte pieces (bf16 rows may start anywhere).
+template <typename E>
+__device__ __forceinline__ bool mlstm_vec8(const E* base, int ldp, int off, int width) {
+  return sizeof(E) == 2 && ((reinterpret_cast<uintptr_t>(base) & 15u) | ((ldp | off | width) & 7)) == 0;
+}
+
 // ---- portions of prompts: the same recurrence, 64 positions at a time ------------------------------------------
 // Within a block of L positions (t = 1..L) let b_t be the running sum of the log forget gates, a_s = i_s - b_s and
 // M_t = max(m_0, max_{s<=t} a_s).  Unrolling the recurrence gives m_t = b_t + M_t and
@@ -164,7 +170,7 @@ mlstm_chunk_kernel(const E* __restrict__ proj, float* __restrict__ o, MlstmArgs 
     const int len = min(kMcL, e.z - t0);
     const E* base = proj + (size_t)(e.y + t0) * a.ldp;
     // q, k transposed (zero beyond len), v slice, gates
-    if (sizeof(E) == 2 && D % 8 == 0 && (a.q_off + h * D) % 8 == 0 && (a.k_off + h * D) % 8 == 0 && a.ldp % 8 == 0) {
+    if (mlstm_vec8(proj, a.ldp, a.q_off + h * D, D) && mlstm_vec8(proj, a.ldp, a.k_off + h * D, D)) {
       // 16-byte loads; consecutive threads take consecutive rows so that the transposed stores do not collide
 #pragma unroll 4
       for (int i = tid; i < kMcL * (D / 8); i += kMcThreads) {
@@ -373,7 +379,7 @@ __device__ __forceinline__ void mlstm_load_kv_gates(const E* base, const MlstmAr
                                                     float ib, float fb, float* qT, float* kT, float* vs, float* av,
                                                     float* bv, bool want_q) {
   const int D = a.D, tid = threadIdx.x;
-  if (sizeof(E) == 2 && D % 8 == 0 && (a.q_off + h * D) % 8 == 0 && (a.k_off + h * D) % 8 == 0 && a.ldp % 8 == 0) {
+  if (mlstm_vec8(base, a.ldp, a.q_off + h * D, D) && mlstm_vec8(base, a.ldp, a.k_off + h * D, D)) {
 #pragma unroll 4
     for (int i = tid; i < kMcL * (D / 8); i += kMcThreads) {
       const int t = i % kMcL, d8 = i / kMcL;
@@ -403,7 +409,7 @@ __device__ __forceinline__ void mlstm_load_kv_gates(const E* base, const MlstmAr
       kT[d * kMcLp + t] = kv;
     }
   }
-  if (sizeof(E) == 2 && a.V % 8 == 0 && (a.v_off + h * a.V) % 8 == 0 && a.ldp % 8 == 0) {
+  if (mlstm_vec8(base, a.ldp, a.v_off + h * a.V, a.V)) {
 #pragma unroll
     for (int i = tid; i < kMcL * (kMcCols / 8); i += kMcThreads) {
       const int t = i / (kMcCols / 8), c = c0 + i % (kMcCols / 8) * 8;

@@ -316,6 +316,51 @@ def test_mlstm_portions_and_dirty_slots(dims, cuts, blocked):
     assert (out.double().cpu() - ref).abs().max() < 3e-4 * max(1.0, ref.abs().max().item())
 
 
+@pytest.mark.parametrize("start,shift,pad", [(0, 0, 0), (1, 0, 0), (4, 0, 0), (0, 1, 7), (0, 4, 4), (3, 5, 3), (0, 8, 1)])
+@pytest.mark.parametrize("dims", [(2, 56, 96), (3, 10, 40), (2, 16, 72), (1, 130, 33), (2, 8, 256)])
+@pytest.mark.parametrize("blocked", [False, True, "parallel"])
+def test_mlstm_rows_of_bf16_that_start_anywhere(dims, start, shift, pad, blocked):
+    """bf16 projections whose first row starts `start` elements past a 16-byte boundary, whose columns are preceded by `shift`
+    others and whose row stride leaves `pad`, against the oracle on the same values.  Value sizes that are a multiple of 8 but not
+    of the 64 columns a block takes, key sizes that are none; states that are whole vectors and states that are not.  Bound: the
+    fp32 recurrence as above, and one rounding of the output to bf16 (half an ulp: 2^-8 of it at most)."""
+    from dli_b200 import ops
+
+    H, D, V = dims
+    torch.manual_seed(7)
+    m = {"heads": H, "dim": D, "vdim": V, "gate_cap": 6.0}
+    cuts, T = [70, 1, 64, 15], 150
+    w = 2 * H * D + 2 * H * V + 2 * H
+    ld = shift + w + pad
+    x = torch.randn(T, w)
+    x[:, -2 * H:] *= 4
+    x = x.bfloat16()
+    q, k, v, g, ig, fg = (c.double() for c in x.split((H * D, H * D, H * V, H * V, H, H), dim=1))
+    ib, fb, nw = torch.randn(H), torch.randn(H), torch.rand(H * V) + 0.5
+    ref = mlstm_oracle(q, k, v, g, ig, fg, m, ib, fb, nw, 1e-5)
+    offs = [shift + o for o in (0, H * D, 2 * H * D, 2 * H * D + 2 * H * V, 2 * H * D + 2 * H * V + H, 2 * H * D + H * V)]
+    S, n, mm = torch.full((3, H, D, V), 9e3, device=DEV), torch.full((3, H, D), -4e3, device=DEV), torch.full((3, H), 55.0, device=DEV)
+    out, at = torch.empty(T, H * V, device=DEV), 0
+    for c in cuts:
+        pr = torch.full((start + c * ld,), float("nan"), dtype=torch.bfloat16, device=DEV)[start:].view(c, ld)
+        pr[:, shift:shift + w] = x[at:at + c].to(DEV)
+        _, ent = meta([(2, c, at)])
+        o, scratch = torch.empty(c, H * V, device=DEV, dtype=torch.bfloat16), torch.empty(c * H * V, device=DEV)
+        if blocked == "parallel":
+            tiles = torch.tensor([[0, q0] for q0 in range(0, c, 64)], dtype=torch.int32, device=DEV)
+            scr = torch.full((ops.mlstm_parallel_scratch_floats(tiles.shape[0], H, D, V),), float("nan"), device=DEV)
+            ops.mlstm_ragged_parallel(pr, scratch, o, ent, tiles, scr, H, D, V, *offs, ib.to(DEV), fb.to(DEV), 6.0, nw.to(DEV), 1e-5,
+                                      S, n, mm)
+        else:
+            ops.mlstm_ragged(pr, scratch, o, ent, H, D, V, *offs, ib.to(DEV), fb.to(DEV), 6.0, nw.to(DEV), 1e-5, S, n, mm,
+                             blocked=blocked)
+        out[at:at + c] = o.float()
+        at += c
+    assert at == T
+    err = (out.double().cpu() - ref).abs()
+    assert bool((err <= 3e-4 * max(1.0, ref.abs().max().item()) + 2.0 ** -8 * ref.abs()).all()), err.max()
+
+
 def test_rot_frequencies_match_the_oracle():
     from dli_b200.ragged_engine import rot_frequencies
 
