@@ -324,14 +324,17 @@ static PrefillShape prefill_tile(int M, int N, int K, bool gated) {
   return p;
 }
 
-// Which kernel takes a projection, by estimated time.  The clusters' estimate errs high from some 250 rows on (28672 x 4096 gated
-// at 301 rows: 91 us, measured 74): 0.88 of it + 1.5 us.  Over 9 matrices x 12 row counts from 150 to 700 what is picked is 0.9 %
-// slower than the faster of the first two on average, 10 % at most.
+// Which kernel takes a projection, by estimated time:
 //  - clusters that split K (gemm_rows.cu), up to 4 096 rows, which bound what was measured, and always up to 128 rows;
-//  - pairs of SMs (gemm_pair.cu) in tiles of 256 rows, from some 400 rows on;
-//  - the persistent kernel above where 256-row tiles would be half padding and the matrix is large (57344 x 8192 at 301 ... 384
-//    rows: 285 us, pairs 320), and for widths that are no multiple of 128, which no matrix of the models has: the only ones it
-//    was measured against the clusters for, whose estimate is taken 10 % high there.  It costs 9.5 us beyond its rounds.
+//  - pairs of SMs (gemm_pair.cu) in tiles of 256 rows, for widths that are multiples of 128; from 129 ... 500 rows on, by matrix;
+//  - the persistent kernel above where 256-row tiles would be half padding and the matrix is large (28672 x 4096 gated at 336
+//    rows: 85 us, clusters 95), and for other widths, at which the pairs were not measured.
+// The clusters' estimate errs high from some 250 rows on, by up to a quarter (28672 x 4096 gated at 301 rows: 91 us, measured 76),
+// and it knows nothing of the power limit, which costs them more than the pairs: 57344 x 8192 gated at 900 / 2 048 rows 751 / 1 504
+// estimated, 787 / 1 717 measured (pairs 636 / 1 345).  So 0.88 of it + 1.5 us, and a quarter more where the work reaches 10^12
+// operations, by its square below.  Against widths that are no multiple of 128 it is taken 10 % high.  The persistent kernel costs
+// 9.5 us beyond its rounds, 4.5 where the gated epilogue, half as many columns, hides under the next tile's long K.
+// Over 29 matrices x 30 row counts from 129 to 4 096 what is picked is 0.3 % slower than the fastest of the three on average.
 enum Route { kRouteRows, kRoutePair, kRoutePersistent };
 struct Choice {
   Route route;
@@ -344,11 +347,12 @@ static int choose(int M, int N, int K, bool gated, Choice* c) {
   c->route = kRoutePersistent;
   if (M > 128 && N < 128) return DLI_OK;
   PrefillShape p;
-  double us, best = pick_prefill(M, N, K, gated, &p) + 9.5;
+  double us, best = pick_prefill(M, N, K, gated, &p) + (gated && K >= 4096 ? 4.5 : 9.5);
   if (pairs && (M > 1024 || ((M + 127) / 128) % 2 == 0)) best = 1e30;  // 256-row tiles are full, or nearly
   if (M <= 4096) {
     if ((rc = plan_gemm_rows(M, N, K, &c->rows, &us)) != DLI_OK) return rc;
-    us = pairs ? 0.88 * us + 1.5 : 1.1 * us;
+    const double tera = 2e-12 * M * N * K, hot = tera < 1.0 ? tera : 1.0;
+    us = pairs ? (0.88 * us + 1.5) * (1.0 + 0.24 * hot * hot) : 1.1 * us;
     if (M <= 128 || us < best) c->route = kRouteRows, best = us;
     if (M <= 128) return DLI_OK;
   }
