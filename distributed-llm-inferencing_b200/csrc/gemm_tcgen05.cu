@@ -334,7 +334,12 @@ static PrefillShape prefill_tile(int M, int N, int K, bool gated) {
 // estimated, 787 / 1 717 measured (pairs 636 / 1 345).  So 0.88 of it + 1.5 us, and a quarter more where the work reaches 10^12
 // operations, by its square below.  Against widths that are no multiple of 128 it is taken 10 % high.  The persistent kernel costs
 // 9.5 us beyond its rounds, 4.5 where the gated epilogue, half as many columns, hides under the next tile's long K.
-// Over 29 matrices x 30 row counts from 129 to 4 096 what is picked is 0.3 % slower than the fastest of the three on average.
+// A matrix of more outputs than inputs may be a qkv projection, which takes the same kernel with its rotation and without: the
+// same K split, so the same bits.  It goes by what the pairs take with whole heads of 128 in a tile, widths of 128 and 256 alone:
+// 6144 x 4096 at 301 rows is estimated at 20.4 us in tiles of 176, at 26.1 in tiles of 256 (with the rotation 27.7 measured,
+// clusters 21.5).
+// Over 29 matrices x 30 row counts from 129 to 4 096 what is picked is 0.6 % slower than the fastest of the three on average, 0.3 %
+// where no rotation has a say.
 enum Route { kRouteRows, kRoutePair, kRoutePersistent };
 struct Choice {
   Route route;
@@ -358,6 +363,8 @@ static int choose(int M, int N, int K, bool gated, Choice* c) {
   }
   if (pairs) {
     if ((rc = plan_gemm_pair(gated ? kPairGated : kPairPlain, M, N, K, 128, &c->pair, &us)) != DLI_OK) return rc;
+    PairShape rotated;
+    if (!gated && N > K && (rc = plan_gemm_pair(kPairRope, M, N, K, 128, &rotated, &us)) != DLI_OK) return rc;
     if (us < best) c->route = kRoutePair;
   }
   return DLI_OK;

@@ -17,6 +17,13 @@ MEASURED = [  # rows, outputs, K, gated, kernel; us of the persistent kernel, th
     (400, 4096, 14336, False, "rows"),     # 90 / 44 / 50
     (450, 4096, 4096, False, "pairs"),     # 32 / 22 / 19
     (2048, 256, 4096, False, "rows"),      # narrow: the pairs 27 % slower
+    # qkv projections, with the rotation in the epilogue (without it they take the same kernel)
+    (129, 10240, 8192, False, "rows"),     # 67 / 37 / 49
+    (301, 6144, 4096, False, "rows"),      # 38 / 22 / 28
+    (384, 6144, 4096, False, "rows"),      # 38 / 23 / 28
+    (600, 6144, 4096, False, "pairs"),     # 38 / 30 / 29
+    (1024, 6144, 4096, False, "pairs"),    # 59 / 54 / 39
+    (512, 10240, 8192, False, "pairs"),    # 104 / 92 / 72
 ]
 
 
