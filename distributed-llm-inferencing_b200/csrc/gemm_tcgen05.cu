@@ -69,12 +69,20 @@ __device__ __forceinline__ void prefill_tile_coords(int tile, int m_tiles, int n
   m_blk = m0 + r - n_blk * gsize;
 }
 
+// kRope (the qkv projection of a prompt pass, head_dim 128, 128 x 256 tiles = two whole heads per tile): the epilogue
+// rotates q and k (rotate-half RoPE with the rounding points of apply_rotary_pos_emb on bf16 tensors,
+// TF:models/llama/modeling_llama.py:138-168, applied to the bf16-rounded projection exactly as the separate
+// rope_kv_append_kernel applies it to the stored one) and appends k and v to the paged cache — the work of
+// dli_rope_kv_append_bf16 without a second pass over the qkv matrix.  For large matrices at an odd number of 128-row tiles:
+// 10240 x 8192 at 350 rows 65 us, the pairs 72.
+//
 // threads: TMA warp + MMA warp + four epilogue warps per 128-row half
-template <int BN, bool kGated, int MT>
+template <int BN, bool kGated, int MT, bool kRope = false>
 __global__ void __launch_bounds__(64 + 128 * MT, 1)
 gemm_prefill_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     const bf16* __restrict__ bias, const bf16* residual, bf16* y, int M, int N, int K,
-                    int epilogue, int m_tiles, int num_tiles) {
+                    int epilogue, int m_tiles, int num_tiles, const __grid_constant__ RopeArgs rope) {
+  static_assert(!kRope || (BN == 256 && !kGated && MT == 1), "the RoPE epilogue works on two whole 128-wide heads");
   using Cfg = PrefillCfg<BN, kGated, MT>;
   constexpr int S = Cfg::kStages;
   constexpr int kMRows = MT * 128;
@@ -190,7 +198,76 @@ gemm_prefill_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       // per 16 columns before).  A chunk of 16 columns ahead instead: 127 -> 198, the store and the load share the line.
       constexpr int kLine = kGated ? 16 : 64;
       const int n_out = kGated ? N / 2 : N;
-      {
+      if constexpr (kRope) {
+        const uint32_t lane_base = tmem_base + as * Cfg::kAccCols + ((uint32_t)(quad * 32) << 16);
+        const int m = m_blk * 128 + quad * 32 + lane;
+        const bool live = m < M;
+        int pos = 0;
+        size_t cache_row = 0;  // ((page * KV) * page_size + slot): + kvh * page_size gives the token's row of a kv head
+        if (live) {
+          pos = rope.positions[m];
+          const int page = rope.page_table[(size_t)rope.seq_ids[m] * rope.max_pages + (pos >> rope.page_shift)];
+          cache_row = ((size_t)page * rope.KV << rope.page_shift) + (pos & ((1 << rope.page_shift) - 1));
+        }
+#pragma unroll 1
+        for (int hh = 0; hh < 2; ++hh) {
+          const int head = (n_tile0 >> 7) + hh;  // q heads, then k heads, then v heads
+          if (head >= rope.H + 2 * rope.KV) break;
+          bf16* yrow = y + (size_t)m * N + (size_t)head * 128;
+          if (head < rope.H + rope.KV) {
+            bf16* crow = head >= rope.H ? rope.k_cache + (cache_row + ((size_t)(head - rope.H) << rope.page_shift)) * 128 : nullptr;
+#pragma unroll 1
+            for (int j = 0; j < 4; ++j) {  // 16 rotation pairs (i, i + 64) per step
+              uint32_t r1[16], r2[16];
+              tmem_ld_32x16(lane_base + hh * 128 + j * 16, r1);
+              tmem_ld_32x16(lane_base + hh * 128 + 64 + j * 16, r2);
+              tmem_ld_wait();
+              if (live) {
+                float c[16], sn[16], o1[16], o2[16];
+                unpack8(ld_16B(rope.cos_t + (size_t)pos * 64 + j * 16), c);
+                unpack8(ld_16B(rope.cos_t + (size_t)pos * 64 + j * 16 + 8), c + 8);
+                unpack8(ld_16B(rope.sin_t + (size_t)pos * 64 + j * 16), sn);
+                unpack8(ld_16B(rope.sin_t + (size_t)pos * 64 + j * 16 + 8), sn + 8);
+#pragma unroll
+                for (int e = 0; e < 16; ++e) {
+                  const float x1 = round_bf16(__uint_as_float(r1[e])), x2 = round_bf16(__uint_as_float(r2[e]));
+                  o1[e] = round_bf16(x1 * c[e]) + round_bf16(-x2 * sn[e]);
+                  o2[e] = round_bf16(x2 * c[e]) + round_bf16(x1 * sn[e]);
+                }
+#pragma unroll
+                for (int v8 = 0; v8 < 2; ++v8) {
+                  const uint4 u1 = pack8(o1 + v8 * 8), u2 = pack8(o2 + v8 * 8);
+                  st_16B(yrow + j * 16 + v8 * 8, u1);
+                  st_16B(yrow + 64 + j * 16 + v8 * 8, u2);
+                  if (crow) {
+                    st_16B(crow + j * 16 + v8 * 8, u1);
+                    st_16B(crow + 64 + j * 16 + v8 * 8, u2);
+                  }
+                }
+              }
+            }
+          } else {
+            bf16* crow = rope.v_cache + (cache_row + ((size_t)(head - rope.H - rope.KV) << rope.page_shift)) * 128;
+#pragma unroll 1
+            for (int j = 0; j < 8; ++j) {
+              uint32_t r1[16];
+              tmem_ld_32x16(lane_base + hh * 128 + j * 16, r1);
+              tmem_ld_wait();
+              if (live) {
+                float v[16];
+#pragma unroll
+                for (int e = 0; e < 16; ++e) v[e] = __uint_as_float(r1[e]);
+#pragma unroll
+                for (int v8 = 0; v8 < 2; ++v8) {
+                  const uint4 u = pack8(v + v8 * 8);
+                  st_16B(yrow + j * 16 + v8 * 8, u);
+                  st_16B(crow + j * 16 + v8 * 8, u);
+                }
+              }
+            }
+          }
+        }
+      } else {
         const int h = (warp - 2) >> 2;  // warps 2-5: rows 0-127 of the tile, warps 6-9 (MT = 2): rows 128-255
         const uint32_t lane_base = tmem_base + as * Cfg::kAccCols + h * BN + ((uint32_t)(quad * 32) << 16);
         const int m = m_blk * kMRows + h * 128 + quad * 32 + lane;
@@ -264,12 +341,13 @@ gemm_prefill_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 }
 
 // ---- host side ---------------------------------------------------------------------------
-template <int BN, bool kGated, int MT = 1>
+template <int BN, bool kGated, int MT = 1, bool kRope = false>
 static int launch_prefill_gemm(const void* x, const void* w, const void* bias, const void* residual, void* y, int M,
-                               int N /* rows of w */, int K, int epilogue, cudaStream_t s) {
+                               int N /* rows of w */, int K, int epilogue, cudaStream_t s,
+                               const RopeArgs& rope = RopeArgs{}) {
   using Cfg = PrefillCfg<BN, kGated, MT>;
   static PerDeviceOnce once;
-  DLI_ONCE_PER_DEVICE(once, dev, DLI_CUDA_CALL(cudaFuncSetAttribute(gemm_prefill_kernel<BN, kGated, MT>,
+  DLI_ONCE_PER_DEVICE(once, dev, DLI_CUDA_CALL(cudaFuncSetAttribute(gemm_prefill_kernel<BN, kGated, MT, kRope>,
                                                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                                     Cfg::kSmemBytes)));
   CUtensorMap tmA, tmB;
@@ -280,9 +358,9 @@ static int launch_prefill_gemm(const void* x, const void* w, const void* bias, c
   const int num_tiles = m_tiles * n_tiles;
   const int sms = sm_count_cached();
   const int grid = num_tiles < sms ? num_tiles : sms;
-  DLI_LAUNCH("gemm_prefill_kernel", (gemm_prefill_kernel<BN, kGated, MT>), dim3(grid), dim3(64 + 128 * MT),
+  DLI_LAUNCH("gemm_prefill_kernel", (gemm_prefill_kernel<BN, kGated, MT, kRope>), dim3(grid), dim3(64 + 128 * MT),
              (size_t)Cfg::kSmemBytes, s, tmA, tmB, (const bf16*)bias, (const bf16*)residual, (bf16*)y, M, N, K, epilogue,
-             m_tiles, num_tiles);
+             m_tiles, num_tiles, rope);
   return DLI_OK;
 }
 
@@ -370,14 +448,20 @@ static int choose(int M, int N, int K, bool gated, Choice* c) {
   return DLI_OK;
 }
 
-// The persistent kernel and the pairs add K in the same order: the same bits whichever of them the projection by itself takes.
-static int launch_pair_rope(const void* x, const void* w, const void* bias, void* qkv, int M, int N, int K, const RopeArgs& rope,
-                            int hd, cudaStream_t s) {
+// The rotating form of the chosen kernel, or of the pairs where the persistent kernel has none for these heads: those two add K in
+// the same order, so the bits are the projection's by itself all the same.
+static int launch_rope(const Choice& c, const void* x, const void* w, const void* bias, void* qkv, int M, int N, int K,
+                       const RopeArgs& rope, int hd, cudaStream_t s) {
+  const int epilogue = bias ? DLI_EPI_BIAS : 0;
+  if (c.route == kRouteRows)
+    return launch_gemm_rows(kRowsRope, x, w, bias, nullptr, qkv, M, N, K, epilogue, c.rows, s, rope, hd);
+  if (c.route == kRoutePersistent && hd == 128 && rope.H % 2 == 0 && rope.KV % 2 == 0 && !bias && rope.cos_t)
+    return launch_prefill_gemm<256, false, 1, true>(x, w, nullptr, nullptr, qkv, M, N, K, 0, s, rope);
   PairShape sh;
   double us;
   const int rc = plan_gemm_pair(kPairRope, M, N, K, hd, &sh, &us);
   if (rc != DLI_OK) return rc;
-  return launch_gemm_pair(kPairRope, x, w, bias, nullptr, qkv, M, N, K, bias ? DLI_EPI_BIAS : 0, sh, s, rope, hd);
+  return launch_gemm_pair(kPairRope, x, w, bias, nullptr, qkv, M, N, K, epilogue, sh, s, rope, hd);
 }
 
 // qkv = x w^T (+ bias), q and k rotated, k and v appended to the cache pages: one kernel where a projection kernel has that
@@ -392,9 +476,7 @@ int linear_qkv_append(const void* x, const void* w, const void* bias, void* qkv,
     Choice c;
     const int rc = choose(M, N, K, false, &c);
     if (rc != DLI_OK) return rc;
-    if (c.route == kRouteRows)
-      return launch_gemm_rows(kRowsRope, x, w, bias, nullptr, qkv, M, N, K, bias ? DLI_EPI_BIAS : 0, c.rows, s, rope, hd);
-    if (N % 128 == 0) return launch_pair_rope(x, w, bias, qkv, M, N, K, rope, hd, s);
+    if (c.route == kRouteRows || N % 128 == 0) return launch_rope(c, x, w, bias, qkv, M, N, K, rope, hd, s);
   }
   const int rc = dli_linear_bf16(x, w, bias, nullptr, qkv, M, N, K, bias ? DLI_EPI_BIAS : 0, s);
   if (rc != DLI_OK) return rc;
@@ -502,9 +584,7 @@ int dli_gemm_qkv_rope_append_bf16(const void* x, const void* w_qkv, void* qkv, i
   Choice c;
   const int rc = choose(M, N, K, false, &c);
   if (rc != DLI_OK) return rc;
-  if (c.route == kRouteRows)
-    return launch_gemm_rows(kRowsRope, x, w_qkv, nullptr, nullptr, qkv, M, N, K, 0, c.rows, s, ra, hd);
-  return launch_pair_rope(x, w_qkv, nullptr, qkv, M, N, K, ra, hd, s);
+  return launch_rope(c, x, w_qkv, nullptr, qkv, M, N, K, ra, hd, s);
 }
 
 static int gemm_gated_act(const void* x, const void* w_gu, void* y, int M, int F, int K, const float* act, dli_stream_t stream);

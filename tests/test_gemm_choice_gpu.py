@@ -3,6 +3,8 @@ others by 4 % and more, around where the choice has its borders.  The times are 
 import pytest
 
 pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+BF = torch.bfloat16
 
 MEASURED = [  # rows, outputs, K, gated, kernel; us of the persistent kernel, the clusters and the pairs
     (1777, 8192, 28672, False, "pairs"),   # 680 / 713 / 545
@@ -34,3 +36,43 @@ def test_the_kernel_measured_to_be_faster(cuda, M, N, K, gated, kernel):
     if ops.sm_count() != 148:
         pytest.skip("the choice counts SMs")
     assert ops.gemm_plan(M, N, K, gated)[0] == kernel
+
+
+@pytest.mark.parametrize("hd,H,KV,bias,kernel", [(128, 64, 8, False, "gemm_prefill_kernel"), (128, 64, 8, True, "gemm_pair_kernel"),
+                                                 (128, 78, 1, False, "gemm_pair_kernel"), (64, 128, 16, False, "gemm_pair_kernel")])
+def test_qkv_where_the_persistent_kernel_is_chosen(cuda, hd, H, KV, bias, kernel):
+    """The rotation and the cache append in the persistent kernel's epilogue where it has them, else in the pairs': the bits of the
+    projection on the persistent kernel and the separate rotation either way."""
+    from dli_b200 import ops
+
+    T, d, ff, page, prefix = 350, 8192, 256, 16, 5
+    g = torch.Generator(device="cuda").manual_seed(H)
+    rnd = lambda *s, std=1.0: (std * torch.randn(*s, device=cuda, generator=g)).to(BF)  # noqa: E731
+    N, pages = (H + 2 * KV) * hd, (T + prefix + 15) // 16
+    if ops.sm_count() == 148:
+        assert ops.gemm_plan(T, N, d)[0] == "persistent"
+    L = {"ln1": rnd(d), "ln2": rnd(d), "wqkv": rnd(N, d, std=0.02), "wo": rnd(d, H * hd, std=0.02), "wdown": rnd(d, ff, std=0.02),
+         "wgu": ops.pack_gate_up(rnd(ff, d, std=0.02), rnd(ff, d, std=0.02))}
+    if bias:
+        L["bqkv"] = rnd(N)
+    ang = torch.rand(T + prefix, hd // 2, device=cuda, generator=g) * 6.28
+    cos, sin = ang.cos().to(BF), ang.sin().to(BF)
+    table = torch.randperm(pages, device=cuda, generator=g).int().view(1, pages)
+    positions, seq_ids, last = (torch.empty(T, device=cuda, dtype=torch.int32) for _ in range(3))
+    ops.prompt_rows(positions, seq_ids, last, 1, T, prefix, 0)
+    h_in = rnd(T, d)
+    kc, vc = (torch.zeros(pages, KV, page, hd, device=cuda, dtype=BF) for _ in range(2))
+    h, x, qkv, attn, act = (torch.empty(T, w, device=cuda, dtype=BF) for w in (d, d, N, H * hd, ff))
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        ops.prompt_layers([L], [kc], [vc], table, table, h_in, h, x, qkv, attn, act, cos, sin, positions, seq_ids, 1, T, prefix,
+                          H, KV, hd, 1e-5, hd ** -0.5)
+        torch.cuda.synchronize()
+    names = [e.name for e in prof.events()]
+    assert not any("rope_kv_append" in n for n in names)
+    if ops.sm_count() == 148:
+        assert kernel in next(n for n in names if "gemm_" in n)  # the first projection
+    ops.add_rmsnorm(h_in, L["ln1"], 1e-5, out=x)
+    want = ops.gemm(x, L["wqkv"], bias=L.get("bqkv"))
+    k2, v2 = torch.zeros_like(kc), torch.zeros_like(vc)
+    ops.rope_kv_append(want, cos, sin, positions, seq_ids, table, k2, v2, H, KV, hd)
+    assert torch.equal(qkv, want) and torch.equal(kc, k2) and torch.equal(vc, v2)
