@@ -16,13 +16,13 @@
 //         are what the parity test compares.
 //
 // What bounds it: latency.  A row is 64 ... 256 KB, a few us of one SM's load bandwidth, so it is cut over a cluster of up
-// to 8 CTAs (16 384 logits each) and read ONCE, with 16-byte loads, into registers, as keys that compare two at a time.  The k-th
-// largest logit is found without a histogram of the row: the k-th largest of a CTA's 512 per-thread maxima is a lower bound of it
-// (k threads hold an element at least that large), the largest such bound of the cluster leaves a few hundred candidates, each CTA
-// writes its own into its region of the first CTA's shared memory, and the exact threshold is a search over the bits in which
-// bound and maximum differ.  Up to 64 that remain are put in order by counting and finished by one warp in registers; the
-// uniform is drawn while the cluster meets.  One row of 128 256 logits, us: load and maxima 0.9, bound 1.5, exchange 0.5,
-// candidates 1.0, gathering 0.9, threshold 1.8, order 0.5, softmax and nucleus 0.9, draw 0.4.
+// to 8 CTAs.  A CTA keeps the first 16 384 logits of its slice in registers, as keys that compare two at a time; what a longer
+// slice has beyond them (many rows, fewer CTAs each) is read twice, for the bound and for the candidates.  The k-th largest logit
+// is found without a histogram of the row: the k-th largest of a CTA's 512 per-thread maxima is a lower bound of it (k threads
+// hold an element at least that large), the largest such bound of the cluster leaves a few hundred candidates, each CTA writes
+// its own into its region of the first CTA's shared memory, and the exact threshold is a search over the bits in which bound and
+// maximum differ.  Up to 64 that remain are put in order by counting and finished by one warp in registers; the uniform is drawn
+// while the cluster meets.  One row of 128 256 logits takes 8.6 us, 48 rows 12.5.
 // (The two 256-bin histograms with shared-memory atomics and their serial scans, three passes of 2-byte loads by one CTA per
 // row, took 62 us for one row as for 48, V = 128 256.  They are left for large k, see launch_sample.)
 #include <math.h>
@@ -104,18 +104,17 @@ __device__ __forceinline__ uint32_t max_keys2(uint32_t a, const uint4& u) {
 }
 
 // The largest t in [base, base + 2^bits) with at least k of the block's keys >= t, where k of them are >= base: a bit a step, a
-// count of the block each (0.1 us).  Two bits a step take three counts, and every way to sum them over 16 warps (reductions, atomics)
-// was slower: 0.28 us a step.
-template <int NQ>
-__device__ __forceinline__ uint32_t kth_key(const uint32_t (&keys)[NQ], int nq, int k, uint32_t base, int bits) {
+// count of the block for each of a thread's first NQ keys (0.1 us; a test of how many there are inside the loop doubles that).
+// Two bits a step take three counts, and every way to sum them over 16 warps (reductions, atomics) was slower: 0.28 us a step.
+template <int NQ, int N>
+__device__ __forceinline__ uint32_t kth_key(const uint32_t (&keys)[N], int k, uint32_t base, int bits) {
   uint32_t t = base;
 #pragma unroll 1
   for (int sh = bits - 1; sh >= 0; --sh) {
     const uint32_t a = t + (1u << sh);
     int count = 0;
 #pragma unroll
-    for (int q = 0; q < NQ; ++q)
-      if (q < nq) count += __syncthreads_count(keys[q] >= a);
+    for (int q = 0; q < NQ; ++q) count += __syncthreads_count(keys[q] >= a);
     if (count >= k) t = a;
   }
   return t;
@@ -267,7 +266,7 @@ sample_kernel(const bf16* __restrict__ logits, int ld, int32_t* __restrict__ out
       if (lane == 0) mths[warp] = mth;
       __syncthreads();
       const uint32_t lo = __reduce_min_sync(0xffffffffu, mths[lane & 15]), hi = __reduce_max_sync(0xffffffffu, mths[lane & 15]);
-      bound = kth_key(top, 1, k, lo, 32 - __clz(hi - lo));
+      bound = kth_key<1>(top, k, lo, 32 - __clz(hi - lo));
       most = __reduce_max_sync(0xffffffffu, tops[lane & 15]);
     }
     cluster_wait();  // every CTA of the cluster runs: from here on its shared memory may be written
@@ -327,7 +326,12 @@ sample_kernel(const bf16* __restrict__ logits, int ld, int32_t* __restrict__ out
 #pragma unroll
       for (int q = 0; q < 8; ++q)
         keys[q] = q < nq && q * per_region + at < mine ? gkey[region * region_slots + q * per_region + at] : 0u;
-      const uint32_t thr = kth_key(keys, nq, k, bound, 32 - __clz(most - bound));
+      const int bits = 32 - __clz(most - bound);
+      const uint32_t thr = nq == 1   ? kth_key<1>(keys, k, bound, bits)
+                           : nq == 2 ? kth_key<2>(keys, k, bound, bits)
+                           : nq == 3 ? kth_key<3>(keys, k, bound, bits)
+                           : nq == 4 ? kth_key<4>(keys, k, bound, bits)
+                                     : kth_key<8>(keys, k, bound, bits);  // keys past the counted ones are 0
       __syncthreads();
 #pragma unroll
       for (int q = 0; q < 8; ++q) {
@@ -567,9 +571,10 @@ static int sample_capacity(int* capacity /*[kMaxRowCtas + 1]*/) {
 }
 
 // A cluster of as many CTAs as the row has slices of 16 384 logits, at most the portable 8, and no more than let all rows'
-// clusters run at once: a second wave is a second chain, a longer slice (read twice beyond 16 384 logits) a few loads.  128 256
-// logits, us with 8 / 4 / 2 / 1 CTAs a row: one row 10.3 / 12.4 / 14.9 / 18.9, 24 rows 13.3 / 13.7 / 15.8 / 20.0, 48 rows 20.6 /
-// 16.0 / 16.0 / 20.4, 128 rows 42 / 30 / 20.0 / 21.0 (48 rows before, always 8: 24.1).
+// clusters run at once (two CTAs share an SM: clusters of 8 / 5 / 4 / 2 hold 264 / 270 / 280 / 296 CTAs at once): a second wave is a
+// second chain, a longer slice a few loads.  128 256 logits, us with 8 / 5 / 4 / 2 / 1 CTAs a row: one row 8.5 / 10.0 / 10.7 / 12.8 /
+// 17.5, 24 rows 10.7 / 11.0 / 11.9 / 13.9 / 18.0, 48 rows 16.8 / 12.4 / 13.8 / 14.3 / 18.2, 64 rows 20.1 / 19.3 / 13.7 / 15.0 / 18.5,
+// 128 rows 33.5 / 27.1 / 25.8 / 17.4 / 19.7: what the rule takes is the fastest of all eight sizes in each line.
 // That way (`narrow`) is for k small enough that few logits lie above the bound: with `per` logits a thread, k of 512 maxima above
 // it means a share of 1 - (1 - k/512)^(1/per) of all logits, and a bf16 step at the bound adds up to some V / 4096 ties.  Larger
 // k would overflow the first CTA's shared memory after all the work; it takes the histograms of one CTA per row at once.

@@ -49,3 +49,12 @@ def test_a_few_tokens_left(cuda, n):
     drawn = set(out.tolist())
     assert all((i - 3) % 50 == 0 and (i - 3) // 50 < n for i in drawn)
     assert len(drawn) >= n - 10
+
+
+@pytest.mark.parametrize("V", [300, 512, 513, 1000, 1024, 1025, 1500, 2000, 2048])
+def test_every_number_of_keys_a_thread(cuda, V):
+    """Short rows are candidates as a whole: one to four keys a thread in the search for the threshold, full and not."""
+    g = torch.Generator(device="cuda").manual_seed(V)
+    x = torch.randn(3, V, device=cuda, generator=g).to(BF)
+    for k in (1, 257, 300):
+        _check(x, top_k=min(k, V), top_p=1.0)
