@@ -681,12 +681,10 @@ mlstm_par_readout_kernel(const E* __restrict__ proj, float* __restrict__ o, Mlst
       Ss[i] = c < a.V ? Sin[(size_t)d * a.V + c] : 0.f;
     }
   }
-  {  // q . n of a row by four threads
+  if (tid < kMcL) {  // one chain a row: split over four threads it saves nothing (ragged steps 2 407 us with it and without)
     float d0 = 0.f;
-    for (int d = tid & 3; d < D; d += 4) d0 = fmaf(ns[d], qT[d * kMcLp + (tid >> 2)], d0);
-    d0 += __shfl_xor_sync(0xffffffffu, d0, 1);
-    d0 += __shfl_xor_sync(0xffffffffu, d0, 2);
-    if ((tid & 3) == 0) qn[tid >> 2] = d0;
+    for (int d = 0; d < D; ++d) d0 = fmaf(ns[d], qT[d * kMcLp + tid], d0);
+    qn[tid] = d0;
   }
   __syncthreads();
   float inter[4][4] = {}, intra[4][4] = {};
@@ -726,8 +724,6 @@ mlstm_par_readout_kernel(const E* __restrict__ proj, float* __restrict__ o, Mlst
     }
   }
 }
-
-static_assert(kMcThreads == 4 * kMcL, "four threads per row");
 
 static size_t mlstm_readout_smem(int D) {
   return sizeof(float) * (2 * (size_t)D * kMcLp + kMcL * kMcLp + kMcL * kMcCols + D + 5 * kMcL);

@@ -361,6 +361,31 @@ def test_mlstm_rows_of_bf16_that_start_anywhere(dims, start, shift, pad, blocked
     assert bool((err <= 3e-4 * max(1.0, ref.abs().max().item()) + 2.0 ** -8 * ref.abs()).all()), err.max()
 
 
+def test_mlstm_parallel_sums_q_n_in_order():
+    """q . n of a read-out is one chain in the order of the keys: a sum whose order shows (2^25, 1, -2^25, 1 and zeros: 1 in order,
+    0 in four interleaved chains) as the denominator of the first row after a state."""
+    from dli_b200 import ops
+
+    H, D, V = 1, 16, 64
+    n = torch.zeros(1, H, D, device=DEV)
+    n[0, 0, :4] = torch.tensor([2.0 ** 25, 1.0, -2.0 ** 25, 1.0])
+    S = torch.zeros(1, H, D, V, device=DEV)
+    S[0, 0, 4] = torch.linspace(1.0, 2.0, V)
+    mm = torch.full((1, H), 20.0, device=DEV)
+    w = 2 * H * D + 2 * H * V + 2 * H
+    proj = torch.zeros(1, w, device=DEV)
+    proj[0, :D] = 4.0                       # q, times D^-1/2: 1
+    proj[0, -2], proj[0, -1] = -100.0, 100.0  # the input's gate shut, the state kept: m stays 20
+    _, ent = meta([(0, 1, 5)])
+    tiles = torch.tensor([[0, 0]], dtype=torch.int32, device=DEV)
+    scr = torch.empty(ops.mlstm_parallel_scratch_floats(1, H, D, V), device=DEV)
+    o, y = torch.empty(H * V, device=DEV), torch.empty(1, H * V, device=DEV)
+    zero, one = torch.zeros(H, device=DEV), torch.ones(H * V, device=DEV)
+    ops.mlstm_ragged_parallel(proj, o, y, ent, tiles, scr, H, D, V, 0, D, 2 * D, 2 * D + 2 * V, 2 * D + 2 * V + 1, 2 * D + V, zero,
+                              zero, 0.0, one, 1e-6, S, n, mm)
+    assert torch.allclose(o.cpu(), torch.linspace(1.0, 2.0, V), rtol=1e-5)  # over a denominator of 1 (of e^-20 if the sum is 0)
+
+
 def test_rot_frequencies_match_the_oracle():
     from dli_b200.ragged_engine import rot_frequencies
 
