@@ -415,7 +415,8 @@ static PrefillShape prefill_tile(int M, int N, int K, bool gated) {
 // A matrix of more outputs than inputs may be a qkv projection, which takes the same kernel with its rotation and without: the
 // same K split, so the same bits.  It goes by what the pairs take with whole heads of 128 in a tile, widths of 128 and 256 alone:
 // 6144 x 4096 at 301 rows is estimated at 20.4 us in tiles of 176, at 26.1 in tiles of 256 (with the rotation 27.7 measured,
-// clusters 21.5).
+// clusters 21.5).  Nor do so few CTAs bring the weights in faster than 4.8 TB/s (15360 x 5120 at 129 rows: 31 us by the MMAs, 50
+// measured, clusters 43).
 // Over 29 matrices x 30 row counts from 129 to 4 096 what is picked is 0.6 % slower than the fastest of the three on average, 0.3 %
 // where no rotation has a say.
 enum Route { kRouteRows, kRoutePair, kRoutePersistent };
@@ -441,8 +442,12 @@ static int choose(int M, int N, int K, bool gated, Choice* c) {
   }
   if (pairs) {
     if ((rc = plan_gemm_pair(gated ? kPairGated : kPairPlain, M, N, K, 128, &c->pair, &us)) != DLI_OK) return rc;
-    PairShape rotated;
-    if (!gated && N > K && (rc = plan_gemm_pair(kPairRope, M, N, K, 128, &rotated, &us)) != DLI_OK) return rc;
+    if (!gated && N > K) {
+      PairShape rotated;
+      if ((rc = plan_gemm_pair(kPairRope, M, N, K, 128, &rotated, &us)) != DLI_OK) return rc;
+      const double weights = 2.5 + (double)N * K * 2 / 4.8e6;
+      if (us < weights) us = weights;
+    }
     if (us < best) c->route = kRoutePair;
   }
   return DLI_OK;

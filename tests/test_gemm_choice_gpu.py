@@ -21,6 +21,7 @@ MEASURED = [  # rows, outputs, K, gated, kernel; us of the persistent kernel, th
     (2048, 256, 4096, False, "rows"),      # narrow: the pairs 27 % slower
     # qkv projections, with the rotation in the epilogue (without it they take the same kernel)
     (129, 10240, 8192, False, "rows"),     # 67 / 37 / 49
+    (129, 15360, 5120, False, "rows"),     # 66 / 43 / 50
     (301, 6144, 4096, False, "rows"),      # 38 / 22 / 28
     (384, 6144, 4096, False, "rows"),      # 38 / 23 / 28
     (600, 6144, 4096, False, "pairs"),     # 38 / 30 / 29
