@@ -1,6 +1,7 @@
 """Which kernel a prompt's projections take (csrc/gemm_tcgen05.cu): sizes at which one of the three was measured to be faster than the
 others by 4 % and more, around where the choice has its borders.  The times are the fastest kernel's and what the others took."""
 import pytest
+from test_gemm_rows_gpu import HALF_ULP, _inputs, _within
 
 pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
@@ -39,6 +40,32 @@ def test_the_kernel_measured_to_be_faster(cuda, M, N, K, gated, kernel):
     assert ops.gemm_plan(M, N, K, gated)[0] == kernel
 
 
+@pytest.mark.parametrize("M,kernel", [(301, "rows"), (336, "persistent"), (400, "pairs"), (560, "persistent")])
+def test_gated_forms_on_each_kernel(cuda, M, kernel):
+    """silu, the clamped activation and gelu of 14 336 gates from 4 096 inputs, against float64.  Bounds as in test_gemm_rows_gpu.py:
+    gate and up carry the sum's slack and a rounding, the activation's slope is below 1.1 (gelu 1.13), silu is rounded before the
+    product."""
+    from dli_b200 import ops
+
+    F, K, limit, alpha = 14336, 4096, 1.1, 1.702
+    if ops.sm_count() == 148:
+        assert ops.gemm_plan(M, 2 * F, K, True)[0] == kernel
+    g, x, wg, gate, s1 = _inputs(M, F, K, M)
+    wu = (torch.randn(F, K, device=cuda, generator=g) * K ** -0.5).to(BF)
+    up, s2 = x.double() @ wu.double().T, 2 * K * 2.0 ** -24 * (x.double().abs() @ wu.double().abs().T)
+    w, e_gate, e_up = ops.pack_gate_up(wg, wu), s1 + HALF_ULP * gate.abs(), s2 + HALF_ULP * up.abs()
+    act = torch.nn.functional.silu(gate)
+    e_act = 1.1 * e_gate + HALF_ULP * (act.abs() + 1.1 * e_gate)
+    _within(ops.linear_gated_silu(x, w), act * up, e_act * (up.abs() + e_up) + act.abs() * e_up + HALF_ULP * 1.1 * (act * up).abs() + 1e-6)
+    held = gate.clamp(max=limit)
+    act, u1 = held * torch.sigmoid(alpha * held), up.clamp(-limit, limit) + 1
+    got = ops.linear_gated_act(x, w, torch.tensor([limit, alpha], device=cuda))
+    _within(got, act * u1, 1.1 * e_gate * (u1.abs() + e_up) + act.abs() * e_up + HALF_ULP * 1.1 * (act * u1).abs() + 1e-6)
+    act = torch.nn.functional.gelu(gate, approximate="tanh")
+    got = ops.linear_gated_act(x, w, torch.zeros(2, device=cuda))
+    _within(got, act * up, 1.13 * e_gate * (up.abs() + e_up) + act.abs() * e_up + HALF_ULP * 1.1 * (act * up).abs() + 1e-6)
+
+
 @pytest.mark.parametrize("hd,H,KV,bias,kernel", [(128, 64, 8, False, "gemm_prefill_kernel"), (128, 64, 8, True, "gemm_pair_kernel"),
                                                  (128, 78, 1, False, "gemm_pair_kernel"), (64, 128, 16, False, "gemm_pair_kernel")])
 def test_qkv_where_the_persistent_kernel_is_chosen(cuda, hd, H, KV, bias, kernel):
@@ -64,7 +91,7 @@ def test_qkv_where_the_persistent_kernel_is_chosen(cuda, hd, H, KV, bias, kernel
     h_in = rnd(T, d)
     kc, vc = (torch.zeros(pages, KV, page, hd, device=cuda, dtype=BF) for _ in range(2))
     h, x, qkv, attn, act = (torch.empty(T, w, device=cuda, dtype=BF) for w in (d, d, N, H * hd, ff))
-    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA], acc_events=True) as prof:
         ops.prompt_layers([L], [kc], [vc], table, table, h_in, h, x, qkv, attn, act, cos, sin, positions, seq_ids, 1, T, prefix,
                           H, KV, hd, 1e-5, hd ** -0.5)
         torch.cuda.synchronize()
