@@ -8,16 +8,19 @@
 // gives out 8 KB instead of the 12 KB of a 128 x 256 tile on one SM, and the tile asks L2 for a third less.  Persistent, one
 // CTA per SM: warp 0 = TMA producer, warp 1 of the leader = MMA issuer, warps 2-9 = epilogue.
 //
-// What bounds it: at 4 096 rows the tensor pipe, busy 93 % of the time at 1.42 GHz under the power limit (28672 x 4096 gated,
-// 1 580 TFLOP/s); below some 1 000 rows whole rounds of tiles, which the width and a tail of narrower tiles even out
-// (pair_cost); at K = 768 ... 2048 what no tile hides: 2.5 us from the predecessor's end to the first load, the last epilogue.
-// Measured on B200 in a chain of launches over rotating weights, us, 128-row tiles on single SMs -> here:
-//   rows            1024           1777           4096
-//   6144 x 4096      55 ->  39     90 ->  64     172 -> 137
-//   4096 x 4096      37 ->  30     53 ->  44     134 -> 100
-//   4096 x 14336    110 ->  94    187 -> 148     386 -> 333
-//   28672 gated     185 -> 165    292 -> 270     645 -> 608
-//   2048 x 5632      28 ->  25     44 ->  34      72 ->  69
+// What bounds it: at 4 096 rows the tensor pipe, busy 93 % of the time under the power limit (28672 x 4096 gated: 588 us by itself,
+// 709 us at 1.29 GHz after a second of nothing else, 1 357 TFLOP/s; profiles/pairs_notes.md); below some 1 000 rows whole rounds
+// of tiles, which the width and a tail of narrower tiles even out (pair_cost); at K = 768 ... 2048 what no tile hides: 2.5 us from
+// the predecessor's end to the first load, the last epilogue.
+// Measured on B200 in chains of launches over rotating weights, in turn with the other kernels, us, 128-row tiles on single SMs /
+// clusters (gemm_rows.cu) / here:
+//   rows            301              450              1024             1777             4096
+//   6144 x 4096      39 /  25 /  24   40 /  29 /  25   55 /  55 /  36   85 /  79 /  60  173 / 219 / 134
+//   4096 x 4096      32 /  19 /  18   32 /  21 /  18   33 /  33 /  25   53 /  60 /  40  117 / 149 /  92
+//   4096 x 14336     91 /  40 /  50   90 /  60 /  51   98 / 106 /  81  161 / 184 / 143  380 / 464 / 360
+//   28672 gated      84 /  76 /  82  113 / 119 /  91  188 / 247 / 165  323 / 410 / 291  711 / 926 / 647
+//   2048 x 5632      39 /  15 /  20   39 /  18 /  20   39 /  25 /  21   40 /  36 /  29   73 /  86 /  64
+//   768 x 3072       26 /   8 /  11   26 /   9 /  11   25 /  12 /  12   26 /  15 /  13   25 /  22 /  16
 #include "gemm_pair.cuh"
 #include "recent.h"
 
@@ -568,7 +571,10 @@ int launch_gemm_pair(PairMode mode, const void* x, const void* w, const void* bi
   if ((rc = make_tmap(&tmA, x, M, K, 128)) != DLI_OK) return rc;
   if ((rc = make_tmap(&tmB, w, N, K, sh.bn / 2)) != DLI_OK) return rc;
   if ((rc = make_tmap(&tmTail, w, N, K, sh.bn_tail / 2)) != DLI_OK) return rc;
-  const auto launch = mode == kPairGated ? launch_pair<kPairGated> : mode == kPairGatedAct ? launch_pair<kPairGatedAct> : mode == kPairRope ? launch_pair<kPairRope> : launch_pair<kPairPlain>;
+  const auto launch = mode == kPairGated      ? launch_pair<kPairGated>
+                      : mode == kPairGatedAct ? launch_pair<kPairGatedAct>
+                      : mode == kPairRope     ? launch_pair<kPairRope>
+                                              : launch_pair<kPairPlain>;
   return launch(tmA, tmB, tmTail, bias, residual, y, M, N, K, epilogue, sh, n_tiles, stages, smem, s, rope, hd);
 }
 

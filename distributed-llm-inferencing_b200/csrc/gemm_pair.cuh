@@ -16,8 +16,9 @@ enum PairMode { kPairPlain = 0, kPairGated = 1, kPairRope = 2, kPairGatedAct = 3
 // The cut for [M, K] x [N, K]^T and its estimated time in us (the rule stands beside the definition).  hd: kPairRope only.
 int plan_gemm_pair(PairMode mode, int M, int N, int K, int hd, PairShape* shape, double* us);
 
-// y = epi(x w^T).  kPairGated: w is the interleaved gate / up matrix, N counts its rows, `bias` is not used; kPairRope: N = (H + 2 KV) hd, no residual, no activation.  The caller has checked the arguments: K % 64 == 0,
-// N % 16 == 0 (gated: N % 256 == 0), 16-byte pointers.
+// y = epi(x w^T).  kPairGated: w is the interleaved gate / up matrix, N counts its rows, `bias` is not used; kPairRope:
+// N = (H + 2 KV) hd, no residual, no activation.  The caller has checked the arguments: K % 64 == 0, N % 16 == 0 (gated:
+// N % 256 == 0), 16-byte pointers.
 int launch_gemm_pair(PairMode mode, const void* x, const void* w, const void* bias, const void* residual, void* y, int M, int N,
                      int K, int epilogue, const PairShape& shape, cudaStream_t s, const RopeArgs& rope = RopeArgs{}, int hd = 128);
 

@@ -14,13 +14,14 @@
 // two cluster barriers, and every CTA finishes its own share of the columns.  Two CTAs fit an SM (at most 108 KB of ring,
 // at most 256 TMEM columns each), and the dependents are released as soon as all CTAs run, so their weight loads
 // start beside this kernel's tail.  Measured on B200 in a chain of launches over rotating weights, us, before -> now:
-//   rows           16            128            301            1024
-//   4096 x 4096    11.6 ->  8.6   19.8 -> 12.5   35.0 -> 17.7   36.0 -> 36.0 (persistent kernel)
-//   4096 x 14336   24.6 -> 21.7   35.2 -> 27.4   94.5 -> 40.1   97.4 -> 97.4 (persistent kernel)
-//   28672 gated    42.4 -> 39.8   62.8 -> 48.9   87.2 -> 79.2  181   -> 181  (persistent kernel)
-//   768 x 3072      9.7 ->  4.6   30.6 ->  6.0   29.2 ->  7.6   28.8 -> 11.8
-// (before: split-K through global memory up to 128 rows, the persistent kernel of 128-row tiles above; from some 400 rows on pairs
-// of SMs take over, gemm_pair.cu: 4096 x 4096 at 1 024 rows 30 us, 4096 x 14336 85, 28672 gated 163.)
+//   rows           16            128            301
+//   4096 x 4096    11.6 ->  8.6   19.8 -> 12.5   35.0 -> 17.7
+//   4096 x 14336   24.6 -> 21.7   35.2 -> 27.4   94.5 -> 40.1
+//   28672 gated    42.4 -> 39.8   62.8 -> 48.9   87.2 -> 79.2
+//   768 x 3072      9.7 ->  4.6   30.6 ->  6.0   29.2 ->  7.6
+// (before: split-K through global memory up to 128 rows, the persistent kernel of 128-row tiles above.  Where the pairs of SMs take
+// over depends on the matrix, at 129 rows for 768 x 768, at 500 to 700 for 6144 x 4096 with rotation and 2048 x 5632: choose in
+// gemm_tcgen05.cu; times of both beside each other in gemm_pair.cu.)
 #include "gemm_rows.cuh"
 #include "recent.h"
 

@@ -404,7 +404,7 @@ static PrefillShape prefill_tile(int M, int N, int K, bool gated) {
 
 // Which kernel takes a projection, by estimated time:
 //  - clusters that split K (gemm_rows.cu), up to 4 096 rows, which bound what was measured, and always up to 128 rows;
-//  - pairs of SMs (gemm_pair.cu) in tiles of 256 rows, for widths that are multiples of 128; from 129 ... 500 rows on, by matrix;
+//  - pairs of SMs (gemm_pair.cu) in tiles of 256 rows, for widths that are multiples of 128; from 129 ... 700 rows on, by matrix;
 //  - the persistent kernel above where 256-row tiles would be half padding and the matrix is large (28672 x 4096 gated at 336
 //    rows: 85 us, clusters 95), and for other widths, at which the pairs were not measured.
 // The clusters' estimate errs high from some 250 rows on, by up to a quarter (28672 x 4096 gated at 301 rows: 91 us, measured 76),

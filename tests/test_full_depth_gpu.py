@@ -1,14 +1,14 @@
 """Parity at FULL DEPTH against the reference's own forward on the same B200.
 
 The reference loads `AutoModelForCausalLM` (reference worker/app.py:121-124, `USE_GPU=1` :23-26) and calls
-`model.generate(...)` (:297-305); with `do_sample=False` that is the parity mode north-star names ("greedy
-token IDs must match exactly, logits within a stated bf16 tolerance").  The other engine tests pin the CUDA path on
-2-4-layer models; here the WHOLE models of BASELINE.json run side by side, from one seeded state dict:
+`model.generate(...)` (:297-305); with `do_sample=False` that is the parity mode: greedy token ids must match
+exactly, logits within a stated bf16 tolerance.  The other engine tests pin the CUDA path on
+2-4-layer models; here WHOLE models run side by side, from one seeded state dict:
 
-  * Llama-3-8B   (32 layers), 2 048-token prompt -> 64 greedy tokens  (configs[2], the headline)
-  * TinyLlama-1.1B (22 layers), 512-token prompt -> 64 tokens         (configs[1])
-  * Mistral-7B   (32 layers), 4 200-token prompt -> 24 tokens, so the 4 096-token window bites (configs[3])
-  * GPT-2 small  (12 layers), 32-token prompt -> 64 tokens: configs[0]'s model and shape on the CUDA path
+  * Llama-3-8B   (32 layers), 2 048-token prompt -> 64 greedy tokens  (the benchmark's model)
+  * TinyLlama-1.1B (22 layers), 512-token prompt -> 64 tokens
+  * Mistral-7B   (32 layers), 4 200-token prompt -> 24 tokens, so the 4 096-token window bites
+  * GPT-2 small  (12 layers), 32-token prompt -> 64 tokens: the reference's default model
 
 three ways: this engine (bf16, CUDA-graph decode = the path bench.py times), transformers bf16 sdpa (what the
 reference would run on this GPU) and transformers fp32 ("truth").  Stated tolerance (the one tests/test_engine_gpu.py
@@ -17,22 +17,20 @@ uses on the small models):
     token == HF-fp32's token at every step whose fp32 top-1/top-2 margin exceeds twice the bf16 error on the
       leading candidates (margin-safe steps), and over all steps as often as HF-bf16's own token does (- 10 %)
     free-running tokens == HF-bf16's up to the first step that is not margin-safe
-Random-init weights give nearly flat logits (SURVEY.md 7.2): at 32 layers and a 2k context the bf16 noise on a logit
+Random-init weights give nearly flat logits: at 32 layers and a 2k context the bf16 noise on a logit
 (~0.1, up to 0.5 somewhere in a 128k-entry row) is of the order of the median top-1/top-2 margin (~0.2), so
 transformers' own bf16 run picks fp32's token on only ~83 % of the steps (measured: 53 of 64, this engine 53 of 64)
-and "exact" can only be asked where the margin clears the noise.  Margins, noise and the counts are printed (-s),
-written to gpurun_out/full_depth_parity.jsonl and asserted to be non-trivial.
+and "exact" can only be asked where the margin clears the noise.  Margins, noise and the counts are printed (-s)
+and asserted to be non-trivial.
 """
 import gc
 import json
-import os
 
 import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
 BF = torch.bfloat16
-ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 def _hf_config(transformers, name):
@@ -162,12 +160,6 @@ def test_full_depth_model_matches_transformers_on_the_same_gpu(cuda, name, T, n_
               "hf_bf16_equal_fp32": int(hf_vs_truth.sum()), "free_running_equal_hf_bf16_prefix": same_hist,
               "margin_safe_prefix": first_unsafe}
     print("\n[full-depth parity] " + json.dumps(report))
-    try:  # kept with the run's other outputs when the box has the directory (gpurun merges it back)
-        os.makedirs(os.path.join(ROOT, "gpurun_out"), exist_ok=True)
-        with open(os.path.join(ROOT, "gpurun_out", "full_depth_parity.jsonl"), "a") as f:
-            f.write(json.dumps(report) + "\n")
-    except OSError:
-        pass
     # logits: within twice transformers' own bf16 error against fp32 truth, worst step and typical step
     assert our_err.max() <= 2.0 * hf_err.max() + 4e-3
     assert our_err.median() <= 2.0 * hf_err.median() + 4e-3

@@ -114,7 +114,7 @@ def _scaled_cfg(transformers, rope):
 
 @pytest.mark.parametrize("rope", [_LLAMA31_ROPE, {"rope_type": "linear", "factor": 4.0, "rope_theta": 10000.0}])
 def test_rope_scaling_matches_transformers(rope):
-    """`llama3` / `linear` rope scaling (SURVEY.md a9 "only if config says so"): the engine's host-side
+    """`llama3` / `linear` rope scaling, only where the config has it: the engine's host-side
     inverse frequencies equal transformers' bit for bit, from the new-style config and from a
     Llama-3.1-style config.json dict; the oracle's forward with the scaled table equals transformers'."""
     transformers = pytest.importorskip("transformers")

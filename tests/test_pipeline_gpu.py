@@ -39,7 +39,7 @@ def test_nccl_mailbox_pipeline_equals_single_engine(cuda, world, vp, hop):
 
 @pytest.mark.parametrize("world,vp,chunks", [(2, 0, 3), (2, 1, 4), (4, 1, 3)])
 def test_nccl_pipeline_with_chunked_prefill(cuda, world, vp, chunks):
-    """Prompts fed in chunks, the stages working on different chunks at once (SURVEY 8e): tokens equal the
+    """Prompts fed in chunks, the stages working on different chunks at once: tokens equal the
     single engine's with the same chunking."""
     if torch.cuda.device_count() < world:
         pytest.skip(f"needs {world} GPUs, have {torch.cuda.device_count()}")

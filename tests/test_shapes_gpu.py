@@ -1,6 +1,6 @@
-"""Full-WIDTH parity at reduced depth (SURVEY.md 7.2: the 70B model cannot be run by the CPU oracle, so
+"""Full-WIDTH parity at reduced depth (the 70B model cannot be run by the CPU oracle, so
 parity is checked on 70B-shaped layers with few of them): the real hidden sizes, head counts, GQA groups and
-MLP widths of the BASELINE models — the shapes the kernels are tuned and routed for (K = 28 672 weight
+MLP widths of the models served — the shapes the kernels are tuned and routed for (K = 28 672 weight
 streams, 8 query heads per KV head, ...) — with 2 layers and a small vocabulary, teacher-forced against the
 oracle on the same seeded weights; once as one engine and once as two single-layer shards chained the way a
 worker runs `shard_ids`."""

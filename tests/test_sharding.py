@@ -57,7 +57,7 @@ def test_write_shards_layout_and_selective_load(tmp_path):
 
 def test_reference_style_full_depth_directory_only_yields_in_range_tensors(tmp_path):
     """A reference shard directory is a full-depth save_pretrained() model whose out-of-range
-    layers are random (SURVEY 0 F2): the loader must read only [start, end]."""
+    layers are random: the loader must read only [start, end]."""
     cfg, spec, sd = _tiny()
     from safetensors.torch import save_file
 

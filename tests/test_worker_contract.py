@@ -104,7 +104,7 @@ def test_shard_registration_health_and_unload_match_reference(tmp_path):
 
 
 def test_shard_id_zero_is_accepted_deliberate_deviation(tmp_path):
-    """The reference answers 400 here (falsy 0 in all([...]), SURVEY A.3 Q1); a first shard
+    """The reference answers 400 here (falsy 0 in all([...])); a first shard
     must be registrable, so this worker accepts it."""
     g = _golden("/load_shard", "shard_id 0 is falsy (Q1)")
     assert g["status"] == 400
