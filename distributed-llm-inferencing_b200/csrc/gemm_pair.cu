@@ -21,6 +21,7 @@
 //   28672 gated      84 /  76 /  82  113 / 119 /  91  188 / 247 / 165  323 / 410 / 291  711 / 926 / 647
 //   2048 x 5632      39 /  15 /  20   39 /  18 /  20   39 /  25 /  21   40 /  36 /  29   73 /  86 /  64
 //   768 x 3072       26 /   8 /  11   26 /   9 /  11   25 /  12 /  12   26 /  15 /  13   25 /  22 /  16
+#include "cta_pair.cuh"
 #include "gemm_pair.cuh"
 #include "recent.h"
 
@@ -33,63 +34,6 @@ constexpr int kPairAccCols = 256;  // TMEM columns per accumulator stage, two st
 constexpr int kPairStageBytes = 32 * 128;  // an epilogue warp's line buffer: 32 rows x 64 bf16
 constexpr int kPairSmemMax = 227 * 1024;
 constexpr int kPairSmemFixed = 1024 + 8 * kPairStageBytes + 256;  // alignment, line buffers, barriers
-
-// ---- PTX of a CTA pair ------------------------------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t pair_map(uint32_t addr, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-  return r;
-}
-__device__ __forceinline__ uint32_t pair_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-// kOrdered = false: a rendezvous alone, which does not wait for this thread's writes to arrive
-template <bool kOrdered = true>
-__device__ __forceinline__ void pair_barrier() {
-  if (kOrdered) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  else asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// Into this CTA's shared memory; the bytes are counted by a barrier of either CTA of the pair.
-__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const void* tmap, uint32_t bar, int c0, int c1) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-      ::"r"(dst), "l"(tmap), "r"(bar), "r"(c0), "r"(c1)
-      : "memory");
-}
-__device__ __forceinline__ void tmem_alloc_pair(uint32_t smem_dst, uint32_t ncols) {
-  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(ncols) : "memory");
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
-  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
-}
-__device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                               uint32_t accumulate) {
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
-      "}\n" ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// Both CTAs' barriers at this offset, once all MMAs issued so far by this thread are complete.
-__device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
-  asm volatile(
-      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
-      "h"((uint16_t)3)
-      : "memory");
-}
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-// kind::f16: D = f32, A = B = bf16, both K-major, M = 256, N = n
-__device__ __forceinline__ uint32_t make_idesc_pair(int n) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
-}
 
 __device__ __forceinline__ uint32_t pair_bias(const bf16* b) {  // two of them, from any address
   return (uint32_t)__bfloat16_as_ushort(b[0]) | ((uint32_t)__bfloat16_as_ushort(b[1]) << 16);
@@ -225,8 +169,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 #pragma unroll
             for (int k = 0; k < kBlockK / kUmmaK; ++k)
               umma_bf16_pair(tacc, adesc0 + off + 2 * k, bdesc0 + off + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
-            umma_commit_pair(empty_bar + 8 * s);
-            if (kb == num_kb - 1) umma_commit_pair(tfull_bar + 8 * as);
+            umma_commit_pair(empty_bar + 8 * s, 3);
+            if (kb == num_kb - 1) umma_commit_pair(tfull_bar + 8 * as, 3);
           }
           __syncwarp();
           if (++s == stages) s = 0, ph ^= 1;

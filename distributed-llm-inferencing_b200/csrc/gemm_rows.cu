@@ -22,6 +22,9 @@
 // (before: split-K through global memory up to 128 rows, the persistent kernel of 128-row tiles above.  Where the pairs of SMs take
 // over depends on the matrix, at 129 rows for 768 x 768, at 500 to 700 for 6144 x 4096 with rotation and 2048 x 5632: choose in
 // gemm_tcgen05.cu; times of both beside each other in gemm_pair.cu.)
+#include <cmath>
+
+#include "cta_pair.cuh"
 #include "gemm_rows.cuh"
 #include "recent.h"
 
@@ -47,6 +50,190 @@ __device__ __forceinline__ void cluster_store(uint32_t addr, uint32_t v) {
 __device__ __forceinline__ void cluster_barrier() {
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// The end of a tile.  Every MMA of every CTA of the cluster is done, the operand rings (smem) take the partial sums; this CTA holds
+// 128 weight rows x `rows` columns of split `rank` in TMEM.  kPair: CTAs per split (the one with this CTA's weight rows is `member`).
+template <int kMode, bool kAnyBias, int kThreads, int kPair>
+__device__ __forceinline__ void rows_finish(uint8_t* smem, uint32_t tmem_base, int splits, int rank, int member, int rows, int m0,
+                                            int n_tile, const bf16* __restrict__ bias, const bf16* residual, bf16* y, int N,
+                                            int epilogue, const RopeArgs& rope, int hd) {
+  constexpr bool kGated = kMode == kRowsGated;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // The tile's columns (activation rows) are dealt to the CTAs in groups of `per`; each CTA sends every owner its fp32
+  // partial of the owner's columns: [source rank][column][128 weight rows], lanes on consecutive weight rows.
+  const int per = (((rows + splits - 1) / splits) + 7) & ~7;
+  const uint32_t red = smem_addr(smem);
+  if (warp >= 2) {
+    constexpr int kDrain = (kThreads / 32 - 2) / 4;  // warps per 32 lanes: each takes every kDrain-th 16 columns
+    const int quad = warp & 3, turn = (warp - 2) >> 2;
+    const uint32_t lane_base = tmem_base + ((uint32_t)(quad * 32) << 16);
+    for (int o = 0; o < splits; ++o) {
+      const int c_end = min((o + 1) * per, rows);
+      const uint32_t base = (splits > 1 ? cluster_map(red, o * kPair + member) : red) + (rank * per * 128 + quad * 32 + lane) * 4;
+      for (int c0 = o * per + turn * 16; c0 < c_end; c0 += kDrain * 16) {
+        uint32_t r1[8], r2[8];
+        tmem_ld_32x8(lane_base + c0, r1);
+        const bool two = c0 + 8 < c_end;
+        if (two) tmem_ld_32x8(lane_base + c0 + 8, r2);
+        tmem_ld_wait();
+        const uint32_t dst = base + (c0 - o * per) * 512;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) cluster_store(dst + j * 512, r1[j]);
+        if (two) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) cluster_store(dst + (8 + j) * 512, r2[j]);
+        }
+      }
+    }
+    tcgen05_fence_before();
+  } else {
+    pdl_wait();  // these warps take part in the epilogue, which reads the residual
+  }
+  if (splits > 1) cluster_barrier();
+  else __syncthreads();
+
+  // ---- epilogue over this CTA's columns: an item is 8 consecutive outputs of one activation row (two groups of 8 where
+  // two belong together: gate and up, or the halves of a rotation pair) ----
+  // A thread keeps its group of outputs (the block is a multiple of kGroups) and takes kBatch rows at a time: what it needs
+  // from global memory for all of them — residual, position, rotation, page — is asked for before any is used.
+  constexpr int kGroups = kMode == kRowsPlain ? 16 : 8;
+  constexpr int kBatch = 4;
+  static_assert(kThreads % kGroups == 0, "a thread keeps its group");
+  const int n_out = kGated ? N / 2 : N;
+  const int col0 = rank * per;
+  const int items = max(0, min(per, rows - col0)) * kGroups;
+  const float* sums = reinterpret_cast<const float*>(smem);
+  const int g = threadIdx.x % kGroups;
+  // first weight row of the group inside the tile, and how much further its second group starts
+  const int half = hd >> 1;
+  const int r0 = kMode == kRowsRope && hd == 64 ? (g >> 2) * 64 + (g & 3) * 8 : g * 8;
+  const int r1 = kMode == kRowsRope ? half : 64;
+  const int n = kGated ? n_tile * 64 + r0 : n_tile * 128 + r0;
+  if (n < n_out) {  // n_out is a multiple of 16 (of hd with heads): a group is whole or absent
+    float bb[8], bb2[8];
+    {
+      uint4 bv = make_uint4(0u, 0u, 0u, 0u), bv2 = bv;
+      if (!kAnyBias && !kGated && (epilogue & DLI_EPI_BIAS)) {
+        bv = ld_16B(bias + n);
+        if (kMode == kRowsRope) bv2 = ld_16B(bias + n + half);
+      }
+      unpack8(bv, bb);
+      unpack8(bv2, bb2);
+      if (kAnyBias && !kGated) {  // a slice of a longer vector may start anywhere
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          bb[e] = __bfloat162float(bias[n + e]);
+          if (kMode == kRowsRope) bb2[e] = __bfloat162float(bias[n + half + e]);
+        }
+      }
+    }
+    const int head = hd == 64 ? n_tile * 2 + (g >> 2) : n_tile;  // kRowsRope: q heads, then k heads, then v heads
+    const int he = hd == 64 ? (g & 3) * 8 : g * 8;               // element of the head's first half
+    const bool turned = kMode == kRowsRope && rope.cos_t && head < rope.H + rope.KV;
+    for (int id0 = threadIdx.x; id0 < items; id0 += kBatch * kThreads) {
+      uint4 pre1[kBatch], pre2[kBatch];  // residual; or cosines and sines
+      int pos[kBatch], page[kBatch];
+#pragma unroll
+      for (int q = 0; q < kBatch; ++q) {
+        const int m = m0 + col0 + (id0 + q * kThreads) / kGroups;
+        const bool on = id0 + q * kThreads < items;
+        pre1[q] = pre2[q] = make_uint4(0u, 0u, 0u, 0u);
+        pos[q] = page[q] = 0;
+        if (kMode == kRowsPlain && on && (epilogue & DLI_EPI_RESIDUAL)) pre1[q] = ld_16B(residual + (size_t)m * n_out + n);
+        if (kMode == kRowsRope && on) {
+          pos[q] = rope.positions[m];
+          if (head >= rope.H) page[q] = rope.seq_ids[m];
+        }
+      }
+      if (kMode == kRowsRope) {
+#pragma unroll
+        for (int q = 0; q < kBatch; ++q) {
+          if (id0 + q * kThreads >= items) continue;
+          if (turned) {
+            pre1[q] = ld_16B(rope.cos_t + (size_t)pos[q] * half + he);
+            pre2[q] = ld_16B(rope.sin_t + (size_t)pos[q] * half + he);
+          }
+          if (head >= rope.H) page[q] = rope.page_table[(size_t)page[q] * rope.max_pages + (pos[q] >> rope.page_shift)];
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < kBatch; ++q) {
+        const int id = id0 + q * kThreads;
+        if (id >= items) continue;
+        const int c = id / kGroups;
+        const size_t at = (size_t)(m0 + col0 + c) * n_out + n;
+        float a[8], b[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) a[e] = 0.f, b[e] = 0.f;
+        for (int sp = 0; sp < splits; ++sp) {  // in split order: deterministic
+          const float4* p = reinterpret_cast<const float4*>(sums + (size_t)(sp * per + c) * 128 + r0);
+          const float4 u = p[0], v = p[1];
+          a[0] += u.x; a[1] += u.y; a[2] += u.z; a[3] += u.w;
+          a[4] += v.x; a[5] += v.y; a[6] += v.z; a[7] += v.w;
+          if (kMode != kRowsPlain) {
+            const float4 u2 = p[r1 / 4], v2 = p[r1 / 4 + 1];
+            b[0] += u2.x; b[1] += u2.y; b[2] += u2.z; b[3] += u2.w;
+            b[4] += v2.x; b[5] += v2.y; b[6] += v2.z; b[7] += v2.w;
+          }
+        }
+        if (kGated) {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) round2_bf16(a[e], b[e]);
+          gated_combine_n(a, b, kAnyBias ? reinterpret_cast<const float*>(bias) : nullptr);
+          st_16B(y + at, pack8(a));
+          continue;
+        }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) a[e] += bb[e];
+#pragma unroll
+        for (int e = 0; e < 8; e += 2) round2_bf16(a[e], a[e + 1]);
+        if (kMode == kRowsPlain) {
+          float rr[8];
+          unpack8(pre1[q], rr);
+          if (epilogue & DLI_EPI_GELU_NEW) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) a[e] = gelu_of_bf16(a[e]);
+#pragma unroll
+            for (int e = 0; e < 8; e += 2) round2_bf16(a[e], a[e + 1]);
+          }
+#pragma unroll
+          for (int e = 0; e < 8; ++e) a[e] += rr[e];
+          st_16B(y + at, pack8(a));
+        } else {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) b[e] += bb2[e];
+#pragma unroll
+          for (int e = 0; e < 8; e += 2) round2_bf16(b[e], b[e + 1]);
+          if (turned) {
+            float cs[8], sn[8];
+            unpack8(pre1[q], cs);
+            unpack8(pre2[q], sn);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              const float x1 = a[e], x2 = b[e];
+              float p = x1 * cs[e], q1 = -x2 * sn[e], q2 = x2 * cs[e], t = x1 * sn[e];
+              round2_bf16(p, q1);
+              round2_bf16(q2, t);
+              a[e] = p + q1;
+              b[e] = q2 + t;
+            }
+          }
+          const uint4 u1 = pack8(a), u2 = pack8(b);
+          st_16B(y + at, u1);
+          st_16B(y + at + half, u2);
+          if (head >= rope.H) {
+            const bool is_k = head < rope.H + rope.KV;
+            const int kvh = head - rope.H - (is_k ? 0 : rope.KV);
+            const size_t row = (((size_t)page[q] * rope.KV + kvh) << rope.page_shift) + (pos[q] & ((1 << rope.page_shift) - 1));
+            bf16* dst = (is_k ? rope.k_cache : rope.v_cache) + row * hd + he;
+            st_16B(dst, u1);
+            st_16B(dst + half, u2);
+          }
+        }
+      }
+    }
+  }
 }
 
 // One tile per cluster: gridDim.x = cluster size c (the K splits), y = activation-row tiles, z = weight-row tiles (so the
@@ -165,179 +352,8 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
   if (splits > 1) cluster_barrier();
   else __syncthreads();
 
-  // The tile's columns (activation rows) are dealt to the CTAs in groups of `per`; each CTA sends every owner its fp32
-  // partial of the owner's columns: [source rank][column][128 weight rows], lanes on consecutive weight rows.
-  const int per = (((rows + splits - 1) / splits) + 7) & ~7;
-  const uint32_t red = smem_addr(smem);
-  if (warp >= 2) {
-    const int quad = warp & 3;
-    const uint32_t lane_base = tmem_base + ((uint32_t)(quad * 32) << 16);
-    for (int o = 0; o < splits; ++o) {
-      const int c_end = min((o + 1) * per, rows);
-      const uint32_t base = (splits > 1 ? cluster_map(red, o) : red) + (rank * per * 128 + quad * 32 + lane) * 4;
-      for (int c0 = o * per; c0 < c_end; c0 += 16) {
-        uint32_t r1[8], r2[8];
-        tmem_ld_32x8(lane_base + c0, r1);
-        const bool two = c0 + 8 < c_end;
-        if (two) tmem_ld_32x8(lane_base + c0 + 8, r2);
-        tmem_ld_wait();
-        const uint32_t dst = base + (c0 - o * per) * 512;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) cluster_store(dst + j * 512, r1[j]);
-        if (two) {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) cluster_store(dst + (8 + j) * 512, r2[j]);
-        }
-      }
-    }
-    tcgen05_fence_before();
-  } else {
-    pdl_wait();  // these warps take part in the epilogue, which reads the residual
-  }
-  if (splits > 1) cluster_barrier();
-  else __syncthreads();
-
-  // ---- epilogue over this CTA's columns: an item is 8 consecutive outputs of one activation row (two groups of 8 where
-  // two belong together: gate and up, or the halves of a rotation pair) ----
-  // A thread keeps its group of outputs (the block is a multiple of kGroups) and takes kBatch rows at a time: what it needs
-  // from global memory for all of them — residual, position, rotation, page — is asked for before any is used.
-  constexpr int kGroups = kMode == kRowsPlain ? 16 : 8;
-  constexpr int kBatch = 4;
-  static_assert(kRowsThreads % kGroups == 0, "a thread keeps its group");
-  const int n_out = kGated ? N / 2 : N;
-  const int col0 = rank * per;
-  const int items = max(0, min(per, rows - col0)) * kGroups;
-  const float* sums = reinterpret_cast<const float*>(smem);
-  const int g = threadIdx.x % kGroups;
-  // first weight row of the group inside the tile, and how much further its second group starts
-  const int half = hd >> 1;
-  const int r0 = kMode == kRowsRope && hd == 64 ? (g >> 2) * 64 + (g & 3) * 8 : g * 8;
-  const int r1 = kMode == kRowsRope ? half : 64;
-  const int n = kGated ? n_tile * 64 + r0 : n_tile * 128 + r0;
-  if (n < n_out) {  // n_out is a multiple of 16 (of hd with heads): a group is whole or absent
-    float bb[8], bb2[8];
-    {
-      uint4 bv = make_uint4(0u, 0u, 0u, 0u), bv2 = bv;
-      if (!kAnyBias && !kGated && (epilogue & DLI_EPI_BIAS)) {
-        bv = ld_16B(bias + n);
-        if (kMode == kRowsRope) bv2 = ld_16B(bias + n + half);
-      }
-      unpack8(bv, bb);
-      unpack8(bv2, bb2);
-      if (kAnyBias && !kGated) {  // a slice of a longer vector may start anywhere
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          bb[e] = __bfloat162float(bias[n + e]);
-          if (kMode == kRowsRope) bb2[e] = __bfloat162float(bias[n + half + e]);
-        }
-      }
-    }
-    const int head = hd == 64 ? n_tile * 2 + (g >> 2) : n_tile;  // kRowsRope: q heads, then k heads, then v heads
-    const int he = hd == 64 ? (g & 3) * 8 : g * 8;               // element of the head's first half
-    const bool turned = kMode == kRowsRope && rope.cos_t && head < rope.H + rope.KV;
-    for (int id0 = threadIdx.x; id0 < items; id0 += kBatch * kRowsThreads) {
-      uint4 pre1[kBatch], pre2[kBatch];  // residual; or cosines and sines
-      int pos[kBatch], page[kBatch];
-#pragma unroll
-      for (int q = 0; q < kBatch; ++q) {
-        const int m = m0 + col0 + (id0 + q * kRowsThreads) / kGroups;
-        const bool on = id0 + q * kRowsThreads < items;
-        pre1[q] = pre2[q] = make_uint4(0u, 0u, 0u, 0u);
-        pos[q] = page[q] = 0;
-        if (kMode == kRowsPlain && on && (epilogue & DLI_EPI_RESIDUAL)) pre1[q] = ld_16B(residual + (size_t)m * n_out + n);
-        if (kMode == kRowsRope && on) {
-          pos[q] = rope.positions[m];
-          if (head >= rope.H) page[q] = rope.seq_ids[m];
-        }
-      }
-      if (kMode == kRowsRope) {
-#pragma unroll
-        for (int q = 0; q < kBatch; ++q) {
-          if (id0 + q * kRowsThreads >= items) continue;
-          if (turned) {
-            pre1[q] = ld_16B(rope.cos_t + (size_t)pos[q] * half + he);
-            pre2[q] = ld_16B(rope.sin_t + (size_t)pos[q] * half + he);
-          }
-          if (head >= rope.H) page[q] = rope.page_table[(size_t)page[q] * rope.max_pages + (pos[q] >> rope.page_shift)];
-        }
-      }
-#pragma unroll
-      for (int q = 0; q < kBatch; ++q) {
-        const int id = id0 + q * kRowsThreads;
-        if (id >= items) continue;
-        const int c = id / kGroups;
-        const size_t at = (size_t)(m0 + col0 + c) * n_out + n;
-        float a[8], b[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) a[e] = 0.f, b[e] = 0.f;
-        for (int sp = 0; sp < splits; ++sp) {  // in split order: deterministic
-          const float4* p = reinterpret_cast<const float4*>(sums + (size_t)(sp * per + c) * 128 + r0);
-          const float4 u = p[0], v = p[1];
-          a[0] += u.x; a[1] += u.y; a[2] += u.z; a[3] += u.w;
-          a[4] += v.x; a[5] += v.y; a[6] += v.z; a[7] += v.w;
-          if (kMode != kRowsPlain) {
-            const float4 u2 = p[r1 / 4], v2 = p[r1 / 4 + 1];
-            b[0] += u2.x; b[1] += u2.y; b[2] += u2.z; b[3] += u2.w;
-            b[4] += v2.x; b[5] += v2.y; b[6] += v2.z; b[7] += v2.w;
-          }
-        }
-        if (kGated) {
-#pragma unroll
-          for (int e = 0; e < 8; ++e) round2_bf16(a[e], b[e]);
-          gated_combine_n(a, b, kAnyBias ? reinterpret_cast<const float*>(bias) : nullptr);
-          st_16B(y + at, pack8(a));
-          continue;
-        }
-#pragma unroll
-        for (int e = 0; e < 8; ++e) a[e] += bb[e];
-#pragma unroll
-        for (int e = 0; e < 8; e += 2) round2_bf16(a[e], a[e + 1]);
-        if (kMode == kRowsPlain) {
-          float rr[8];
-          unpack8(pre1[q], rr);
-          if (epilogue & DLI_EPI_GELU_NEW) {
-#pragma unroll
-            for (int e = 0; e < 8; ++e) a[e] = gelu_of_bf16(a[e]);
-#pragma unroll
-            for (int e = 0; e < 8; e += 2) round2_bf16(a[e], a[e + 1]);
-          }
-#pragma unroll
-          for (int e = 0; e < 8; ++e) a[e] += rr[e];
-          st_16B(y + at, pack8(a));
-        } else {
-#pragma unroll
-          for (int e = 0; e < 8; ++e) b[e] += bb2[e];
-#pragma unroll
-          for (int e = 0; e < 8; e += 2) round2_bf16(b[e], b[e + 1]);
-          if (turned) {
-            float cs[8], sn[8];
-            unpack8(pre1[q], cs);
-            unpack8(pre2[q], sn);
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-              const float x1 = a[e], x2 = b[e];
-              float p = x1 * cs[e], q1 = -x2 * sn[e], q2 = x2 * cs[e], t = x1 * sn[e];
-              round2_bf16(p, q1);
-              round2_bf16(q2, t);
-              a[e] = p + q1;
-              b[e] = q2 + t;
-            }
-          }
-          const uint4 u1 = pack8(a), u2 = pack8(b);
-          st_16B(y + at, u1);
-          st_16B(y + at + half, u2);
-          if (head >= rope.H) {
-            const bool is_k = head < rope.H + rope.KV;
-            const int kvh = head - rope.H - (is_k ? 0 : rope.KV);
-            const size_t row = (((size_t)page[q] * rope.KV + kvh) << rope.page_shift) + (pos[q] & ((1 << rope.page_shift) - 1));
-            bf16* dst = (is_k ? rope.k_cache : rope.v_cache) + row * hd + he;
-            st_16B(dst, u1);
-            st_16B(dst + half, u2);
-          }
-        }
-      }
-    }
-  }
+  rows_finish<kMode, kAnyBias, kRowsThreads, 1>(smem, tmem_base, splits, rank, 0, rows, m0, n_tile, bias, residual, y, N, epilogue,
+                                                rope, hd);
   __syncthreads();
   if (warp == 1) {
     tcgen05_fence_after();
@@ -345,16 +361,150 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
   }
 }
 
+// The same on pairs of SMs for 257 to 320 activation rows: 256 weight rows x all of them are one tile of two
+// tcgen05.mma.cta_group::2 (half of the rows each) per 16 elements of K, each SM holds its 128 weight rows and HALF of the activation
+// rows.  What bounds it: two tiles of 128 x 160 on one SM take in and give out 72 KB of shared memory for 640 clocks of MMAs,
+// which at 128 bytes a clock is 1 150; here it is 35 KB for 608 (304 rows).  Measured 650; what is left are the last wave (112
+// tiles of a 28672-row matrix on 74 pairs) and the epilogue, 7 us a wave that nothing hides, since 512 columns of TMEM are one CTA's.
+// us at 301 rows in chains over rotating weights, single SMs -> pairs: 28672 x 4096 gated 73.4 -> 68.5, 57344 x 8192 gated 299 -> 253,
+// 8192 x 28672 132 -> 113, 8192 x 8192 41.6 -> 38.2, 15360 x 5120 49.6 -> 45.0, 5120 x 13824 46.9 -> 42.6, 128256 x 4096 314 -> 290.
+// Up to 256 rows it gains nothing: one tile of 128 weight rows is fed once, or the paired projections' tiles are full.
+// gridDim.x = 2 x splits, y = 1.
+constexpr int kWideThreads = 64 + 8 * 32;
+template <int kMode, bool kAnyBias = false>
+__global__ void __launch_bounds__(kWideThreads, 1)
+gemm_rows_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX,
+                      const bf16* __restrict__ bias, const bf16* residual, bf16* y, int M, int N, int K, int epilogue, int BN,
+                      int stages, int tmem_cols, const __grid_constant__ RopeArgs rope, int hd) {
+  constexpr bool kGated = kMode == kRowsGated;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  const int width = BN / 2, half = width / 2;  // activation rows of an MMA, of them in this CTA
+  const int stage_bytes = (128 + width) * (kBlockK * 2);
+  uint8_t* bar_mem = smem + stages * stage_bytes;
+  const uint32_t full_bar = smem_addr(bar_mem);          // leader's: both CTAs' operands of a stage have landed
+  const uint32_t empty_bar = full_bar + 8 * stages;      // each CTA's: the stage's MMAs are done
+  const uint32_t done_bar = empty_bar + 8 * stages;      // each CTA's: all MMAs are done
+  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(bar_mem + 8 * (2 * stages + 1));
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int member = blockIdx.x & 1, split = blockIdx.x >> 1, splits = gridDim.x >> 1;
+  const int total_kb = K / kBlockK;
+  const int kb0 = (int)((long long)total_kb * split / splits);
+  const int num_kb = (int)((long long)total_kb * (split + 1) / splits) - kb0;
+  const int n_tile = blockIdx.z * 2 + member;  // of 128 weight rows; an odd last one has no partner: zeros, nothing is stored
+
+  if (warp == 0 && lane == 0) {
+    tma_prefetch_desc(&tmW);
+    tma_prefetch_desc(&tmX);
+    for (int s = 0; s < stages; ++s) {
+      mbar_init(full_bar + 8 * s, 1);
+      mbar_init(empty_bar + 8 * s, 1);
+    }
+    mbar_init(done_bar, 1);
+    fence_barrier_init();
+  }
+  if (warp == 1) tmem_alloc_pair(smem_addr(tmem_ptr_smem), tmem_cols);
+  tcgen05_fence_before();
+  pair_barrier();  // the other CTAs' barriers exist before anything arrives there
+  tcgen05_fence_after();
+  const uint32_t tmem_base = *tmem_ptr_smem;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      const uint32_t lead_full = pair_map(full_bar, blockIdx.x & ~1u);
+      auto load_w = [&](int kb, int s) {
+        if (member == 0) mbar_expect_tx(full_bar + 8 * s, 2 * stage_bytes);
+        const uint32_t dst = smem_addr(smem) + s * stage_bytes;
+        if (kGated) {
+          const int row = (n_tile >> 1) * 256 + (n_tile & 1) * 64;  // 64 gate rows; their up rows are 128 further
+          tma_load_2d_pair(dst, &tmW, lead_full + 8 * s, (kb0 + kb) * kBlockK, row);
+          tma_load_2d_pair(dst + 64 * kBlockK * 2, &tmW, lead_full + 8 * s, (kb0 + kb) * kBlockK, row + 128);
+        } else {
+          tma_load_2d_pair(dst, &tmW, lead_full + 8 * s, (kb0 + kb) * kBlockK, n_tile * 128);
+        }
+      };
+      auto load_x = [&](int kb, int s) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+          tma_load_2d_pair(smem_addr(smem) + s * stage_bytes + (128 + i * half) * kBlockK * 2, &tmX, lead_full + 8 * s,
+                           (kb0 + kb) * kBlockK, i * width + member * half);
+      };
+      const int pre = min(stages, num_kb);
+      for (int kb = 0; kb < pre; ++kb) load_w(kb, kb);  // before the dependency wait: weights depend on nothing
+      pdl_wait();
+      pdl_trigger();
+      for (int kb = 0; kb < pre; ++kb) load_x(kb, kb);
+      int s = pre == stages ? 0 : pre;
+      uint32_t ph = pre == stages ? 0 : 1;  // parity of the empty barrier's phase this lap waits for
+      for (int kb = pre; kb < num_kb; ++kb) {
+        mbar_wait(empty_bar + 8 * s, ph);
+        load_w(kb, s);
+        load_x(kb, s);
+        if (++s == stages) s = 0, ph ^= 1;
+      }
+      for (int i = 0; i < stages; ++i) {  // the leader's last arrivals have come before the ring is used again
+        mbar_wait(empty_bar + 8 * s, ph);
+        if (++s == stages) s = 0, ph ^= 1;
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    if (member == 0) {
+      const uint32_t idesc = make_idesc_pair(width);
+      const uint64_t adesc0 = make_smem_desc(smem_addr(smem));
+      const uint64_t bdesc0 = make_smem_desc(smem_addr(smem) + 128 * kBlockK * 2);
+      const uint16_t both = (uint16_t)(3u << blockIdx.x);
+      int s = 0;
+      uint32_t ph = 0;
+      for (int kb = 0; kb < num_kb; ++kb) {
+        mbar_wait(full_bar + 8 * s, ph);
+        tcgen05_fence_after();
+        const uint64_t off = (uint64_t)(s * (stage_bytes >> 4));  // start-address field: bytes >> 4
+        if (elect_one()) {
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            const uint64_t b = bdesc0 + off + (uint64_t)(i * ((half * kBlockK * 2) >> 4));
+#pragma unroll
+            for (int k = 0; k < kBlockK / kUmmaK; ++k)
+              umma_bf16_pair(tmem_base + i * width, adesc0 + off + 2 * k, b + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+          }
+          umma_commit_pair(empty_bar + 8 * s, both);
+          if (kb == num_kb - 1) umma_commit_pair(done_bar, both);
+        }
+        __syncwarp();
+        if (++s == stages) s = 0, ph ^= 1;
+      }
+    }
+  } else {
+    pdl_wait();  // residual and bias may come from the previous kernel
+    mbar_wait(done_bar, 0);
+    tcgen05_fence_after();
+  }
+  if (splits > 1) cluster_barrier();
+  else __syncthreads();
+  rows_finish<kMode, kAnyBias, kWideThreads, 2>(smem, tmem_base, splits, split, member, M, 0, n_tile, bias, residual, y, N,
+                                                epilogue, rope, hd);
+  tcgen05_fence_before();
+  pair_barrier<false>();  // both epilogues have read their accumulators
+  if (warp == 1) {
+    tcgen05_fence_after();
+    tmem_dealloc_pair(tmem_base, tmem_cols);
+  }
+}
+
 // ---- host side -------------------------------------------------------------------------------------------------------
 constexpr int kRowsMaxSmem = 227 * 1024;
+constexpr int kRowsPairMax = 320;  // activation rows of the form on pairs (from 257 on)
 constexpr size_t kSmemPerSm = 228 * 1024;  // of which each resident CTA also takes 1 KB for the system
 
-static size_t rows_smem(int bn, int stages) { return (size_t)stages * (128 + bn) * kBlockK * 2 + 1024 + 256; }
+static size_t rows_ring(int bn, int stages, bool pair) { return (size_t)stages * (128 + (pair ? bn / 2 : bn)) * kBlockK * 2; }
+static size_t rows_smem(int bn, int stages, bool pair) { return rows_ring(bn, stages, pair) + 1024 + 256; }
 static int rows_per_owner(int bn, int splits) { return (((bn + splits - 1) / splits) + 7) & ~7; }
-static bool rows_fits(int bn, int splits, int stages) {
+static bool rows_fits(int bn, int splits, int stages, bool pair) {
   // the ring also takes the partial sums: `splits` times the columns a CTA owns
-  return rows_smem(bn, stages) <= (size_t)kRowsMaxSmem &&
-         (size_t)splits * rows_per_owner(bn, splits) * 512 <= (size_t)stages * (128 + bn) * kBlockK * 2;
+  return rows_smem(bn, stages, pair) <= (size_t)kRowsMaxSmem &&
+         (size_t)splits * rows_per_owner(bn, splits) * 512 <= rows_ring(bn, stages, pair);
 }
 
 static int rows_setup(int* capacity /*[kRowsMaxCluster + 1]: CTAs that run at once with one CTA per SM*/) {
@@ -370,6 +520,12 @@ static int rows_setup(int* capacity /*[kRowsMaxCluster + 1]: CTAs that run at on
     DLI_CUDA_CALL(ring((const void*)gemm_rows_kernel<kRowsPlain, true>));
     DLI_CUDA_CALL(ring((const void*)gemm_rows_kernel<kRowsRope, true>));
     DLI_CUDA_CALL(ring((const void*)gemm_rows_kernel<kRowsGated, true>));
+    DLI_CUDA_CALL(ring((const void*)gemm_rows_pair_kernel<kRowsPlain>));
+    DLI_CUDA_CALL(ring((const void*)gemm_rows_pair_kernel<kRowsGated>));
+    DLI_CUDA_CALL(ring((const void*)gemm_rows_pair_kernel<kRowsRope>));
+    DLI_CUDA_CALL(ring((const void*)gemm_rows_pair_kernel<kRowsPlain, true>));
+    DLI_CUDA_CALL(ring((const void*)gemm_rows_pair_kernel<kRowsRope, true>));
+    DLI_CUDA_CALL(ring((const void*)gemm_rows_pair_kernel<kRowsGated, true>));
     for (int c = 1; c <= kRowsMaxCluster; ++c) {
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3(c, 64, 64);
@@ -402,7 +558,7 @@ static int rows_setup(int* capacity /*[kRowsMaxCluster + 1]: CTAs that run at on
 static double rows_cost(int M, int N, int K, const RowsShape& sh, const int* cap) {
   const int kb = K / kBlockK, kbp = (kb + sh.splits - 1) / sh.splits;
   const long long ctas = (long long)((M + sh.bn - 1) / sh.bn) * ((N + 127) / 128) * sh.splits;
-  const int r = 2 * (rows_smem(sh.bn, sh.stages) + 1024) <= kSmemPerSm ? 2 : 1;
+  const int r = 2 * (rows_smem(sh.bn, sh.stages, false) + 1024) <= kSmemPerSm ? 2 : 1;
   const long long at_once = (long long)cap[sh.splits] * r;
   const long long waves = (ctas + at_once - 1) / at_once, rest = ctas - (waves - 1) * at_once;
   const long long last = (rest + cap[sh.splits] - 1) / cap[sh.splits];
@@ -421,22 +577,37 @@ static double rows_cost(int M, int N, int K, const RowsShape& sh, const int* cap
   return t + 2.55 + 0.0323 * sh.bn + 5.0 * (double)(waves - 1);
 }
 
+// The same of the form on pairs, fitted to 20 matrices (768 x 768 ... 10240 x 8192) at 272 ... 320 rows x 1 to 4 splits, B200: 6 % off
+// on average.
+//   time = (feed^6 + mem^6)^(1/6) + 1.78 + waves x 0.0219 bn + 0.52 (splits - 1) + 4.6 (waves - 1) us
+//   feed = waves x k-blocks x (0.001 + 0.00113 bn) us; mem = weight bytes / 6.24 TB/s, and up to 55 % more for few CTAs
+// A further wave of an ungated matrix, whose epilogues write twice as much, takes 0.012 bn more.
+static double rows_pair_cost(int N, int K, bool gated, const RowsShape& sh, const int* cap) {
+  const int kbp = (K / kBlockK + sh.splits - 1) / sh.splits, at_once = cap[2 * sh.splits];
+  const long long ctas = 2ll * ((N + 255) / 256) * sh.splits, waves = (ctas + at_once - 1) / at_once;
+  const double feed = (double)waves * kbp * (0.001 + 0.00113 * sh.bn);
+  const double mem = (double)N * K * 2 / 6.24e6 * (ctas < 250 ? 1.0 + 0.55 * (double)(250 - ctas) / 250.0 : 1.0);
+  return std::pow(std::pow(feed, 6) + std::pow(mem, 6), 1.0 / 6) + 1.78 + 0.0219 * sh.bn * (double)waves + 0.52 * (sh.splits - 1) +
+         (4.6 + (gated ? 0.0 : 0.012 * sh.bn)) * (double)(waves - 1);
+}
+
 namespace {
 struct PlanKey {
   int dev, M, N, K;
-  bool operator==(const PlanKey& o) const { return dev == o.dev && M == o.M && N == o.N && K == o.K; }
+  bool gated;
+  bool operator==(const PlanKey& o) const { return dev == o.dev && M == o.M && N == o.N && K == o.K && gated == o.gated; }
 };
-struct Plan { RowsShape shape; double us; };
+struct Plan { RowsShape shape; double us; RowsShape pair; double pair_us; };
 }  // namespace
 
-int plan_gemm_rows(int M, int N, int K, RowsShape* shape, double* us) {
+int plan_gemm_rows(int M, int N, int K, bool gated, RowsShape* shape, double* us, RowsShape* pair, double* pair_us) {
   // A plan is a pure function of the sizes (and the device); the search takes about as long as a launch.  A pass has up
   // to five matrices at one M, a head and a few decode sizes beside them: the last 32 are kept per thread.  Host time of a
   // call from Python, four matrices in turn at 19 and 301 rows: 9.9 us with a search each time, 8.3 without.
   static thread_local RecentResults<PlanKey, Plan, 32> plans;
   const int dev = current_device_slot();
   if (dev < 0) return DLI_ERR_CUDA;
-  const PlanKey key{dev, M, N, K};
+  const PlanKey key{dev, M, N, K, gated};
   const Plan* plan = plans.find(key);
   Plan made;
   if (plan == nullptr) {
@@ -456,29 +627,43 @@ int plan_gemm_rows(int M, int N, int K, RowsShape* shape, double* us) {
         for (int budget : {108, 216}) {
           int stages = budget * 1024 / ((128 + bn) * kBlockK * 2);
           if (stages > 8) stages = 8;
-          if (!rows_fits(bn, splits, stages)) continue;
-          const RowsShape sh{bn, splits, stages};
+          if (!rows_fits(bn, splits, stages, false)) continue;
+          const RowsShape sh{bn, splits, stages, false};
           const double t = rows_cost(M, N, K, sh, cap);
           if (t < best) best = t, pick = sh;
         }
       }
     }
-    made = Plan{pick, best};
+    made = Plan{pick, best, {}, 1e30};
+    if (M > 256 && M <= kRowsPairMax) {
+      const int bn = (M + 31) / 32 * 32;
+      for (int splits = 1; splits <= kRowsMaxCluster / 2; ++splits) {
+        if ((splits > 1 && splits > K / (8 * kBlockK)) || cap[2 * splits] <= 0) continue;
+        const RowsShape sh{bn, splits, (int)((kRowsMaxSmem - 1280) / rows_ring(bn, 1, true)), true};
+        if (!rows_fits(bn, splits, sh.stages, true)) continue;
+        const double t = rows_pair_cost(N, K, gated, sh, cap);
+        if (t < made.pair_us) made.pair_us = t, made.pair = sh;
+      }
+    }
     plans.put(key, made);
     plan = &made;
   }
   *shape = plan->shape;
   *us = plan->us;
+  *pair = plan->pair;
+  *pair_us = plan->pair_us;
   return DLI_OK;
 }
 
 template <int kMode, bool kAnyBias = false>
 static int launch_rows(const CUtensorMap& tmW, const CUtensorMap& tmX, const void* bias, const void* residual, void* y, int M,
                        int N, int K, int epilogue, const RowsShape& sh, cudaStream_t s, const RopeArgs& rope, int hd) {
-  const int cols = sh.bn <= 32 ? 32 : sh.bn <= 64 ? 64 : sh.bn <= 128 ? 128 : 256;
-  const dim3 grid(sh.splits, (M + sh.bn - 1) / sh.bn, (N + 127) / 128);
-  const cudaError_t e = launch_kernel_cluster(gemm_rows_kernel<kMode, kAnyBias>, grid, dim3(kRowsThreads), rows_smem(sh.bn, sh.stages), s,
-                                              (unsigned)sh.splits, tmW, tmX, (const bf16*)bias, (const bf16*)residual,
+  const int cols = sh.bn <= 32 ? 32 : sh.bn <= 64 ? 64 : sh.bn <= 128 ? 128 : sh.bn <= 256 ? 256 : 512;
+  const int ctas = sh.pair ? 2 : 1;
+  const dim3 grid(ctas * sh.splits, (M + sh.bn - 1) / sh.bn, (N + 128 * ctas - 1) / (128 * ctas));
+  const auto kernel = sh.pair ? gemm_rows_pair_kernel<kMode, kAnyBias> : gemm_rows_kernel<kMode, kAnyBias>;
+  const cudaError_t e = launch_kernel_cluster(kernel, grid, dim3(sh.pair ? kWideThreads : kRowsThreads), rows_smem(sh.bn, sh.stages, sh.pair),
+                                              s, (unsigned)(ctas * sh.splits), tmW, tmX, (const bf16*)bias, (const bf16*)residual,
                                               (bf16*)y, M, N, K, epilogue, sh.bn, sh.stages, cols, rope, hd);
   if (e != cudaSuccess) return fail(DLI_ERR_CUDA, "gemm_rows_kernel: %s", cudaGetErrorString(e));
   return DLI_OK;
@@ -489,13 +674,14 @@ int launch_gemm_rows(RowsMode mode, const void* x, const void* w, const void* bi
   int cap[kRowsMaxCluster + 1];
   int rc = rows_setup(cap);
   if (rc != DLI_OK) return rc;
-  if (sh.bn < 16 || sh.bn > 256 || sh.bn % 16 || sh.splits < 1 || sh.splits > kRowsMaxCluster || sh.splits > K / kBlockK ||
-      !rows_fits(sh.bn, sh.splits, sh.stages) || (N + 127) / 128 > 65535 || (M + sh.bn - 1) / sh.bn > 65535)
+  if (sh.bn < 16 || sh.bn > (sh.pair ? kRowsPairMax : 256) || (sh.pair ? sh.bn % 32 || sh.bn <= 256 || M > sh.bn : sh.bn % 16) || sh.splits < 1 ||
+      sh.splits > kRowsMaxCluster / (sh.pair ? 2 : 1) || sh.splits > K / kBlockK || !rows_fits(sh.bn, sh.splits, sh.stages, sh.pair) ||
+      (N + 127) / 128 > 65535 || (M + sh.bn - 1) / sh.bn > 65535)
     return fail(DLI_ERR_INVALID, "gemm_rows: M=%d N=%d K=%d in tiles of %d rows, %d splits, %d stages does not fit", M, N, K,
                 sh.bn, sh.splits, sh.stages);
   CUtensorMap tmW, tmX;
   if ((rc = make_tmap(&tmW, w, N, K, mode == kRowsGated ? 64 : 128)) != DLI_OK) return rc;
-  if ((rc = make_tmap(&tmX, x, M, K, sh.bn)) != DLI_OK) return rc;
+  if ((rc = make_tmap(&tmX, x, M, K, sh.pair ? sh.bn / 4 : sh.bn)) != DLI_OK) return rc;
   const bool any_bias = mode == kRowsGated ? bias != nullptr : (epilogue & DLI_EPI_BIAS) && !aligned16(bias);
   const auto launch = mode == kRowsGated ? (any_bias ? launch_rows<kRowsGated, true> : launch_rows<kRowsGated>)
                       : mode == kRowsRope ? (any_bias ? launch_rows<kRowsRope, true> : launch_rows<kRowsRope>)

@@ -17,15 +17,18 @@ struct RopeArgs {
 };
 
 // How a projection is cut: `bn` activation rows per tile (a multiple of 16, at most 256), K split over a cluster of
-// `splits` CTAs (1..8, at most K / 64), a ring of `stages` operand tiles.
+// `splits` CTAs (1..8, at most K / 64), a ring of `stages` operand tiles.  pair: the splits are pairs of CTAs (1..4 of them), all
+// rows are one tile (288 or 320, a multiple of 32).
 struct RowsShape {
   int bn, splits, stages;
+  bool pair;
 };
 
 enum RowsMode { kRowsPlain = 0, kRowsGated = 1, kRowsRope = 2 };
 
-// The cut for [M, K] x [N, K]^T and its estimated time in us (the rule stands beside the definition).
-int plan_gemm_rows(int M, int N, int K, RowsShape* shape, double* us);
+// The cut for [M, K] x [N, K]^T and its estimated time in us, on single CTAs and on pairs of them (1e30 us: no such cut); the rules
+// stand beside the definitions.
+int plan_gemm_rows(int M, int N, int K, bool gated, RowsShape* shape, double* us, RowsShape* pair, double* pair_us);
 
 // y = epi(x w^T).  kRowsGated: w is the interleaved gate / up matrix, N counts its rows, `bias` carries the activation's
 // parameters; kRowsRope: N = (H + 2 KV) hd, no residual, no activation.  The caller has checked the arguments:

@@ -403,7 +403,8 @@ static PrefillShape prefill_tile(int M, int N, int K, bool gated) {
 }
 
 // Which kernel takes a projection, by estimated time:
-//  - clusters that split K (gemm_rows.cu), up to 4 096 rows, which bound what was measured, and always up to 128 rows;
+//  - clusters that split K (gemm_rows.cu), up to 4 096 rows, which bound what was measured, and always up to 128 rows; from 257 to
+//    320 rows also on pairs of SMs, where their estimate is 3 % below the others';
 //  - pairs of SMs (gemm_pair.cu) in tiles of 256 rows, for widths that are multiples of 128; from 129 ... 700 rows on, by matrix;
 //  - the persistent kernel above where 256-row tiles would be half padding and the matrix is large (28672 x 4096 gated at 336
 //    rows: 85 us, clusters 95), and for other widths, at which the pairs were not measured.
@@ -431,10 +432,11 @@ static int choose(int M, int N, int K, bool gated, Choice* c) {
   c->route = kRoutePersistent;
   if (M > 128 && N < 128) return DLI_OK;
   PrefillShape p;
-  double us, best = pick_prefill(M, N, K, gated, &p) + (gated && K >= 4096 ? 4.5 : 9.5);
+  double us, pair_us = 1e30, best = pick_prefill(M, N, K, gated, &p) + (gated && K >= 4096 ? 4.5 : 9.5);
+  RowsShape on_pairs;
   if (pairs && (M > 1024 || ((M + 127) / 128) % 2 == 0)) best = 1e30;  // 256-row tiles are full, or nearly
   if (M <= 4096) {
-    if ((rc = plan_gemm_rows(M, N, K, &c->rows, &us)) != DLI_OK) return rc;
+    if ((rc = plan_gemm_rows(M, N, K, gated, &c->rows, &us, &on_pairs, &pair_us)) != DLI_OK) return rc;
     const double tera = 2e-12 * M * N * K, hot = tera < 1.0 ? tera : 1.0;
     us = pairs ? (0.88 * us + 1.5) * (1.0 + 0.24 * hot * hot) : 1.1 * us;
     if (M <= 128 || us < best) c->route = kRouteRows, best = us;
@@ -448,8 +450,9 @@ static int choose(int M, int N, int K, bool gated, Choice* c) {
       const double weights = 2.5 + (double)N * K * 2 / 4.8e6;
       if (us < weights) us = weights;
     }
-    if (us < best) c->route = kRoutePair;
+    if (us < best) c->route = kRoutePair, best = us;
   }
+  if (1.03 * pair_us < best) c->route = kRouteRows, c->rows = on_pairs;
   return DLI_OK;
 }
 

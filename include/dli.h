@@ -340,8 +340,8 @@ int dli_gemm_qkv_rope_append_bf16(const void* x, const void* w_qkv, void* qkv, i
  * kernel.  dli_gemm_splitk_scratch_bytes keeps the size it has always returned. */
 size_t dli_gemm_splitk_scratch_bytes(int M, int N);
 /* What dli_gemm_bf16 (gated: dli_gemm_gated_silu_bf16, N = 2 F) runs for these sizes on the current device, for tests and
- * measurements, as three numbers: plan[0] = 1: K split over clusters, plan[1] activation rows per tile, plan[2] splits; plan[0] = 0: the
- * persistent kernel, plan[1] weight rows per tile, plan[2] 128-row halves per tile; plan[0] = 2: pairs of SMs in tiles of 256
+ * measurements, as three numbers: plan[0] = 1: K split over clusters, plan[1] activation rows per tile (above 256: on pairs of SMs),
+ * plan[2] splits; plan[0] = 0: the persistent kernel, plan[1] weight rows per tile, plan[2] 128-row halves per tile; plan[0] = 2: pairs of SMs in tiles of 256
  * activation rows, plan[1] weight rows per tile, plan[2] those of the narrower tiles at the end, or 0. */
 int dli_gemm_plan(int M, int N, int K, int gated, int* plan);
 int dli_gemm_splitk_bf16(const void* x, const void* w, const void* bias,

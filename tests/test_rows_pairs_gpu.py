@@ -1,0 +1,77 @@
+"""K-split projections of 257 to 320 rows on pairs of SMs (csrc/gemm_rows.cu), against float64.  Bounds as in test_gemm_rows_gpu.py."""
+import pytest
+from test_gemm_rows_gpu import HALF_ULP, _inputs, _within
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+BF = torch.bfloat16
+
+
+@pytest.mark.parametrize("M", [257, 288, 289, 320])  # both tiles, full and one row over
+@pytest.mark.parametrize("N,K,splits", [(8192, 8192, 2), (8144, 8192, 2), (15360, 5120, 1), (5120, 13824, 3), (32000, 4096, 1)])
+def test_projection(cuda, M, N, K, splits):
+    """Whole pairs of weight tiles, a last one without a partner (8144 = 63.6 x 128), 1 to 3 splits, more tiles than pairs."""
+    from dli_b200 import ops
+
+    if ops.sm_count() == 148 and N % 128 == 0:
+        assert ops.gemm_plan(M, N, K) == ("rows", (M + 31) // 32 * 32, splits)
+    g, x, w, acc, slack = _inputs(M, N, K, M + N)
+    bias = torch.randn(N + 1, device=cuda, generator=g).to(BF)
+    res = torch.randn(M, N, device=cuda, generator=g).to(BF)
+    y = ops.gemm(x, w)
+    _within(y, acc, slack + HALF_ULP * acc.abs())
+    assert torch.equal(y, ops.gemm(x, w))  # the order of the sums is fixed
+    for b in (bias[:N], bias[1:]):  # one that starts anywhere
+        z = acc + b.double()
+        _within(ops.gemm(x, w, bias=b, residual=res), z + res.double(), slack + HALF_ULP * (z.abs() + slack + (z + res.double()).abs() * 1.01))
+
+
+@pytest.mark.parametrize("M", [257, 301, 320])
+@pytest.mark.parametrize("F,K", [(14336, 4096), (28672, 1024)])
+def test_gated_projection(cuda, M, F, K):
+    from dli_b200 import ops
+
+    if ops.sm_count() == 148 and K == 4096:
+        assert ops.gemm_plan(M, 2 * F, K, True) == ("rows", (M + 31) // 32 * 32, 1)
+    g, x, wg, gate, s1 = _inputs(M, F, K, M + F)
+    wu = (torch.randn(F, K, device="cuda", generator=g) * K ** -0.5).to(BF)
+    up, s2 = x.double() @ wu.double().T, 2 * K * 2.0 ** -24 * (x.double().abs() @ wu.double().abs().T)
+    w, e_gate, e_up = ops.pack_gate_up(wg, wu), s1 + HALF_ULP * gate.abs(), s2 + HALF_ULP * up.abs()
+    act = torch.nn.functional.silu(gate)
+    e_act = 1.1 * e_gate + HALF_ULP * (act.abs() + 1.1 * e_gate)
+    _within(ops.gemm_gated_silu(x, w), act * up, e_act * (up.abs() + e_up) + act.abs() * e_up + HALF_ULP * 1.1 * (act * up).abs() + 1e-6)
+    act = torch.nn.functional.gelu(gate, approximate="tanh")
+    got = ops.linear_gated_act(x, w, torch.zeros(2, device=cuda))
+    _within(got, act * up, 1.13 * e_gate * (up.abs() + e_up) + act.abs() * e_up + HALF_ULP * 1.1 * (act * up).abs() + 1e-6)
+
+
+@pytest.mark.parametrize("hd,H,KV,K,bias", [(128, 104, 8, 5120, False), (128, 105, 7, 5120, True), (64, 208, 16, 5120, True)])
+def test_qkv_with_rotation(cuda, hd, H, KV, K, bias):
+    """Rotation and cache append in the epilogue: the bits of the projection by itself and the separate rotation."""
+    from dli_b200 import ops
+
+    T, ff, page, prefix = 301, 256, 16, 5
+    g = torch.Generator(device="cuda").manual_seed(H)
+    rnd = lambda *s, std=1.0: (std * torch.randn(*s, device=cuda, generator=g)).to(BF)  # noqa: E731
+    N, pages = (H + 2 * KV) * hd, (T + prefix + 15) // 16
+    if ops.sm_count() == 148:
+        assert ops.gemm_plan(T, N, K)[:2] == ("rows", 320)
+    L = {"ln1": rnd(K), "ln2": rnd(K), "wqkv": rnd(N, K, std=0.02), "wo": rnd(K, H * hd, std=0.02), "wdown": rnd(K, ff, std=0.02),
+         "wgu": ops.pack_gate_up(rnd(ff, K, std=0.02), rnd(ff, K, std=0.02))}
+    if bias:
+        L["bqkv"] = rnd(N)
+    ang = torch.rand(T + prefix, hd // 2, device=cuda, generator=g) * 6.28
+    cos, sin = ang.cos().to(BF), ang.sin().to(BF)
+    table = torch.randperm(pages, device=cuda, generator=g).int().view(1, pages)
+    positions, seq_ids, last = (torch.empty(T, device=cuda, dtype=torch.int32) for _ in range(3))
+    ops.prompt_rows(positions, seq_ids, last, 1, T, prefix, 0)
+    h_in = rnd(T, K)
+    kc, vc = (torch.zeros(pages, KV, page, hd, device=cuda, dtype=BF) for _ in range(2))
+    h, x, qkv, attn, act = (torch.empty(T, w, device=cuda, dtype=BF) for w in (K, K, N, H * hd, ff))
+    ops.prompt_layers([L], [kc], [vc], table, table, h_in, h, x, qkv, attn, act, cos, sin, positions, seq_ids, 1, T, prefix,
+                      H, KV, hd, 1e-5, hd ** -0.5)
+    ops.add_rmsnorm(h_in, L["ln1"], 1e-5, out=x)
+    want = ops.gemm(x, L["wqkv"], bias=L.get("bqkv"))
+    k2, v2 = torch.zeros_like(kc), torch.zeros_like(vc)
+    ops.rope_kv_append(want, cos, sin, positions, seq_ids, table, k2, v2, H, KV, hd)
+    assert torch.equal(qkv, want) and torch.equal(kc, k2) and torch.equal(vc, v2)
