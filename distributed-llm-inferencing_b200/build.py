@@ -24,6 +24,7 @@ SOURCES = [
     "attn_decode.cu",
     "attn_prefill.cu",
     "attn_prefill_tc.cu",
+    "attn_prefill_streams.cu",
     "gemv.cu",
     "gemv_mma.cu",
     "gemm_tcgen05.cu",

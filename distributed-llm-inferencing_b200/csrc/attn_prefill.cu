@@ -232,7 +232,8 @@ int launch_attn_prefill_tc_paged(const void* qkv, void* out, const void* k_cache
 // estimated time, because how many items a call has, how long the longest is and how many of its keys a window leaves all
 // shift the line: 32 heads, T = 512: 10.8 / 9.4, 2 heads 8.8 / 9.0; T = 1777 of 12 heads 35 / 20, in a window of 100 8.8 / 12.8.
 //   mma.sync, CTA per 64 queries: c0 + hypot(c1 x longest, (c2 x tiles + c3 x CTAs) / SMs), tiles of 64 keys
-//   tcgen05, 128 queries an item: d0 + d1 x tiles + d2 x items of the fullest CTA of the serpentine deal, tiles of 128 keys
+//   tcgen05, 128 queries an item, or two of them: d0 + d1 x tiles + d2 x items of the fullest CTA of the serpentine deal, tiles of
+//   128 keys
 // fitted to 2 700 calls (2 ... 64 heads, 1 ... 16 sequences, 1 ... 2048 queries, up to 8 000 keys, windows), within 4 and 6 %.
 // Taken where it is estimated 5 % faster: over those calls 0.4 % slower than the better kernel on average, and at most 13 %
 // than mma.sync.  (448 keys as the line: 9.8 % on average, up to 58 %.)
@@ -254,41 +255,66 @@ static void key_tiles(KeyTiles& n, int T, int prefix, int window, int q_tile, in
     if (t > n.longest) n.longest = t;
   }
 }
-static bool prefill64_on_tc(int B, int T, int prefix, int H, int window, bool paged) {
+// Time of a tcgen05 kernel whose items are a query tile, or two of them that share their keys (streams).  n: key tiles of 128 of each
+// query tile, sorted by length.
+static double tc_time(const KeyTiles& n, int B, int H, int KV, bool streams, double start, double per_tile, double per_item) {
   const int sms = sm_count_cached() > 0 ? sm_count_cached() : 148;
-  const double copies = (double)H * B;
+  const int per_kv = H / KV;
+  const long long levels = streams ? ((long long)n.count * per_kv + 1) / 2 : n.count, copies = (long long)B * (streams ? KV : H);
+  const long long items = levels * copies, rounds = (items + sms - 1) / sms;
+  if (rounds > 16 || n.count > kMaxListed)
+    return start + per_tile * n.total * B * H / (streams ? 2.0 : 1.0) / sms + per_item * (double)rounds;
+  // the first and the last CTA, and those at either side of where the last round ends
+  const int last = (int)(items - (rounds - 1) * sms);
+  const int side = rounds % 2 ? last - 1 : sms - last, other = rounds % 2 ? (last < sms ? last : sms - 1) : (side > 0 ? side - 1 : 0);
+  double most = 0;
+  for (const int c : {0, sms - 1, side, other}) {
+    double t = 0;
+    for (long long r = 0; r < rounds; ++r) {
+      const long long at = r * sms + (r % 2 ? sms - 1 - c : c);
+      if (at < items) t += per_item + per_tile * n.of[streams ? at / copies * 2 / per_kv : at / copies];
+    }
+    if (t > most) most = t;
+  }
+  return start + most;
+}
+static void tc_tiles(KeyTiles& n, int T, int prefix, int window) {
+  key_tiles(n, T, prefix, window, 128, 128);
+  if (n.count <= kMaxListed) std::sort(n.of, n.of + n.count, std::greater<int>());
+}
+static double items_time(const KeyTiles& n, int B, int H, int KV, int hd, bool paged) {
+  if (hd == 64) return paged ? tc_time(n, B, H, KV, false, 3.4, 1.08, 3.4) : tc_time(n, B, H, KV, false, 3.2, 1.11, 2.1);
+  return paged ? tc_time(n, B, H, KV, false, 4.6, 1.64, 2.45) : tc_time(n, B, H, KV, false, 3.2, 1.09, 3.0);
+}
+static double streams_time(const KeyTiles& n, int B, int H, int KV, int hd, bool paged) {
+  if (n.longest < 4) return 1e30;
+  if (hd == 64) return paged ? tc_time(n, B, H, KV, true, 1.2, 1.40, 8.3) : tc_time(n, B, H, KV, true, 2.8, 1.55, 4.6);
+  return paged ? tc_time(n, B, H, KV, true, 2.3, 1.72, 7.9) : tc_time(n, B, H, KV, true, 3.1, 1.80, 5.4);
+}
+// Two streams per CTA (attn_prefill_streams.cu) or one item at a time (attn_prefill_tc.cu): two query tiles in 1.4 ... 1.8 us per key
+// tile against one in 1.05 ... 1.64, but half as many items to spread over the SMs.  By estimated time, fitted to 268 calls (8 ... 64
+// heads, 1 ... 32 sequences of 128 ... 8 000 tokens, windows, chunks) within 8 %; taken where it is 6 % faster and the longest item has
+// four key tiles.  Over those calls never more than 2 % slower than the other kernel, and up to 66 % faster (us, one item at a time /
+// streams; 32 heads, 8 of keys): head size 64, 8000 tokens 467 / 353, 2048 43 / 38; 128, 2 x 2048 89 / 78, 2048 behind 2048 in the
+// cache 167 / 101; not taken: 1024 tokens 17.7 / 23.6, 512 behind 512 20.1 / 23.5.
+bool attn_streams_faster(int B, int T, int prefix, int H, int KV, int hd, int window, bool paged) {
+  KeyTiles n;
+  tc_tiles(n, T, prefix, window);
+  return 1.06 * streams_time(n, B, H, KV, hd, paged) < items_time(n, B, H, KV, hd, paged);
+}
+static bool prefill64_on_tc(int B, int T, int prefix, int H, int KV, int window, bool paged) {
+  const int sms = sm_count_cached() > 0 ? sm_count_cached() : 148;
   KeyTiles n;
   key_tiles(n, T, prefix, window, 64, 64);
-  const double even = copies * (paged ? 0.65 * n.total + 0.6 * n.count : 0.5 * n.total + 0.8 * n.count) / sms;
+  const double even = (double)H * B * (paged ? 0.65 * n.total + 0.6 * n.count : 0.5 * n.total + 0.8 * n.count) / sms;
   const double mma = paged ? 2.0 + hypot(1.0 * n.longest, even) : 2.5 + hypot(0.8 * n.longest, even);
-  key_tiles(n, T, prefix, window, 128, 128);
-  const long long items = (long long)(copies * n.count), rounds = (items + sms - 1) / sms;
-  double tiles = 0, count = 0;
-  if (rounds > 16 || n.count > kMaxListed) {
-    tiles = copies * n.total / sms;
-    count = (double)rounds;
-  } else {
-    std::sort(n.of, n.of + n.count, std::greater<int>());
-    // the first and the last CTA, and those at either side of where the last round ends
-    const int last = (int)(items - (rounds - 1) * sms);
-    const int side = rounds % 2 ? last - 1 : sms - last, other = rounds % 2 ? (last < sms ? last : sms - 1) : (side > 0 ? side - 1 : 0);
-    double most = -1;
-    for (const int c : {0, sms - 1, side, other}) {
-      double t = 0, k = 0;
-      for (long long r = 0; r < rounds; ++r) {
-        const long long at = r * sms + (r % 2 ? sms - 1 - c : c);
-        if (at < items) t += n.of[at / (long long)copies], k += 1;
-      }
-      if (t + 2 * k > most) most = t + 2 * k, tiles = t, count = k;
-    }
-  }
-  const double tc = paged ? 3.4 + 1.08 * tiles + 3.4 * count : 3.2 + 1.11 * tiles + 2.1 * count;
-  return 1.05 * tc < mma;
+  tc_tiles(n, T, prefix, window);
+  return 1.05 * items_time(n, B, H, KV, 64, paged) < mma || 1.05 * streams_time(n, B, H, KV, 64, paged) < mma;
 }
-static bool prefill_on_tc(int B, int T, int prefix, int H, int hd, int window, bool paged) {
+static bool prefill_on_tc(int B, int T, int prefix, int H, int KV, int hd, int window, bool paged) {
   const char* choice = getenv("DLI_PREFILL_ATTN");
   if (choice && strcmp(choice, "mma") == 0) return false;
-  return hd == 64 ? prefill64_on_tc(B, T, prefix, H, window, paged) : prefix + T > 64;
+  return hd == 64 ? prefill64_on_tc(B, T, prefix, H, KV, window, paged) : prefix + T > 64;
 }
 
 }  // namespace dli
@@ -306,7 +332,7 @@ static int attn_prefill(const void* qkv, void* out, int B, int T, int H, int KV,
   if (B == 0 || T == 0) return DLI_OK;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (hd == 128) return launch_prefill<128, false>(qkv, out, B, T, H, KV, scale, window, s);
-  if (by_rule && prefill_on_tc(B, T, 0, H, hd, window, false)) return launch_attn_prefill_tc(qkv, out, B, T, H, KV, hd, scale, window, s);
+  if (by_rule && prefill_on_tc(B, T, 0, H, KV, hd, window, false)) return launch_attn_prefill_tc(qkv, out, B, T, H, KV, hd, scale, window, s);
   return launch_prefill<64, false>(qkv, out, B, T, H, KV, scale, window, s);
 }
 
@@ -342,7 +368,7 @@ extern "C" int dli_attn_prefill_paged_bf16(const void* qkv, void* out, const voi
   while ((1 << shift) < page_size) ++shift;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   // both attention GEMMs on tcgen05, K/V pages brought in by TMA (num_pages > 0 says how large the pools are)
-  if (num_pages > 0 && page_size <= 128 && prefill_on_tc(B, T, prefix, H, hd, window, true))
+  if (num_pages > 0 && page_size <= 128 && prefill_on_tc(B, T, prefix, H, KV, hd, window, true))
     return launch_attn_prefill_tc_paged(qkv, out, k_cache, v_cache, page_table, max_pages, num_pages, B, T, prefix, H,
                                         KV, hd, page_size, scale, window, s);
   if (hd == 128)

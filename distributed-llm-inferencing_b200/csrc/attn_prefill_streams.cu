@@ -1,0 +1,512 @@
+// Causal prefill attention on the 5th-generation tensor cores, two query tiles at a time (head_dim 128 and 64).
+//
+// Work item = two 128-row query tiles that share a K / V head (two heads of a group, or two tiles of one head), each a STREAM with its
+// own Q, scores, probabilities and output; they read the same K and V tiles.  As in attn_prefill_tc.cu the GEMMs are tcgen05.mma with
+// the accumulators in tensor memory, P goes back there as the A operand of P V, a persistent CTA per SM walks a list of items
+// sorted by length, the maximum is lazy.  What differs:
+//  - one thread per query row: no exchange of maxima, and the row's 128 scores stay in registers;
+//  - one stream's softmax runs beside the other's MMAs.  With one stream both wait for each other: 2 000 clocks per key tile at head
+//    size 128 for 1 024 of MMAs and 1 030 of exponentials (16 a clock and SM; 1 400 with everything else of a softmax);
+//  - K and V are read from L2 once for 256 rows, and from the paged cache in half as many boxes, which is what bounded the chunks;
+//  - an MMA warp per stream: one warp for both made each stream wait for the other's probabilities.
+// Tensor memory: S0 | S1 | O0 | O1 (128 columns each) at head size 128, P in the first half of the columns its scores came from, so that
+// a stream's next scores wait for its P V (which starts on the first half of P); at 64 there is room for P and they do not.
+// A stream's chain at head size 128 is what bounds it now: 1 300 clocks of exponentials, 1 200 from P to the next scores, 800 of loads,
+// maxima and turns; 3 100 per two tiles.  us, this / one item at a time, 32 heads: 4096 tokens, head size 128 124 / 148, 64 108 / 136.
+#include "attn_tc.cuh"
+
+namespace dli {
+
+// A warpgroup with the TMA warp and the MMA warp, then two streams of softmax warps, a thread per query row.  A row's 128 scores want
+// more registers than the 168 a thread of 384 is launched with: 104 + 2 x 200 = 3 x 168.
+constexpr int kStreamThreads = 384, kRegsFew = 104, kRegsMany = 200;
+
+template <int HD>
+struct StreamCfg {
+  static constexpr int kSpans = HD / 64;
+  static constexpr int kTileBytes = kSpans * kSpanBytes;  // a [128 x HD] bf16 operand tile
+  static constexpr int kStages = HD == 64 ? 4 : 2;        // K and V tiles in shared memory, each
+  static constexpr bool kOwnP = HD == 64;                 // P has columns of its own; else it takes those of the scores it came from
+  // smem: Q0 Q1 | K stages | V stages | barriers, + alignment slack
+  static constexpr int kSmem = (2 + 2 * kStages) * kTileBytes + 1024 + 256;
+};
+
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{ .reg .b64 a, b, c, d; mov.b64 a, {%2, %3}; mov.b64 b, {%4, %5}; mov.b64 c, {%6, %7}; fma.rn.f32x2 d, a, b, c; mov.b64 {%0, %1}, d; }"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 d;
+  asm("{ .reg .b64 a, b, d; mov.b64 a, {%2, %3}; mov.b64 b, {%4, %5}; add.rn.f32x2 d, a, b; mov.b64 {%0, %1}, d; }"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+
+struct StreamItem {
+  int b, kvh, row_base, tb, te;      // key tiles [tb, te) of the item
+  int h[2], q0[2], first[2], end[2];  // of each stream: head, first query row of the chunk, key tiles
+};
+
+// kPaged (chunked prefill): the T query rows are a chunk at positions prefix .. prefix+T-1; K and V tiles come
+// from the paged cache through two more tensor maps (the cache seen as [pages*KV*page_size, hd] rows, box = one
+// page x 64 columns): the 32 lanes of the producer warp each issue one page-sized box of a 128-token tile.
+// A box whose first token lies beyond the context is requested out of bounds, i.e. zero-filled.
+template <int HD, bool kPaged>
+__global__ void __launch_bounds__(kStreamThreads, 1)
+attn_streams_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant__ CUtensorMap tmK,
+                       const __grid_constant__ CUtensorMap tmV, bf16* __restrict__ out, int T, int H, int KV,
+                       float scale_log2, int window, const int32_t* __restrict__ page_table, int max_pages,
+                       int page_shift, int prefix, int cache_rows, int n_items, int groups, int n_qtiles) {
+  using Cfg = StreamCfg<HD>;
+  constexpr int kTileBytes = Cfg::kTileBytes, kStages = Cfg::kStages;
+  constexpr bool kOwnP = Cfg::kOwnP;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  const uint32_t sQ = smem_addr(smem);
+  const uint32_t sK = sQ + 2 * kTileBytes;
+  const uint32_t sV = sK + kStages * kTileBytes;
+  uint8_t* bar_mem = smem + (2 + 2 * kStages) * kTileBytes;
+  const uint32_t bars = smem_addr(bar_mem);
+  // barrier slots (8 B each); from s_full to p_half: one per stream
+  const uint32_t q_full = bars, q_empty = bars + 8, s_full = bars + 16, s_empty = bars + 32, p_full = bars + 48, pv_done = bars + 64,
+                 p_half = bars + 80, k_full = bars + 96, k_empty = k_full + 8 * kStages, v_full = k_empty + 8 * kStages,
+                 v_empty = v_full + 8 * kStages;
+  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(bar_mem + 96 + 32 * kStages);
+  static_assert(96 + 32 * kStages + 4 <= 256, "barriers");
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int G = gridDim.x, cta = blockIdx.x, per_kv = H / KV;
+  const int past = kPaged ? prefix : 0;
+
+  // item r of this CTA (serpentine deal of the length-sorted list); false when the list is exhausted
+  auto get_item = [&](int r, StreamItem& it) -> bool {
+    const int idx = r * G + ((r & 1) ? G - 1 - cta : cta);
+    if (idx >= n_items) return false;
+    const int level = idx / groups, grp = idx - level * groups;
+    it.b = grp / KV;
+    it.kvh = grp - it.b * KV;
+    it.row_base = it.b * T;  // row of token 0 of this sequence in the packed qkv matrix
+#pragma unroll
+    for (int x = 0; x < 2; ++x) {
+      const int u = 2 * level + x;  // longest first
+      const int back = u / per_kv, qtile = n_qtiles - 1 - back;
+      it.h[x] = it.kvh * per_kv + u - back * per_kv;
+      it.q0[x] = qtile * kTcTile;
+      const int qpos0 = past + it.q0[x];  // absolute position of the tile's first query row
+      it.first[x] = window > 0 && qpos0 - window + 1 > 0 ? (qpos0 - window + 1) / kTcTile : 0;
+      // last key tile: the one holding the last query row's own position (the diagonal tile when prefix == 0)
+      it.end[x] = kPaged ? min((prefix + T + kTcTile - 1) / kTcTile, (qpos0 + kTcTile - 1) / kTcTile + 1) : qtile + 1;
+      if (qtile < 0) it.first[x] = it.end[x] = 0x7fffffff;  // an odd number of query tiles: the last item has one
+    }
+    it.tb = min(it.first[0], it.first[1]);
+    it.te = it.end[0];  // stream 0 has the later or an equal query tile
+    return true;
+  };
+
+  if (warp == 0 && lane == 0) {
+    tma_prefetch_desc(&tm);
+    mbar_init(q_full, 1);
+    mbar_init(q_empty, 2);  // both streams, as below
+    for (int x = 0; x < 2; ++x) {
+      mbar_init(s_full + 8 * x, 1);
+      mbar_init(s_empty + 8 * x, 4);  // one arrive per softmax warp
+      mbar_init(p_full + 8 * x, 4);
+      mbar_init(p_half + 8 * x, 4);
+      mbar_init(pv_done + 8 * x, 1);
+    }
+    for (int i = 0; i < kStages; ++i) {
+      mbar_init(k_full + 8 * i, 1);
+      mbar_init(k_empty + 8 * i, 2);
+      mbar_init(v_full + 8 * i, 1);
+      mbar_init(v_empty + 8 * i, 2);
+    }
+    fence_barrier_init();
+  }
+  if (warp == 1) tmem_alloc(smem_addr(tmem_ptr_smem), 512);
+  pdl_wait();
+  tcgen05_fence_before();
+  __syncthreads();
+  tcgen05_fence_after();
+  // Behind the barrier, that is with the tensor memory in hand: one thread's trigger counts for the CTA, and a projection's CTA may fit
+  // beside this one.  It would take columns and wait for this grid, which would wait for the columns.
+  pdl_trigger();
+  const uint32_t tmem_base = *tmem_ptr_smem;
+  // S0 | S1 (128 columns each) | O0 | O1 (HD each) | P0 | P1 (64 each: two bf16 probabilities a column) where they have their own
+  const uint32_t tS = tmem_base, tO = tmem_base + 256, tP = kOwnP ? tO + 2 * HD : tS;
+  constexpr int kPStep = kOwnP ? 64 : 128;
+
+  // Running counters, the same in every role by construction: n = items this CTA has started, g = key tiles loaded over all
+  // items (K and V stages alternate with it), and per stream the tiles it has worked on (S, P and PV).
+  // O needs no second buffer: the first P.V of an item waits for P, which the softmax warps write only after they
+  // have read the previous item's O in its output pass.
+  if (warp < 4) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsFew));
+    if (warp == 0 && kPaged) {
+      // ---------------- TMA producer, paged K/V: one page-sized box per lane ----------------
+      if (lane == 0) {
+        tma_prefetch_desc(&tmK);
+        tma_prefetch_desc(&tmV);
+      }
+      const int page_size = 1 << page_shift;
+      const int nb = kTcTile >> page_shift;  // boxes per 64-column span of a tile (<= 16)
+      const int half = lane / nb, bi = lane - half * nb;
+      const int total = prefix + T;
+      int g = 0;
+      StreamItem w;
+      for (int n = 0; get_item(n, w); ++n) {
+        if (lane == 0) {
+          mbar_wait(q_empty, (n & 1) ^ 1);  // the last S = Q K^T of the previous item has read Q
+          const int tiles = w.end[1] != 0x7fffffff ? 2 : 1;
+          mbar_expect_tx(q_full, tiles * kTileBytes);
+#pragma unroll
+          for (int x = 0; x < 2; ++x)
+#pragma unroll
+            for (int sp = 0; sp < Cfg::kSpans; ++sp)
+              if (x < tiles) tma_load_2d(sQ + x * kTileBytes + sp * kSpanBytes, &tm, q_full, w.h[x] * HD + 64 * sp, w.row_base + w.q0[x]);
+        }
+        for (int t = w.tb; t < w.te; ++t, ++g) {
+          const int st = g % kStages;
+          const uint32_t ph = (g / kStages) & 1;
+          const int tok0 = t * kTcTile + bi * page_size;
+          int row = cache_rows;  // out of bounds: the box is zero-filled
+          if (lane < Cfg::kSpans * nb && tok0 < total)
+            row = (page_table[(size_t)w.b * max_pages + (tok0 >> page_shift)] * KV + w.kvh) << page_shift;
+          const uint32_t dst = (uint32_t)(st * kTileBytes + half * kSpanBytes + bi * page_size * 128);
+          if (lane == 0) {
+            mbar_wait(k_empty + 8 * st, ph ^ 1);
+            mbar_expect_tx(k_full + 8 * st, kTileBytes);
+          }
+          __syncwarp();
+          if (lane < Cfg::kSpans * nb) tma_load_2d(sK + dst, &tmK, k_full + 8 * st, half * 64, row);
+          if (lane == 0) {
+            mbar_wait(v_empty + 8 * st, ph ^ 1);
+            mbar_expect_tx(v_full + 8 * st, kTileBytes);
+          }
+          __syncwarp();
+          if (lane < Cfg::kSpans * nb) tma_load_2d(sV + dst, &tmV, v_full + 8 * st, half * 64, row);
+        }
+      }
+    } else if (warp == 0) {
+      if (lane == 0) {
+        // ---------------- TMA producer ----------------
+        int g = 0;
+        StreamItem w;
+        for (int n = 0; get_item(n, w); ++n) {
+          mbar_wait(q_empty, (n & 1) ^ 1);
+          const int tiles = w.end[1] != 0x7fffffff ? 2 : 1;
+          mbar_expect_tx(q_full, tiles * kTileBytes);
+#pragma unroll
+          for (int x = 0; x < 2; ++x)
+#pragma unroll
+            for (int sp = 0; sp < Cfg::kSpans; ++sp)
+              if (x < tiles) tma_load_2d(sQ + x * kTileBytes + sp * kSpanBytes, &tm, q_full, w.h[x] * HD + 64 * sp, w.row_base + w.q0[x]);
+          for (int t = w.tb; t < w.te; ++t, ++g) {
+            const int st = g % kStages;
+            const uint32_t ph = (g / kStages) & 1;
+            const int krow = w.row_base + t * kTcTile;
+            mbar_wait(k_empty + 8 * st, ph ^ 1);
+            mbar_expect_tx(k_full + 8 * st, kTileBytes);
+#pragma unroll
+            for (int sp = 0; sp < Cfg::kSpans; ++sp)
+              tma_load_2d(sK + st * kTileBytes + sp * kSpanBytes, &tm, k_full + 8 * st, (H + w.kvh) * HD + 64 * sp, krow);
+            mbar_wait(v_empty + 8 * st, ph ^ 1);
+            mbar_expect_tx(v_full + 8 * st, kTileBytes);
+#pragma unroll
+            for (int sp = 0; sp < Cfg::kSpans; ++sp)
+              tma_load_2d(sV + st * kTileBytes + sp * kSpanBytes, &tm, v_full + 8 * st, (H + KV + w.kvh) * HD + 64 * sp, krow);
+          }
+        }
+      }
+    } else if (warp < 3) {
+      // ---------------- MMA issuers, a warp per stream: the whole warp runs the loop (uniform values stay in uniform registers), one
+      // elected lane issues each tcgen05 instruction ----------------
+      const int x = warp - 1;
+      constexpr uint32_t idesc_s = make_idesc_attn(false, kTcTile), idesc_o = make_idesc_attn(true, HD);
+      // operand descriptors: the 14-bit start-address field (bytes >> 4) advances with the k-step, so a k-step is
+      // an add on the low word.  Q/K: 16 elements = 32 B inside a 64-element span, spans kSpanBytes apart;
+      // V (MN-major): 16 tokens = two 8-row groups = 2048 B
+      const uint64_t qdesc = make_smem_desc(sQ + x * kTileBytes);
+      const uint64_t kdesc0 = make_smem_desc(sK), vdesc0 = make_smem_desc_mn(sV);
+      const bool leader = elect_one();
+      const uint32_t myS = tS + x * 128, myO = tO + x * HD, myP = tP + x * kPStep;
+      int g = 0, scores = 0, products = 0;  // key tiles loaded; S and P.V of this stream
+      StreamItem w;
+      for (int n = 0; get_item(n, w); ++n) {
+        const int t0 = x ? w.first[1] : w.first[0], t1 = x ? w.end[1] : w.end[0];
+        auto issue_s = [&](int t) {  // scores against key tile t
+          const int gt = g + t - w.tb, st = gt % kStages;
+          mbar_wait(k_full + 8 * st, (gt / kStages) & 1);
+          // P's own columns: the softmax has the scores of the tile before in registers.  Else its P.V, issued before, has read them.
+          if (kOwnP) mbar_wait(s_empty + 8 * x, (scores & 1) ^ 1);
+          ++scores;
+          tcgen05_fence_after();
+          if (leader) {
+            const uint64_t kdesc = kdesc0 + (uint64_t)(st * (kTileBytes >> 4));
+#pragma unroll
+            for (int kk = 0; kk < HD / kUmmaK; ++kk) {
+              const uint32_t off = ((kk >> 2) * kSpanBytes + (kk & 3) * 32) >> 4;
+              umma_bf16(myS, qdesc + off, kdesc + off, idesc_s, kk > 0 ? 1u : 0u);
+            }
+            umma_commit(s_full + 8 * x);
+            umma_commit(k_empty + 8 * st);
+            if (t == t1 - 1) umma_commit(q_empty);  // Q may be replaced by the next item's
+          }
+          __syncwarp();
+        };
+        auto issue_pv = [&](int t) {  // O += P V of key tile t
+          const int gt = g + t - w.tb, st = gt % kStages;
+          mbar_wait((kOwnP ? p_full : p_half) + 8 * x, products & 1);  // P (or half of it) in tensor memory, O rescaled (or read out)
+          mbar_wait(v_full + 8 * st, (gt / kStages) & 1);
+          // Rows of the last key tile past the context hold whatever follows in memory: the rest of the last cache page,
+          // or the next sequence's rows.  Their probabilities are 0, but 0 x inf is not: zero them before P V.  (Both streams may.)
+          const int tile0 = t * kTcTile, ctx = past + T;
+          int dirty_end = 0;
+          if (ctx < tile0 + kTcTile) {
+            const int page_end = kPaged ? (((ctx - 1) >> page_shift) + 1) << page_shift : 0;
+            dirty_end = kPaged ? min(page_end - tile0, kTcTile) : (w.b + 1) * KV < groups ? kTcTile : 0;
+          }
+          if (dirty_end > ctx - tile0) {
+            // a row is 128 bytes per span whatever the swizzle does inside it: eight lanes a row
+#pragma unroll
+            for (int sp = 0; sp < Cfg::kSpans; ++sp)
+              for (int r = ctx - tile0 + (lane >> 3); r < dirty_end; r += 4)
+                *reinterpret_cast<uint4*>(smem + (sV - sQ) + st * kTileBytes + sp * kSpanBytes + r * 128 + (lane & 7) * 16) =
+                    make_uint4(0u, 0u, 0u, 0u);
+            fence_proxy_async();
+            __syncwarp();
+          }
+          // A = P from tensor memory: k-step = 16 tokens = 8 columns; B = V, 16 tokens further per k-step
+          const uint64_t vdesc = vdesc0 + (uint64_t)(st * (kTileBytes >> 4));
+          const bool more = t > t0;
+          auto steps = [&](int from, int to) {
+            tcgen05_fence_after();
+            if (leader) {
+#pragma unroll
+              for (int kk = from; kk < to; ++kk)
+                umma_bf16_ts(myO, myP + kk * 8, vdesc + (uint64_t)(kk * (2048 >> 4)), idesc_o, (more || kk > 0) ? 1u : 0u);
+            }
+          };
+          if (kOwnP) {
+            steps(0, 8);
+          } else {
+            steps(0, 4);
+            mbar_wait(p_full + 8 * x, products & 1);
+            steps(4, 8);
+          }
+          if (leader) {
+            umma_commit(pv_done + 8 * x);
+            umma_commit(v_empty + 8 * st);
+          }
+          __syncwarp();
+          ++products;
+        };
+        mbar_wait(q_full, n & 1);
+        // A tile that only the other stream works on.  Waiting for it keeps the two arrivals of a phase those of the two streams.
+        auto skip = [&](int t) {
+          const int gt = g + t - w.tb, st = gt % kStages;
+          mbar_wait(k_full + 8 * st, (gt / kStages) & 1);
+          mbar_wait(v_full + 8 * st, (gt / kStages) & 1);
+          if (lane == 0) {
+            mbar_arrive(k_empty + 8 * st);
+            mbar_arrive(v_empty + 8 * st);
+          }
+        };
+        for (int t = w.tb; t < w.te && t < t0; ++t) skip(t);
+        if (t0 < t1) {
+          issue_s(t0);
+          for (int t = t0 + 1; t < t1; ++t) {
+            if (kOwnP) issue_s(t);
+            issue_pv(t - 1);
+            if (!kOwnP) issue_s(t);
+          }
+          issue_pv(t1 - 1);
+        } else if (lane == 0) {
+          mbar_arrive(q_empty);
+        }
+        for (int t = max(w.tb, t1); t < w.te; ++t) skip(t);
+        g += w.te - w.tb;
+      }
+    }
+  } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsMany));
+    // ---------------- softmax + output pass: four warps per stream, a thread per query row ----------------
+    const int x = (warp - 4) >> 2, quad = warp & 3;
+    const int row = quad * 32 + lane;  // TMEM lane
+    const uint32_t lane_off = (uint32_t)(quad * 32) << 16;
+    const uint32_t myS = tS + x * 128 + lane_off, myO = tO + x * HD + lane_off, myP = tP + x * kPStep + lane_off;
+    int g = 0;                                              // tiles of this stream so far
+    // Head size 128: the exponentials of the two streams take turns on a scheduler's special function unit, so that one's maxima, loads,
+    // stores and MMAs run beside the other's exponentials.  Left alone both fall into step and wait at the same time (4 096 tokens of
+    // 32 heads: 157 us, 124 in turns).  At head size 64 the MMAs are shorter and nothing waits for them: 358 us for 8 192 tokens, 401.
+    auto take_turn = [&] {
+      if (!kOwnP) asm volatile("bar.sync %0, 64;" ::"r"(1 + 4 * x + quad) : "memory");
+    };
+    auto pass_turn = [&] {
+      if (!kOwnP) asm volatile("bar.arrive %0, 64;" ::"r"(1 + 4 * (x ^ 1) + quad) : "memory");
+    };
+    if (x == 1) pass_turn();
+    StreamItem w;
+    for (int n = 0; get_item(n, w); ++n) {
+      const int q0 = x ? w.q0[1] : w.q0[0], h = x ? w.h[1] : w.h[0];
+      const int qrel = q0 + row;                        // row of the chunk / prompt
+      const int qpos0 = past + q0, qrow = qpos0 + row;  // absolute position in the sequence
+      float m_run = -INFINITY, l_run = 0.f;
+      const int t0 = x ? w.first[1] : w.first[0], t1 = x ? w.end[1] : w.end[0];
+      for (int t = w.tb; t < w.te; ++t) {
+        if (t < t0 || t >= t1) {
+          take_turn();
+          pass_turn();
+          continue;
+        }
+        mbar_wait(s_full + 8 * x, g & 1);
+        tcgen05_fence_after();
+        uint32_t r[4][32];  // all pieces requested before the one wait: one TMEM round trip per tile
+#pragma unroll
+        for (int c = 0; c < 4; ++c) tmem_ld_32x32(myS + 32 * c, r[c]);
+        tmem_ld_wait();
+        if (kOwnP) {
+          tcgen05_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(s_empty + 8 * x);
+        }
+        if ((t * kTcTile + kTcTile - 1 > qpos0) || (window > 0 && t * kTcTile < qpos0 + kTcTile - window + 1)) {
+#pragma unroll
+          for (int i = 0; i < 128; ++i) {
+            const int tok = t * kTcTile + i;
+            if (tok > qrow || (window > 0 && tok <= qrow - window)) r[i >> 5][i & 31] = 0xff800000u;  // -inf
+          }
+        }
+        float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};  // four chains: one long chain is latency-bound
+#pragma unroll
+        for (int i = 0; i < 128; i += 8)
+#pragma unroll
+          for (int v = 0; v < 4; ++v)
+            mx4[v] = fmaxf(mx4[v], fmaxf(__uint_as_float(r[i >> 5][(i & 31) + v]), __uint_as_float(r[i >> 5][(i & 31) + v + 4])));
+        const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+        // Lazy reference maximum: the exponentials only need a COMMON reference per row, not the true running
+        // maximum, so m_run moves only when the tile's maximum exceeds it by more than 2^kLazyLog2 (p stays
+        // <= 256, exact in bf16's range; sums are fp32).  Then corr == 1 on almost every tile and the
+        // TMEM round trip that rescales O below is skipped.  (-inf - -inf = NaN compares false: a fully
+        // masked tile leaves m_run alone.)
+        constexpr float kLazyLog2 = 8.f;
+        const float m_new = ((mx - m_run) * scale_log2 > kLazyLog2) ? mx : m_run;
+        const float m_use = (m_new == -INFINITY) ? 0.f : m_new;
+        const float corr = ex2_ftz((m_run - m_use) * scale_log2);
+        m_run = m_new;
+        take_turn();
+        // p = 2^(s*scale - m*scale); P (bf16, two tokens per 32-bit column) -> tensor memory
+        const float2 sc2 = make_float2(scale_log2, scale_log2), ms2 = make_float2(-m_use * scale_log2, -m_use * scale_log2);
+        float2 rs[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+        uint32_t pk[2][16];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            float2 e = fma2(make_float2(__uint_as_float(r[c][2 * i]), __uint_as_float(r[c][2 * i + 1])), sc2, ms2);
+            e.x = ex2_ftz(e.x);
+            e.y = ex2_ftz(e.y);
+            rs[i & 1] = add2(rs[i & 1], e);
+            pk[c & 1][i] = pack_bf16(e.x, e.y);
+          }
+          if (c == 0) continue;
+          if (c == 1) {
+            // P's own columns were read by the P.V of the tile before; O is rescaled behind it too.  (Where P takes the scores' columns, that
+            // P.V was issued before these scores, and they are here.)
+            if (kOwnP && t > t0) {
+              mbar_wait(pv_done + 8 * x, (g - 1) & 1);
+              tcgen05_fence_after();
+            }
+            // (skipped when no row of this warp moved its maximum: corr == 1 exactly, nothing to do)
+            if (t > t0 && !__all_sync(0xffffffffu, corr == 1.f)) {
+#pragma unroll
+              for (int c = 0; c < HD / 16; ++c) {
+                uint32_t o[16];
+                tmem_ld_32x16(myO + 16 * c, o);
+                tmem_ld_wait();
+#pragma unroll
+                for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * corr);
+                tmem_st_32x16(myO + 16 * c, o);
+              }
+            }
+            tmem_st_32x16(myP, pk[0]);
+          }
+          tmem_st_32x16(myP + 16 * c, pk[c & 1]);
+          if (!kOwnP && c == 1) {
+            tmem_st_wait();  // half of P, and O, are in tensor memory before the MMA warp is told
+            tcgen05_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(p_half + 8 * x);
+          }
+        }
+        pass_turn();
+        l_run = l_run * corr + ((rs[0].x + rs[0].y) + (rs[1].x + rs[1].y));
+        tmem_st_wait();
+        tcgen05_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(p_full + 8 * x);
+        ++g;
+      }
+      // ---- output pass: O / l -> bf16 ----
+      if (t1 > t0) mbar_wait(pv_done + 8 * x, (g - 1) & 1);  // the stream's last P.V
+      tcgen05_fence_after();
+      bf16* dst = out + ((size_t)(w.row_base + qrel)) * ((size_t)H * HD) + (size_t)h * HD;
+      if (t1 > t0) {
+        const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
+#pragma unroll
+        for (int c = 0; c < HD / 32; ++c) {
+          uint32_t o[32];
+          tmem_ld_32x32(myO + 32 * c, o);
+          tmem_ld_wait();
+          if (qrel < T) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              float v[8];
+#pragma unroll
+              for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(o[q * 8 + i]) * inv;
+              st_16B(dst + 32 * c + q * 8, pack8(v));
+            }
+          }
+        }
+        tcgen05_fence_before();  // O has been read: the next item's first P.V (after its P) may overwrite it
+      }
+    }
+    if (x == 0) take_turn();  // the last one passed
+  }
+  __syncthreads();
+  if (warp == 1) {
+    tcgen05_fence_after();
+    tmem_dealloc(tmem_base, 512);
+  }
+}
+
+
+template <int HD, bool kPaged>
+static int launch_streams(const CUtensorMap& tm, const CUtensorMap& tmK, const CUtensorMap& tmV, void* out, int B, int T, int H, int KV,
+                          float scale, int window, const int32_t* page_table, int max_pages, int page_shift, int prefix, int cache_rows,
+                          cudaStream_t s) {
+  static PerDeviceOnce once;
+  DLI_ONCE_PER_DEVICE(once, dev,
+                      DLI_CUDA_CALL(cudaFuncSetAttribute(attn_streams_kernel<HD, kPaged>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                         StreamCfg<HD>::kSmem)));
+  const int n_qtiles = (T + kTcTile - 1) / kTcTile, units = n_qtiles * (H / KV);  // query tiles that share K and V
+  const int items = (units + 1) / 2 * KV * B;
+  const int sms = sm_count_cached();
+  DLI_LAUNCH("attn_streams_kernel", (attn_streams_kernel<HD, kPaged>), dim3(items < sms ? items : sms), dim3(kStreamThreads),
+             (size_t)StreamCfg<HD>::kSmem, s, tm, tmK, tmV, (bf16*)out, T, H, KV, scale * 1.4426950408889634f, window, page_table,
+             max_pages, page_shift, prefix, cache_rows, items, B * KV, n_qtiles);
+  return DLI_OK;
+}
+
+int launch_attn_streams(bool paged, int hd, const CUtensorMap& tm, const CUtensorMap& tmK, const CUtensorMap& tmV, void* out, int B, int T,
+                        int H, int KV, float scale, int window, const int32_t* page_table, int max_pages, int page_shift, int prefix,
+                        int cache_rows, cudaStream_t s) {
+  const auto launch = hd == 64 ? (paged ? launch_streams<64, true> : launch_streams<64, false>)
+                               : (paged ? launch_streams<128, true> : launch_streams<128, false>);
+  return launch(tm, tmK, tmV, out, B, T, H, KV, scale, window, page_table, max_pages, page_shift, prefix, cache_rows, s);
+}
+
+}  // namespace dli

@@ -14,7 +14,7 @@
 // works on the next scores while the SFUs exponentiate the current ones; P/V of tile j are
 // multiplied as soon as P(j) is in tensor memory and (rarely, see the lazy maximum) O has been rescaled.
 // The T x T score matrix never leaves the SM.  FLOPs per head: 4 * T^2/2 * hd (causal).
-#include "tcgen05_utils.cuh"
+#include "attn_tc.cuh"
 
 namespace dli {
 
@@ -23,9 +23,6 @@ constexpr int kSmWarps = 4 * kRowThreads;      // softmax warps: kRowThreads per
 constexpr int kSmCols = 128 / kRowThreads;     // score columns per softmax thread
 constexpr int kTcThreads = 64 + 32 * kSmWarps;  // TMA warp + MMA warp + softmax warps
 static_assert(kRowThreads == 4, "the P store writes 16 packed columns per thread; the TMEM map assumes 4 x 32 columns");
-constexpr int kTcTile = 128;      // query rows per item and tokens per KV tile
-constexpr int kSpanBytes = 128 * 64 * 2;  // one [128 rows x 64 elements] swizzled sub-tile: 16 KB
-
 template <int HD>
 struct TcCfg {
   static_assert(HD == 64 || HD == 128, "whole 64-element swizzle spans");
@@ -37,49 +34,11 @@ struct TcCfg {
   static constexpr int kSmem = 5 * kTileBytes + 1024 + 256 + 3 * kRowThreads * 128 * 4;
 };
 
-__device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t (&r)[32]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-      "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
-      "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};" ::"r"(taddr),
-      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
-      "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]),
-      "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]),
-      "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
-      : "memory");
-}
-__device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-      "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr),
-      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
-      "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-      : "memory");
-}
 // a thread's output columns: 32 (head size 128) or 16 (64)
 __device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&r)[32]) { tmem_ld_32x32(taddr, r); }
 __device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&r)[16]) { tmem_ld_32x16(taddr, r); }
 __device__ __forceinline__ void tmem_st_cols(uint32_t taddr, const uint32_t (&r)[32]) { tmem_st_32x32(taddr, r); }
 __device__ __forceinline__ void tmem_st_cols(uint32_t taddr, const uint32_t (&r)[16]) { tmem_st_32x16(taddr, r); }
-__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-
-// MN-major SWIZZLE_128B operand (V as B: N = hd contiguous, K = tokens): 64-element MN groups are
-// LBO apart (the two hd halves = two TMA boxes, 16 KB), 8-row K groups are SBO = 1024 B apart.
-__device__ __forceinline__ uint64_t make_smem_desc_mn(uint32_t saddr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((saddr & 0x3ffffu) >> 4);
-  d |= (uint64_t)(kSpanBytes >> 4) << 16;  // leading (MN) byte offset
-  d |= (uint64_t)64 << 32;                 // stride (K) byte offset = 1024 B
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)2 << 61;
-  return d;
-}
-// D=f32, A=bf16 K-major, B=bf16 (K-major or MN-major), M=128, N=n
-__host__ __device__ constexpr uint32_t make_idesc_attn(bool b_mn_major, int n) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((b_mn_major ? 1u : 0u) << 16) | ((uint32_t)(n >> 3) << 17) |
-         ((uint32_t)(128 >> 4) << 24);
-}
-
 // One work item = one 128-row query tile of one head of one sequence.  The kernel is PERSISTENT: a CTA per SM walks a
 // static list of items, so the TMEM allocation, the barrier set-up and the launch of a CTA are paid once per SM and
 // the output pass of an item (O from TMEM, normalise, store) runs while the producer loads the next item's Q, K, V and
@@ -480,6 +439,8 @@ static int launch_tc(const void* qkv, void* out, int B, int T, int H, int KV, fl
   CUtensorMap tm;
   const int rc = make_tmap(&tm, qkv, B * T, (H + 2 * KV) * HD, 128);
   if (rc != DLI_OK) return rc;
+  if (attn_streams_faster(B, T, 0, H, KV, HD, window, false))
+    return launch_attn_streams(false, HD, tm, tm, tm, out, B, T, H, KV, scale, window, nullptr, 0, 0, 0, 0, s);
   const int n_qtiles = (T + kTcTile - 1) / kTcTile;
   const long long n_items = (long long)n_qtiles * H * B;
   dim3 grid((unsigned)(n_items < sm_count_cached() ? n_items : sm_count_cached()));  // persistent: one CTA per SM
@@ -515,6 +476,8 @@ static int launch_tc_paged(const void* qkv, void* out, const void* k_cache, cons
   if (rc != DLI_OK) return rc;
   int shift = 0;
   while ((1 << shift) < page_size) ++shift;
+  if (attn_streams_faster(B, T, prefix, H, KV, HD, window, true))
+    return launch_attn_streams(true, HD, tm, tmK, tmV, out, B, T, H, KV, scale, window, page_table, max_pages, shift, prefix, (int)rows, s);
   const int n_qtiles = (T + kTcTile - 1) / kTcTile;
   const long long n_items = (long long)n_qtiles * H * B;
   dim3 grid((unsigned)(n_items < sm_count_cached() ? n_items : sm_count_cached()));

@@ -1,0 +1,56 @@
+// What the two causal prefill kernels on tcgen05 share (attn_prefill_tc.cu, attn_prefill_streams.cu).
+#pragma once
+#include "tcgen05_utils.cuh"
+
+namespace dli {
+
+constexpr int kTcTile = 128;      // query rows per item and tokens per KV tile
+constexpr int kSpanBytes = 128 * 64 * 2;  // one [128 rows x 64 elements] swizzled sub-tile: 16 KB
+
+__device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t (&r)[32]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+      "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
+      "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};" ::"r"(taddr),
+      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+      "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]),
+      "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]),
+      "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+      "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr),
+      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+      "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+// MN-major SWIZZLE_128B operand (V as B: N = hd contiguous, K = tokens): 64-element MN groups are
+// LBO apart (the two hd halves = two TMA boxes, 16 KB), 8-row K groups are SBO = 1024 B apart.
+__device__ __forceinline__ uint64_t make_smem_desc_mn(uint32_t saddr) {
+  uint64_t d = 0;
+  d |= (uint64_t)((saddr & 0x3ffffu) >> 4);
+  d |= (uint64_t)(kSpanBytes >> 4) << 16;  // leading (MN) byte offset
+  d |= (uint64_t)64 << 32;                 // stride (K) byte offset = 1024 B
+  d |= (uint64_t)1 << 46;
+  d |= (uint64_t)2 << 61;
+  return d;
+}
+// D=f32, A=bf16 K-major, B=bf16 (K-major or MN-major), M=128, N=n
+__host__ __device__ constexpr uint32_t make_idesc_attn(bool b_mn_major, int n) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((b_mn_major ? 1u : 0u) << 16) | ((uint32_t)(n >> 3) << 17) |
+         ((uint32_t)(128 >> 4) << 24);
+}
+
+// The form with two streams per CTA (attn_prefill_streams.cu); tmK, tmV and what follows them: the paged cache, or tm, tm, null, 0 ...
+int launch_attn_streams(bool paged, int hd, const CUtensorMap& tm, const CUtensorMap& tmK, const CUtensorMap& tmV, void* out, int B, int T,
+                        int H, int KV, float scale, int window, const int32_t* page_table, int max_pages, int page_shift, int prefix,
+                        int cache_rows, cudaStream_t s);
+
+// The rule between the two, beside the others in attn_prefill.cu.
+bool attn_streams_faster(int B, int T, int prefix, int H, int KV, int hd, int window, bool paged);
+
+}  // namespace dli
