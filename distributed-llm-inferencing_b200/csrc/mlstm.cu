@@ -754,6 +754,123 @@ mlstm_out_kernel(const float* __restrict__ o, const E* __restrict__ proj, const 
   }
 }
 
+// Decode rows: the scan and mlstm_out in one kernel.  The slices of a head (32 columns of V each, at most 8) are a thread-block CLUSTER:
+// each works out its columns, and the head's mean square is added from all of them over distributed shared memory.  Both kernels
+// were bound by latency (3 MB of state for 3 sequences of 8 heads of 128 x 256): the scan took its state through shared memory, a few
+// loads at a time, and the second kernel waited for the first one's end.  Here a thread asks for all of its state at once and keeps it
+// in registers.  Every sum has the order of the two kernels, so the bits are theirs.
+// 3 rows, 8 heads of 128 x 256 behind a projection: 8.3 + 6.6 -> 5.8 us.
+// All slices have read n and m before one of them writes them, whatever the grid (the cluster barrier of the first row).
+template <typename E, int I>  // I: rows of the state per thread, D <= 8 I
+__global__ void __launch_bounds__(kMlThreads)
+mlstm_decode_kernel(const E* __restrict__ proj, const float* __restrict__ w, E* __restrict__ y, int g_off, float eps, MlstmArgs a) {
+  __shared__ float qs[kMlGroups * I], ks[kMlGroups * I], red[kMlThreads], rnq[kMlGroups], os[2][kMlCols];
+  const int h = blockIdx.y, slice = blockIdx.x, slices = gridDim.x;
+  const int tid = threadIdx.x, col = tid % kMlCols, grp = tid / kMlCols, c = slice * kMlCols + col;
+  const bool col_ok = c < a.V;
+  const float wc = col_ok ? w[h * a.V + c] : 0.f, ib = a.i_bias ? a.i_bias[h] : 0.f, fb = a.f_bias ? a.f_bias[h] : 0.f;
+  pdl_wait();
+  pdl_trigger();
+  const int4 e = reinterpret_cast<const int4*>(a.ent)[blockIdx.z];  // slot, row0, n, start
+  const bool fresh = e.w == 0;
+  float* Sg = a.S + ((size_t)e.x * a.H + h) * a.D * a.V;
+  float* ng = a.n + ((size_t)e.x * a.H + h) * a.D;
+  float* mg = a.m + (size_t)e.x * a.H + h;
+  float S[I], ns[I];  // rows grp, grp + 8, ...; n: the threads of column 0
+#pragma unroll
+  for (int i = 0; i < I; ++i) {
+    const int d = grp + kMlGroups * i;
+    S[i] = d < a.D && !fresh && col_ok ? Sg[(size_t)d * a.V + c] : 0.f;
+    ns[i] = d < a.D && !fresh && col == 0 ? ng[d] : 0.f;
+  }
+  float m = fresh ? 0.f : *mg;
+  const float qscale = 1.f / sqrtf((float)a.D);
+  for (int t = 0; t < e.z; ++t) {
+    const int row = e.y + t;
+    const E* pr = proj + (size_t)row * a.ldp;
+    for (int d = tid; d < a.D; d += kMlThreads) {
+      qs[d] = m_to_f(pr[a.q_off + h * a.D + d]) * qscale;
+      ks[d] = m_to_f(pr[a.k_off + h * a.D + d]);
+    }
+    const float v = col_ok ? m_to_f(pr[a.v_off + h * a.V + c]) : 0.f;
+    const float gate = col_ok && grp == 0 ? m_to_f(pr[g_off + h * a.V + c]) : 0.f;
+    const float ig = soft_cap(m_to_f(pr[a.i_off + h]) + ib, a.cap);
+    const float fg = log_sigmoid(soft_cap(m_to_f(pr[a.f_off + h]) + fb, a.cap));
+    const float m_new = fmaxf(fg + m, ig);
+    const float da = expf(fg + m - m_new), db = expf(ig - m_new);
+    __syncthreads();
+    float num = 0.f, nq = 0.f;
+#pragma unroll
+    for (int i = 0; i < I; ++i) {
+      const int d = grp + kMlGroups * i;
+      if (d < a.D) {
+        const float kd = ks[d], qd = qs[d];
+        const float s = da * S[i] + db * kd * v;
+        S[i] = s;
+        num = fmaf(s, qd, num);
+        const float nn = da * ns[i] + db * kd;
+        ns[i] = nn;
+        nq = fmaf(nn, qd, nq);
+      }
+    }
+    red[grp * kMlCols + col] = num;
+    if (col == 0) rnq[grp] = nq;
+    __syncthreads();
+    float mine = 0.f;
+    if (grp == 0) {
+      float s = 0.f, q = 0.f;
+#pragma unroll
+      for (int g = 0; g < kMlGroups; ++g) { s += red[g * kMlCols + col]; q += rnq[g]; }
+      const float den = fmaxf(fabsf(q), expf(-m_new)) + 1e-6f;
+      mine = col_ok ? s / den : 0.f;
+      os[t & 1][col] = mine;
+    }
+    m = m_new;
+    // the outputs of all slices are there; the place of the row before last, read before this barrier, is free again
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (grp == 0) {
+      const uint32_t at = (uint32_t)__cvta_generic_to_shared(&os[t & 1][col]);
+      float ss = 0.f, v8[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        v8[k] = 0.f;
+        if (k < slices) {
+          uint32_t far;
+          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(far) : "r"(at), "r"(k));
+          asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v8[k]) : "r"(far) : "memory");
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        if (k * kMlCols + col < a.V) ss += v8[k] * v8[k];
+      ss = warp_sum(ss);
+      const float r = 1.f / sqrtf(ss / a.V + eps);
+      if (col_ok) y[((size_t)row * a.H + h) * a.V + c] = m_from_f<E>(mine * r * wc * (1.f / (1.f + expf(-gate))));
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < I; ++i) {
+    const int d = grp + kMlGroups * i;
+    if (d < a.D && col_ok) Sg[(size_t)d * a.V + c] = S[i];
+    if (d < a.D && slice == 0 && col == 0 && e.z > 0) ng[d] = ns[i];
+  }
+  if (slice == 0 && tid == 0 && e.z > 0) *mg = m;
+  // a slice's shared memory lives until all have read it
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+template <typename E>
+static int launch_mlstm_decode(const void* proj, const float* out_w, void* y, int n_ent, int g_off, float eps, const MlstmArgs& a,
+                               cudaStream_t s) {
+  const int slices = (a.V + kMlCols - 1) / kMlCols;
+  const auto kernel = a.D <= 64 ? mlstm_decode_kernel<E, 8> : a.D <= 128 ? mlstm_decode_kernel<E, 16> : mlstm_decode_kernel<E, 32>;
+  const cudaError_t err = launch_kernel_cluster(kernel, dim3(slices, a.H, n_ent), dim3(kMlThreads), (size_t)0, s, (unsigned)slices,
+                                                (const E*)proj, out_w, (E*)y, g_off, eps, a);
+  return err == cudaSuccess ? DLI_OK : fail(DLI_ERR_CUDA, "mlstm_decode: %s", cudaGetErrorString(err));
+}
+
 }  // namespace dli
 
 using namespace dli;
@@ -777,6 +894,10 @@ int dli_mlstm_ragged(const void* proj, float* o_scratch, void* y, const int32_t*
   const size_t csmem = mlstm_chunk_smem(D);
   const bool chunked = blocked && csmem <= 220 * 1024;  // larger key sizes: the token-by-token kernel
   const dim3 cgrid(n_ent, H, (V + kMcCols - 1) / kMcCols);
+  // decode (one row an entry), of sizes whose slices are one portable cluster and whose state fits the registers
+  if (!chunked && rows == n_ent && V <= 8 * kMlCols && D <= 256 && H <= 65535 && n_ent <= 65535)
+    return dt == 0 ? launch_mlstm_decode<bf16>(proj, out_w, y, n_ent, g_off, eps, a, s)
+                   : launch_mlstm_decode<float>(proj, out_w, y, n_ent, g_off, eps, a, s);
   if (dt == 0) {
     static PerDeviceOnce once;
     DLI_ONCE_PER_DEVICE(once, dev, DLI_CUDA_CALL(cudaFuncSetAttribute(mlstm_scan_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));

@@ -1,0 +1,40 @@
+"""Decode rows of the matrix-memory recurrence in one kernel: the bits (outputs and states) of the two kernels that walk entries of any
+number of rows, which one more entry without rows selects."""
+import pytest
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("D,V", [(8, 32), (64, 40), (72, 224), (128, 256), (200, 1), (256, 256), (128, 264), (264, 64)])
+@pytest.mark.parametrize("rows,H,cap", [(1, 8, 15.0), (5, 3, 0.0)])
+def test_same_bits_as_any_number_of_rows(cuda, D, V, rows, H, cap, dt):
+    from dli_b200 import ops
+
+    before = ops.set_pdl(True)
+    g = torch.Generator(device="cuda").manual_seed(D * V + rows)
+    rnd = lambda *s: torch.randn(*s, device=cuda, generator=g)  # noqa: E731
+    slots, ld = rows + 3, H * (2 * D + 2 * V + 2) + 5
+    q, k, v, gate = 0, H * D, 2 * H * D, 2 * H * D + H * V
+    i_off, f_off = gate + H * V, gate + H * V + H
+    ib, fb, w = rnd(H), rnd(H) + 2, 1 + 0.2 * rnd(H * V)
+    state = [rnd(slots, H, D, V), rnd(slots, H, D), rnd(slots, H)]
+    slot = torch.randperm(slots, device=cuda, generator=g).int()
+    got = [[t.clone() for t in state] for _ in range(2)]
+    outs = [[], []]
+    for step in range(3):
+        proj = rnd(rows, ld).to(dt)
+        ent = torch.tensor([[int(slot[r]), r, 1, (0 if r % 2 else 7) + step] for r in range(rows)] + [[int(slot[rows]), 0, 0, 5]],
+                           device=cuda, dtype=torch.int32)
+        torch.cuda.synchronize()
+        for at, n in ((0, rows), (1, rows + 1)):
+            out = torch.empty(rows, H * V, device=cuda, dtype=dt)
+            S, nn, m = got[at]
+            ops.mlstm_ragged(proj, torch.empty(rows, H * V, device=cuda), out, ent[:n].contiguous().view(-1), H, D, V, q, k, v, i_off,
+                             f_off, gate, ib, fb, cap, w, 1e-6, S, nn, m)
+            outs[at].append(out)
+    torch.cuda.synchronize()
+    ops.set_pdl(before)
+    assert all(torch.equal(a, b) for a, b in zip(*outs)) and torch.isfinite(outs[0][-1].float()).all()
+    assert all(torch.equal(a, b) for a, b in zip(*got))
