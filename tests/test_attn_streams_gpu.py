@@ -2,6 +2,10 @@
 
 Bound per output: probabilities are rounded to bf16 (8 bits: 2^-8 relative each, the sum is of the unrounded ones), the output once more; the
 fp32 scores move a probability by less than 2e-4 of itself."""
+import os
+import subprocess
+import sys
+
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -9,13 +13,45 @@ torch = pytest.importorskip("torch")
 BF = torch.bfloat16
 
 
-def _kernels(f):
-    f()
+PROMPTS = [
+    (1, 2048, 32, 8, 0),      # pairs of heads
+    (1, 2177, 32, 32, 0),     # pairs of query tiles of one head, 18 tiles, one row in the last
+    (1, 4097, 14, 2, 0),      # groups of 7: both kinds, 33 tiles: the last one alone
+    (3, 1500, 32, 8, 0),      # rows behind a sequence are the next one's
+    (1, 4000, 32, 8, 1000),   # windows: key tiles that only one of the two needs
+    (1, 4224, 32, 32, 900),
+]
+CHUNKS = [(1, 1024, 3072, 32, 8, 16, 0), (2, 907, 1500, 32, 8, 8, 0), (4, 515, 1021, 32, 4, 128, 0), (2, 1025, 2047, 14, 2, 32, 0),
+          (1, 2048, 2048, 32, 32, 16, 1100)]
+# in a process of its own: a profile taken here would be one of several of a test run
+ROUTE = """
+import torch
+from test_attn_streams_gpu import CHUNKS, PROMPTS
+from dli_b200 import ops
+z = lambda *s: torch.zeros(*s, device="cuda", dtype=torch.bfloat16)
+with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA], acc_events=True) as p:
+    for hd in (64, 128):
+        for B, T, H, KV, w in PROMPTS:
+            ops.attn_prefill(z(B * T, (H + 2 * KV) * hd), z(B * T, H * hd), B, T, H, KV, hd, 1.0, w)
+        for B, T, prefix, H, KV, page, w in CHUNKS:
+            n = (prefix + T + page - 1) // page
+            cache, table = z(B * n, KV, page, hd), torch.arange(B * n, device="cuda", dtype=torch.int32).view(B, n)
+            ops.attn_prefill_paged(z(B * T, (H + 2 * KV) * hd), z(B * T, H * hd), cache, cache, table, B, T, prefix, H, KV, hd, 1.0, w)
     torch.cuda.synchronize()
-    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as p:
-        f()
-        torch.cuda.synchronize()
-    return " ".join(e.name for e in p.events())
+print("streams", sum("attn_streams_kernel" in e.name for e in p.events()), "of", 2 * (len(PROMPTS) + len(CHUNKS)))
+"""
+
+
+def test_the_rule_takes_these_sizes(cuda):
+    from dli_b200 import ops
+
+    if ops.sm_count() != 148:
+        pytest.skip("the rule counts SMs")
+    here = os.path.dirname(os.path.abspath(__file__))
+    env = dict(os.environ, PYTHONPATH=os.pathsep.join([here, os.path.dirname(here), os.environ.get("PYTHONPATH", "")]))
+    out = subprocess.run([sys.executable, "-c", ROUTE], env=env, capture_output=True, text=True, timeout=300)
+    n = 2 * (len(PROMPTS) + len(CHUNKS))
+    assert f"streams {n} of {n}" in out.stdout, out.stdout + out.stderr
 
 
 def _check(out, q, k, v, rows, pos, window, H, KV):
@@ -35,14 +71,7 @@ def _rows(T):
 
 
 @pytest.mark.parametrize("hd", [64, 128])
-@pytest.mark.parametrize("B,T,H,KV,window", [
-    (1, 2048, 32, 8, 0),      # pairs of heads
-    (1, 2177, 32, 32, 0),     # pairs of query tiles of one head, 18 tiles, one row in the last
-    (1, 4097, 14, 2, 0),      # groups of 7: both kinds, 33 tiles: the last one alone
-    (3, 1500, 32, 8, 0),      # rows behind a sequence are the next one's
-    (1, 4000, 32, 8, 1000),   # windows: key tiles that only one of the two needs
-    (1, 4224, 32, 32, 900),
-])
+@pytest.mark.parametrize("B,T,H,KV,window", PROMPTS)
 def test_prompt(cuda, hd, B, T, H, KV, window):
     from dli_b200 import ops
 
@@ -53,8 +82,6 @@ def test_prompt(cuda, hd, B, T, H, KV, window):
     x[-1, T // 2:T // 2 + 3, H] *= 4
     out = torch.empty(B * T, H * hd, device=cuda, dtype=BF)
     run = lambda: ops.attn_prefill(qkv, out, B, T, H, KV, hd, hd ** -0.5, window)  # noqa: E731
-    if ops.sm_count() == 148:
-        assert "attn_streams_kernel" in _kernels(run)
     run()
     first = out.clone()
     run()
@@ -70,9 +97,7 @@ def test_prompt(cuda, hd, B, T, H, KV, window):
 
 
 @pytest.mark.parametrize("hd", [64, 128])
-@pytest.mark.parametrize("B,T,prefix,H,KV,page,window", [
-    (1, 1024, 3072, 32, 8, 16, 0), (2, 907, 1500, 32, 8, 8, 0), (4, 515, 1021, 32, 4, 128, 0), (2, 1025, 2047, 14, 2, 32, 0),
-    (1, 2048, 2048, 32, 32, 16, 1100)])
+@pytest.mark.parametrize("B,T,prefix,H,KV,page,window", CHUNKS)
 def test_chunk(cuda, hd, B, T, prefix, H, KV, page, window):
     from dli_b200 import ops
 
@@ -88,8 +113,6 @@ def test_chunk(cuda, hd, B, T, prefix, H, KV, page, window):
     qkv = torch.randn(B * T, (H + 2 * KV) * hd, device=cuda, generator=g).to(BF)
     out = torch.empty(B * T, H * hd, device=cuda, dtype=BF)
     run = lambda: ops.attn_prefill_paged(qkv, out, kc, vc, table, B, T, prefix, H, KV, hd, hd ** -0.5, window)  # noqa: E731
-    if ops.sm_count() == 148:
-        assert "attn_streams_kernel" in _kernels(run)
     run()
     for b in {0, B - 1}:
         rows = _rows(T)
