@@ -387,7 +387,7 @@ attn_ragged_kernel(const float* __restrict__ qbuf, const E* __restrict__ kc, con
     }
   }
   __syncthreads();
-  if constexpr (kCluster) {
+  if (kCluster) {
     __shared__ float wz[kAttnMaxCluster], lz[kAttnMaxCluster];
     for (int d = tid; d < a.V; d += kAttnThreads) {  // this CTA's sums, where its first key group's were
       float u = 0.f;
@@ -967,7 +967,7 @@ static int attn_wide_clusters(int* wide) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(kAttnMaxCluster, 64, 64);
     cfg.blockDim = dim3(kAttnThreads);
-    cfg.dynamicSmemBytes = 47 * 1024;
+    cfg.dynamicSmemBytes = 48 * 1024;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = kAttnMaxCluster;
@@ -1055,8 +1055,7 @@ int dli_attn_ragged(const float* qbuf, const void* k_cache, const void* v_cache,
                        : launch_shared_kv<float, 2>(qbuf, k_cache, v_cache, out, rows, a, s);
     if (rc != DLI_OK) return rc;
   } else {
-    constexpr size_t kFixed = 2 * kAttnMaxCluster * sizeof(float);  // shared memory of the cluster form beside `smem`
-    if (splits > 1 && splits <= kAttnMaxCluster && rows <= 65535 && H <= 65535 && smem + kFixed <= 48 * 1024) {
+    if (splits > 1 && splits <= kAttnMaxCluster && rows <= 65535 && H <= 65535) {
       int wide = 0;
       const int rc = attn_wide_clusters(&wide);
       if (rc != DLI_OK) return rc;
