@@ -238,26 +238,9 @@ __host__ __device__ inline int attn_value_groups(int V, int ldv) {
 }
 constexpr int kAttnMaxVPerThread = 4;  // V <= 512
 
-constexpr int kAttnMaxCluster = 16;  // key splits that may be one cluster (above 8: not portable, asked for)
-__device__ __forceinline__ void attn_cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ float attn_peer(const float* mine, int rank) {  // what a CTA of the cluster has at the same place
-  uint32_t far;
-  float v;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(far) : "r"((uint32_t)__cvta_generic_to_shared(mine)), "r"(rank));
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(far) : "memory");
-  return v;
-}
-
-// One CTA per (row, query head) and key split.  Keys in tiles of 128: one score per thread, a block-wide running maximum,
+// One CTA per (row, query head).  Keys in tiles of 128: one score per thread, a block-wide running maximum,
 // then the weighted value sum with the threads across the value dimensions (V < 128: several key groups).
-// kCluster: the splits of a (row, head) are a thread-block cluster (grid.x) and add their partial sums over distributed shared memory,
-// each for its share of the value dimensions, in the order and so with the bits of attn_ragged_merge_kernel below, which
-// is bound by its launch, two dependent loads and its end.  12 splits of 3 rows of 16 heads behind a projection, us:
-// 7.5 + 4.1 -> 7.2.
-template <typename E, bool kCluster>
+template <typename E>
 __global__ void __launch_bounds__(kAttnThreads)
 attn_ragged_kernel(const float* __restrict__ qbuf, const E* __restrict__ kc, const E* __restrict__ vc,
                    const E* __restrict__ proj, E* __restrict__ out, AttnRun a) {
@@ -268,8 +251,7 @@ attn_ragged_kernel(const float* __restrict__ qbuf, const E* __restrict__ kc, con
   float* ov = red + 8;                // [groups * Vpad]
   pdl_wait();
   pdl_trigger();
-  const int row = kCluster ? blockIdx.y : blockIdx.x, h = kCluster ? blockIdx.z : blockIdx.y, tid = threadIdx.x;
-  const int split = kCluster ? blockIdx.x : blockIdx.z;
+  const int row = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
   const int g = h / (a.H / a.G);
   const int4 e = reinterpret_cast<const int4*>(a.ent)[a.row_ent[row]];
   const int pos = e.w + (row - e.y);
@@ -284,7 +266,7 @@ attn_ragged_kernel(const float* __restrict__ qbuf, const E* __restrict__ kc, con
   int jb = shift, je = pos;    // this CTA's keys
   if (a.splits > 1) {
     const int per = (pos - shift + a.splits) / a.splits;
-    jb = shift + split * per;
+    jb = shift + (int)blockIdx.z * per;
     je = min(pos, jb + per - 1);
   }
   auto key_pos = [&](int idx) { return idx < lo ? idx - shift : idx; };
@@ -297,7 +279,7 @@ attn_ragged_kernel(const float* __restrict__ qbuf, const E* __restrict__ kc, con
   const int d0 = vec ? (tid % (a.V / 4)) * 4 : (a.V >= kAttnThreads ? tid : tid % a.V);
   const int dstep = vec ? 1 : kAttnThreads;  // acc[i] belongs to dimension d0 + i * dstep
   float acc[kAttnMaxVPerThread] = {0.f, 0.f, 0.f, 0.f};
-  const bool has_sink = a.sink && split == 0;
+  const bool has_sink = a.sink && blockIdx.z == 0;
   float m = has_sink ? a.sink[h] : -INFINITY;  // the sink enters as a term exp(sink - m) = 1 of the denominator
   float l = has_sink ? 1.f : 0.f;
   __syncthreads();
@@ -387,54 +369,8 @@ attn_ragged_kernel(const float* __restrict__ qbuf, const E* __restrict__ kc, con
     }
   }
   __syncthreads();
-  if (kCluster) {
-    __shared__ float wz[kAttnMaxCluster], lz[kAttnMaxCluster];
-    for (int d = tid; d < a.V; d += kAttnThreads) {  // this CTA's sums, where its first key group's were
-      float u = 0.f;
-      for (int gg = 0; gg < groups; ++gg) u += ov[gg * a.V + d];
-      ov[d] = u;
-    }
-    if (tid == 0) { red[0] = m; red[1] = l; }
-    attn_cluster_sync();
-    if (tid < kAttnMaxCluster) {
-      wz[tid] = tid < a.splits ? attn_peer(red, tid) : -INFINITY;
-      lz[tid] = tid < a.splits ? attn_peer(red + 1, tid) : 0.f;
-    }
-    __syncthreads();
-    float M = -INFINITY;
-    for (int z = 0; z < a.splits; ++z) M = fmaxf(M, wz[z]);
-    __syncthreads();
-    if (tid < kAttnMaxCluster) wz[tid] = wz[tid] == -INFINITY ? 0.f : expf(wz[tid] - M);
-    __syncthreads();
-    float L = 0.f;
-    for (int z = 0; z < a.splits; ++z) L += wz[z] * lz[z];
-    const float inv = 1.f / L;
-    E* orow = out + (size_t)row * a.ldo + h * a.V;
-    const int per = (a.V / 2 + a.splits - 1) / a.splits, end = min(a.V / 2, (split + 1) * per);
-    for (int i = split * per + tid; i < end; i += kAttnThreads) {
-      float fu[kAttnMaxCluster], fv[kAttnMaxCluster], u = 0.f, v = 0.f;
-#pragma unroll
-      for (int z = 0; z < kAttnMaxCluster; ++z) {
-        fu[z] = z < a.splits ? attn_peer(ov + 2 * i, z) : 0.f;
-        fv[z] = z < a.splits ? attn_peer(ov + 2 * i + 1, z) : 0.f;
-      }
-#pragma unroll
-      for (int z = 0; z < kAttnMaxCluster; ++z)
-        if (z < a.splits) { u = fmaf(wz[z], fu[z], u); v = fmaf(wz[z], fv[z], v); }
-      u *= inv; v *= inv;
-      if (a.cos_v) {
-        const float c = a.cos_v[(size_t)pos * (a.V / 2) + i], s = a.sin_v[(size_t)pos * (a.V / 2) + i];
-        const float u2 = u * c + v * s, v2 = v * c - u * s;
-        u = u2; v = v2;
-      }
-      orow[2 * i] = a_from_f<E>(u * out_gate(proj, a, row, h, 2 * i));
-      orow[2 * i + 1] = a_from_f<E>(v * out_gate(proj, a, row, h, 2 * i + 1));
-    }
-    attn_cluster_sync();  // a CTA's shared memory lives until all have read it
-    return;
-  }
   if (a.splits > 1) {
-    float* pr = a.part + (((size_t)row * a.H + h) * a.splits + split) * (a.V + 2);
+    float* pr = a.part + (((size_t)row * a.H + h) * a.splits + blockIdx.z) * (a.V + 2);
     for (int d = tid; d < a.V; d += kAttnThreads) {
       float u = 0.f;
       for (int gg = 0; gg < groups; ++gg) u += ov[gg * a.V + d];
@@ -959,39 +895,6 @@ static int launch_ragged_tc(const float* qbuf, const void* kc, const void* vc, c
   return launch_ragged_tc_as<DK, DV, true>(qbuf, kc, vc, proj, out, tiles, n_tiles, a, s);
 }
 
-// Whether clusters of up to kAttnMaxCluster CTAs run on this device (1) or only portable ones of 8 (0): more than 8 are asked for, and
-// room for one such cluster is looked up, once per device.
-static int attn_wide_clusters(int* wide) {
-  static PerDeviceOnce once;
-  DLI_ONCE_PER_DEVICE(once, dev, {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(kAttnMaxCluster, 64, 64);
-    cfg.blockDim = dim3(kAttnThreads);
-    cfg.dynamicSmemBytes = 48 * 1024;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = kAttnMaxCluster;
-    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    int n = 0;
-    DLI_CUDA_CALL(cudaFuncSetAttribute(attn_ragged_kernel<bf16, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    DLI_CUDA_CALL(cudaFuncSetAttribute(attn_ragged_kernel<float, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    DLI_CUDA_CALL(cudaOccupancyMaxActiveClusters(&n, attn_ragged_kernel<float, true>, &cfg));
-    once.value[dev] = n > 0;
-  });
-  *wide = once.value[dev];
-  return DLI_OK;
-}
-
-template <typename E>
-static int launch_attn_cluster(const E* kc, const E* vc, const E* proj, E* out, const float* qbuf, int rows, size_t smem, const AttnRun& a,
-                               cudaStream_t s) {
-  const cudaError_t err = launch_kernel_cluster(attn_ragged_kernel<E, true>, dim3(a.splits, rows, a.H), dim3(kAttnThreads), smem, s,
-                                                (unsigned)a.splits, qbuf, kc, vc, proj, out, a);
-  return err == cudaSuccess ? DLI_OK : fail(DLI_ERR_CUDA, "attn_ragged: %s", cudaGetErrorString(err));
-}
-
 }  // namespace dli
 
 using namespace dli;
@@ -1054,18 +957,9 @@ int dli_attn_ragged(const float* qbuf, const void* k_cache, const void* v_cache,
     else rc = hpc == 4 ? launch_shared_kv<float, 4>(qbuf, k_cache, v_cache, out, rows, a, s)
                        : launch_shared_kv<float, 2>(qbuf, k_cache, v_cache, out, rows, a, s);
     if (rc != DLI_OK) return rc;
-  } else {
-    if (splits > 1 && splits <= kAttnMaxCluster && rows <= 65535 && H <= 65535) {
-      int wide = 0;
-      const int rc = attn_wide_clusters(&wide);
-      if (rc != DLI_OK) return rc;
-      if (splits <= 8 || wide)
-        return dt == 0 ? launch_attn_cluster((const bf16*)k_cache, (const bf16*)v_cache, (const bf16*)proj, (bf16*)out, qbuf, rows, smem, a, s)
-                       : launch_attn_cluster((const float*)k_cache, (const float*)v_cache, (const float*)proj, (float*)out, qbuf, rows, smem, a, s);
-    }
-    if (dt == 0) DLI_LAUNCH("attn_ragged", (attn_ragged_kernel<bf16, false>), dim3(rows, H, splits), dim3(kAttnThreads), smem, s, qbuf, (const bf16*)k_cache, (const bf16*)v_cache, (const bf16*)proj, (bf16*)out, a);
-    else DLI_LAUNCH("attn_ragged", (attn_ragged_kernel<float, false>), dim3(rows, H, splits), dim3(kAttnThreads), smem, s, qbuf, (const float*)k_cache, (const float*)v_cache, (const float*)proj, (float*)out, a);
-  }
+  } else
+  if (dt == 0) DLI_LAUNCH("attn_ragged", attn_ragged_kernel<bf16>, dim3(rows, H, splits), dim3(kAttnThreads), smem, s, qbuf, (const bf16*)k_cache, (const bf16*)v_cache, (const bf16*)proj, (bf16*)out, a);
+  else DLI_LAUNCH("attn_ragged", attn_ragged_kernel<float>, dim3(rows, H, splits), dim3(kAttnThreads), smem, s, qbuf, (const float*)k_cache, (const float*)v_cache, (const float*)proj, (float*)out, a);
   if (splits > 1) {
     const int mz = (V / 2 + kAttnThreads - 1) / kAttnThreads;
     if (dt == 0) DLI_LAUNCH("attn_ragged_merge", attn_ragged_merge_kernel<bf16>, dim3(rows, H, mz), dim3(kAttnThreads), 0, s, (const bf16*)proj, (bf16*)out, a);

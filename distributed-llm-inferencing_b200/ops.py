@@ -702,8 +702,7 @@ def attn_ragged(qbuf, k_cache, v_cache, proj, out, row_ent, ent, page_table, H, 
     _f32(qbuf, sink, cos_v, sin_v, part, r1, r2), _i32(row_ent, ent, page_table), _cols(out, H * V, k_cache.dtype), _req(proj, k_cache.dtype)
     if splits > 1 and part.numel() < qbuf.shape[0] * H * splits * (V + 2):
         raise ValueError("attn_ragged: scratch too small for the key splits")
-    # up to 16 splits of a head are one cluster of one kernel; more, and one key head shared by all heads, have a second one
-    _call("dli_attn_ragged", 2 if splits > 1 and (splits > 16 or G == 1) else 1, _p(qbuf), _p(k_cache), _p(v_cache), _p(proj), _p(out), _p(row_ent), _p(ent),
+    _call("dli_attn_ragged", 2 if splits > 1 else 1, _p(qbuf), _p(k_cache), _p(v_cache), _p(proj), _p(out), _p(row_ent), _p(ent),
           _p(page_table), page_table.shape[1], k_cache.shape[2], qbuf.shape[0], H, G, D, V, float(scale), int(chunk),
           int(window), int(first), _p(sink), proj.shape[1] if proj is not None else 0, g_off, _p(cos_v), _p(sin_v), int(ldv),
           int(splits), _p(part), _dt(k_cache), _p(r1), _p(r2), float(cap), int(bool(g_chan)), float(out_scale), out.stride(0), _stream())
