@@ -894,8 +894,13 @@ int dli_mlstm_ragged(const void* proj, float* o_scratch, void* y, const int32_t*
   const size_t csmem = mlstm_chunk_smem(D);
   const bool chunked = blocked && csmem <= 220 * 1024;  // larger key sizes: the token-by-token kernel
   const dim3 cgrid(n_ent, H, (V + kMcCols - 1) / kMcCols);
-  // decode (one row an entry), of sizes whose slices are one portable cluster and whose state fits the registers
-  if (!chunked && rows == n_ent && V <= 8 * kMlCols && D <= 256 && H <= 65535 && n_ent <= 65535)
+  // decode (one row an entry), of sizes whose slices are one portable cluster and whose state fits the registers, where all CTAs
+  // are resident at once: up to 3, 2 or 1 per SM by key size, of which clusters fill some 85 %.  Above, the state streams and the scan's
+  // eight CTAs per SM keep more of it in flight.  us, two kernels / one: heads of 128 x 256, 3 rows of 8 8.8 / 5.1, 16 rows 15.7 / 19.1,
+  // 64 47.5 / 83; 64 x 64, 16 rows of 16 8.2 / 6.1, 64 rows 17.5 / 18.7; 256 x 256, 3 rows of 4 9.9 / 7.0, 16 rows 15.8 / 33.8.
+  const long long ctas = (long long)n_ent * H * ((V + kMlCols - 1) / kMlCols);
+  const int sms = sm_count_cached() > 0 ? sm_count_cached() : 148, per_sm = D <= 64 ? 3 : D <= 128 ? 2 : 1;
+  if (!chunked && rows == n_ent && V <= 8 * kMlCols && D <= 256 && 20 * ctas <= 17ll * per_sm * sms)
     return dt == 0 ? launch_mlstm_decode<bf16>(proj, out_w, y, n_ent, g_off, eps, a, s)
                    : launch_mlstm_decode<float>(proj, out_w, y, n_ent, g_off, eps, a, s);
   if (dt == 0) {
