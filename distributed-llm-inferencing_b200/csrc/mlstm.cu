@@ -42,9 +42,43 @@ constexpr int kMlCols = 32, kMlGroups = 8, kMlThreads = kMlCols * kMlGroups;
 __device__ __forceinline__ float soft_cap(float x, float cap) { return cap > 0.f ? cap * tanhf(x / cap) : x; }
 __device__ __forceinline__ float log_sigmoid(float x) { return fminf(x, 0.f) - log1pf(expf(-fabsf(x))); }
 
+// The column slices of a head (grid.z) all start from its n and m, which slice 0 replaces in the end: none may read them after that, and
+// a late slice of a grid that does not fit the SMs did (40 rows of 8 heads).  Up to 8 slices are a cluster, and these are the
+// two halves of its barrier; more are two launches, slice 0 after the others.  (The barrier of a CTA that is its own cluster is free.)
+__device__ __forceinline__ void slices_read() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void slices_have_read() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+template <typename E>
+static int launch_slices(void (*kernel)(const E*, float*, MlstmArgs, int), dim3 grid, int threads, size_t smem, cudaStream_t s, const void* proj,
+                         float* o, const MlstmArgs& a) {
+  const auto launch = [&](unsigned count, unsigned cluster, int slice0) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid.x, grid.y, count);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = cluster;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl_enabled() ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<const E*>(proj), o, a, slice0);
+  };
+  if (grid.z <= 8) {
+    DLI_CUDA_CALL(launch(grid.z, grid.z, 0));
+  } else {
+    DLI_CUDA_CALL(launch(grid.z - 1, 1, 1));
+    DLI_CUDA_CALL(launch(1, 1, 0));
+  }
+  return DLI_OK;
+}
+
 template <typename E>
 __global__ void __launch_bounds__(kMlThreads)
-mlstm_scan_kernel(const E* __restrict__ proj, float* __restrict__ o, MlstmArgs a) {
+mlstm_scan_kernel(const E* __restrict__ proj, float* __restrict__ o, MlstmArgs a, int slice0) {
   extern __shared__ float sm[];
   float* S = sm;                         // [D][kMlCols]
   float* qs = S + (size_t)a.D * kMlCols;  // [D]
@@ -55,7 +89,7 @@ mlstm_scan_kernel(const E* __restrict__ proj, float* __restrict__ o, MlstmArgs a
   pdl_wait();
   pdl_trigger();
   const int4 e = reinterpret_cast<const int4*>(a.ent)[blockIdx.x];  // slot, row0, n, start
-  const int h = blockIdx.y, c0 = blockIdx.z * kMlCols;
+  const int h = blockIdx.y, slice = blockIdx.z + slice0, c0 = slice * kMlCols;
   const int tid = threadIdx.x, col = tid % kMlCols, grp = tid / kMlCols;
   const int c = c0 + col;
   const bool col_ok = c < a.V;
@@ -69,6 +103,7 @@ mlstm_scan_kernel(const E* __restrict__ proj, float* __restrict__ o, MlstmArgs a
   const float qscale = 1.f / sqrtf((float)a.D);
   const float ib = a.i_bias ? a.i_bias[h] : 0.f, fb = a.f_bias ? a.f_bias[h] : 0.f;
   __syncthreads();
+  slices_read();
   for (int t = 0; t < e.z; ++t) {
     const int row = e.y + t;
     const E* pr = proj + (size_t)row * a.ldp;
@@ -109,7 +144,8 @@ mlstm_scan_kernel(const E* __restrict__ proj, float* __restrict__ o, MlstmArgs a
   }
   if (col_ok)
     for (int d = grp; d < a.D; d += kMlGroups) Sg[(size_t)d * a.V + c] = S[d * kMlCols + col];
-  if (blockIdx.z == 0) {
+  slices_have_read();
+  if (slice == 0) {
     for (int d = tid; d < a.D; d += kMlThreads) ng[d] = ns[d];
     if (tid == 0) *mg = m;
   }
@@ -133,7 +169,7 @@ constexpr int kMcL = 64, kMcLp = 68, kMcCols = 64, kMcThreads = 256;
 
 template <typename E>
 __global__ void __launch_bounds__(kMcThreads)
-mlstm_chunk_kernel(const E* __restrict__ proj, float* __restrict__ o, MlstmArgs a) {
+mlstm_chunk_kernel(const E* __restrict__ proj, float* __restrict__ o, MlstmArgs a, int slice0) {
   extern __shared__ __align__(16) float smc[];
   const int D = a.D;
   float* qT = smc;                          // [D][kMcLp]
@@ -150,7 +186,7 @@ mlstm_chunk_kernel(const E* __restrict__ proj, float* __restrict__ o, MlstmArgs 
   pdl_wait();
   pdl_trigger();
   const int4 e = reinterpret_cast<const int4*>(a.ent)[blockIdx.x];
-  const int h = blockIdx.y, c0 = blockIdx.z * kMcCols;
+  const int h = blockIdx.y, slice = blockIdx.z + slice0, c0 = slice * kMcCols;
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   const bool fresh = e.w == 0;
   float* Sg = a.S + ((size_t)e.x * a.H + h) * D * a.V;
@@ -165,6 +201,7 @@ mlstm_chunk_kernel(const E* __restrict__ proj, float* __restrict__ o, MlstmArgs 
   const float qscale = 1.f / sqrtf((float)D);
   const float ib = a.i_bias ? a.i_bias[h] : 0.f, fb = a.f_bias ? a.f_bias[h] : 0.f;
   __syncthreads();
+  slices_read();
 
   for (int t0 = 0; t0 < e.z; t0 += kMcL) {
     const int len = min(kMcL, e.z - t0);
@@ -351,7 +388,8 @@ mlstm_chunk_kernel(const E* __restrict__ proj, float* __restrict__ o, MlstmArgs 
     const int d = i / kMcCols, c = c0 + i % kMcCols;
     if (c < a.V) Sg[(size_t)d * a.V + c] = Ss[i];
   }
-  if (blockIdx.z == 0) {
+  slices_have_read();
+  if (slice == 0) {
     for (int d = tid; d < D; d += kMcThreads) ng[d] = ns[d];
     if (tid == 0) *mg = m0;
   }
@@ -907,15 +945,17 @@ int dli_mlstm_ragged(const void* proj, float* o_scratch, void* y, const int32_t*
     static PerDeviceOnce once;
     DLI_ONCE_PER_DEVICE(once, dev, DLI_CUDA_CALL(cudaFuncSetAttribute(mlstm_scan_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
                         DLI_CUDA_CALL(cudaFuncSetAttribute(mlstm_chunk_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024)));
-    if (chunked) DLI_LAUNCH("mlstm_chunk", mlstm_chunk_kernel<bf16>, cgrid, dim3(kMcThreads), csmem, s, (const bf16*)proj, o_scratch, a);
-    else DLI_LAUNCH("mlstm_scan", mlstm_scan_kernel<bf16>, grid, dim3(kMlThreads), smem, s, (const bf16*)proj, o_scratch, a);
+    const int rc = chunked ? launch_slices<bf16>(mlstm_chunk_kernel<bf16>, cgrid, kMcThreads, csmem, s, proj, o_scratch, a)
+                           : launch_slices<bf16>(mlstm_scan_kernel<bf16>, grid, kMlThreads, smem, s, proj, o_scratch, a);
+    if (rc != DLI_OK) return rc;
     DLI_LAUNCH("mlstm_out", mlstm_out_kernel<bf16>, dim3((rows * H + 3) / 4), dim3(128), 0, s, (const float*)o_scratch, (const bf16*)proj, out_w, (bf16*)y, rows, H, V, ldp, g_off, eps);
   } else {
     static PerDeviceOnce once;
     DLI_ONCE_PER_DEVICE(once, dev, DLI_CUDA_CALL(cudaFuncSetAttribute(mlstm_scan_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
                         DLI_CUDA_CALL(cudaFuncSetAttribute(mlstm_chunk_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024)));
-    if (chunked) DLI_LAUNCH("mlstm_chunk", mlstm_chunk_kernel<float>, cgrid, dim3(kMcThreads), csmem, s, (const float*)proj, o_scratch, a);
-    else DLI_LAUNCH("mlstm_scan", mlstm_scan_kernel<float>, grid, dim3(kMlThreads), smem, s, (const float*)proj, o_scratch, a);
+    const int rc = chunked ? launch_slices<float>(mlstm_chunk_kernel<float>, cgrid, kMcThreads, csmem, s, proj, o_scratch, a)
+                           : launch_slices<float>(mlstm_scan_kernel<float>, grid, kMlThreads, smem, s, proj, o_scratch, a);
+    if (rc != DLI_OK) return rc;
     DLI_LAUNCH("mlstm_out", mlstm_out_kernel<float>, dim3((rows * H + 3) / 4), dim3(128), 0, s, (const float*)o_scratch, (const float*)proj, out_w, (float*)y, rows, H, V, ldp, g_off, eps);
   }
   return DLI_OK;

@@ -8,7 +8,7 @@ torch = pytest.importorskip("torch")
 
 @pytest.mark.parametrize("dt", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("D,V", [(8, 32), (64, 40), (72, 224), (128, 256), (200, 1), (256, 256), (128, 264), (264, 64)])
-@pytest.mark.parametrize("rows,H,cap", [(1, 8, 15.0), (5, 3, 0.0)])
+@pytest.mark.parametrize("rows,H,cap", [(1, 8, 15.0), (5, 3, 0.0), (40, 8, 0.0)])  # the last: too many for one kernel, at most sizes
 def test_same_bits_as_any_number_of_rows(cuda, D, V, rows, H, cap, dt):
     from dli_b200 import ops
 
@@ -38,3 +38,29 @@ def test_same_bits_as_any_number_of_rows(cuda, D, V, rows, H, cap, dt):
     ops.set_pdl(before)
     assert all(torch.equal(a, b) for a, b in zip(*outs)) and torch.isfinite(outs[0][-1].float()).all()
     assert all(torch.equal(a, b) for a, b in zip(*got))
+
+
+@pytest.mark.parametrize("V,blocked", [(224, False), (256, True), (264, False), (520, True)])
+def test_many_entries_as_few(cuda, V, blocked):
+    """More column slices than run at once: each starts from the state before the call.  Entries by themselves give the same bits."""
+    from dli_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(V)
+    rnd = lambda *s: torch.randn(*s, device=cuda, generator=g)  # noqa: E731
+    n_ent, per, H, D = 90, 2, 8, 72
+    rows, ld = n_ent * per, H * (2 * D + 2 * V + 2)
+    q, k, v, gate = 0, H * D, 2 * H * D, 2 * H * D + H * V
+    i_off, f_off = gate + H * V, gate + H * V + H
+    ib, fb, w = rnd(H), rnd(H) + 2, 1 + 0.2 * rnd(H * V)
+    state, proj = [rnd(n_ent, H, D, V), rnd(n_ent, H, D), rnd(n_ent, H)], rnd(rows, ld).to(torch.bfloat16)
+
+    def run(st, lo, hi):
+        out = torch.empty((hi - lo) * per, H * V, device=cuda, dtype=torch.bfloat16)
+        ent = torch.tensor([[e, (e - lo) * per, per, 9] for e in range(lo, hi)], device=cuda, dtype=torch.int32).view(-1)
+        ops.mlstm_ragged(proj[lo * per:hi * per], torch.empty((hi - lo) * per, H * V, device=cuda), out, ent, H, D, V, q, k, v, i_off, f_off,
+                         gate, ib, fb, 0.0, w, 1e-6, *st, blocked=blocked)
+        return out
+
+    one, many = [t.clone() for t in state], [t.clone() for t in state]
+    want = torch.cat([run(one, e, e + 3) for e in range(0, n_ent, 3)])
+    assert torch.equal(run(many, 0, n_ent), want) and all(torch.equal(a, b) for a, b in zip(one, many))
